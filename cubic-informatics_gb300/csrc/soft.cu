@@ -10,6 +10,9 @@
 // by tau, tau^2, tau^3.  Loss = mean score at the positive points - mean score at the
 // negative points.
 //
+// With few sample points the DoG, its derivatives and the transposed Gaussians are evaluated at the
+// points' neighbourhoods (k_soft_points_local); with many, over the volume as follows.
+//
 // Backward recomputes every intermediate from the input, or (the _kept entry) takes the
 // forward chain's intermediates from the workspace the forward call filled, which the
 // backward does not overwrite, and runs the adjoints in reverse: the score's derivative scattered through the
@@ -30,6 +33,7 @@
 // the float32 sigma gradients are sensitive to the last bits of the normalized volume, so
 // that order is kept.  Min / max windows and their first extremes, which do not round, come
 // from doubling in the tile.
+#include <algorithm>
 #include <cmath>
 
 #include "kernels.cuh"
@@ -177,7 +181,8 @@ __device__ __forceinline__ double soft_warp_dot(float hi, float lo) {
 constexpr int kSoftRowsX = 4;
 
 __global__ void __launch_bounds__(kSoftTileX) k_soft_pass_x(const float *in, float *out, SoftGeom g, int mode, int R,
-                                                            SoftTaps T) {
+                                                            SoftTaps T, const unsigned *skip) {
+  if (skip && *skip) return;   // the output is already there
   __shared__ float tile[kSoftRowsX][kSoftTileX + 2 * kSoftTileMaxR];
   const int nseg = (g.W + kSoftTileX - 1) / kSoftTileX;
   const int64_t row0 = (int64_t)(blockIdx.x / nseg) * kSoftRowsX;
@@ -227,8 +232,10 @@ enum { kEpiStore = 0, kEpiDot = 1, kEpiDiff = 2 };
 
 template <int AXIS, int EPI = kEpiStore>
 __global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *out, SoftGeom g, int mode, int R,
-                                                      SoftTaps T, const float *aux = nullptr,
-                                                      double *dot_out = nullptr, float scale = 0.0f) {
+                                                      SoftTaps T, const unsigned *skip = nullptr,
+                                                      const float *aux = nullptr, double *dot_out = nullptr,
+                                                      float scale = 0.0f) {
+  if (skip && *skip) return;
   extern __shared__ float slab[];   // [kSoftTileYZ + 2R][32]
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int n = AXIS == 1 ? g.H : g.D;
@@ -529,10 +536,14 @@ __global__ void k_soft_box_adj(const float *g_out, float *g_in, SoftGeom g, int 
   g_in[i] = acc / (float)(2 * r + 1);
 }
 
-__global__ void k_soft_norm(const float *I, const float *e, const float *d, float *norm, float min_intensity, int64_t N) {
+// *bad is set when a normalized value is not finite (a window without contrast).
+__global__ void k_soft_norm(const float *I, const float *e, const float *d, float *norm, float min_intensity, int64_t N,
+                            unsigned *bad) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  norm[i] = I[i] >= min_intensity ? (I[i] - e[i]) / (d[i] - e[i]) : 0.0f;
+  const float v = I[i] >= min_intensity ? (I[i] - e[i]) / (d[i] - e[i]) : 0.0f;
+  norm[i] = v;
+  if (!isfinite(v)) *bad = 1u;
 }
 
 // Quotient rule of the normalization: g_I (direct term, written), g_e, g_d.
@@ -617,7 +628,8 @@ __device__ void soft_hessian(const float *f, const SoftGeom &g, SoftPoint p, flo
   }
 }
 
-__device__ void soft_hessian_adj(float *gf, const SoftGeom &g, SoftPoint p, const float gh[6]) {
+// (in doubles: many points may meet in one voxel)
+__device__ void soft_hessian_adj(double *gf, const SoftGeom &g, SoftPoint p, const float gh[6]) {
   for (int e = 0; e < 6; e++) {
     for (int sb = -1; sb <= 1; sb += 2) {
       int qx = p.x, qy = p.y, qz = p.z;
@@ -627,8 +639,8 @@ __device__ void soft_hessian_adj(float *gf, const SoftGeom &g, SoftPoint p, cons
       int ax = qx, ay = qy, az = qz, bx = qx, by = qy, bz = qz;
       soft_step(h_inner(e), 1, ax, ay, az);
       soft_step(h_inner(e), -1, bx, by, bz);
-      if (soft_in(g, ax, ay, az)) atomicAdd(gf + ((int64_t)az * g.H + ay) * g.W + ax, c);
-      if (soft_in(g, bx, by, bz)) atomicAdd(gf + ((int64_t)bz * g.H + by) * g.W + bx, -c);
+      if (soft_in(g, ax, ay, az)) atomicAdd(gf + ((int64_t)az * g.H + ay) * g.W + ax, (double)c);
+      if (soft_in(g, bx, by, bz)) atomicAdd(gf + ((int64_t)bz * g.H + by) * g.W + bx, -(double)c);
     }
   }
 }
@@ -678,7 +690,7 @@ __global__ void k_soft_points(const float *dog, SoftGeom g, const int32_t *pos, 
 // Backward at the points: d loss / d dog scattered into gdog (which must start at zero), and
 // d loss / d thresholds summed into gb[0..2] (double, zeroed first) when gb is given.
 __global__ void k_soft_points_adj(const float *dog, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg,
-                                  int n_neg, float tau, SoftThresh b, float grad_loss, float *gdog, double *gb) {
+                                  int n_neg, float tau, SoftThresh b, float grad_loss, double *gdog, double *gb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos + n_neg) return;
   const int32_t *q = i < n_pos ? pos + 3 * i : neg + 3 * (i - n_pos);
@@ -698,6 +710,347 @@ __global__ void k_soft_to_float(const double *in, float *out, int n) {
   if (i < n) out[i] = (float)in[i];
 }
 
+__global__ void k_soft_gdog(const double *in, float *out, int64_t N) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) out[i] = (float)in[i];
+}
+
+// ---- the DoG and its derivatives at the points' own neighbourhoods
+//
+// The loss reads the DoG at 19 positions around each sample point (the Hessian's stencil), and
+// d loss / d DoG is zero everywhere else, so with few points the dense Gaussian passes (6
+// forward, 16 for the sigma gradients, 6 for the input gradient) compute values that nothing
+// reads.  Here a block takes one point at a time: it stages the normalized volume around the
+// point (stencil plus the taps' reach) in shared memory, runs the separable passes on the 5 x 5 x 5
+// stencil only (x on the lines the y and z taps reach, then y, then z at the 19 positions; both
+// scales in one phase), and forms score, derivatives and sums from them.  Every DoG value is the
+// dense passes' fold, tap by tap in the same order; a tap outside the volume multiplies a staged
+// zero instead of being skipped, which leaves the sum as it is.  The adjoint spreads the stencil's
+// gradient through the same taps (z, y, then x) and adds the patch to the normalized volume's
+// gradient, one float reduction per voxel and point.
+// What bounds it: the phases' latency (twelve barriers a point) and shared-memory loads; 48 KB and
+// 256 threads a block at sigmas 2.0 / 3.2, four blocks per SM.  128x512x512, 4000 points, sigmas
+// (2.0, 2.0, 1.5, 3.2, 3.2, 2.4): 98 us forward and 209 us backward, where the 28 dense passes took
+// 4.8 ms (the whole forward + backward 10.99 -> 6.23 ms).
+constexpr int kSoftPtThreads = 256;
+constexpr int kSoftStencil = 19;
+constexpr int kSoftPadX = 2 * kSoftMaxRadius + 6;
+
+struct SoftTapSet {
+  SoftTaps plain[6], deriv[6];   // x1, y1, z1, x2, y2, z2
+};
+
+// Reaches of the staged box (the larger scale's per axis) and the layout of the shared memory.
+struct SoftBox {
+  int r[3];   // x, y, z
+  __host__ __device__ int e(int a) const { return 5 + 2 * r[a]; }
+  __host__ __device__ int tile() const { return e(0) * e(1) * e(2); }
+  __host__ __device__ int lines() const { return e(1) * e(2); }
+  // floats: the tile; per scale two x-pass buffers of 5 outputs per line (the adjoint's y buffers) and
+  // three y-pass buffers of 25 columns (the adjoint's z buffers); the plain taps, the x ones padded
+  __host__ __device__ int floats() const {
+    return tile() + 20 * lines() + 150 * e(2) + 6 * kSoftMaxTaps + 2 * kSoftPadX;
+  }
+};
+
+// the stencil's position k as offsets from the point (0: the point; 1-6: +-2 along an axis; 7-18: the
+// twelve edge neighbours, xy, xz and yz pairs)
+__device__ __forceinline__ void soft_stencil(int k, int &dx, int &dy, int &dz) {
+  dx = dy = dz = 0;
+  if (k == 0) return;
+  if (k < 7) {
+    const int v = (k & 1) ? 2 : -2, a = (k - 1) >> 1;
+    if (a == 0) dx = v;
+    else if (a == 1) dy = v;
+    else dz = v;
+    return;
+  }
+  const int m = k - 7, pair = m >> 2, u = (m & 1) ? 1 : -1, v = (m & 2) ? 1 : -1;
+  if (pair == 0) { dx = u; dy = v; }
+  else if (pair == 1) { dx = u; dz = v; }
+  else { dy = u; dz = v; }
+}
+__device__ __forceinline__ int soft_at(int dx, int dy, int dz) { return ((dz + 2) * 5 + dy + 2) * 5 + dx + 2; }
+
+// element e of soft_hessian on the 5 x 5 x 5 cube around p instead of the volume
+__device__ __forceinline__ float soft_hessian_cube(const float *f, const SoftGeom &g, SoftPoint p, int e) {
+  float v = 0.0f;
+  for (int sb = -1; sb <= 1; sb += 2) {
+    int qx = 0, qy = 0, qz = 0;
+    soft_step(h_outer(e), sb, qx, qy, qz);
+    if (!soft_in(g, p.x + qx, p.y + qy, p.z + qz)) continue;
+    int ax = qx, ay = qy, az = qz, bx = qx, by = qy, bz = qz;
+    soft_step(h_inner(e), 1, ax, ay, az);
+    soft_step(h_inner(e), -1, bx, by, bz);
+    const float ga = 0.5f * (f[soft_at(ax, ay, az)] - f[soft_at(bx, by, bz)]);
+    v += sb > 0 ? ga : -ga;
+  }
+  return 0.5f * v;
+}
+
+// what soft_hessian_adj adds at the stencil's position k: +-gh / 4 of the element whose two steps lead
+// there, where the step between them (along the outer axis) stays inside the volume
+__device__ __forceinline__ float soft_hessian_coef(const SoftGeom &g, SoftPoint p, int k, const float gh[6]) {
+  if (k == 0) {
+    const float gd[3] = {gh[0], gh[3], gh[5]};
+    float c = 0.0f;
+    for (int a = 0; a < 3; a++)
+      for (int sb = -1; sb <= 1; sb += 2) {
+        int qx = 0, qy = 0, qz = 0;
+        soft_step(a, sb, qx, qy, qz);
+        if (soft_in(g, p.x + qx, p.y + qy, p.z + qz)) c -= 0.25f * gd[a];
+      }
+    return c;
+  }
+  int dx, dy, dz;
+  soft_stencil(k, dx, dy, dz);
+  if (k < 7) {
+    const int a = (k - 1) >> 1;
+    return soft_in(g, p.x + dx / 2, p.y + dy / 2, p.z + dz / 2) ? 0.25f * (a == 0 ? gh[0] : a == 1 ? gh[3] : gh[5]) : 0.0f;
+  }
+  const int pair = (k - 7) >> 2;   // xy: outer y; xz, yz: outer z
+  const int qy = pair == 0 ? dy : 0, qz = pair == 0 ? 0 : dz;
+  const float s = (float)((dx ? dx : 1) * (dy ? dy : 1) * (dz ? dz : 1));
+  return soft_in(g, p.x, p.y + qy, p.z + qz) ? 0.25f * s * (pair == 0 ? gh[1] : pair == 1 ? gh[2] : gh[4]) : 0.0f;
+}
+
+// BWD false: scores (optional) and the loss into acc[0].  BWD true: the sums the sigma
+// gradients are formed from into acc[0..6] (as soft_backward's dense passes leave them), the
+// threshold gradients into gb[0..2], and, when gnorm is given, the gradient of the normalized volume
+// added to it.  All sums are doubles that must start at zero.
+template <bool BWD>
+__global__ void __launch_bounds__(kSoftPtThreads, 4)
+    k_soft_points_local(const float *norm, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
+                        const __grid_constant__ SoftTapSet T, SoftBox box, float nrm, float tau, SoftThresh b,
+                        float grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+  extern __shared__ float sm[];
+  __shared__ float fv[2][4][kSoftStencil];   // per scale: plain, d/dz, d/dy, d/dx
+  __shared__ float cube[125], coef[125];     // DoG and d loss / d DoG around the point (0 off the stencil)
+  __shared__ float hs[6], ds[6];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int ex = box.e(0), ey = box.e(1), ez = box.e(2), L = box.lines();
+  float *tile = sm;
+  float *xl = tile + box.tile();             // [scale][plain, derivative][lines][5]
+  float *yl = xl + 20 * L;                   // [scale][3][25][ez]
+  float *tap = yl + 150 * ez;                // [6][kSoftMaxTaps] plain taps: the adjoint's lanes read different ones
+  float *padx = tap + 6 * kSoftMaxTaps;      // [2][kSoftPadX] x taps by staged column, zeros around
+  for (int i = t; i < 6 * kSoftMaxTaps; i += kSoftPtThreads) tap[i] = T.plain[i / kSoftMaxTaps].k[i % kSoftMaxTaps];
+  for (int i = t; i < 2 * kSoftPadX; i += kSoftPtThreads) {
+    const SoftTaps &P = T.plain[3 * (i / kSoftPadX)];
+    const int j = i % kSoftPadX - (box.r[0] - P.r);
+    padx[i] = j >= 0 && j <= 2 * P.r ? P.k[j] : 0.0f;
+  }
+  for (int i = t; i < 125; i += kSoftPtThreads) cube[i] = coef[i] = 0.0f;
+  const int l1y = 5 + 2 * T.plain[1].r, l1z = 5 + 2 * T.plain[2].r, l2y = 5 + 2 * T.plain[4].r, l2z = 5 + 2 * T.plain[5].r;
+  const int lines1 = l1y * l1z, lines2 = l2y * l2z, cols1 = 5 * l1z, cols2 = 5 * l2z;
+  // this thread's walk over the tile: element t, then 256 further each time
+  const int sx = kSoftPtThreads % ex, sl = kSoftPtThreads / ex;
+  const int xi0 = t % ex, yi0 = (t / ex) % ey, zi0 = t / (ex * ey);
+  int kx, ky, kz;                            // the stencil position of lane % 19's products
+  soft_stencil(lane < kSoftStencil ? lane : 0, kx, ky, kz);
+  double sum = 0.0;                          // lane 0 of warp w < 7: acc[w]; thread 0 without BWD: the loss
+  double gsum[3] = {0.0, 0.0, 0.0};
+  const int n = n_pos + n_neg;
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int32_t *q = i < n_pos ? pos + 3 * (int64_t)i : neg + 3 * (int64_t)(i - n_pos);
+    const SoftPoint p{q[2], q[1], q[0]};
+    const int x0 = p.x - 2 - box.r[0], y0 = p.y - 2 - box.r[1], z0 = p.z - 2 - box.r[2];
+    __syncthreads();   // the previous point is done with the shared memory
+    for (int k = t, xi = xi0, yi = yi0, zi = zi0; k < box.tile(); k += kSoftPtThreads) {
+      const int x = x0 + xi, y = y0 + yi, z = z0 + zi;
+      tile[k] = soft_in(g, x, y, z) ? __ldg(norm + ((int64_t)z * g.H + y) * g.W + x) : 0.0f;
+      xi += sx;
+      yi += sl;
+      if (xi >= ex) { xi -= ex; yi++; }
+      while (yi >= ey) { yi -= ey; zi++; }
+    }
+    __syncthreads();
+    // x: five outputs per line, plain taps and (BWD) derivative taps
+    for (int m = t; m < lines1 + lines2; m += kSoftPtThreads) {
+      const int sc = m >= lines1, l = sc ? m - lines1 : m, ly_n = sc ? l2y : l1y;
+      const SoftTaps &px = T.plain[3 * sc];
+      const int ly = l % ly_n, lz = l / ly_n, rx = px.r;
+      const float *w = tile + ((lz + box.r[2] - T.plain[3 * sc + 2].r) * ey + ly + box.r[1] - T.plain[3 * sc + 1].r) * ex +
+                       box.r[0] - rx;
+      float a[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, d[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+      float v[5] = {w[0], w[1], w[2], w[3], 0.f};
+      for (int j = 0; j <= 2 * rx; j++) {
+        v[4] = w[j + 4];
+        const float k0 = px.k[j], k1 = BWD ? T.deriv[3 * sc].k[j] : 0.0f;
+#pragma unroll
+        for (int o = 0; o < 5; o++) {
+          a[o] = __fmaf_rn(k0, v[o], a[o]);
+          if (BWD) d[o] = __fmaf_rn(k1, v[o], d[o]);
+        }
+#pragma unroll
+        for (int o = 0; o < 4; o++) v[o] = v[o + 1];
+      }
+      float *out = xl + (2 * sc * L + l) * 5;
+#pragma unroll
+      for (int o = 0; o < 5; o++) {
+        out[o] = a[o];
+        if (BWD) out[L * 5 + o] = d[o];
+      }
+    }
+    __syncthreads();
+    // y: field 0 plain of plain, 1 derivative of plain, 2 plain of the x derivative
+    constexpr int NY = BWD ? 3 : 1, NF = BWD ? 4 : 1;
+    for (int m = t; m < NY * (cols1 + cols2); m += kSoftPtThreads) {
+      const int sc = m >= NY * cols1, mm = sc ? m - NY * cols1 : m, cols = sc ? cols2 : cols1, ly_n = sc ? l2y : l1y;
+      const int f = mm / cols, c = mm % cols, x = c % 5, z = c / 5, ry = T.plain[3 * sc + 1].r;
+      const float *w = xl + ((2 * sc + (f == 2)) * L + z * ly_n) * 5 + x;
+      const float *kk = f == 1 ? T.deriv[3 * sc + 1].k : T.plain[3 * sc + 1].k;
+      float a[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, v[5] = {w[0], w[5], w[10], w[15], 0.f};
+      for (int j = 0; j <= 2 * ry; j++) {
+        v[4] = w[(j + 4) * 5];
+        const float k0 = kk[j];
+#pragma unroll
+        for (int o = 0; o < 5; o++) a[o] = __fmaf_rn(k0, v[o], a[o]);
+#pragma unroll
+        for (int o = 0; o < 4; o++) v[o] = v[o + 1];
+      }
+#pragma unroll
+      for (int o = 0; o < 5; o++) yl[((3 * sc + f) * 25 + o * 5 + x) * ez + z] = a[o];
+    }
+    __syncthreads();
+    // z at the stencil: plain, d/dz, d/dy, d/dx
+    for (int m = t; m < 2 * NF * kSoftStencil; m += kSoftPtThreads) {
+      const int k = m % kSoftStencil, f = (m / kSoftStencil) % NF, sc = m / (kSoftStencil * NF);
+      int dx, dy, dz;
+      soft_stencil(k, dx, dy, dz);
+      const float *w = yl + ((3 * sc + (f < 2 ? 0 : f - 1)) * 25 + (dy + 2) * 5 + dx + 2) * ez + dz + 2;
+      const float *kk = f == 1 ? T.deriv[3 * sc + 2].k : T.plain[3 * sc + 2].k;
+      const int rz = T.plain[3 * sc + 2].r;
+      float a = 0.0f;
+      for (int j = 0; j <= 2 * rz; j++) a = __fmaf_rn(kk[j], w[j], a);
+      fv[sc][f][k] = a;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const bool in = lane < kSoftStencil && soft_in(g, p.x + kx, p.y + ky, p.z + kz);
+      if (lane < kSoftStencil) cube[soft_at(kx, ky, kz)] = in ? nrm * (fv[0][0][lane] - fv[1][0][lane]) : 0.0f;
+      __syncwarp();
+      if (lane < 6) hs[lane] = soft_hessian_cube(cube, g, p, lane);
+      __syncwarp();
+      if (lane == 0) {
+        float h[6];
+        for (int k = 0; k < 6; k++) h[k] = hs[k];
+        if (BWD) {
+          float dh[6], db[3];
+          soft_score(h, tau, b.v, dh, db);
+          const float w = i < n_pos ? grad_loss / (float)n_pos : -grad_loss / (float)n_neg;
+          for (int k = 0; k < 6; k++) ds[k] = dh[k] * w;
+          for (int k = 0; k < 3; k++) gsum[k] += (double)db[k] * (double)w;
+        } else {
+          const float s = soft_score(h, tau, b.v, nullptr, nullptr);
+          if (scores) scores[i] = s;
+          sum += i < n_pos ? (double)s / n_pos : -(double)s / n_neg;
+        }
+      }
+      if (BWD) {
+        __syncwarp();
+        float gh[6];
+        for (int k = 0; k < 6; k++) gh[k] = ds[k];
+        if (lane < kSoftStencil) coef[soft_at(kx, ky, kz)] = in ? soft_hessian_coef(g, p, lane, gh) : 0.0f;
+      }
+    }
+    if (!BWD) continue;
+    __syncthreads();
+    if (acc && warp < 7) {
+      // <gradient, field> of warp w: w = 3 scale + axis, or the DoG itself
+      double v = 0.0;
+      if (lane < kSoftStencil && soft_in(g, p.x + kx, p.y + ky, p.z + kz)) {
+        const int at = soft_at(kx, ky, kz);
+        v = (double)coef[at] * (double)(warp == 6 ? cube[at] : fv[warp / 3][3 - warp % 3][lane]);
+      }
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+      sum += v;
+    }
+    if (!gnorm) continue;
+    // the transposed passes: z (25 columns), y (5 columns of lines), x into the tile
+    for (int m = t; m < 2 * 25 * ez; m += kSoftPtThreads) {
+      const int sc = m >= 25 * ez, r = sc ? m - 25 * ez : m, c = r / ez, z = r % ez;
+      const int rz = T.plain[3 * sc + 2].r;
+      const float *kk = tap + (3 * sc + 2) * kSoftMaxTaps;
+      float a = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        const int j = z - (box.r[2] - rz) - k;
+        if (j >= 0 && j <= 2 * rz) a = __fmaf_rn(coef[k * 25 + c], kk[j], a);
+      }
+      yl[m] = a;
+    }
+    __syncthreads();
+    for (int m = t; m < 10 * L; m += kSoftPtThreads) {
+      const int xs = m / L, l = m % L, sc = xs >= 5, x = sc ? xs - 5 : xs;   // xs = 5 scale + column
+      const int y = l % ey, z = l / ey, ry = T.plain[3 * sc + 1].r, off = box.r[1] - ry;
+      const float *kk = tap + (3 * sc + 1) * kSoftMaxTaps;
+      const float *w = yl + (sc * 25 + x) * ez + z;
+      float a = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        const int j = y - off - k;
+        if (j >= 0 && j <= 2 * ry) a = __fmaf_rn(w[k * 5 * ez], kk[j], a);
+      }
+      xl[m] = a;
+    }
+    __syncthreads();
+    for (int l = t; l < L; l += kSoftPtThreads) {
+      float c1[5], c2[5], t1[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, t2[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int o = 0; o < 5; o++) {
+        c1[o] = xl[o * L + l];
+        c2[o] = xl[(5 + o) * L + l];
+      }
+      for (int xi = 0; xi < ex; xi++) {
+#pragma unroll
+        for (int o = 4; o > 0; o--) { t1[o] = t1[o - 1]; t2[o] = t2[o - 1]; }
+        t1[0] = padx[xi];
+        t2[0] = padx[kSoftPadX + xi];
+        float a = 0.0f, c = 0.0f;
+#pragma unroll
+        for (int o = 0; o < 5; o++) {
+          a = __fmaf_rn(c1[o], t1[o], a);
+          c = __fmaf_rn(c2[o], t2[o], c);
+        }
+        tile[l * ex + xi] = nrm * (a - c);
+      }
+    }
+    __syncthreads();
+    for (int k = t, xi = xi0, yi = yi0, zi = zi0; k < box.tile(); k += kSoftPtThreads) {
+      const int x = x0 + xi, y = y0 + yi, z = z0 + zi;
+      const float v = tile[k];
+      if (v != 0.0f && soft_in(g, x, y, z)) atomicAdd(gnorm + ((int64_t)z * g.H + y) * g.W + x, v);
+      xi += sx;
+      yi += sl;
+      if (xi >= ex) { xi -= ex; yi++; }
+      while (yi >= ey) { yi -= ey; zi++; }
+    }
+  }
+  if (!BWD) {
+    if (t == 0) atomicAdd(acc, sum);
+    return;
+  }
+  if (acc && warp < 7 && lane == 0) atomicAdd(acc + warp, sum);
+  if (gb && t == 0)
+    for (int k = 0; k < 3; k++) atomicAdd(gb + k, gsum[k]);
+}
+
+// d loss / d sigma from the sums <gradient, derivative fields> (h[0..5]) and <gradient, DoG>
+// (h[6]): the normalizer times the field's sum, plus the normalizer's own derivative
+// gamma normalizer / sigma.  A normalized volume with a value that is not finite (*bad) makes every
+// dense field, and so every sum, NaN; sums taken at the points alone say so here.
+struct SoftSigma {
+  float v[6];
+};
+__global__ void k_soft_sigma_grad(const double *h, const unsigned *bad, SoftSigma s, float nrm, float gamma, float *out) {
+  const int k = threadIdx.x;
+  if (k >= 6) return;
+  double v = (double)(k < 3 ? nrm : -nrm) * h[k];
+  if (k < 3) v = __dadd_rn(v, __dmul_rn((double)gamma / s.v[k], h[6]));
+  out[k] = bad && *bad ? __int_as_float(0x7FC00000) : (float)v;
+}
+
 // ------------------------------------------------------------------ host side
 namespace {
 
@@ -707,7 +1060,9 @@ struct SoftRun {
   int64_t N;
   cudaStream_t st;
   float *w;      // workspace slots of N floats (after the accumulators)
-  double *acc;   // 16 doubles at the start of the workspace
+  double *acc;   // 16 doubles at the start of the workspace: sums [0, 14), then the flags
+  // set by the forward chain: [0] a normalized value is not finite, [1] the DoG slot is filled
+  unsigned *flags() const { return reinterpret_cast<unsigned *>(acc + 14); }
   unsigned blocks() const { return ceil_div(N, 256); }
   float *slot(int k) const { return w + (int64_t)k * N; }
 };
@@ -739,7 +1094,8 @@ SoftTaps gauss_taps_f(double sigma, bool derivative) {
   return t;
 }
 
-void pass(const SoftRun &R, const float *in, float *out, int axis, int mode, int r, const SoftTaps &T) {
+void pass(const SoftRun &R, const float *in, float *out, int axis, int mode, int r, const SoftTaps &T,
+          const unsigned *skip = nullptr) {
   const int reach = mode == kConv ? T.r : r;
   const SoftGeom &g = R.g;
   if (reach > kSoftTileMaxR) {
@@ -748,7 +1104,7 @@ void pass(const SoftRun &R, const float *in, float *out, int axis, int mode, int
   }
   if (axis == 0) {
     const unsigned blocks = (unsigned)(ceil_div(g.W, kSoftTileX) * ceil_div((int64_t)g.H * g.D, kSoftRowsX));
-    KLAUNCH("k_soft_pass_x", R.st, (k_soft_pass_x<<<blocks, kSoftTileX, 0, R.st>>>(in, out, g, mode, reach, T)));
+    KLAUNCH("k_soft_pass_x", R.st, (k_soft_pass_x<<<blocks, kSoftTileX, 0, R.st>>>(in, out, g, mode, reach, T, skip)));
     return;
   }
   const size_t smem = (size_t)(kSoftTileYZ + 2 * reach) * 32 * sizeof(float);
@@ -762,9 +1118,9 @@ void pass(const SoftRun &R, const float *in, float *out, int axis, int mode, int
     return;
   }
   if (axis == 1)
-    KLAUNCH("k_soft_pass_y", R.st, (k_soft_pass_yz<1><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T)));
+    KLAUNCH("k_soft_pass_y", R.st, (k_soft_pass_yz<1><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T, skip)));
   else
-    KLAUNCH("k_soft_pass_z", R.st, (k_soft_pass_yz<2><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T)));
+    KLAUNCH("k_soft_pass_z", R.st, (k_soft_pass_yz<2><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T, skip)));
 }
 
 // the correlation along z with T, summed against w into *acc (double) instead of stored
@@ -774,20 +1130,20 @@ void pass_z_dot(const SoftRun &R, const float *in, const SoftTaps &T, const floa
   const size_t smem = (size_t)(kSoftTileYZ + 2 * T.r) * 32 * sizeof(float);
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(g.D, kSoftTileYZ), (unsigned)g.H);
   KLAUNCH("k_soft_pass_z_dot", R.st, (k_soft_pass_yz<2, kEpiDot><<<grid, dim3(32, 8), smem, R.st>>>(
-                                         in, nullptr, g, kConv, T.r, T, w, acc)));
+                                         in, nullptr, g, kConv, T.r, T, nullptr, w, acc)));
 }
 
 // the separable Gaussian (x, y, then z) with the DoG difference folded into the z pass:
 // out = scale * (sub - in * G), the same operations as a separate difference kernel
 void conv3_diff(const SoftRun &R, const float *in, float *out, const SoftTaps &tx, const SoftTaps &ty,
-                const SoftTaps &tz, float *t1, float *t2, const float *sub, float scale) {
-  pass(R, in, t1, 0, kConv, 0, tx);
-  pass(R, t1, t2, 1, kConv, 0, ty);
+                const SoftTaps &tz, float *t1, float *t2, const float *sub, float scale, const unsigned *skip) {
+  pass(R, in, t1, 0, kConv, 0, tx, skip);
+  pass(R, t1, t2, 1, kConv, 0, ty, skip);
   const SoftGeom &g = R.g;
   const size_t smem = (size_t)(kSoftTileYZ + 2 * tz.r) * 32 * sizeof(float);
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(g.D, kSoftTileYZ), (unsigned)g.H);
   KLAUNCH("k_soft_pass_z_diff", R.st, (k_soft_pass_yz<2, kEpiDiff><<<grid, dim3(32, 8), smem, R.st>>>(
-                                          t2, out, g, kConv, tz.r, tz, sub, nullptr, scale)));
+                                          t2, out, g, kConv, tz.r, tz, skip, sub, nullptr, scale)));
 }
 
 // a transposed pass along `axis`: box gather (src = g_out, into g_in) or min / max scatter
@@ -829,14 +1185,26 @@ void adj_pass(const SoftRun &R, const float *src, const float *g_out, float *g_i
 
 // conv of `in` with taps (tx, ty, tz) along x, y, z -> out (t1, t2 as temporaries)
 void conv3(const SoftRun &R, const float *in, float *out, const SoftTaps &tx, const SoftTaps &ty, const SoftTaps &tz,
-           float *t1, float *t2) {
-  pass(R, in, t1, 0, kConv, 0, tx);
-  pass(R, t1, t2, 1, kConv, 0, ty);
-  pass(R, t2, out, 2, kConv, 0, tz);
+           float *t1, float *t2, const unsigned *skip = nullptr) {
+  pass(R, in, t1, 0, kConv, 0, tx, skip);
+  pass(R, t1, t2, 1, kConv, 0, ty, skip);
+  pass(R, t2, out, 2, kConv, 0, tz, skip);
 }
 
-// The forward chain into the workspace: min/max chains, box means, norm, dog.
-void forward_chain(const SoftRun &R, const float *vol) {
+// The DoG slot from the normalized one (temporaries T1-T3); skip: a device flag that says it is filled.
+void dense_dog(const SoftRun &R, const unsigned *skip) {
+  const float *s = R.p.sigma;
+  const float nrm = (float)pow((double)s[0] * s[1] * s[2], (double)R.p.gamma);
+  conv3(R, R.slot(S_NORM), R.slot(S_T3), gauss_taps_f(s[0], false), gauss_taps_f(s[1], false), gauss_taps_f(s[2], false),
+        R.slot(S_T1), R.slot(S_T2), skip);
+  conv3_diff(R, R.slot(S_NORM), R.slot(S_DOG), gauss_taps_f(s[3], false), gauss_taps_f(s[4], false),
+             gauss_taps_f(s[5], false), R.slot(S_T1), R.slot(S_T2), R.slot(S_T3), nrm, skip);
+}
+
+// The forward chain into the workspace: min/max chains, box means, norm, and the DoG when the
+// score is to be read from the volume.
+void forward_chain(const SoftRun &R, const float *vol, bool want_dog) {
+  cudaMemsetAsync(R.acc, 0, 16 * sizeof(double), R.st);
   const hdog_soft_params &p = R.p;
   const SoftTaps none = no_taps();
   const int rr[3] = {p.radius_norm_xy, p.radius_norm_xy, p.radius_norm_z};
@@ -855,13 +1223,51 @@ void forward_chain(const SoftRun &R, const float *vol) {
   pass(R, R.slot(S_T1), R.slot(S_T2), 1, kBox, rr[1], none);
   pass(R, R.slot(S_T2), R.slot(S_D), 2, kBox, rr[2], none);
   KLAUNCH("k_soft_norm", R.st, (k_soft_norm<<<R.blocks(), 256, 0, R.st>>>(vol, R.slot(S_E), R.slot(S_D), R.slot(S_NORM),
-                                                                        p.min_intensity, R.N)));
+                                                                        p.min_intensity, R.N, R.flags())));
+  if (want_dog) {
+    dense_dog(R, nullptr);
+    cudaMemsetAsync(R.flags() + 1, 1, sizeof(unsigned), R.st);
+  }
+}
+
+// Whether the DoG is evaluated at the points' neighbourhoods (k_soft_points_local) instead of
+// over the volume: when a block's box fits twice on an SM, and the points cost less than the 28 dense
+// passes.  Measured (forward + backward, ns): a point 34, 57 and 185 at patches of 1859, 4335 and
+// 14297 voxels, so about 20 + 0.011 per voxel; the dense passes 0.16 per voxel of the volume plus about
+// 150 us of launches (665-830 us at 64x256x256, 200 us at 32x80x96).  At 64x256x256 that puts the
+// line at 12 k points for the middle patch: 8 k took 1.60 against 1.95 ms, 32 k 3.00 against 2.09.
+constexpr size_t kSoftLocalSmem = 110 * 1024;
+
+bool points_local(const SoftRun &R, int64_t n, SoftBox &box) {
+  for (int a = 0; a < 3; a++)
+    box.r[a] = std::max((int)(2.0 * R.p.sigma[a] + 0.5), (int)(2.0 * R.p.sigma[a + 3] + 0.5));
+  if ((size_t)box.floats() * sizeof(float) > kSoftLocalSmem) return false;
+  return (double)n * (20.0 + 0.011 * box.tile()) <= 0.16 * (double)R.N + 150e3;
+}
+
+template <bool BWD>
+void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
+                   float grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+  const hdog_soft_params &p = R.p;
+  const int64_t n = (int64_t)n_pos + n_neg;
+  if (n == 0) return;
+  SoftTapSet T;
+  for (int k = 0; k < 6; k++) {
+    T.plain[k] = gauss_taps_f(p.sigma[k], false);
+    T.deriv[k] = gauss_taps_f(p.sigma[k], true);
+  }
+  SoftThresh b;
+  for (int k = 0; k < 3; k++) b.v[k] = p.thresh[k];
   const float *s = p.sigma;
-  conv3(R, R.slot(S_NORM), R.slot(S_T3), gauss_taps_f(s[0], false), gauss_taps_f(s[1], false), gauss_taps_f(s[2], false),
-        R.slot(S_T1), R.slot(S_T2));
   const float nrm = (float)pow((double)s[0] * s[1] * s[2], (double)p.gamma);
-  conv3_diff(R, R.slot(S_NORM), R.slot(S_DOG), gauss_taps_f(s[3], false), gauss_taps_f(s[4], false),
-             gauss_taps_f(s[5], false), R.slot(S_T1), R.slot(S_T2), R.slot(S_T3), nrm);
+  const size_t smem = (size_t)box.floats() * sizeof(float);
+  if (smem > 44 * 1024)   // 48 KB without it, static shared memory included
+    cudaFuncSetAttribute(k_soft_points_local<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoftLocalSmem);
+  const unsigned grid = (unsigned)std::min<int64_t>(n, 152 * 8);
+  KLAUNCH(BWD ? "k_soft_points_local_adj" : "k_soft_points_local", R.st,
+          (k_soft_points_local<BWD><<<grid, kSoftPtThreads, smem, R.st>>>(R.slot(S_NORM), R.g, pos, n_pos, neg, n_neg, T,
+                                                                          box, nrm, p.tau, b, grad_loss, scores, acc, gb,
+                                                                          gnorm)));
 }
 
 SoftThresh thresh_of(const hdog_soft_params &p) {
@@ -896,9 +1302,12 @@ int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos
             static_cast<float *>(work), nullptr};
   R.acc = static_cast<double *>(work);
   R.w = reinterpret_cast<float *>(R.acc + 16);
-  forward_chain(R, vol);
-  cudaMemsetAsync(R.acc, 0, sizeof(double), st);
-  if (n_pos + n_neg > 0)
+  SoftBox box;
+  const bool local = points_local(R, (int64_t)n_pos + n_neg, box);
+  forward_chain(R, vol, !local);
+  if (local)
+    points_launch<false>(R, box, pos, n_pos, neg, n_neg, 0.0f, scores, R.acc, nullptr, nullptr);
+  else if (n_pos + n_neg > 0)
     KLAUNCH("k_soft_points", st, (k_soft_points<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
                                      R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), scores,
                                      R.acc)));
@@ -918,60 +1327,70 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
   const unsigned nb = R.blocks();
   // The backward reads the forward chain's slots (S_MN1 .. S_DOG) and writes only the others,
   // so a workspace that soft_forward filled for the same inputs still holds them.
-  if (!forward_kept) forward_chain(R, vol);
-  float *gdog = R.slot(S_GDOG);
-  cudaMemsetAsync(gdog, 0, R.N * sizeof(float), st);
-  double *gb = R.acc + 8;   // threshold gradients
-  cudaMemsetAsync(gb, 0, 3 * sizeof(double), st);
-  if (n_pos + n_neg > 0)
-    KLAUNCH("k_soft_points_adj", st, (k_soft_points_adj<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
-                                         R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), grad_loss,
-                                         gdog, gb)));
-  if (grad_thresh) k_soft_to_float<<<1, 32, 0, st>>>(gb, grad_thresh, 3);
+  SoftBox box;
+  const bool local = points_local(R, (int64_t)n_pos + n_neg, box);
+  if (!forward_kept) forward_chain(R, vol, !local);
   const float *s = p->sigma;
   const float nrm = (float)pow((double)s[0] * s[1] * s[2], (double)p->gamma);
+  // acc[0..5]: <gdog, d dog / d sigma_k> without the normalizer term; acc[6]: <gdog, dog>
+  double *gb = R.acc + 8;   // threshold gradients
+  cudaMemsetAsync(R.acc, 0, 14 * sizeof(double), st);
+  float *gdog = R.slot(S_GDOG);
+  if (local) {
+    float *gnorm = grad_vol ? R.slot(S_GB) : nullptr;
+    if (gnorm) cudaMemsetAsync(gnorm, 0, R.N * sizeof(float), st);
+    points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, nullptr, grad_sigma ? R.acc : nullptr,
+                        grad_thresh ? gb : nullptr, gnorm);
+  } else {
+    // a forward call with fewer points may have left the DoG slot empty
+    if (forward_kept) dense_dog(R, R.flags() + 1);
+    static_assert(S_GB == S_GA + 1 && S_GA % 2 == 0, "an 8-byte aligned volume of doubles");
+    double *gsum = reinterpret_cast<double *>(R.slot(S_GA));
+    cudaMemsetAsync(gsum, 0, R.N * sizeof(double), st);
+    if (n_pos + n_neg > 0)
+      KLAUNCH("k_soft_points_adj", st, (k_soft_points_adj<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
+                                           R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), grad_loss,
+                                           gsum, gb)));
+    KLAUNCH("k_soft_gdog", st, (k_soft_gdog<<<nb, 256, 0, st>>>(gsum, gdog, R.N)));
+  }
+  if (grad_thresh) k_soft_to_float<<<1, 32, 0, st>>>(gb, grad_thresh, 3);
   if (grad_sigma) {
-    // acc[0..5]: <gdog, d dog / d sigma_k> without the normalizer term; acc[6]: <gdog, dog>
-    cudaMemsetAsync(R.acc, 0, 8 * sizeof(double), st);
-    const unsigned db = 152 * 4;
-    // Per scale: <gdog, C_z C_y C_x norm> with the derivative taps on one axis.  The plain x
-    // pass serves the y and z derivatives, and every z pass folds straight into the dot.
-    float *nm = R.slot(S_NORM), *t1 = R.slot(S_T1), *t2 = R.slot(S_T2);
-    for (int sc = 0; sc < 2; sc++) {
-      SoftTaps pl[3], dv[3];
-      for (int a = 0; a < 3; a++) {
-        pl[a] = gauss_taps_f(s[3 * sc + a], false);
-        dv[a] = gauss_taps_f(s[3 * sc + a], true);
+    if (!local) {
+      const unsigned db = 152 * 4;
+      // Per scale: <gdog, C_z C_y C_x norm> with the derivative taps on one axis.  The plain x
+      // pass serves the y and z derivatives, and every z pass folds straight into the dot.
+      float *nm = R.slot(S_NORM), *t1 = R.slot(S_T1), *t2 = R.slot(S_T2);
+      for (int sc = 0; sc < 2; sc++) {
+        SoftTaps pl[3], dv[3];
+        for (int a = 0; a < 3; a++) {
+          pl[a] = gauss_taps_f(s[3 * sc + a], false);
+          dv[a] = gauss_taps_f(s[3 * sc + a], true);
+        }
+        double *acc = R.acc + 3 * sc;
+        pass(R, nm, t1, 0, kConv, 0, pl[0]);
+        pass(R, t1, t2, 1, kConv, 0, pl[1]);
+        pass_z_dot(R, t2, dv[2], gdog, acc + 2);
+        pass(R, t1, t2, 1, kConv, 0, dv[1]);
+        pass_z_dot(R, t2, pl[2], gdog, acc + 1);
+        pass(R, nm, t1, 0, kConv, 0, dv[0]);
+        pass(R, t1, t2, 1, kConv, 0, pl[1]);
+        pass_z_dot(R, t2, pl[2], gdog, acc + 0);
       }
-      double *acc = R.acc + 3 * sc;
-      pass(R, nm, t1, 0, kConv, 0, pl[0]);
-      pass(R, t1, t2, 1, kConv, 0, pl[1]);
-      pass_z_dot(R, t2, dv[2], gdog, acc + 2);
-      pass(R, t1, t2, 1, kConv, 0, dv[1]);
-      pass_z_dot(R, t2, pl[2], gdog, acc + 1);
-      pass(R, nm, t1, 0, kConv, 0, dv[0]);
-      pass(R, t1, t2, 1, kConv, 0, pl[1]);
-      pass_z_dot(R, t2, pl[2], gdog, acc + 0);
+      KLAUNCH("k_soft_dot", st, (k_soft_dot<<<db, 256, 0, st>>>(gdog, R.slot(S_DOG), R.N, R.acc + 6)));
     }
-    KLAUNCH("k_soft_dot", st, (k_soft_dot<<<db, 256, 0, st>>>(gdog, R.slot(S_DOG), R.N, R.acc + 6)));
-    double h[8];
-    HDOG_CUDA_TRY(cudaMemcpyAsync(h, R.acc, sizeof(h), cudaMemcpyDeviceToHost, st));
-    HDOG_CUDA_TRY(cudaStreamSynchronize(st));
-    float gs[6];
-    for (int k = 0; k < 6; k++) {
-      double v = (k < 3 ? nrm : -nrm) * h[k];
-      if (k < 3) v += (double)p->gamma / s[k] * h[6];   // d normalizer / d sigma = gamma normalizer / sigma
-      gs[k] = (float)v;
-    }
-    HDOG_CUDA_TRY(cudaMemcpyAsync(grad_sigma, gs, sizeof(gs), cudaMemcpyHostToDevice, st));
-    HDOG_CUDA_TRY(cudaStreamSynchronize(st));
+    SoftSigma sg;
+    for (int k = 0; k < 6; k++) sg.v[k] = s[k];
+    KLAUNCH("k_soft_sigma_grad", st, (k_soft_sigma_grad<<<1, 32, 0, st>>>(R.acc, local ? R.flags() : nullptr, sg, nrm,
+                                                                         p->gamma, grad_sigma)));
   }
   if (grad_vol) {
-    // g_norm = normalizer (G1 - G2)^T gdog = normalizer (G1 gdog - G2 gdog)
-    conv3(R, gdog, R.slot(S_T3), gauss_taps_f(s[0], false), gauss_taps_f(s[1], false), gauss_taps_f(s[2], false),
-          R.slot(S_T1), R.slot(S_T2));
-    conv3_diff(R, gdog, R.slot(S_GB), gauss_taps_f(s[3], false), gauss_taps_f(s[4], false), gauss_taps_f(s[5], false),
-               R.slot(S_T1), R.slot(S_T2), R.slot(S_T3), nrm);
+    if (!local) {
+      // g_norm = normalizer (G1 - G2)^T gdog = normalizer (G1 gdog - G2 gdog)
+      conv3(R, gdog, R.slot(S_T3), gauss_taps_f(s[0], false), gauss_taps_f(s[1], false), gauss_taps_f(s[2], false),
+            R.slot(S_T1), R.slot(S_T2));
+      conv3_diff(R, gdog, R.slot(S_GB), gauss_taps_f(s[3], false), gauss_taps_f(s[4], false), gauss_taps_f(s[5], false),
+                 R.slot(S_T1), R.slot(S_T2), R.slot(S_T3), nrm, nullptr);
+    }
     // quotient rule: direct term into grad_vol, g_e -> S_T1, g_d -> S_T2
     KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<<<nb, 256, 0, st>>>(vol, R.slot(S_E), R.slot(S_D), R.slot(S_GB),
                                                                        grad_vol, R.slot(S_T1), R.slot(S_T2),
