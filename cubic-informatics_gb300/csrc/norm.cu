@@ -12,9 +12,9 @@
 // sequential float sum `val = 0; for j in 0..2r: val += s[j]` times 1.0f/(2r+1).
 // Five passes, each one read and one write of the volume:
 //
-//   mm_z      uint16 -> packed u32     z window, four columns per thread
-//   mm_y      u32 -> u32               van Herk / Gil-Werman column window in smem
-//   mm_x_box  u32 -> float2            van Herk / Gil-Werman row window, then the x box
+//   mm_z      uint16 -> packed u32     van Herk / Gil-Werman z window in registers
+//   mm_y      u32 -> u32               column window from short blocks (window.cuh)
+//   mm_x_box  u32 -> float2            row window from short blocks, then the x box
 //                                      sum as exact integer sliding sums (2r+1 <= 256:
 //                                      every partial sum of the reference's float chain
 //                                      is an integer below 2^24, hence exact)
@@ -24,7 +24,10 @@
 //
 // Erosion and dilation travel as one packed u32 per voxel: low half the running min,
 // high half 65535 minus the running max, so one __vminu2 combines both.
+#include <algorithm>
+
 #include "kernels.cuh"
+#include "window.cuh"
 
 namespace hdog {
 
@@ -84,28 +87,47 @@ __global__ void __launch_bounds__(256) k_mm_z(const Sub *subs, int rz, uint32_t 
   }
 }
 
-// The same z pass with nearest borders and a compile-time radius, streaming van Herk /
-// Gil-Werman in registers: a thread owns two neighbouring columns and runs down z, every
-// input slice loaded once (the windowed loop above reads each one 2R+1 times).  Both
-// voxels are packed as (v, 65535 - v), so one __vminu2 carries the min and the max.
-template <int R>
+// The same z pass with a compile-time radius, streaming van Herk / Gil-Werman in registers: a
+// thread owns VEC neighbouring columns (two where the slices' 4-byte words hold two columns each)
+// and runs down z, every input slice loaded once (the windowed loop above reads each one 2R+1
+// times).  A voxel is packed as (v, 65535 - v), so one __vminu2 carries the min and the max.
+template <int R, int BORDER, int VEC>
 __global__ void __launch_bounds__(128) k_mm_z_stream(const Sub *subs, uint32_t *mm) {
   constexpr int L = 2 * R + 1;
   const Sub S = subs[blockIdx.y];
   const int64_t plane = (int64_t)S.W * S.H;
-  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
+  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (p >= plane) return;
   const int D = S.D, dv = S.depth_valid;
   const uint16_t *col = S.src + p;
   uint32_t *oc = mm + S.vox + p;
-  auto ld = [&](int z) -> uint2 {
-    z = clampi(z, 0, D - 1);
-    if (z >= dv) return make_uint2(kZeroPacked, kZeroPacked);
-    const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(col + (int64_t)z * plane));
-    return make_uint2(__byte_perm(v, ~v, 0x5410), __byte_perm(v, ~v, 0x7632));
+  struct Cols {
+    uint32_t c[VEC];
   };
-  auto vmin = [](uint2 a, uint2 b) { return make_uint2(__vminu2(a.x, b.x), __vminu2(a.y, b.y)); };
-  uint2 suf[L], cur[L];
+  auto ld = [&](int z) -> Cols {
+    Cols r;
+    const bool out = BORDER == 1 && (z < 0 || z >= D);
+    z = clampi(z, 0, D - 1);
+    if (out || z >= dv) {
+#pragma unroll
+      for (int k = 0; k < VEC; k++) r.c[k] = kZeroPacked;
+    } else if constexpr (VEC == 2) {
+      const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(col + (int64_t)z * plane));
+      r.c[0] = __byte_perm(v, ~v, 0x5410);
+      r.c[1] = __byte_perm(v, ~v, 0x7632);
+    } else {
+      const uint32_t v = __ldg(col + (int64_t)z * plane);
+      r.c[0] = __byte_perm(v, ~v, 0x5410);
+    }
+    return r;
+  };
+  auto vmin = [](Cols a, Cols b) {
+    Cols r;
+#pragma unroll
+    for (int k = 0; k < VEC; k++) r.c[k] = __vminu2(a.c[k], b.c[k]);
+    return r;
+  };
+  Cols suf[L], cur[L];
 #pragma unroll
   for (int j = 0; j < L; j++) suf[j] = ld(j - R);
 #pragma unroll
@@ -113,11 +135,17 @@ __global__ void __launch_bounds__(128) k_mm_z_stream(const Sub *subs, uint32_t *
   for (int t0 = 0; t0 < D; t0 += L) {
 #pragma unroll
     for (int j = 0; j < L; j++) cur[j] = ld(t0 - R + L + j);
-    uint2 pre = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+    Cols pre;
+#pragma unroll
+    for (int k = 0; k < VEC; k++) pre.c[k] = 0xFFFFFFFFu;
 #pragma unroll
     for (int i = 0; i < L; i++) {
-      const uint2 m = i == 0 ? suf[0] : vmin(suf[i], pre);
-      if (t0 + i < D) *reinterpret_cast<uint2 *>(oc + (int64_t)(t0 + i) * plane) = m;
+      const Cols m = i == 0 ? suf[0] : vmin(suf[i], pre);
+      if (t0 + i < D) {
+        uint32_t *o = oc + (int64_t)(t0 + i) * plane;
+        if constexpr (VEC == 2) *reinterpret_cast<uint2 *>(o) = make_uint2(m.c[0], m.c[1]);
+        else *o = m.c[0];
+      }
       pre = vmin(pre, cur[i]);
     }
     suf[L - 1] = cur[L - 1];
@@ -282,175 +310,242 @@ __global__ void __launch_bounds__(256) k_mm_x(const Sub *subs, int r, int ry, in
   }
 }
 
-// ---------------------------------------------------------------- streaming y / x passes
-// Radius-specialised min/max passes (L = 2R+1 known at compile time).  Each thread walks
-// one line in blocks of L inputs and keeps, in registers, the suffix minima of the
-// previous block and the running prefix minimum of the current one (van Herk /
-// Gil-Werman): the window [t-R, t+R] starting at index i of block b is
-// min(suffix_b[i], prefix_{b+1}[i-1]).  The loops over a block are unrolled, so every
-// register index is a constant.  Nearest border (BORDER 0) clamps the line index; the
-// zero border (BORDER 1) reads the packed zero outside the line.
+// ---------------------------------------------------------------- y / x passes for any reach
+// Windows from short blocks (window.cuh), for reaches from 4 up.
+struct PackedMin {
+  typedef uint32_t T;
+  __device__ __forceinline__ static T op(T a, T b) { return __vminu2(a, b); }
+};
 
-// y pass: one thread per (column, segment of rows) of a slice; a warp reads 32
-// consecutive columns of a row per load.
-template <int R, int BORDER>
-__global__ void __launch_bounds__(128, 8) k_mm_y_stream(const Sub *subs, int seg, const uint32_t *in, uint32_t *out) {
-  constexpr int L = 2 * R + 1;
+constexpr int kColWarps = 8;
+
+// y pass: a block of 32 columns x kColWarps warps runs down `seg` rows of one slice, B rows per warp
+// and step, every input row read once (the 2r halo rows twice per segment).
+// HBM and latency: at reach 20 67% of the DRAM cycles at 28 warps per SM.  2560x2160x32 substacks:
+// eight with reach 20 2.16 -> 1.89 ms (against columns of 41 entries in registers), four with reach
+// 100 9.26 -> 1.33 ms (against chains of 201 in shared memory).
+template <int BORDER, int B>
+__global__ void __launch_bounds__(32 * kColWarps) k_mm_y_cols(const Sub *subs, int r, int seg, const uint32_t *in,
+                                                              uint32_t *out) {
+  extern __shared__ uint32_t ring_y[];
   const Sub S = subs[blockIdx.z];
   const int W = S.W, H = S.H;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int nseg = (H + seg - 1) / seg;
   const int z = blockIdx.y / nseg, ys = (blockIdx.y % nseg) * seg;
-  if (x >= W || z >= S.D) return;
-  const int ye = min(ys + seg, H);
-  const int64_t plane = (int64_t)W * H;
-  const uint32_t *col = in + S.vox + z * plane + x;
-  uint32_t *oc = out + S.vox + z * plane + x;
-  auto ld = [&](int y) -> uint32_t {
-    if (BORDER == 1 && (y < 0 || y >= H)) return kZeroPacked;
-    return __ldg(col + (int64_t)clampi(y, 0, H - 1) * W);
-  };
-  uint32_t suf[L], cur[L];
+  if (z >= S.D) return;
+  const int x = blockIdx.x * 32 + threadIdx.x, n = min(seg, H - ys);
+  const bool xin = x < W;
+  const int64_t base = S.vox + (int64_t)z * W * H + min(x, W - 1);
+  const uint32_t *col = in + base;
+  uint32_t *oc = out + base + (int64_t)ys * W;
+  ext_cols<PackedMin, B, kColWarps>(
+      ring_y, n, r,
+      [&](int a, uint32_t (&v)[B]) {
+        const int y = ys - r + a;
+        if (y >= 0 && y + B <= H) {
+          const uint32_t *p = col + (int64_t)y * W;
 #pragma unroll
-  for (int j = 0; j < L; j++) suf[j] = ld(ys - R + j);
+          for (int j = 0; j < B; j++, p += W) v[j] = __ldg(p);
+        } else {
 #pragma unroll
-  for (int j = L - 2; j >= 0; j--) suf[j] = __vminu2(suf[j], suf[j + 1]);
-  for (int t0 = ys; t0 < ye; t0 += L) {
-#pragma unroll
-    for (int j = 0; j < L; j++) cur[j] = ld(t0 - R + L + j);
-    uint32_t pre = 0xFFFFFFFFu;
-#pragma unroll
-    for (int i = 0; i < L; i++) {
-      const uint32_t m = i == 0 ? suf[0] : __vminu2(suf[i], pre);
-      if (t0 + i < ye) oc[(int64_t)(t0 + i) * W] = m;
-      pre = __vminu2(pre, cur[i]);
-    }
-    suf[L - 1] = cur[L - 1];
-#pragma unroll
-    for (int j = L - 2; j >= 0; j--) suf[j] = __vminu2(cur[j], suf[j + 1]);
-  }
+          for (int j = 0; j < B; j++) {
+            const bool zero = BORDER == 1 && (y + j < 0 || y + j >= H);
+            v[j] = zero ? kZeroPacked : __ldg(col + (int64_t)clampi(y + j, 0, H - 1) * W);
+          }
+        }
+      },
+      [&](int t, uint32_t m) {
+        if (xin) oc[(int64_t)t * W] = m;
+      });
 }
 
-// x pass (nearest border) with the exact x box sum -> float2 (ero_x, dil_x): one warp per
-// 32 rows, one row per lane.  Each block of L inputs of the warp's rows is staged in
-// shared memory by cp.async, one block ahead of the one in use (two buffers), then read
-// one row per lane (L is odd, so the lanes' rows fall in distinct banks).  The box sum
-// over the window minima M slides one position per step as an exact integer sum; the box
-// output of u is formed when M(u + R) is, with M(0) standing for positions left of the
-// row and M(W-1) right of it.  Outputs return through a shared tile for row-wise
-// coalesced stores.
-constexpr int kXsWarps = 2;
+// x pass, G lanes per row, outputs as k_mm_x's MODE: 0 the exact x box sums of the extremes -> float2
+// (2r + 1 <= 255), 1 the min -> uint16, 2 the packed extremes.  A lane's 8 neighbours are loaded as
+// one 32-byte word and its 8 box means stored as two where the addresses allow it: the row starts `pad`
+// entries early, so that for even reaches inputs and outputs both fall on 32 bytes (for odd ones the
+// outputs do, and the inputs on 8).  The next chunk's inputs are loaded before this one is worked on.
+// MODE 0: a lane's first box sum is the difference of two prefix sums of the extremes (a scan of
+// the lanes' totals, and the prefix at the one place of a block where its windows start, from the lane
+// that many blocks back); the other seven slide, taking the extremes that leave from a second ring. All in
+// wrapping integers; the row's first and last extreme stand for the positions outside it.
+// G = 8 for reaches up to 31: chunks of 64 entries waste less of a short row, and the scan is three steps.
+// Bound by instruction issue and the shared-memory pipe.
+// 2560x2160x32 substacks: eight with reach 20 3.85 -> 3.41 ms (against rows of 41 entries in
+// registers), four with reach 100 9.85 -> 1.62 ms (against chains of 201 in shared memory); 256x256
+// and half frames with reach 20 83 -> 59 us a batch.
+constexpr int kRowWarps = 4;
 
-__device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
+// 32-byte global accesses (sm_100 on)
+__device__ __forceinline__ void ld8(const uint32_t *p, uint32_t (&v)[8]) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void st8(float2 *p, float2 a, float2 b, float2 c, float2 d) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y),
+               "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// acc +- one half of a packed pair
+template <int HALF, int SIGN>
+__device__ __forceinline__ uint32_t add_half(uint32_t pair, uint32_t acc) {
+  int r;
+  asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(pair), "r"((SIGN & 0xFF) << (8 * HALF)), "r"((int)acc));
+  return (uint32_t)r;
 }
 
-template <int R>
-__global__ void __launch_bounds__(32 * kXsWarps) k_mm_x_stream(const Sub *subs, const uint32_t *in, float2 *out) {
-  constexpr int L = 2 * R + 1;
-  static_assert(L <= 255, "the integer box sum needs 2R+1 <= 256");
-  __shared__ uint32_t sin_[kXsWarps][2][32 * L];
-  __shared__ float2 sout[kXsWarps][32 * L];
+template <int BORDER, int MODE, int G, int Q>
+__global__ void __launch_bounds__(32 * kRowWarps) k_mm_x_rows(const Sub *subs, int r, const uint32_t *in, void *out) {
+  using R = RowRing<G>;
+  __shared__ uint32_t smr[kRowWarps][R::WORDS * (MODE == 0 ? 2 : 1)];
   const Sub S = subs[blockIdx.y];
-  const int W = S.W;
+  const int W = S.W, gl = threadIdx.x & (G - 1), w = threadIdx.x >> 5;
   const int64_t rows = (int64_t)S.H * S.D;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t row0 = ((int64_t)blockIdx.x * kXsWarps + w) * 32;
+  const int64_t row0 = ((int64_t)blockIdx.x * kRowWarps + w) * R::LINES;
   if (row0 >= rows) return;
-  const int nr = (int)min((int64_t)32, rows - row0);
-  float2 *tout = sout[w];
-  const uint32_t *lines = in + S.vox + row0 * W;
-  float2 *olines = out + S.vox + row0 * W;
-
-  // inputs [p, p + L) of the warp's rows (clamped to the row) -> buffer, asynchronously
-  auto issue = [&](int p, uint32_t *buf) {
-#pragma unroll 4
-    for (int k = 0; k < 32; k++) {
-      const uint32_t *line = lines + (int64_t)min(k, nr - 1) * W;
-#pragma unroll
-      for (int i = lane; i < L; i += 32) cp_async4(buf + k * L + i, line + clampi(p + i, 0, W - 1));
-    }
-    cp_async_commit();
-  };
-
+  const int64_t mine = row0 + (threadIdx.x & 31) / G, row = min(mine, rows - 1);
+  const bool live = mine < rows;
+  uint32_t *suf = smr[w], *ring = suf + R::WORDS;   // ring: MODE 0, the extremes
+  const uint32_t *line = in + S.vox + row * W;
+  const int n_in = W + 2 * r, n_e = MODE == 0 ? W + 3 * r : n_in;
+  const int L = 2 * r + 1;
   const float inv = 1.0f / (float)L;
   const uint32_t full = (uint32_t)L * 0xFFFFu;
-  uint32_t suf[L], cur[L], mp[L];
-  issue(-R, sin_[w][0]);
-  issue(-R + L, sin_[w][1]);
-  cp_async_wait<1>();
-  __syncwarp();
+  constexpr int QP = Q == 0 ? 7 : Q - 1;            // 8 ceil(L / 8) - L
+  const int backp = (L + 7) / 8;
+  // entry e is position e - r; entries -pad .. -1 are there for the alignment only
+  const uintptr_t in0 = reinterpret_cast<uintptr_t>(line - r);
+  float2 *o2 = reinterpret_cast<float2 *>(out) + S.vox + row * W;
+  const uintptr_t out0 = reinterpret_cast<uintptr_t>(o2 - 3 * r);
+  const int pad = MODE != 0 ? 0 : Q % 4 == 0 ? (int)((in0 >> 2) & 7) : (int)((out0 >> 3) & 3);
+  const int in_al = (int)(((in0 >> 2) - pad) & 7);
+  const bool out_al = (((out0 >> 3) - pad) & 3) == 0;
+  uint32_t nv[8], hist[6] = {0, 0, 0, 0, 0, 0};
+  uint32_t m0 = 0, mlast = 0, clo = 0, chi = 0, plo = 0, phi = 0;
+  auto fetch = [&](int c) {
+    const int x = c + 8 * gl - r;
+    const uint32_t *p = line + x;
+    if (x >= 0 && x + 8 <= W && (in_al & 1) == 0) {
+      if (in_al == 0) {
+        ld8(p, nv);
+      } else {
 #pragma unroll
-  for (int j = 0; j < L; j++) suf[j] = sin_[w][0][lane * L + j];
-#pragma unroll
-  for (int j = L - 2; j >= 0; j--) suf[j] = __vminu2(suf[j], suf[j + 1]);
-  uint32_t slo = 0, shi = 0, m0 = 0, mlast = 0;
-  int b = 0;
-  for (int t0 = 0; t0 < W + R; t0 += L, b ^= 1) {
-    __syncwarp();                                  // every lane is done with buffer b
-    issue(t0 - R + 2 * L, sin_[w][b]);            // block after next
-    cp_async_wait<1>();                            // block after this one has landed
-    __syncwarp();
-    const uint32_t *cb = sin_[w][b ^ 1];
-#pragma unroll
-    for (int j = 0; j < L; j++) cur[j] = cb[lane * L + j];
-    uint32_t pre = 0xFFFFFFFFu;
-    if (t0 >= L && t0 + L < W) {   // interior: every M(t - L) is in mp, no border
-#pragma unroll
-      for (int i = 0; i < L; i++) {
-        const uint32_t m = i == 0 ? suf[0] : __vminu2(suf[i], pre);
-        pre = __vminu2(pre, cur[i]);
-        const uint32_t o = mp[i];
-        slo += (m & 0xFFFFu) - (o & 0xFFFFu);
-        shi += (m >> 16) - (o >> 16);
-        mp[i] = m;
-        tout[lane * L + i] = make_float2((float)slo * inv, (float)(full - shi) * inv);
+        for (int o = 0; o < 8; o += 2) {
+          const uint2 a = __ldg(reinterpret_cast<const uint2 *>(p + o));
+          nv[o] = a.x;
+          nv[o + 1] = a.y;
+        }
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < L; i++) {
-        const int t = t0 + i;
-        uint32_t m = i == 0 ? suf[0] : __vminu2(suf[i], pre);
-        pre = __vminu2(pre, cur[i]);
-        if (t == W - 1) mlast = m;
-        if (t >= W) m = mlast;
-        if (t == 0) {
-          m0 = m;
-          slo = (uint32_t)L * (m & 0xFFFFu);
-          shi = (uint32_t)L * (m >> 16);
-        } else {
-          const uint32_t o = t >= L ? mp[i] : m0;
-          slo += (m & 0xFFFFu) - (o & 0xFFFFu);
-          shi += (m >> 16) - (o >> 16);
+      for (int o = 0; o < 8; o++)
+        nv[o] = (BORDER == 1 && (x + o < 0 || x + o >= W)) ? kZeroPacked : __ldg(line + clampi(x + o, 0, W - 1));
+    }
+  };
+  int c = -pad;   // the chunk's first entry; the warp's rows may differ by up to 7
+  fetch(c);
+  int pc = 0;
+  for (int i = 0; i < n_e + (MODE == 0 ? 7 : 0); i += R::CHUNK, c += R::CHUNK) {
+    uint32_t v[8], m[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++) v[o] = nv[o];
+    if (i < n_in) fetch(c + R::CHUNK);
+    ext_row_chunk<PackedMin, G, Q>(suf, pc, r, v, hist, m);
+    const int e0 = c + 8 * gl;   // the window that ends with entry e is centred on position e - 2r
+    if (MODE == 0) {
+      const int ef = 2 * r, el = W - 1 + 2 * r;   // the first and the last position's entries
+      const bool inside = __all_sync(0xFFFFFFFFu, c >= ef + L && c + R::CHUNK - 1 < el);
+      if (!inside) {
+        uint32_t tf = m[0], tl = m[0];
+#pragma unroll
+        for (int o = 1; o < 8; o++) {
+          tf = o == ((ef - c) & 7) ? m[o] : tf;
+          tl = o == ((el - c) & 7) ? m[o] : tl;
         }
-        mp[i] = m;
-        tout[lane * L + i] = make_float2((float)slo * inv, (float)(full - shi) * inv);
+        tf = __shfl_sync(0xFFFFFFFFu, tf, ((ef - c) >> 3) & (G - 1), G);
+        tl = __shfl_sync(0xFFFFFFFFu, tl, ((el - c) >> 3) & (G - 1), G);
+        if (ef >= c && ef < c + R::CHUNK) m0 = tf;
+        if (el >= c && el < c + R::CHUNK) mlast = tl;
+        // left of the row: nothing here, the first extreme's share comes with the box; right of it: the last extreme
+#pragma unroll
+        for (int o = 0; o < 8; o++) m[o] = e0 + o < ef ? 0u : e0 + o > el ? mlast : m[o];
+      }
+      const RowAt<G> at(pc);
+      const int own = at(0);
+      uint32_t tlo = 0, thi = 0, qlo = 0, qhi = 0;
+#pragma unroll
+      for (int o = 0; o < 8; o++) {
+        ring[o * R::PITCH + own] = m[o];
+        tlo = add_half<0, 1>(m[o], tlo);
+        thi = add_half<1, 1>(m[o], thi);
+        if (o == QP) {
+          qlo = tlo;
+          qhi = thi;
+        }
+      }
+      uint32_t blo = tlo, bhi = thi;   // inclusive scan of the lanes' totals
+#pragma unroll
+      for (int d = 1; d < G; d <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, blo, d, G), b = __shfl_up_sync(0xFFFFFFFFu, bhi, d, G);
+        if (gl >= d) {
+          blo += a;
+          bhi += b;
+        }
+      }
+      const uint32_t slo = __shfl_sync(0xFFFFFFFFu, blo, G - 1, G), shi = __shfl_sync(0xFFFFFFFFu, bhi, G - 1, G);
+      blo += clo - tlo;   // the sum before the lane
+      bhi += chi - thi;
+      clo += slo;
+      chi += shi;
+      qlo += blo;         // the prefix at the place where windows start
+      qhi += bhi;
+      uint32_t a = blo - row_lag<G>(qlo, plo, backp), d = bhi - row_lag<G>(qhi, phi, backp);
+      plo = qlo;
+      phi = qhi;
+      __syncwarp();
+      const uint32_t *p0 = ring + at(backp), *p1 = ring + at(backp - 1);
+      if (!inside) {
+        const uint32_t left = (uint32_t)max(0, 4 * r - e0);   // positions of the box left of the row
+        a += left * (m0 & 0xFFFFu);
+        d += left * (m0 >> 16);
+      }
+      a = add_half<0, 1>(m[0], a);
+      d = add_half<1, 1>(m[0], d);
+      float2 res[8];
+#pragma unroll
+      for (int o = 0; o < 8; o++) {
+        if (o) {
+          uint32_t x = QP + o < 8 ? p0[(QP + o) * R::PITCH] : p1[(QP + o - 8) * R::PITCH];
+          if (!inside) x = e0 + o - L < ef ? m0 : x;
+          a = add_half<0, -1>(x, add_half<0, 1>(m[o], a));
+          d = add_half<1, -1>(x, add_half<1, 1>(m[o], d));
+        }
+        res[o] = make_float2((float)a * inv, (float)(full - d) * inv);
+      }
+      const int u = e0 - 3 * r;
+      if (live) {
+        if (out_al && u >= 0 && u + 8 <= W) {
+          st8(o2 + u, res[0], res[1], res[2], res[3]);
+          st8(o2 + u + 4, res[4], res[5], res[6], res[7]);
+        } else {
+#pragma unroll
+          for (int o = 0; o < 8; o++)
+            if (u + o >= 0 && u + o < W) o2[u + o] = res[o];
+        }
+      }
+    } else if (live) {
+      const int u = e0 - 2 * r;
+#pragma unroll
+      for (int o = 0; o < 8; o++) {
+        if (u + o < 0 || u + o >= W) continue;
+        if (MODE == 1) reinterpret_cast<uint16_t *>(out)[S.vox + row * W + u + o] = (uint16_t)(m[o] & 0xFFFFu);
+        else reinterpret_cast<uint32_t *>(out)[S.vox + row * W + u + o] = m[o];
       }
     }
-    __syncwarp();
-    const int u0 = t0 - R;
-#pragma unroll 4
-    for (int k = 0; k < 32; k++) {
-      if (k >= nr) break;
-#pragma unroll
-      for (int i = lane; i < L; i += 32) {
-        const int u = u0 + i;
-        if (u >= 0 && u < W) olines[(int64_t)k * W + u] = tout[k * L + i];
-      }
-    }
-    __syncwarp();                                  // the tile is rewritten next block
-    suf[L - 1] = cur[L - 1];
-#pragma unroll
-    for (int j = L - 2; j >= 0; j--) suf[j] = __vminu2(cur[j], suf[j + 1]);
+    __syncwarp();   // the rings' oldest blocks are rewritten next chunk
+    pc += G;
+    if (pc >= R::NB) pc = 0;
   }
-  cp_async_wait<0>();                              // no copy outlives the block
 }
 
 // ---------------------------------------------------------------- x pass (box, float chain)
@@ -482,38 +577,6 @@ __global__ void k_box_x_chain(const Sub *subs, int r, const uint32_t *in, float2
 }
 
 // ---------------------------------------------------------------- y / z passes (box mean)
-// Register-blocked sequential sums: a thread produces K consecutive outputs along the
-// axis; slot (u + k) % K of a K-entry rotating window feeds output k at tap u of each
-// block of K taps, so the window never moves between registers.  Every output still
-// sums its 2r+1 inputs from 0.0f in the reference order.  load(i) returns input
-// c0 - r + i.
-template <int K, class LoadF>
-__device__ __forceinline__ void box_chain(int L, LoadF load, float2 (&acc)[K]) {
-  float2 win[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    win[k] = load(k);
-    acc[k] = make_float2(0.f, 0.f);
-  }
-  int jb = 0;
-  for (; jb + K <= L; jb += K) {
-#pragma unroll
-    for (int u = 0; u < K; u++) {
-#pragma unroll
-      for (int k = 0; k < K; k++) acc[k] = add2(acc[k], win[(u + k) % K]);
-      win[u] = load(jb + u + K);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < K; u++) {
-    if (jb + u < L) {
-#pragma unroll
-      for (int k = 0; k < K; k++) acc[k] = add2(acc[k], win[(u + k) % K]);
-      if (jb + u + K < L + K - 1) win[u] = load(jb + u + K);
-    }
-  }
-}
-
 // The y box chain with a compile-time window: K outputs from a window of K registers
 // (input j + k feeds output k at step j, in the reference's order: 0 + s0 + s1 + ...).
 template <int K, int L, class LoadF>
@@ -698,12 +761,25 @@ static void allow_smem(F *fn, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// vec: the widest of 4, 2, 1 neighbouring columns that the inputs' alignment allows
 template <int BORDER>
-static void mm_z(const Sub *d_subs, int nsub, int plane, int rz, bool vec4, uint32_t *mm, cudaStream_t s) {
-  if (BORDER == 0 && vec4 && rz == 5) {
-    dim3 grid(ceil_div(plane / 2, 128), nsub);
-    KLAUNCH("k_mm_z", s, (k_mm_z_stream<5><<<grid, 128, 0, s>>>(d_subs, mm)));
-  } else if (vec4) {
+static void mm_z(const Sub *d_subs, int nsub, int plane, int rz, int vec, uint32_t *mm, cudaStream_t s) {
+  const dim3 g2(ceil_div(plane / 2, 128), nsub), g1(ceil_div(plane, 128), nsub);
+  switch (rz) {
+#define HDOG_MMZ_CASE(R)                                                                      \
+  case R:                                                                                     \
+    if (vec >= 2)                                                                             \
+      KLAUNCH("k_mm_z", s, (k_mm_z_stream<R, BORDER, 2><<<g2, 128, 0, s>>>(d_subs, mm)));     \
+    else                                                                                      \
+      KLAUNCH("k_mm_z", s, (k_mm_z_stream<R, BORDER, 1><<<g1, 128, 0, s>>>(d_subs, mm)));     \
+    return;
+    HDOG_MMZ_CASE(1) HDOG_MMZ_CASE(2) HDOG_MMZ_CASE(3) HDOG_MMZ_CASE(4)
+    HDOG_MMZ_CASE(5) HDOG_MMZ_CASE(6) HDOG_MMZ_CASE(7) HDOG_MMZ_CASE(8)
+#undef HDOG_MMZ_CASE
+    default:
+      break;
+  }
+  if (vec == 4) {
     dim3 grid(ceil_div(plane / 4, 256), nsub);
     KLAUNCH("k_mm_z", s, (k_mm_z<BORDER, 4><<<grid, 256, 0, s>>>(d_subs, rz, mm)));
   } else {
@@ -712,9 +788,32 @@ static void mm_z(const Sub *d_subs, int nsub, int plane, int rz, bool vec4, uint
   }
 }
 
+// Rows per block of the y pass: whole columns when the columns fill the chip, else segments of at
+// least one step of the block and one window.
+static int mm_y_seg(int64_t cols, int H, int r) {
+  const int64_t want = 2048;
+  const int64_t nseg = std::max<int64_t>(1, (want + cols - 1) / cols);
+  const int seg = (int)std::max<int64_t>(ceil_div(H, nseg), std::max(2 * r, 128));
+  return std::min(seg, H);
+}
+
+template <int BORDER, int B>
+static bool mm_y_cols(const Sub *d_subs, int nsub, int W, int H, int D, int r, const uint32_t *in, uint32_t *out,
+                      cudaStream_t s) {
+  const int seg = mm_y_seg((int64_t)ceil_div(W, 32) * D * nsub, H, r);
+  if ((int64_t)ceil_div(H, seg) * D > 65535) return false;   // the grid's second extent
+  const size_t smem = (size_t)ext_cols_rows(r, B, kColWarps) * 32 * sizeof(uint32_t);
+  allow_smem(k_mm_y_cols<BORDER, B>, smem);
+  const dim3 grid(ceil_div(W, 32), ceil_div(H, seg) * D, nsub);
+  KLAUNCH("k_mm_y", s, (k_mm_y_cols<BORDER, B><<<grid, dim3(32, kColWarps), smem, s>>>(d_subs, r, seg, in, out)));
+  return true;
+}
+
 template <int BORDER>
 static void mm_y(const Sub *d_subs, int nsub, int W, int H, int D, int r, const uint32_t *in, uint32_t *out,
                  cudaStream_t s) {
+  if (r >= 8 && mm_y_cols<BORDER, 16>(d_subs, nsub, W, H, D, r, in, out, s)) return;
+  if (r >= 4 && r < 8 && mm_y_cols<BORDER, 8>(d_subs, nsub, W, H, D, r, in, out, s)) return;
   // rows per block: 128, fewer when the staged window would not fit in shared memory
   const int cap_rows = max_optin_smem() / (2 * 32 * 4);
   int ty = 128;
@@ -723,34 +822,6 @@ static void mm_y(const Sub *d_subs, int nsub, int W, int H, int D, int r, const 
   allow_smem(k_mm_y<BORDER>, smem);
   dim3 grid((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, ty) * D), nsub);
   KLAUNCH("k_mm_y", s, (k_mm_y<BORDER><<<grid, 256, smem, s>>>(d_subs, r, ty, in, out)));
-}
-
-// The streaming passes where the radius has an instantiation (false: use the staged ones).
-template <int BORDER>
-static bool mm_y_stream(const Sub *d_subs, int nsub, int W, int H, int D, int r, const uint32_t *in, uint32_t *out,
-                        cudaStream_t s) {
-  const int L = 2 * r + 1;
-  const int seg = (ceil_div(H, 4) + L - 1) / L * L;   // about four segments a column, whole blocks
-  const dim3 grid(ceil_div(W, 128), ceil_div(H, seg) * D, nsub);
-  switch (r) {
-    case 20:
-      KLAUNCH("k_mm_y", s, (k_mm_y_stream<20, BORDER><<<grid, 128, 0, s>>>(d_subs, seg, in, out)));
-      return true;
-    default:
-      return false;
-  }
-}
-
-static bool mm_x_stream(const Sub *d_subs, int nsub, int64_t rows, int r, const uint32_t *in, float2 *out,
-                        cudaStream_t s) {
-  const dim3 grid(ceil_div(rows, 32 * kXsWarps), nsub);
-  switch (r) {
-    case 20:
-      KLAUNCH("k_mm_x", s, (k_mm_x_stream<20><<<grid, 32 * kXsWarps, 0, s>>>(d_subs, in, out)));
-      return true;
-    default:
-      return false;
-  }
 }
 
 static size_t mm_x_smem(int mode, int r, int ry, int tx) {
@@ -767,6 +838,21 @@ static size_t mm_x_smem(int mode, int r, int ry, int tx) {
 template <int BORDER, int MODE>
 static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const uint32_t *in, void *out,
                  cudaStream_t s) {
+  if (r >= 4 && r <= (MODE == 0 ? 127 : 255)) {
+    switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+#define HDOG_MMX_CASE(Q)                                                                                     \
+  case Q:                                                                                                    \
+    KLAUNCH("k_mm_x", s, (k_mm_x_rows<BORDER, MODE, 32, Q><<<dim3(ceil_div(rows, kRowWarps), nsub), 32 * kRowWarps, 0, s>>>( \
+                             d_subs, r, in, out)));                                                          \
+    return;                                                                                                  \
+  case Q + 1:                                                                                                \
+    KLAUNCH("k_mm_x", s, (k_mm_x_rows<BORDER, MODE, 8, Q><<<dim3(ceil_div(rows, 4 * kRowWarps), nsub), 32 * kRowWarps, 0, s>>>( \
+                             d_subs, r, in, out)));                                                          \
+    return;
+      HDOG_MMX_CASE(0) HDOG_MMX_CASE(2) HDOG_MMX_CASE(4) HDOG_MMX_CASE(6)
+#undef HDOG_MMX_CASE
+    }
+  }
   // 16 rows x 256 outputs per block, narrower until the staged rows fit in shared
   // memory; MODE 0 runs one thread per (row, chunk of kBoxC outputs).
   int ry = 16, tx = 256;
@@ -778,15 +864,16 @@ static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const 
   KLAUNCH("k_mm_x", s, (k_mm_x<BORDER, MODE><<<grid, threads, smem, s>>>(d_subs, r, ry, tx, in, out)));
 }
 
+static int mm_z_vec(bool src_aligned8, int plane) { return !src_aligned8 ? 1 : plane % 4 == 0 ? 4 : plane % 2 == 0 ? 2 : 1; }
+
 void launch_normalize(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, int rz, float min_intensity,
                       bool src_aligned8, uint32_t *ma, uint32_t *mb, float2 *fa, float2 *fb, float *norm,
                       cudaStream_t s, float *ero_l, float *dil_l) {
   const int plane = W * H;
   const int64_t rows = (int64_t)H * D;
-  mm_z<0>(d_subs, nsub, plane, rz, src_aligned8 && plane % 4 == 0, ma, s);
-  if (!mm_y_stream<0>(d_subs, nsub, W, H, D, rxy, ma, mb, s)) mm_y<0>(d_subs, nsub, W, H, D, rxy, ma, mb, s);
-  if (mm_x_stream(d_subs, nsub, rows, rxy, mb, fa, s)) {
-  } else if (2 * rxy + 1 <= 256) {
+  mm_z<0>(d_subs, nsub, plane, rz, mm_z_vec(src_aligned8, plane), ma, s);
+  mm_y<0>(d_subs, nsub, W, H, D, rxy, ma, mb, s);
+  if (2 * rxy + 1 <= 256) {
     mm_x<0, 0>(d_subs, nsub, W, rows, rxy, mb, fa, s);
   } else {
     mm_x<0, 2>(d_subs, nsub, W, rows, rxy, mb, ma, s);
@@ -835,7 +922,7 @@ void launch_erosion(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, i
   const int plane = W * H;
   const int64_t n = (int64_t)plane * D;
   uint32_t *a = tmp, *b = tmp + n * nsub;
-  mm_z<1>(d_subs, nsub, plane, rz, src_aligned8 && plane % 4 == 0, a, s);
+  mm_z<1>(d_subs, nsub, plane, rz, mm_z_vec(src_aligned8, plane), a, s);
   mm_y<1>(d_subs, nsub, W, H, D, rxy, a, b, s);
   mm_x<1, 1>(d_subs, nsub, W, (int64_t)H * D, rxy, b, dst, s);
 }
