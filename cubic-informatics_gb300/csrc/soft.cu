@@ -26,17 +26,11 @@
 // window's gradient goes to its first extreme, recomputed from the filter's input).
 // Tap radii are (int)(2 sigma + 0.5), held fixed for the derivatives.
 //
-// The windowed passes (and their transposes) run from shared-memory tiles that stage a line
-// segment or column slab with the window's reach once (k_soft_pass_x / _yz, k_soft_adj_x /
-// _yz, k_soft_ext_yz, k_soft_ext_adj_yz), and fall back to the untiled kernels for reaches
-// above kSoftTileMaxR.  Box means and Gaussians fold each output's window in one fixed order:
-// the float32 sigma gradients are sensitive to the last bits of the normalized volume, so
-// that order is kept.  Min / max windows and their first extremes, which do not round, come
-// from doubling in the tile.
 #include <algorithm>
 #include <cmath>
 
 #include "kernels.cuh"
+#include "window.cuh"
 
 namespace hdog {
 
@@ -46,7 +40,6 @@ struct SoftTaps {
   float k[kSoftMaxTaps];
   int r;
 };
-enum { kMin = 0, kMax = 1, kBox = 2, kConv = 3 };
 struct SoftGeom {
   int W, H, D;
 };
@@ -58,95 +51,24 @@ __device__ __forceinline__ void soft_axis(const SoftGeom &g, int axis, int64_t i
   else { c = z; stride = (int64_t)g.W * g.H; n = g.D; }
 }
 
-// One separable pass along `axis` (0 x, 1 y, 2 z): min / max / box mean with nearest
-// borders, or the correlation with T (zero border).
-__global__ void k_soft_pass(const float *in, float *out, SoftGeom g, int axis, int mode, int r, SoftTaps T, int64_t N) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  int c, n;
-  int64_t s;
-  soft_axis(g, axis, i, c, s, n);
-  const float *line = in + (i - (int64_t)c * s);
-  float acc;
-  if (mode == kConv) {
-    acc = 0.0f;
-    for (int j = -T.r; j <= T.r; j++) {
-      const int p = c + j;
-      if (p >= 0 && p < n) acc = __fmaf_rn(T.k[j + T.r], line[(int64_t)p * s], acc);
-    }
-  } else if (mode == kBox) {
-    acc = 0.0f;
-    for (int j = -r; j <= r; j++) acc += line[(int64_t)clampi(c + j, 0, n - 1) * s];
-    acc = acc / (float)(2 * r + 1);
-  } else {
-    acc = line[(int64_t)clampi(c - r, 0, n - 1) * s];
-    for (int j = -r + 1; j <= r; j++) {
-      const float v = line[(int64_t)clampi(c + j, 0, n - 1) * s];
-      acc = mode == kMin ? fminf(acc, v) : fmaxf(acc, v);
-    }
-  }
-  out[i] = acc;
-}
+// One separable Gaussian pass (zero border) from a shared-memory tile: a block stages the inputs of
+// its outputs once (along x a row segment of kSoftTileX outputs plus the taps' reach on each side;
+// along y or z a 32-column slab of kSoftTileYZ outputs plus the reach), zero outside the line, and every
+// output folds its taps in ascending order, skipping those outside the line.
+constexpr int kSoftTileX = 256, kSoftTileYZ = 64;
 
-// The same pass from a shared-memory tile: a block stages the inputs of its outputs once
-// (along x a row segment of kSoftTileX outputs plus the window's reach on each side; along y
-// or z a 32-column slab of kSoftTileYZ outputs plus the reach), out-of-line positions already
-// clamped (min / max / box) or zero (conv), and every output folds its window in the same
-// order and with the same operations as k_soft_pass, so the results are identical; only
-// the repeated global loads of overlapping windows are gone.  For reaches up to
-// kSoftTileMaxR.
-constexpr int kSoftTileX = 256, kSoftTileYZ = 64, kSoftTileMaxR = 64;
-
-__device__ __forceinline__ float soft_fold(const float *w, int step, int c, int n, int mode, int R, const SoftTaps &T) {
-  // w[k * step] is the input at line position c - R + k
-  float acc;
-  if (mode == kConv) {
-    acc = 0.0f;
-    for (int j = -R; j <= R; j++) {
-      const int p = c + j;
-      if (p >= 0 && p < n) acc = __fmaf_rn(T.k[j + R], w[(j + R) * step], acc);
-    }
-  } else if (mode == kBox) {
-    acc = 0.0f;
-    for (int j = -R; j <= R; j++) acc += w[(j + R) * step];
-    acc = acc / (float)(2 * R + 1);
-  } else {
-    acc = w[0];
-    for (int j = -R + 1; j <= R; j++) {
-      const float v = w[(j + R) * step];
-      acc = mode == kMin ? fminf(acc, v) : fmaxf(acc, v);
-    }
+__device__ __forceinline__ float soft_fold(const float *w, int step, int c, int n, const SoftTaps &T) {
+  // w[k * step] is the input at line position c - T.r + k
+  float acc = 0.0f;
+  for (int j = -T.r; j <= T.r; j++) {
+    const int p = c + j;
+    if (p >= 0 && p < n) acc = __fmaf_rn(T.k[j + T.r], w[(j + T.r) * step], acc);
   }
   return acc;
 }
 
-__device__ __forceinline__ float soft_stage(const float *line, int64_t s, int p, int n, int mode) {
-  if (mode == kConv) return (p >= 0 && p < n) ? line[(int64_t)p * s] : 0.0f;
-  return line[(int64_t)clampi(p, 0, n - 1) * s];
-}
-
-// Min / max windows from the staged tile by doubling: after the steps with spans 1, 2, ..., q
-// an entry holds the extreme of the q staged values from it on, where q is the largest power
-// of two <= w = 2R + 1; a window [t, t + 2R] is then the extreme of the entries t and
-// t + w - q (two spans that overlap and cover it).  Min and max do not round, so the values
-// equal the sequential fold's (for inputs without NaN).  With indices, an entry also carries
-// the staged position of its span's first extreme: a later span replaces it only when
-// strictly better, which keeps the first extreme of the union (a tie inside the overlap is
-// already the earlier span's).  Along y and z a block of 32 x 16 threads doubles a slab of
-// kSoftTileYZ + 2R rows (R <= kSoftExtMaxR), kSoftExtPer rows per thread.
-constexpr int kSoftExtMaxR = 32, kSoftExtPer = (kSoftTileYZ + 2 * kSoftExtMaxR) / 16;
-
-__device__ __forceinline__ float soft_ext(float a, float b, bool is_max) { return is_max ? fmaxf(a, b) : fminf(a, b); }
-
-__device__ __forceinline__ void soft_ext_at(float &a, int &ia, float b, int ib, bool is_max) {
-  if (is_max ? b > a : b < a) {
-    a = b;
-    ia = ib;
-  }
-}
-
-__device__ __forceinline__ int soft_span(int R) {   // the largest power of two <= 2R + 1
-  return 1 << (31 - __clz(2 * R + 1));
+__device__ __forceinline__ float soft_stage(const float *line, int64_t s, int p, int n) {
+  return (p >= 0 && p < n) ? line[(int64_t)p * s] : 0.0f;
 }
 
 // Dot products as compensated float32 sums (GB300's FP64 pipe is a small fraction of its
@@ -180,47 +102,21 @@ __device__ __forceinline__ double soft_warp_dot(float hi, float lo) {
 // several loads in flight before the barrier), one output per thread and row
 constexpr int kSoftRowsX = 4;
 
-__global__ void __launch_bounds__(kSoftTileX) k_soft_pass_x(const float *in, float *out, SoftGeom g, int mode, int R,
-                                                            SoftTaps T, const unsigned *skip) {
+__global__ void __launch_bounds__(kSoftTileX) k_soft_pass_x(const float *in, float *out, SoftGeom g, SoftTaps T,
+                                                            const unsigned *skip) {
   if (skip && *skip) return;   // the output is already there
-  __shared__ float tile[kSoftRowsX][kSoftTileX + 2 * kSoftTileMaxR];
+  __shared__ float tile[kSoftRowsX][kSoftTileX + 2 * kSoftMaxRadius];
   const int nseg = (g.W + kSoftTileX - 1) / kSoftTileX;
   const int64_t row0 = (int64_t)(blockIdx.x / nseg) * kSoftRowsX;
   const int nr = (int)min((int64_t)kSoftRowsX, (int64_t)g.H * g.D - row0);
   const int x0 = (int)(blockIdx.x % nseg) * kSoftTileX, t = threadIdx.x;
-  const int L = kSoftTileX + 2 * R;
+  const int L = kSoftTileX + 2 * T.r;
   for (int r = 0; r < nr; r++)
-    for (int k = t; k < L; k += kSoftTileX) tile[r][k] = soft_stage(in + (row0 + r) * g.W, 1, x0 - R + k, g.W, mode);
+    for (int k = t; k < L; k += kSoftTileX) tile[r][k] = soft_stage(in + (row0 + r) * g.W, 1, x0 - T.r + k, g.W);
   __syncthreads();
   const int x = x0 + t;
-  if (mode == kMin || mode == kMax) {
-    const bool is_max = mode == kMax;
-    const int q_end = soft_span(R);
-    for (int q = 1; q < q_end; q *= 2) {
-      const int lim = L - 2 * q + 1;   // entries whose span of 2q stays inside the tile
-      float a[kSoftRowsX][2];
-#pragma unroll
-      for (int r = 0; r < kSoftRowsX; r++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int k = t + h * kSoftTileX;
-          a[r][h] = r < nr && k < lim ? soft_ext(tile[r][k], tile[r][k + q], is_max) : 0.0f;
-        }
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < kSoftRowsX; r++)
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-          if (r < nr && t + h * kSoftTileX < lim) tile[r][t + h * kSoftTileX] = a[r][h];
-      __syncthreads();
-    }
-    if (x < g.W)
-      for (int r = 0; r < nr; r++)
-        out[(row0 + r) * g.W + x] = soft_ext(tile[r][t], tile[r][t + 2 * R + 1 - q_end], is_max);
-    return;
-  }
   if (x < g.W)
-    for (int r = 0; r < nr; r++) out[(row0 + r) * g.W + x] = soft_fold(tile[r] + t, 1, x, g.W, mode, R, T);
+    for (int r = 0; r < nr; r++) out[(row0 + r) * g.W + x] = soft_fold(tile[r] + t, 1, x, g.W, T);
 }
 
 // along y (AXIS 1) or z (AXIS 2): a block of 32 x 8 threads owns 32 columns and
@@ -231,13 +127,13 @@ __global__ void __launch_bounds__(kSoftTileX) k_soft_pass_x(const float *in, flo
 enum { kEpiStore = 0, kEpiDot = 1, kEpiDiff = 2 };
 
 template <int AXIS, int EPI = kEpiStore>
-__global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *out, SoftGeom g, int mode, int R,
-                                                      SoftTaps T, const unsigned *skip = nullptr,
+__global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *out, SoftGeom g, SoftTaps T,
+                                                      const unsigned *skip = nullptr,
                                                       const float *aux = nullptr, double *dot_out = nullptr,
                                                       float scale = 0.0f) {
   if (skip && *skip) return;
   extern __shared__ float slab[];   // [kSoftTileYZ + 2R][32]
-  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int tx = threadIdx.x, ty = threadIdx.y, R = T.r;
   const int n = AXIS == 1 ? g.H : g.D;
   const int64_t s = AXIS == 1 ? (int64_t)g.W : (int64_t)g.W * g.H;
   const int x = blockIdx.x * 32 + tx;
@@ -246,7 +142,7 @@ __global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *ou
   const int64_t other = AXIS == 1 ? (int64_t)blockIdx.z * g.W * g.H : (int64_t)blockIdx.z * g.W;
   const float *line = in + other + x;
   const int rows = kSoftTileYZ + 2 * R;
-  for (int k = ty; k < rows; k += 8) slab[k * 32 + tx] = x < g.W ? soft_stage(line, s, c0 - R + k, n, mode) : 0.0f;
+  for (int k = ty; k < rows; k += 8) slab[k * 32 + tx] = x < g.W ? soft_stage(line, s, c0 - R + k, n) : 0.0f;
   __syncthreads();
   float hi = 0.0f, lo = 0.0f;
   if (x < g.W)
@@ -254,7 +150,7 @@ __global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *ou
       const int c = c0 + m;
       if (c >= n) break;
       const int64_t i = other + x + (int64_t)c * s;
-      const float v = soft_fold(slab + m * 32 + tx, 32, c, n, mode, R, T);
+      const float v = soft_fold(slab + m * 32 + tx, 32, c, n, T);
       if (EPI == kEpiDot) soft_dot_add(hi, lo, aux[i], v);
       else if (EPI == kEpiDiff) out[i] = scale * (aux[i] - v);
       else out[i] = v;
@@ -272,302 +168,562 @@ __global__ void __launch_bounds__(256) k_soft_pass_yz(const float *in, float *ou
   }
 }
 
-// min / max along y (AXIS 1) or z (AXIS 2) by doubling, 32 columns x kSoftTileYZ outputs
+// ---- normalization windows: min and max (and their box means) travel as one float2 per voxel
+//
+// All passes handle both sides at once, so a volume is read and written once per axis.  Extremes come
+// from short blocks (window.cuh); their adjoints find each window's first extreme the same way, every
+// combination taking a later entry only when it is strictly better, and a thread adds up the gradients
+// of its consecutive windows with one extreme before the atomic add.  Box means fold each output's
+// window from 0 in ascending order (the sigma gradients are sensitive to the last bits of the
+// normalized volume), K neighbouring outputs per thread from a rotating register window.  Reaches that
+// the rings or tiles do not hold, and those below a block (r < 4), take the *_far kernels, which read each
+// window from global memory.
+struct MinMaxF {
+  typedef float2 T;
+  __device__ __forceinline__ static float2 op(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fmaxf(a.y, b.y)); }
+};
+
+// A window's first min and first max, and their entries.
+struct ExtAt {
+  float2 v;
+  int a, b;
+};
+// the extremes of a span and of one after it (or overlapping its end)
+__device__ __forceinline__ ExtAt ext_join(const ExtAt &p, const ExtAt &q) {
+  ExtAt r = p;
+  if (q.v.x < p.v.x) {
+    r.v.x = q.v.x;
+    r.a = q.a;
+  }
+  if (q.v.y > p.v.y) {
+    r.v.y = q.v.y;
+    r.b = q.b;
+  }
+  return r;
+}
+
+// Adds the gradients of consecutive windows that share their extreme (the entries never decrease along
+// a line) and puts each run's sum where the extreme lies.
+template <class PutF>
+struct RunSum {
+  int at = -1;
+  float sum = 0.0f;
+  PutF put;
+  __device__ __forceinline__ RunSum(PutF p) : put(p) {}
+  __device__ __forceinline__ void add(int a, float g) {
+    if (a != at) {
+      flush();
+      at = a;
+      sum = 0.0f;
+    }
+    sum += g;
+  }
+  __device__ __forceinline__ void flush() {
+    if (sum != 0.0f) put(at, sum);
+  }
+};
+
+// Line geometry of a pass along y (AXIS 1) or z (AXIS 2): block x = 32 columns, block y = the other coordinate.
 template <int AXIS>
-__global__ void __launch_bounds__(512) k_soft_ext_yz(const float *in, float *out, SoftGeom g, int is_max, int R) {
-  __shared__ float slab[(kSoftTileYZ + 2 * kSoftExtMaxR) * 32];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int n = AXIS == 1 ? g.H : g.D;
-  const int64_t s = AXIS == 1 ? (int64_t)g.W : (int64_t)g.W * g.H;
-  const int x = blockIdx.x * 32 + tx;
-  const int c0 = blockIdx.y * kSoftTileYZ;
-  const int64_t other = AXIS == 1 ? (int64_t)blockIdx.z * g.W * g.H : (int64_t)blockIdx.z * g.W;
-  const float *line = in + other + x;
-  const int rows = kSoftTileYZ + 2 * R, q_end = soft_span(R);
-  for (int k = ty; k < rows; k += 16) slab[k * 32 + tx] = x < g.W ? soft_stage(line, s, c0 - R + k, n, kMin) : 0.0f;
-  __syncthreads();
-  for (int q = 1; q < q_end; q *= 2) {
-    const int lim = rows - 2 * q + 1;
-    float v[kSoftExtPer];
-#pragma unroll
-    for (int e = 0; e < kSoftExtPer; e++) {
-      const int k = ty + 16 * e;
-      v[e] = k < lim ? soft_ext(slab[k * 32 + tx], slab[(k + q) * 32 + tx], is_max) : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < kSoftExtPer; e++)
-      if (ty + 16 * e < lim) slab[(ty + 16 * e) * 32 + tx] = v[e];
-    __syncthreads();
+struct SoftLine {
+  int n, x;
+  int64_t base, s;
+  bool in;
+  __device__ __forceinline__ SoftLine(const SoftGeom &g) {
+    n = AXIS == 1 ? g.H : g.D;
+    s = AXIS == 1 ? (int64_t)g.W : (int64_t)g.W * g.H;
+    x = blockIdx.x * 32 + threadIdx.x;
+    in = x < g.W;
+    base = (AXIS == 1 ? (int64_t)blockIdx.y * g.W * g.H : (int64_t)blockIdx.y * g.W) + min(x, g.W - 1);
   }
-  if (x >= g.W) return;
-  for (int m = ty; m < kSoftTileYZ; m += 16) {
-    const int c = c0 + m;
-    if (c >= n) break;
-    out[other + x + (int64_t)c * s] = soft_ext(slab[m * 32 + tx], slab[(m + 2 * R + 1 - q_end) * 32 + tx], is_max);
-  }
+};
+
+constexpr int kSoftB = 8;   // block of the column passes
+
+// min / max along y or z, segments of `seg` positions (blockIdx.z)
+template <int AXIS, int NW>
+__global__ void __launch_bounds__(32 * NW) k_soft_ext_cols(const float2 *in, float2 *out, SoftGeom g, int r, int seg) {
+  extern __shared__ float2 ring2[];
+  const SoftLine<AXIS> l(g);
+  const int t0 = blockIdx.z * seg;
+  ext_cols<MinMaxF, kSoftB, NW>(
+      ring2, min(seg, l.n - t0), r,
+      [&](int a, float2 (&v)[kSoftB]) {
+#pragma unroll
+        for (int j = 0; j < kSoftB; j++) v[j] = __ldg(in + l.base + (int64_t)clampi(t0 - r + a + j, 0, l.n - 1) * l.s);
+      },
+      [&](int t, float2 m) {
+        if (l.in) out[l.base + (int64_t)(t0 + t) * l.s] = m;
+      });
 }
 
-// The two transposed passes from the same tiles, again with the old operations in the old
-// order: the box mean's gather (kAdjBox; the tile holds g_out, zero outside the line), and
-// the min / max scatter to each window's first extreme (kAdjMin / kAdjMax; the tile holds
-// the filter's input, clamped).  Window positions outside the line are clamped exactly as
-// in k_soft_box_adj / k_soft_minmax_adj.
-enum { kAdjBox = 0, kAdjMin = 1, kAdjMax = 2 };
-
-__device__ __forceinline__ void soft_adj_one(const float *w, int step, int c, int n, int R, int adj, int64_t base,
-                                             int64_t s, const float *g_out, float *g_in) {
-  // w[k * step] is the staged value at line position c - R + k
-  if (adj == kAdjBox) {
-    float acc = 0.0f;
-    for (int t = max(0, c - R); t <= min(n - 1, c + R); t++) acc += w[(t - c + R) * step];
-    if (c == 0)
-      for (int t = 0; t < min(n, R); t++) acc += (float)(R - t) * w[(t - c + R) * step];
-    if (c == n - 1)
-      for (int t = max(0, n - 1 - R + 1); t < n; t++) acc += (float)(t + R - (n - 1)) * w[(t - c + R) * step];
-    g_in[base + (int64_t)c * s] = acc / (float)(2 * R + 1);
-    return;
-  }
-  const float go = g_out[base + (int64_t)c * s];
-  if (go == 0.0f) return;
-  int arg = clampi(c - R, 0, n - 1);
-  float best = w[0];
-  for (int j = -R + 1; j <= R; j++) {
-    const float v = w[(j + R) * step];
-    if (adj == kAdjMax ? v > best : v < best) {
-      best = v;
-      arg = clampi(c + j, 0, n - 1);
-    }
-  }
-  atomicAdd(g_in + base + (int64_t)arg * s, go);
-}
-
-__global__ void __launch_bounds__(kSoftTileX) k_soft_adj_x(const float *src, const float *g_out, float *g_in,
-                                                           SoftGeom g, int adj, int R) {
-  __shared__ float tile[kSoftRowsX][kSoftTileX + 2 * kSoftTileMaxR];
-  __shared__ int at[kSoftRowsX][kSoftTileX + 2 * kSoftTileMaxR];
-  const int nseg = (g.W + kSoftTileX - 1) / kSoftTileX;
-  const int64_t row0 = (int64_t)(blockIdx.x / nseg) * kSoftRowsX;
-  const int nr = (int)min((int64_t)kSoftRowsX, (int64_t)g.H * g.D - row0);
-  const int x0 = (int)(blockIdx.x % nseg) * kSoftTileX, t = threadIdx.x;
-  const int L = kSoftTileX + 2 * R;
-  const int stage_mode = adj == kAdjBox ? kConv : kMin;   // zero outside / clamped
-  for (int r = 0; r < nr; r++)
-    for (int k = t; k < L; k += kSoftTileX) {
-      tile[r][k] = soft_stage(src + (row0 + r) * g.W, 1, x0 - R + k, g.W, stage_mode);
-      at[r][k] = k;
-    }
-  __syncthreads();
-  const int x = x0 + t;
-  if (adj != kAdjBox) {
-    // first extreme of every window by doubling over (value, staged position) pairs
-    const bool is_max = adj == kAdjMax;
-    const int q_end = soft_span(R);
-    for (int q = 1; q < q_end; q *= 2) {
-      const int lim = L - 2 * q + 1;
-      float a[kSoftRowsX][2];
-      int ia[kSoftRowsX][2];
+// The adjoint along y or z: src the pass's input, gout its output's gradient, added to gin (zeroed before).
+// As ext_cols, with the suffixes' places in their blocks kept beside them.
+template <int AXIS, int NW>
+__global__ void __launch_bounds__(32 * NW) k_soft_ext_adj_cols(const float2 *src, const float2 *gout, float2 *gin,
+                                                               SoftGeom g, int r, int seg) {
+  constexpr int B = kSoftB;
+  extern __shared__ float2 ring2[];
+  const SoftLine<AXIS> l(g);
+  const int lane = threadIdx.x, w = threadIdx.y, t0 = blockIdx.z * seg, n = min(seg, l.n - t0);
+  const int rows = ext_cols_rows(r, B, NW), total = n + 2 * r, back = (2 * r + B - 1) / B, q = back * B - 2 * r;
+  uint16_t *place = reinterpret_cast<uint16_t *>(ring2 + rows * 32);
+  float *gi = reinterpret_cast<float *>(gin);
+  auto put = [&](int side) {
+    return [=](int e, float v) {
+      atomicAdd(gi + 2 * (l.base + (int64_t)clampi(t0 - r + e, 0, l.n - 1) * l.s) + side, v);
+    };
+  };
+  int pos = w * B;
+  for (int c = 0; c < total; c += NW * B) {
+    const int a = c + w * B;
+    float2 v[B];
+    if (a < total) {
 #pragma unroll
-      for (int r = 0; r < kSoftRowsX; r++)
+      for (int j = 0; j < B; j++) v[j] = __ldg(src + l.base + (int64_t)clampi(t0 - r + a + j, 0, l.n - 1) * l.s);
+      ExtAt s{v[B - 1], B - 1, B - 1};
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int k = t + h * kSoftTileX;
-          a[r][h] = 0.0f;
-          ia[r][h] = 0;
-          if (r < nr && k < lim) {
-            a[r][h] = tile[r][k];
-            ia[r][h] = at[r][k];
-            soft_ext_at(a[r][h], ia[r][h], tile[r][k + q], at[r][k + q], is_max);
-          }
-        }
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < kSoftRowsX; r++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int k = t + h * kSoftTileX;
-          if (r < nr && k < lim) {
-            tile[r][k] = a[r][h];
-            at[r][k] = ia[r][h];
-          }
-        }
-      __syncthreads();
-    }
-    if (x < g.W)
-      for (int r = 0; r < nr; r++) {
-        const int64_t row = (row0 + r) * g.W;
-        const float go = g_out[row + x];
-        if (go == 0.0f) continue;
-        float v = tile[r][t];
-        int iv = at[r][t];
-        soft_ext_at(v, iv, tile[r][t + 2 * R + 1 - q_end], at[r][t + 2 * R + 1 - q_end], is_max);
-        atomicAdd(g_in + row + clampi(x0 - R + iv, 0, g.W - 1), go);
-      }
-    return;
-  }
-  if (x < g.W)
-    for (int r = 0; r < nr; r++) soft_adj_one(tile[r] + t, 1, x, g.W, R, adj, (row0 + r) * g.W, 1, g_out, g_in);
-}
-
-template <int AXIS>
-__global__ void __launch_bounds__(256) k_soft_adj_yz(const float *src, const float *g_out, float *g_in, SoftGeom g,
-                                                     int adj, int R) {
-  extern __shared__ float slab[];   // [kSoftTileYZ + 2R][32]
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int n = AXIS == 1 ? g.H : g.D;
-  const int64_t s = AXIS == 1 ? (int64_t)g.W : (int64_t)g.W * g.H;
-  const int x = blockIdx.x * 32 + tx;
-  const int c0 = blockIdx.y * kSoftTileYZ;
-  const int64_t other = AXIS == 1 ? (int64_t)blockIdx.z * g.W * g.H : (int64_t)blockIdx.z * g.W;
-  const float *line = src + other + x;
-  const int stage_mode = adj == kAdjBox ? kConv : kMin;
-  const int rows = kSoftTileYZ + 2 * R;
-  for (int k = ty; k < rows; k += 8) slab[k * 32 + tx] = x < g.W ? soft_stage(line, s, c0 - R + k, n, stage_mode) : 0.0f;
-  __syncthreads();
-  if (x >= g.W) return;
-  for (int m = ty; m < kSoftTileYZ; m += 8) {
-    const int c = c0 + m;
-    if (c >= n) break;
-    soft_adj_one(slab + m * 32 + tx, 32, c, n, R, adj, other + x, s, g_out, g_in);
-  }
-}
-
-// the transposed min / max along y or z: each window's output gradient to its first extreme,
-// found by doubling over (value, staged position) pairs; g_in must start at zero
-template <int AXIS>
-__global__ void __launch_bounds__(512) k_soft_ext_adj_yz(const float *src, const float *g_out, float *g_in, SoftGeom g,
-                                                         int is_max, int R) {
-  __shared__ float slab[(kSoftTileYZ + 2 * kSoftExtMaxR) * 32];
-  __shared__ int at[(kSoftTileYZ + 2 * kSoftExtMaxR) * 32];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int n = AXIS == 1 ? g.H : g.D;
-  const int64_t s = AXIS == 1 ? (int64_t)g.W : (int64_t)g.W * g.H;
-  const int x = blockIdx.x * 32 + tx;
-  const int c0 = blockIdx.y * kSoftTileYZ;
-  const int64_t other = AXIS == 1 ? (int64_t)blockIdx.z * g.W * g.H : (int64_t)blockIdx.z * g.W;
-  const float *line = src + other + x;
-  const int rows = kSoftTileYZ + 2 * R, q_end = soft_span(R);
-  for (int k = ty; k < rows; k += 16) {
-    slab[k * 32 + tx] = x < g.W ? soft_stage(line, s, c0 - R + k, n, kMin) : 0.0f;
-    at[k * 32 + tx] = k;
-  }
-  __syncthreads();
-  for (int q = 1; q < q_end; q *= 2) {
-    const int lim = rows - 2 * q + 1;
-    float v[kSoftExtPer];
-    int iv[kSoftExtPer];
-#pragma unroll
-    for (int e = 0; e < kSoftExtPer; e++) {
-      const int k = ty + 16 * e;
-      v[e] = 0.0f;
-      iv[e] = 0;
-      if (k < lim) {
-        v[e] = slab[k * 32 + tx];
-        iv[e] = at[k * 32 + tx];
-        soft_ext_at(v[e], iv[e], slab[(k + q) * 32 + tx], at[(k + q) * 32 + tx], is_max);
+      for (int j = B - 1; j >= 0; j--) {
+        if (j < B - 1) s = ext_join(ExtAt{v[j], j, j}, s);
+        ring2[(pos + j) * 32 + lane] = s.v;
+        place[(pos + j) * 32 + lane] = (uint16_t)(s.a | s.b << 8);
       }
     }
     __syncthreads();
-#pragma unroll
-    for (int e = 0; e < kSoftExtPer; e++) {
-      const int k = ty + 16 * e;
-      if (k < lim) {
-        slab[k * 32 + tx] = v[e];
-        at[k * 32 + tx] = iv[e];
+    if (a < total && a + B > 2 * r && l.in) {
+      auto row = [&](int d) {
+        const int p = pos - d * B;
+        return p < 0 ? p + rows : p;
+      };
+      auto get = [&](int p, int blk0) {   // ring row p, whose block starts at entry blk0
+        const int k = place[p * 32 + lane];
+        return ExtAt{ring2[p * 32 + lane], blk0 + (k & 0xFF), blk0 + (k >> 8)};
+      };
+      ExtAt mid1, mid0;
+      if (back >= 3) {
+        mid1 = get(row(back - 2), a - (back - 2) * B);
+        for (int d = back - 3; d >= 1; d--) mid1 = ext_join(mid1, get(row(d), a - d * B));
       }
+      if (back >= 2) {
+        mid0 = get(row(back - 1), a - (back - 1) * B);
+        if (back >= 3) mid0 = ext_join(mid0, mid1);
+      }
+      RunSum<decltype(put(0))> lo(put(0)), hi(put(1));
+      const int r0 = row(back), r1 = back >= 2 ? row(back - 1) : r0;
+      ExtAt p{v[0], a, a};
+#pragma unroll
+      for (int o = 0; o < B; o++) {
+        const int e = a + o;
+        if (o) p = ext_join(p, ExtAt{v[o], e, e});
+        if (e < 2 * r || e >= total) continue;
+        const bool first = o < B - q;
+        ExtAt m = first ? get(r0 + q + o, a - back * B) : get(r1 + q + o - B, a - (back - 1) * B);
+        if (first ? back >= 2 : back >= 3) m = ext_join(m, first ? mid0 : mid1);
+        m = ext_join(m, p);
+        const float2 go = __ldg(gout + l.base + (int64_t)(t0 + e - 2 * r) * l.s);
+        lo.add(m.a, go.x);
+        hi.add(m.b, go.y);
+      }
+      lo.flush();
+      hi.flush();
     }
-    __syncthreads();
-  }
-  if (x >= g.W) return;
-  for (int m = ty; m < kSoftTileYZ; m += 16) {
-    const int c = c0 + m;
-    if (c >= n) break;
-    const float go = g_out[other + x + (int64_t)c * s];
-    if (go == 0.0f) continue;
-    float a = slab[m * 32 + tx];
-    int ia = at[m * 32 + tx];
-    const int m2 = m + 2 * R + 1 - q_end;
-    soft_ext_at(a, ia, slab[m2 * 32 + tx], at[m2 * 32 + tx], is_max);
-    atomicAdd(g_in + other + x + (int64_t)clampi(c0 - R + ia, 0, n - 1) * s, go);
+    pos += NW * B;
+    if (pos >= rows) pos -= rows;
   }
 }
 
-// Transposed min / max pass: the output gradient of each window goes to the window's first
-// extreme (the index the forward filter took it from).  g_in must start at zero.
-__global__ void k_soft_minmax_adj(const float *in, const float *g_out, float *g_in, SoftGeom g, int axis, int r,
-                                  int is_max, int64_t N) {
+// 32-byte global accesses where the address allows them (sm_100 on), else entry by entry
+__device__ __forceinline__ void soft_ld8(const float *p, float (&v)[8]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "l"(p));
+  } else {
+#pragma unroll
+    for (int o = 0; o < 8; o++) v[o] = __ldg(p + o);
+  }
+}
+__device__ __forceinline__ void soft_st8(float *p, const float (&v)[8]) {
+  if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+  } else {
+#pragma unroll
+    for (int o = 0; o < 8; o++) p[o] = v[o];
+  }
+}
+
+// min / max along x of the volume itself, G lanes per row (window.cuh); rows start `pad` entries early
+// so that a lane's eight outputs start on 32 bytes
+constexpr int kSoftRowWarps = 4;
+
+template <int G, int Q>
+__global__ void __launch_bounds__(32 * kSoftRowWarps) k_soft_ext_rows(const float *in, float2 *out, SoftGeom g, int r) {
+  using R = RowRing<G>;
+  __shared__ float2 smr[kSoftRowWarps][R::WORDS];
+  const int W = g.W, gl = threadIdx.x & (G - 1), w = threadIdx.x >> 5;
+  const int64_t rows = (int64_t)g.H * g.D, row0 = ((int64_t)blockIdx.x * kSoftRowWarps + w) * R::LINES;
+  if (row0 >= rows) return;
+  const int64_t mine = row0 + (threadIdx.x & 31) / G, row = min(mine, rows - 1);
+  const bool live = mine < rows;
+  const float *line = in + row * W;
+  float2 *o2 = out + row * W;
+  // (for reaches that are multiples of 4 the inputs do too)
+  const int pad = r % 4 == 0 ? (int)((reinterpret_cast<uintptr_t>(line - r) >> 2) & 7)
+                             : (int)((reinterpret_cast<uintptr_t>(o2 - 2 * r) >> 3) & 3);
+  const int n_in = W + 2 * r;
+  float nv[8];
+  float2 hist[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) hist[k] = make_float2(0.0f, 0.0f);
+  auto fetch = [&](int c) {
+    const int x = c + 8 * gl - r;
+    if (x >= 0 && x + 8 <= W) {
+      soft_ld8(line + x, nv);
+    } else {
+#pragma unroll
+      for (int o = 0; o < 8; o++) nv[o] = __ldg(line + clampi(x + o, 0, W - 1));
+    }
+  };
+  int c = -pad, pc = 0;
+  fetch(c);
+  for (int i = 0; i < n_in + 7; i += R::CHUNK, c += R::CHUNK) {
+    float2 v[8], m[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++) v[o] = make_float2(nv[o], nv[o]);
+    if (i < n_in) fetch(c + R::CHUNK);
+    ext_row_chunk<MinMaxF, G, Q>(smr[w], pc, r, v, hist, m);
+    const int u = c + 8 * gl - 2 * r;
+    if (live) {
+      if (u >= 0 && u + 8 <= W) {
+        const float a[8] = {m[0].x, m[0].y, m[1].x, m[1].y, m[2].x, m[2].y, m[3].x, m[3].y};
+        const float b[8] = {m[4].x, m[4].y, m[5].x, m[5].y, m[6].x, m[6].y, m[7].x, m[7].y};
+        soft_st8(reinterpret_cast<float *>(o2 + u), a);
+        soft_st8(reinterpret_cast<float *>(o2 + u + 4), b);
+      } else {
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+          if (u + o >= 0 && u + o < W) o2[u + o] = m[o];
+      }
+    }
+    __syncwarp();
+    pc += G;
+    if (pc >= R::NB) pc = 0;
+  }
+}
+
+template <int G>
+__device__ __forceinline__ ExtAt row_lag_at(const ExtAt &cur, const ExtAt &prev, int lag) {
+  return ExtAt{make_float2(row_lag<G>(cur.v.x, prev.v.x, lag), row_lag<G>(cur.v.y, prev.v.y, lag)),
+               row_lag<G>(cur.a, prev.a, lag), row_lag<G>(cur.b, prev.b, lag)};
+}
+
+// The adjoint along x: both sides' gradients go to the volume's gradient gin, at the first min and first max of each
+// window of the volume src.  As ext_row_chunk, with places.
+template <int G, int Q>
+__global__ void __launch_bounds__(32 * kSoftRowWarps) k_soft_ext_adj_rows(const float *src, const float2 *gout, float *gin,
+                                                                          SoftGeom g, int r) {
+  using R = RowRing<G>;
+  __shared__ float2 smv[kSoftRowWarps][R::WORDS];
+  __shared__ uint16_t smp[kSoftRowWarps][R::WORDS];
+  const int W = g.W, gl = threadIdx.x & (G - 1), w = threadIdx.x >> 5;
+  const int64_t rows = (int64_t)g.H * g.D, row0 = ((int64_t)blockIdx.x * kSoftRowWarps + w) * R::LINES;
+  if (row0 >= rows) return;
+  const int64_t mine = row0 + (threadIdx.x & 31) / G, row = min(mine, rows - 1);
+  const bool live = mine < rows;
+  const float *line = src + row * W;
+  const float2 *go2 = gout + row * W;
+  float *gi = gin + row * W;
+  float2 *suf = smv[w];
+  uint16_t *place = smp[w];
+  const int pad = r % 4 == 0 ? (int)((reinterpret_cast<uintptr_t>(line - r) >> 2) & 7)
+                             : (int)((reinterpret_cast<uintptr_t>(go2 - 2 * r) >> 3) & 3);
+  const int n_in = W + 2 * r, back = (2 * r + 7) / 8, n1 = back - 2;
+  float nv[8];
+  ExtAt hist[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) hist[k] = ExtAt{make_float2(0.0f, 0.0f), 0, 0};
+  auto fetch = [&](int c) {
+    const int x = c + 8 * gl - r;
+    if (x >= 0 && x + 8 <= W) {
+      soft_ld8(line + x, nv);
+    } else {
+#pragma unroll
+      for (int o = 0; o < 8; o++) nv[o] = __ldg(line + clampi(x + o, 0, W - 1));
+    }
+  };
+  auto put = [=](int e, float v) { atomicAdd(gi + clampi(e - r, 0, W - 1), v); };
+  int c = -pad, pc = 0;
+  fetch(c);
+  for (int i = 0; i < n_in + 7; i += R::CHUNK, c += R::CHUNK) {
+    float v[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++) v[o] = nv[o];
+    if (i < n_in) fetch(c + R::CHUNK);
+    const int e0 = c + 8 * gl, u = e0 - 2 * r;
+    float2 go[8];
+    if (u >= 0 && u + 8 <= W) {
+      float a[8], b[8];
+      soft_ld8(reinterpret_cast<const float *>(go2 + u), a);
+      soft_ld8(reinterpret_cast<const float *>(go2 + u + 4), b);
+#pragma unroll
+      for (int o = 0; o < 4; o++) {
+        go[o] = make_float2(a[2 * o], a[2 * o + 1]);
+        go[4 + o] = make_float2(b[2 * o], b[2 * o + 1]);
+      }
+    } else {
+#pragma unroll
+      for (int o = 0; o < 8; o++) go[o] = u + o >= 0 && u + o < W ? __ldg(go2 + u + o) : make_float2(0.0f, 0.0f);
+    }
+    const RowAt<G> at(pc);
+    const int own = at(0);
+    ExtAt s{make_float2(v[7], v[7]), e0 + 7, e0 + 7};
+#pragma unroll
+    for (int o = 7; o >= 0; o--) {
+      if (o < 7) s = ext_join(ExtAt{make_float2(v[o], v[o]), e0 + o, e0 + o}, s);
+      suf[o * R::PITCH + own] = s.v;
+      place[o * R::PITCH + own] = (uint16_t)((s.a - e0) | (s.b - e0) << 8);
+    }
+    __syncwarp();
+    ExtAt mid1, mid0, d = s;
+#pragma unroll
+    for (int k = 0; k < (G == 8 ? 3 : 6); k++) {
+      if ((1 << k) <= n1) {
+        const bool last = (2 << k) > n1;
+        if (last) mid1 = ext_join(row_lag_at<G>(d, hist[k], 1 + n1 - (1 << k)), row_lag_at<G>(d, hist[k], 1));
+        const ExtAt h = hist[k];
+        hist[k] = d;
+        if (!last) d = ext_join(row_lag_at<G>(d, h, 1 << k), d);
+      }
+    }
+    auto get = [&](int o, int b, int blk0) {
+      const int k = place[o * R::PITCH + b];
+      return ExtAt{suf[o * R::PITCH + b], blk0 + (k & 0xFF), blk0 + (k >> 8)};
+    };
+    const int b0 = at(back), b1 = at(back >= 2 ? back - 1 : 1);
+    if (back >= 2) {
+      mid0 = get(0, b1, e0 - 8 * (back - 1));
+      if (n1 >= 1) mid0 = ext_join(mid0, mid1);
+    }
+    RunSum<decltype(put)> lo(put), hi(put);
+    ExtAt p{make_float2(v[0], v[0]), e0, e0};
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+      const int e = e0 + o;
+      if (o) p = ext_join(p, ExtAt{make_float2(v[o], v[o]), e, e});
+      ExtAt m;
+      if (Q + o < 8) {
+        m = get(Q + o, b0, e0 - 8 * back);
+        if (back >= 2) m = ext_join(m, mid0);
+      } else {
+        m = get(Q + o - 8, b1, e0 - 8 * (back - 1));
+        if (n1 >= 1) m = ext_join(m, mid1);
+      }
+      m = ext_join(m, p);
+      if (live && u + o >= 0 && u + o < W) {
+        lo.add(m.a, go[o].x);
+        hi.add(m.b, go[o].y);
+      }
+    }
+    lo.flush();
+    hi.flush();
+    __syncwarp();
+    pc += G;
+    if (pc >= R::NB) pc = 0;
+  }
+}
+
+// One input of a box fold: clamped to the line (the mean), or zero outside it (ADJ, the transposed mean,
+// whose edge outputs take the repeated edge taps on top).
+__device__ __forceinline__ float2 soft_fma2(float k, float2 v, float2 a) {
+  return make_float2(__fmaf_rn(k, v.x, a.x), __fmaf_rn(k, v.y, a.y));
+}
+// the extra taps of the transposed mean at the line's ends: output t's window ran past position 0 (n - 1) R - t
+// (t + R - (n - 1)) times; ld(t): the gradient at t
+template <class LoadF>
+__device__ __forceinline__ float2 soft_box_ends(int c, int n, int R, LoadF ld, float2 acc) {
+  if (c == 0)
+    for (int t = 0; t < min(n, R); t++) acc = soft_fma2((float)(R - t), ld(t), acc);
+  if (c == n - 1)
+    for (int t = max(0, n - R); t < n; t++) acc = soft_fma2((float)(t + R - (n - 1)), ld(t), acc);
+  return acc;
+}
+__device__ __forceinline__ float2 soft_div(float2 a, float n) { return make_float2(a.x / n, a.y / n); }
+
+// Box mean along x (or its transpose): a tile of 32 rows x kSoftBoxX outputs with the reach on both sides in shared
+// memory (odd pitch: a lane's row starts in its own bank), one row per lane and kSoftBoxK outputs per thread.
+constexpr int kSoftBoxK = 16, kSoftBoxX = 128;
+
+template <bool ADJ>
+__global__ void __launch_bounds__(256, 2) k_soft_box_x(const float2 *in, float2 *out, SoftGeom g, int R) {
+  extern __shared__ float2 tile2[];
+  const int pitch = (kSoftBoxX + 2 * R) | 1, n0 = kSoftBoxX + 2 * R;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nseg = (g.W + kSoftBoxX - 1) / kSoftBoxX;
+  const int64_t rows = (int64_t)g.H * g.D, row0 = (int64_t)(blockIdx.x / nseg) * 32;
+  const int x0 = (int)(blockIdx.x % nseg) * kSoftBoxX, nr = (int)min((int64_t)32, rows - row0);
+  for (int k = w; k < nr; k += 8) {
+    const float2 *line = in + (row0 + k) * g.W;
+    for (int i = lane; i < n0; i += 32) {
+      const int x = x0 - R + i;
+      tile2[k * pitch + i] = ADJ && (x < 0 || x >= g.W) ? make_float2(0.0f, 0.0f) : __ldg(line + clampi(x, 0, g.W - 1));
+    }
+  }
+  __syncthreads();
+  float2 acc[kSoftBoxK];
+  const float2 *mine = tile2 + lane * pitch;
+  const int xw = w * kSoftBoxK;
+  const bool work = lane < nr && x0 + xw < g.W;
+  if (work) {
+    box_chain<kSoftBoxK>(2 * R + 1, [&](int i) { return mine[xw + i]; }, acc);
+    const float L = (float)(2 * R + 1);
+#pragma unroll
+    for (int k = 0; k < kSoftBoxK; k++) {
+      if (ADJ) acc[k] = soft_box_ends(x0 + xw + k, g.W, R, [&](int t) { return mine[t - x0 + R]; }, acc[k]);
+      acc[k] = soft_div(acc[k], L);
+    }
+  }
+  __syncthreads();
+  if (work)
+#pragma unroll
+    for (int k = 0; k < kSoftBoxK; k++) tile2[lane * pitch + xw + k] = acc[k];
+  __syncthreads();
+  for (int k = w; k < nr; k += 8)
+    for (int i = lane; i < min(kSoftBoxX, g.W - x0); i += 32) out[(row0 + k) * g.W + x0 + i] = tile2[k * pitch + i];
+}
+
+// Box mean along y or z (or its transpose), K outputs of one column per thread; NORM (z, the last
+// pass): also the normalized volume, *bad set when a value of it is not finite (a window without contrast).
+template <int AXIS, int K, bool ADJ, bool NORM>
+__global__ void __launch_bounds__(128) k_soft_box_cols(const float2 *in, float2 *out, SoftGeom g, int R, const float *I,
+                                                       float *norm, float min_intensity, unsigned *bad) {
+  const SoftLine<AXIS> l(g);
+  const int c0 = (blockIdx.z * blockDim.y + threadIdx.y) * K;
+  if (!l.in || c0 >= l.n) return;
+  const float2 *col = in + l.base;
+  float2 acc[K];
+  if (c0 - R >= 0 && c0 + K + R < l.n) {   // the chain loads one input past its last window
+    const float2 *p = col + (int64_t)(c0 - R) * l.s;
+    box_chain<K>(2 * R + 1, [&](int i) { return __ldg(p + (int64_t)i * l.s); }, acc);
+  } else {
+    box_chain<K>(2 * R + 1, [&](int i) {
+      const int c = c0 - R + i;
+      return ADJ && (c < 0 || c >= l.n) ? make_float2(0.0f, 0.0f) : __ldg(col + (int64_t)clampi(c, 0, l.n - 1) * l.s);
+    }, acc);
+  }
+  const float L = (float)(2 * R + 1);
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int c = c0 + k;
+    if (c >= l.n) break;
+    const int64_t i = l.base + (int64_t)c * l.s;
+    if (ADJ) acc[k] = soft_box_ends(c, l.n, R, [&](int t) { return __ldg(col + (int64_t)t * l.s); }, acc[k]);
+    const float2 m = soft_div(acc[k], L);
+    out[i] = m;
+    if (NORM) {
+      const float iv = __ldg(I + i);
+      const float v = iv >= min_intensity ? (iv - m.x) / (m.y - m.x) : 0.0f;
+      norm[i] = v;
+      if (!isfinite(v)) *bad = 1u;
+    }
+  }
+}
+
+// Any reach, from global memory: the extremes of a line of float2 (or, FIRST, of the volume itself)
+template <bool FIRST>
+__device__ __forceinline__ float2 soft_far_ld(const void *p, int64_t i) {
+  if (FIRST) {
+    const float v = __ldg(static_cast<const float *>(p) + i);
+    return make_float2(v, v);
+  }
+  return __ldg(static_cast<const float2 *>(p) + i);
+}
+
+template <bool FIRST>
+__global__ void k_soft_ext_far(const void *in, float2 *out, SoftGeom g, int axis, int r, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const float go = g_out[i];
-  if (go == 0.0f) return;
   int c, n;
   int64_t s;
   soft_axis(g, axis, i, c, s, n);
   const int64_t base = i - (int64_t)c * s;
-  int arg = clampi(c - r, 0, n - 1);
-  float best = in[base + (int64_t)arg * s];
-  for (int j = -r + 1; j <= r; j++) {
-    const int p = clampi(c + j, 0, n - 1);
-    const float v = in[base + (int64_t)p * s];
-    if (is_max ? v > best : v < best) {
-      best = v;
-      arg = p;
-    }
-  }
-  atomicAdd(g_in + base + (int64_t)arg * s, go);
+  float2 m = soft_far_ld<FIRST>(in, i);
+  for (int t = max(0, c - r); t <= min(n - 1, c + r); t++) m = MinMaxF::op(m, soft_far_ld<FIRST>(in, base + (int64_t)t * s));
+  out[i] = m;
 }
 
-// Transposed box mean (nearest border), as a gather: input i receives every output t within
-// r of it, and an edge input additionally receives each output whose window ran past that
-// edge once per clamped tap.
-__global__ void k_soft_box_adj(const float *g_out, float *g_in, SoftGeom g, int axis, int r, int64_t N) {
+template <bool FIRST>
+__global__ void k_soft_ext_adj_far(const void *src, const float2 *gout, float *gin, SoftGeom g, int axis, int r, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int c, n;
   int64_t s;
   soft_axis(g, axis, i, c, s, n);
-  const float *line = g_out + (i - (int64_t)c * s);
-  float acc = 0.0f;
-  for (int t = max(0, c - r); t <= min(n - 1, c + r); t++) acc += line[(int64_t)t * s];
-  if (c == 0)
-    for (int t = 0; t < min(n, r); t++) acc += (float)(r - t) * line[(int64_t)t * s];
-  if (c == n - 1)
-    for (int t = max(0, n - 1 - r + 1); t < n; t++) acc += (float)(t + r - (n - 1)) * line[(int64_t)t * s];
-  g_in[i] = acc / (float)(2 * r + 1);
+  const int64_t base = i - (int64_t)c * s;
+  const int t0 = max(0, c - r);
+  ExtAt m{soft_far_ld<FIRST>(src, base + (int64_t)t0 * s), t0, t0};
+  for (int t = t0 + 1; t <= min(n - 1, c + r); t++)
+    m = ext_join(m, ExtAt{soft_far_ld<FIRST>(src, base + (int64_t)t * s), t, t});
+  const float2 go = gout[i];
+  const int step = FIRST ? 1 : 2;
+  if (go.x != 0.0f) atomicAdd(gin + step * (base + (int64_t)m.a * s), go.x);
+  if (go.y != 0.0f) atomicAdd(gin + step * (base + (int64_t)m.b * s) + step - 1, go.y);
 }
 
-// *bad is set when a normalized value is not finite (a window without contrast).
-__global__ void k_soft_norm(const float *I, const float *e, const float *d, float *norm, float min_intensity, int64_t N,
-                            unsigned *bad) {
+// (sums of over 731 values: compensated, a plain float32 chain that long is off by 1e-5 of a score)
+template <bool ADJ>
+__global__ void k_soft_box_far(const float2 *in, float2 *out, SoftGeom g, int axis, int R, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const float v = I[i] >= min_intensity ? (I[i] - e[i]) / (d[i] - e[i]) : 0.0f;
+  int c, n;
+  int64_t s;
+  soft_axis(g, axis, i, c, s, n);
+  const float2 *line = in + (i - (int64_t)c * s);
+  float2 hi = make_float2(0.0f, 0.0f), lo = hi;
+  for (int j = -R; j <= R; j++) {
+    const int t = c + j;
+    if (ADJ && (t < 0 || t >= n)) continue;
+    const float2 v = line[(int64_t)clampi(t, 0, n - 1) * s];
+    soft_two_sum(hi.x, lo.x, v.x);
+    soft_two_sum(hi.y, lo.y, v.y);
+  }
+  float2 acc = add2(hi, lo);
+  if (ADJ) acc = soft_box_ends(c, n, R, [&](int t) { return line[(int64_t)t * s]; }, acc);
+  out[i] = soft_div(acc, (float)(2 * R + 1));
+}
+
+// The normalized volume from the box means where no other pass forms it (see k_soft_box_cols).
+__global__ void k_soft_norm(const float *I, const float2 *ed, float *norm, float min_intensity, int64_t N, unsigned *bad) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const float iv = I[i];
+  const float2 m = ed[i];
+  const float v = iv >= min_intensity ? (iv - m.x) / (m.y - m.x) : 0.0f;
   norm[i] = v;
   if (!isfinite(v)) *bad = 1u;
 }
 
-// Quotient rule of the normalization: g_I (direct term, written), g_e, g_d.
-__global__ void k_soft_norm_adj(const float *I, const float *e, const float *d, const float *g_norm, float *g_I,
-                                float *g_e, float *g_d, float min_intensity, int64_t N) {
+// Quotient rule of the normalization: g_I (direct term, written) and the gradients of both box means.
+__global__ void k_soft_norm_adj(const float *I, const float2 *ed, const float *g_norm, float *g_I, float2 *g_ed,
+                                float min_intensity, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const float g = g_norm[i];
-  if (I[i] >= min_intensity) {
-    const float den = d[i] - e[i], inv = 1.0f / den, inv2 = inv * inv;
+  const float g = g_norm[i], v = I[i];
+  const float2 m = ed[i];
+  if (v >= min_intensity) {
+    const float den = m.y - m.x, inv = 1.0f / den, inv2 = inv * inv;
     g_I[i] = g * inv;
-    g_e[i] = g * (I[i] - d[i]) * inv2;
-    g_d[i] = -g * (I[i] - e[i]) * inv2;
+    g_ed[i] = make_float2(g * (v - m.y) * inv2, -g * (v - m.x) * inv2);
   } else {
     g_I[i] = 0.0f;
-    g_e[i] = 0.0f;
-    g_d[i] = 0.0f;
+    g_ed[i] = make_float2(0.0f, 0.0f);
   }
 }
 
-// out = scale * (a - b)
-__global__ void k_soft_add(float *a, const float *b, int64_t N) {
+// a += b.x + b.y (no window along any of x and y: both sides' gradients belong where they are)
+__global__ void k_soft_add(float *a, const float2 *b, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) a[i] += b[i];
+  if (i < N) a[i] += b[i].x + b[i].y;
 }
 
 // sum_i a[i] * b[i] into *out (a double, which must start at zero; compensated float32 sums
@@ -1059,26 +1215,26 @@ struct SoftRun {
   SoftGeom g;
   int64_t N;
   cudaStream_t st;
-  float *w;      // workspace slots of N floats (after the accumulators)
+  float *w;      // workspace slots of slot_floats(N) floats (after the accumulators)
   double *acc;   // 16 doubles at the start of the workspace: sums [0, 14), then the flags
   // set by the forward chain: [0] a normalized value is not finite, [1] the DoG slot is filled
   unsigned *flags() const { return reinterpret_cast<unsigned *>(acc + 14); }
   unsigned blocks() const { return ceil_div(N, 256); }
-  float *slot(int k) const { return w + (int64_t)k * N; }
+  static int64_t slot_floats(int64_t n) { return (n + 31) / 32 * 32; }   // whole 128-byte lines
+  float *slot(int k) const { return w + k * slot_floats(N); }
+  float2 *pair(int k) const { return reinterpret_cast<float2 *>(slot(k)); }   // slots k and k + 1
 };
 
-enum { S_MN1, S_MN2, S_MN, S_MX1, S_MX2, S_MX, S_E, S_D, S_NORM, S_DOG, S_T1, S_T2, S_T3, S_GDOG, S_GA, S_GB, S_GC,
-       kSoftSlots };
-
-SoftTaps no_taps() {
-  SoftTaps t;
-  memset(&t, 0, sizeof(t));
-  return t;
-}
+// Kept for the backward: the extremes after the x and the y pass, the box means (pairs, min and max
+// side in one float2), the normalized volume, the DoG; scratch: two pairs and one volume.  The dense
+// Gaussian passes use the pairs' halves.
+enum { S_MM1 = 0, S_MM2 = 2, S_ED = 4, S_NORM = 6, S_DOG = 7, S_PA = 8, S_PB = 10, S_GB = 12, kSoftSlots = 13,
+       S_T1 = S_PA, S_T2 = S_PA + 1, S_T3 = S_PB, S_GDOG = S_PB + 1 };
 
 // Normalized Gaussian taps of sigma (or their derivative in sigma), radius (int)(2 sigma + 0.5).
 SoftTaps gauss_taps_f(double sigma, bool derivative) {
-  SoftTaps t = no_taps();
+  SoftTaps t;
+  memset(&t, 0, sizeof(t));
   const int r = (int)(2.0 * sigma + 0.5);
   t.r = r;
   double e[kSoftMaxTaps], sum = 0.0, m2 = 0.0;
@@ -1094,101 +1250,190 @@ SoftTaps gauss_taps_f(double sigma, bool derivative) {
   return t;
 }
 
-void pass(const SoftRun &R, const float *in, float *out, int axis, int mode, int r, const SoftTaps &T,
-          const unsigned *skip = nullptr) {
-  const int reach = mode == kConv ? T.r : r;
+void pass(const SoftRun &R, const float *in, float *out, int axis, const SoftTaps &T, const unsigned *skip = nullptr) {
   const SoftGeom &g = R.g;
-  if (reach > kSoftTileMaxR) {
-    KLAUNCH("k_soft_pass", R.st, (k_soft_pass<<<R.blocks(), 256, 0, R.st>>>(in, out, g, axis, mode, r, T, R.N)));
-    return;
-  }
   if (axis == 0) {
     const unsigned blocks = (unsigned)(ceil_div(g.W, kSoftTileX) * ceil_div((int64_t)g.H * g.D, kSoftRowsX));
-    KLAUNCH("k_soft_pass_x", R.st, (k_soft_pass_x<<<blocks, kSoftTileX, 0, R.st>>>(in, out, g, mode, reach, T, skip)));
+    KLAUNCH("k_soft_pass_x", R.st, (k_soft_pass_x<<<blocks, kSoftTileX, 0, R.st>>>(in, out, g, T, skip)));
     return;
   }
-  const size_t smem = (size_t)(kSoftTileYZ + 2 * reach) * 32 * sizeof(float);
+  const size_t smem = (size_t)(kSoftTileYZ + 2 * T.r) * 32 * sizeof(float);
   const int n = axis == 1 ? g.H : g.D, other = axis == 1 ? g.D : g.H;
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(n, kSoftTileYZ), (unsigned)other);
-  if ((mode == kMin || mode == kMax) && reach <= kSoftExtMaxR) {
-    if (axis == 1)
-      KLAUNCH("k_soft_ext_y", R.st, (k_soft_ext_yz<1><<<grid, dim3(32, 16), 0, R.st>>>(in, out, g, mode == kMax, reach)));
-    else
-      KLAUNCH("k_soft_ext_z", R.st, (k_soft_ext_yz<2><<<grid, dim3(32, 16), 0, R.st>>>(in, out, g, mode == kMax, reach)));
-    return;
-  }
   if (axis == 1)
-    KLAUNCH("k_soft_pass_y", R.st, (k_soft_pass_yz<1><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T, skip)));
+    KLAUNCH("k_soft_pass_y", R.st, (k_soft_pass_yz<1><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, T, skip)));
   else
-    KLAUNCH("k_soft_pass_z", R.st, (k_soft_pass_yz<2><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, mode, reach, T, skip)));
+    KLAUNCH("k_soft_pass_z", R.st, (k_soft_pass_yz<2><<<grid, dim3(32, 8), smem, R.st>>>(in, out, g, T, skip)));
 }
 
 // the correlation along z with T, summed against w into *acc (double) instead of stored
 void pass_z_dot(const SoftRun &R, const float *in, const SoftTaps &T, const float *w, double *acc) {
-  static_assert(kSoftMaxRadius <= kSoftTileMaxR, "Gaussian taps fit the z tile");
   const SoftGeom &g = R.g;
   const size_t smem = (size_t)(kSoftTileYZ + 2 * T.r) * 32 * sizeof(float);
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(g.D, kSoftTileYZ), (unsigned)g.H);
   KLAUNCH("k_soft_pass_z_dot", R.st, (k_soft_pass_yz<2, kEpiDot><<<grid, dim3(32, 8), smem, R.st>>>(
-                                         in, nullptr, g, kConv, T.r, T, nullptr, w, acc)));
+                                         in, nullptr, g, T, nullptr, w, acc)));
 }
 
 // the separable Gaussian (x, y, then z) with the DoG difference folded into the z pass:
 // out = scale * (sub - in * G), the same operations as a separate difference kernel
 void conv3_diff(const SoftRun &R, const float *in, float *out, const SoftTaps &tx, const SoftTaps &ty,
                 const SoftTaps &tz, float *t1, float *t2, const float *sub, float scale, const unsigned *skip) {
-  pass(R, in, t1, 0, kConv, 0, tx, skip);
-  pass(R, t1, t2, 1, kConv, 0, ty, skip);
+  pass(R, in, t1, 0, tx, skip);
+  pass(R, t1, t2, 1, ty, skip);
   const SoftGeom &g = R.g;
   const size_t smem = (size_t)(kSoftTileYZ + 2 * tz.r) * 32 * sizeof(float);
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(g.D, kSoftTileYZ), (unsigned)g.H);
   KLAUNCH("k_soft_pass_z_diff", R.st, (k_soft_pass_yz<2, kEpiDiff><<<grid, dim3(32, 8), smem, R.st>>>(
-                                          t2, out, g, kConv, tz.r, tz, skip, sub, nullptr, scale)));
+                                          t2, out, g, tz, skip, sub, nullptr, scale)));
 }
 
-// a transposed pass along `axis`: box gather (src = g_out, into g_in) or min / max scatter
-// (src = the filter's input, g_out into the zeroed g_in)
-void adj_pass(const SoftRun &R, const float *src, const float *g_out, float *g_in, int axis, int adj, int r) {
+// ---- the normalization's windows
+constexpr size_t kSoftMaxSmem = 220 * 1024;
+constexpr int kSoftColWarps[3] = {0, 8, 4};   // warps of the column passes along y and z
+
+template <class F>
+void allow_smem(F *fn, size_t bytes) {
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+// Grid of a column pass: 32 columns x the other coordinate x segments of the line, which is cut while the
+// columns alone leave the chip idle and a segment stays as long as a block's step and a window.
+dim3 col_grid(const SoftGeom &g, int axis, int r, int step, int &seg) {
+  const int n = axis == 1 ? g.H : g.D, other = axis == 1 ? g.D : g.H;
+  const int64_t cols = (int64_t)ceil_div(g.W, 32) * other;
+  const int64_t want = std::max<int64_t>(1, (1216 + cols - 1) / cols);
+  seg = std::min<int64_t>(n, std::max<int64_t>(ceil_div(n, want), std::max(step, 2 * r)));
+  return dim3((unsigned)ceil_div(g.W, 32), (unsigned)other, (unsigned)ceil_div(n, seg));
+}
+
+// Extremes along `axis`: the volume itself (axis 0) or a pair in, a pair out.
+void ext_pass(const SoftRun &R, const void *in, float2 *out, int axis, int r) {
   const SoftGeom &g = R.g;
-  const unsigned nb = R.blocks();
-  if (r > kSoftTileMaxR) {
-    if (adj == kAdjBox)
-      KLAUNCH("k_soft_box_adj", R.st, (k_soft_box_adj<<<nb, 256, 0, R.st>>>(src, g_in, g, axis, r, R.N)));
-    else
-      KLAUNCH("k_soft_minmax_adj", R.st, (k_soft_minmax_adj<<<nb, 256, 0, R.st>>>(src, g_out, g_in, g, axis, r,
-                                                                                 adj == kAdjMax, R.N)));
+  const float2 *in2 = static_cast<const float2 *>(in);
+  if (axis == 0) {
+    const float *v = static_cast<const float *>(in);
+    const int64_t rows = (int64_t)g.H * g.D;
+    if (r >= 4 && r <= 255) {
+      switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+#define HDOG_CASE(Q)                                                                                                  \
+  case Q:                                                                                                             \
+    KLAUNCH("k_soft_ext_rows", R.st, (k_soft_ext_rows<32, Q><<<ceil_div(rows, kSoftRowWarps), 32 * kSoftRowWarps, 0,  \
+                                                               R.st>>>(v, out, g, r)));                               \
+    return;                                                                                                           \
+  case Q + 1:                                                                                                         \
+    KLAUNCH("k_soft_ext_rows", R.st, (k_soft_ext_rows<8, Q><<<ceil_div(rows, 4 * kSoftRowWarps), 32 * kSoftRowWarps,  \
+                                                              0, R.st>>>(v, out, g, r)));                             \
+    return;
+        HDOG_CASE(0) HDOG_CASE(2) HDOG_CASE(4) HDOG_CASE(6)
+#undef HDOG_CASE
+      }
+    }
+    KLAUNCH("k_soft_ext_far", R.st, (k_soft_ext_far<true><<<R.blocks(), 256, 0, R.st>>>(in, out, g, axis, r, R.N)));
+    return;
+  }
+  const int nw = kSoftColWarps[axis];
+  const size_t smem = (size_t)ext_cols_rows(r, kSoftB, nw) * 32 * sizeof(float2);
+  if (2 * r < kSoftB || smem > kSoftMaxSmem) {
+    KLAUNCH("k_soft_ext_far", R.st, (k_soft_ext_far<false><<<R.blocks(), 256, 0, R.st>>>(in, out, g, axis, r, R.N)));
+    return;
+  }
+  int seg;
+  const dim3 grid = col_grid(g, axis, r, nw * kSoftB, seg);
+  if (axis == 1) {
+    allow_smem(k_soft_ext_cols<1, kSoftColWarps[1]>, smem);
+    KLAUNCH("k_soft_ext_y", R.st, (k_soft_ext_cols<1, kSoftColWarps[1]><<<grid, dim3(32, nw), smem, R.st>>>(in2, out, g, r, seg)));
+  } else {
+    allow_smem(k_soft_ext_cols<2, kSoftColWarps[2]>, smem);
+    KLAUNCH("k_soft_ext_z", R.st, (k_soft_ext_cols<2, kSoftColWarps[2]><<<grid, dim3(32, nw), smem, R.st>>>(in2, out, g, r, seg)));
+  }
+}
+
+// The adjoint of ext_pass: the gradient pair gout, through the pass's input src, added to gin (axis 0: the
+// volume's gradient; else a zeroed pair).
+void ext_adj(const SoftRun &R, const void *src, const float2 *gout, float *gin, int axis, int r) {
+  const SoftGeom &g = R.g;
+  if (axis == 0) {
+    const float *v = static_cast<const float *>(src);
+    const int64_t rows = (int64_t)g.H * g.D;
+    if (r >= 4 && r <= 255) {
+      switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+#define HDOG_CASE(Q)                                                                                                      \
+  case Q:                                                                                                                 \
+    KLAUNCH("k_soft_ext_adj_rows", R.st, (k_soft_ext_adj_rows<32, Q><<<ceil_div(rows, kSoftRowWarps), 32 * kSoftRowWarps, \
+                                                                       0, R.st>>>(v, gout, gin, g, r)));                  \
+    return;                                                                                                               \
+  case Q + 1:                                                                                                             \
+    KLAUNCH("k_soft_ext_adj_rows", R.st, (k_soft_ext_adj_rows<8, Q><<<ceil_div(rows, 4 * kSoftRowWarps),                  \
+                                                                      32 * kSoftRowWarps, 0, R.st>>>(v, gout, gin, g, r))); \
+    return;
+        HDOG_CASE(0) HDOG_CASE(2) HDOG_CASE(4) HDOG_CASE(6)
+#undef HDOG_CASE
+      }
+    }
+    KLAUNCH("k_soft_ext_adj_far", R.st, (k_soft_ext_adj_far<true><<<R.blocks(), 256, 0, R.st>>>(src, gout, gin, g, axis, r, R.N)));
+    return;
+  }
+  const int nw = kSoftColWarps[axis];
+  const size_t smem = (size_t)ext_cols_rows(r, kSoftB, nw) * 32 * (sizeof(float2) + sizeof(uint16_t));
+  if (2 * r < kSoftB || smem > kSoftMaxSmem) {
+    KLAUNCH("k_soft_ext_adj_far", R.st, (k_soft_ext_adj_far<false><<<R.blocks(), 256, 0, R.st>>>(src, gout, gin, g, axis, r, R.N)));
+    return;
+  }
+  int seg;
+  const dim3 grid = col_grid(g, axis, r, nw * kSoftB, seg);
+  const float2 *s2 = static_cast<const float2 *>(src);
+  float2 *g2 = reinterpret_cast<float2 *>(gin);
+  if (axis == 1) {
+    allow_smem(k_soft_ext_adj_cols<1, kSoftColWarps[1]>, smem);
+    KLAUNCH("k_soft_ext_adj_y", R.st, (k_soft_ext_adj_cols<1, kSoftColWarps[1]><<<grid, dim3(32, nw), smem, R.st>>>(s2, gout, g2, g, r, seg)));
+  } else {
+    allow_smem(k_soft_ext_adj_cols<2, kSoftColWarps[2]>, smem);
+    KLAUNCH("k_soft_ext_adj_z", R.st, (k_soft_ext_adj_cols<2, kSoftColWarps[2]><<<grid, dim3(32, nw), smem, R.st>>>(s2, gout, g2, g, r, seg)));
+  }
+}
+
+// Box means of a pair along `axis`, or (ADJ) the transpose; vol given (axis 2): also the normalized volume.
+template <bool ADJ>
+void box_pass(const SoftRun &R, const float2 *in, float2 *out, int axis, int r, const float *vol = nullptr) {
+  const SoftGeom &g = R.g;
+  const size_t smem = (size_t)32 * ((kSoftBoxX + 2 * r) | 1) * sizeof(float2);
+  if (smem > kSoftMaxSmem) {   // reaches above 365
+    KLAUNCH("k_soft_box_far", R.st, (k_soft_box_far<ADJ><<<R.blocks(), 256, 0, R.st>>>(in, out, g, axis, r, R.N)));
+    if (vol)
+      KLAUNCH("k_soft_norm", R.st, (k_soft_norm<<<R.blocks(), 256, 0, R.st>>>(vol, out, R.slot(S_NORM), R.p.min_intensity, R.N,
+                                                                             R.flags())));
     return;
   }
   if (axis == 0) {
-    const unsigned blocks = (unsigned)(ceil_div(g.W, kSoftTileX) * ceil_div((int64_t)g.H * g.D, kSoftRowsX));
-    KLAUNCH("k_soft_adj_x", R.st, (k_soft_adj_x<<<blocks, kSoftTileX, 0, R.st>>>(src, g_out, g_in, g, adj, r)));
+    allow_smem(k_soft_box_x<ADJ>, smem);
+    const unsigned blocks = (unsigned)(ceil_div(g.W, kSoftBoxX) * ceil_div((int64_t)g.H * g.D, 32));
+    KLAUNCH(ADJ ? "k_soft_box_adj_x" : "k_soft_box_x", R.st, (k_soft_box_x<ADJ><<<blocks, 256, smem, R.st>>>(in, out, g, r)));
     return;
   }
-  const int n = axis == 1 ? g.H : g.D, other = axis == 1 ? g.D : g.H;
-  if (adj != kAdjBox && r <= kSoftExtMaxR) {
-    const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(n, kSoftTileYZ), (unsigned)other);
-    if (axis == 1)
-      KLAUNCH("k_soft_ext_adj_y", R.st, (k_soft_ext_adj_yz<1><<<grid, dim3(32, 16), 0, R.st>>>(src, g_out, g_in, g,
-                                                                                              adj == kAdjMax, r)));
-    else
-      KLAUNCH("k_soft_ext_adj_z", R.st, (k_soft_ext_adj_yz<2><<<grid, dim3(32, 16), 0, R.st>>>(src, g_out, g_in, g,
-                                                                                              adj == kAdjMax, r)));
+  if (axis == 1) {
+    constexpr int K = 16;
+    const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)g.D, (unsigned)ceil_div(g.H, 4 * K));
+    KLAUNCH(ADJ ? "k_soft_box_adj_y" : "k_soft_box_y", R.st,
+            (k_soft_box_cols<1, K, ADJ, false><<<grid, dim3(32, 4), 0, R.st>>>(in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));
     return;
   }
-  const size_t smem = (size_t)(kSoftTileYZ + 2 * r) * 32 * sizeof(float);
-  const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)ceil_div(n, kSoftTileYZ), (unsigned)other);
-  if (axis == 1)
-    KLAUNCH("k_soft_adj_y", R.st, (k_soft_adj_yz<1><<<grid, dim3(32, 8), smem, R.st>>>(src, g_out, g_in, g, adj, r)));
+  constexpr int K = 8;
+  const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)g.H, (unsigned)ceil_div(g.D, 4 * K));
+  if (vol)
+    KLAUNCH("k_soft_box_z_norm", R.st, (k_soft_box_cols<2, K, false, true><<<grid, dim3(32, 4), 0, R.st>>>(
+                                           in, out, g, r, vol, R.slot(S_NORM), R.p.min_intensity, R.flags())));
   else
-    KLAUNCH("k_soft_adj_z", R.st, (k_soft_adj_yz<2><<<grid, dim3(32, 8), smem, R.st>>>(src, g_out, g_in, g, adj, r)));
+    KLAUNCH("k_soft_box_adj_z", R.st, (k_soft_box_cols<2, K, ADJ, false><<<grid, dim3(32, 4), 0, R.st>>>(
+                                          in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));
 }
 
 // conv of `in` with taps (tx, ty, tz) along x, y, z -> out (t1, t2 as temporaries)
 void conv3(const SoftRun &R, const float *in, float *out, const SoftTaps &tx, const SoftTaps &ty, const SoftTaps &tz,
            float *t1, float *t2, const unsigned *skip = nullptr) {
-  pass(R, in, t1, 0, kConv, 0, tx, skip);
-  pass(R, t1, t2, 1, kConv, 0, ty, skip);
-  pass(R, t2, out, 2, kConv, 0, tz, skip);
+  pass(R, in, t1, 0, tx, skip);
+  pass(R, t1, t2, 1, ty, skip);
+  pass(R, t2, out, 2, tz, skip);
 }
 
 // The DoG slot from the normalized one (temporaries T1-T3); skip: a device flag that says it is filled.
@@ -1205,25 +1450,14 @@ void dense_dog(const SoftRun &R, const unsigned *skip) {
 // score is to be read from the volume.
 void forward_chain(const SoftRun &R, const float *vol, bool want_dog) {
   cudaMemsetAsync(R.acc, 0, 16 * sizeof(double), R.st);
-  const hdog_soft_params &p = R.p;
-  const SoftTaps none = no_taps();
-  const int rr[3] = {p.radius_norm_xy, p.radius_norm_xy, p.radius_norm_z};
-  const float *src_mn = vol, *src_mx = vol;
-  const int smn[3] = {S_MN1, S_MN2, S_MN}, smx[3] = {S_MX1, S_MX2, S_MX};
-  for (int a = 0; a < 3; a++) {
-    pass(R, src_mn, R.slot(smn[a]), a, kMin, rr[a], none);
-    pass(R, src_mx, R.slot(smx[a]), a, kMax, rr[a], none);
-    src_mn = R.slot(smn[a]);
-    src_mx = R.slot(smx[a]);
-  }
-  pass(R, R.slot(S_MN), R.slot(S_T1), 0, kBox, rr[0], none);
-  pass(R, R.slot(S_T1), R.slot(S_T2), 1, kBox, rr[1], none);
-  pass(R, R.slot(S_T2), R.slot(S_E), 2, kBox, rr[2], none);
-  pass(R, R.slot(S_MX), R.slot(S_T1), 0, kBox, rr[0], none);
-  pass(R, R.slot(S_T1), R.slot(S_T2), 1, kBox, rr[1], none);
-  pass(R, R.slot(S_T2), R.slot(S_D), 2, kBox, rr[2], none);
-  KLAUNCH("k_soft_norm", R.st, (k_soft_norm<<<R.blocks(), 256, 0, R.st>>>(vol, R.slot(S_E), R.slot(S_D), R.slot(S_NORM),
-                                                                        p.min_intensity, R.N, R.flags())));
+  const int rxy = R.p.radius_norm_xy, rz = R.p.radius_norm_z;
+  float2 *mm1 = R.pair(S_MM1), *mm2 = R.pair(S_MM2), *pa = R.pair(S_PA), *pb = R.pair(S_PB);
+  ext_pass(R, vol, mm1, 0, rxy);
+  ext_pass(R, mm1, mm2, 1, rxy);
+  ext_pass(R, mm2, pa, 2, rz);
+  box_pass<false>(R, pa, pb, 0, rxy);
+  box_pass<false>(R, pb, pa, 1, rxy);
+  box_pass<false>(R, pa, R.pair(S_ED), 2, rz, vol);
   if (want_dog) {
     dense_dog(R, nullptr);
     cudaMemsetAsync(R.flags() + 1, 1, sizeof(unsigned), R.st);
@@ -1291,7 +1525,7 @@ int check_params(const hdog_soft_params *p, const float *vol, const int32_t *pos
 }  // namespace
 
 size_t soft_workspace_bytes(const hdog_soft_params &p) {
-  return 16 * sizeof(double) + (size_t)kSoftSlots * p.width * p.height * p.depth * sizeof(float);
+  return 16 * sizeof(double) + (size_t)kSoftSlots * SoftRun::slot_floats((int64_t)p.width * p.height * p.depth) * sizeof(float);
 }
 
 int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos, int n_pos, const int32_t *neg,
@@ -1325,7 +1559,7 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
   R.acc = static_cast<double *>(work);
   R.w = reinterpret_cast<float *>(R.acc + 16);
   const unsigned nb = R.blocks();
-  // The backward reads the forward chain's slots (S_MN1 .. S_DOG) and writes only the others,
+  // The backward reads the forward chain's slots (S_MM1 .. S_DOG) and writes only the others,
   // so a workspace that soft_forward filled for the same inputs still holds them.
   SoftBox box;
   const bool local = points_local(R, (int64_t)n_pos + n_neg, box);
@@ -1344,8 +1578,7 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
   } else {
     // a forward call with fewer points may have left the DoG slot empty
     if (forward_kept) dense_dog(R, R.flags() + 1);
-    static_assert(S_GB == S_GA + 1 && S_GA % 2 == 0, "an 8-byte aligned volume of doubles");
-    double *gsum = reinterpret_cast<double *>(R.slot(S_GA));
+    double *gsum = reinterpret_cast<double *>(R.slot(S_PA));   // a pair's two slots
     cudaMemsetAsync(gsum, 0, R.N * sizeof(double), st);
     if (n_pos + n_neg > 0)
       KLAUNCH("k_soft_points_adj", st, (k_soft_points_adj<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
@@ -1367,13 +1600,13 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
           dv[a] = gauss_taps_f(s[3 * sc + a], true);
         }
         double *acc = R.acc + 3 * sc;
-        pass(R, nm, t1, 0, kConv, 0, pl[0]);
-        pass(R, t1, t2, 1, kConv, 0, pl[1]);
+        pass(R, nm, t1, 0, pl[0]);
+        pass(R, t1, t2, 1, pl[1]);
         pass_z_dot(R, t2, dv[2], gdog, acc + 2);
-        pass(R, t1, t2, 1, kConv, 0, dv[1]);
+        pass(R, t1, t2, 1, dv[1]);
         pass_z_dot(R, t2, pl[2], gdog, acc + 1);
-        pass(R, nm, t1, 0, kConv, 0, dv[0]);
-        pass(R, t1, t2, 1, kConv, 0, pl[1]);
+        pass(R, nm, t1, 0, dv[0]);
+        pass(R, t1, t2, 1, pl[1]);
         pass_z_dot(R, t2, pl[2], gdog, acc + 0);
       }
       KLAUNCH("k_soft_dot", st, (k_soft_dot<<<db, 256, 0, st>>>(gdog, R.slot(S_DOG), R.N, R.acc + 6)));
@@ -1391,42 +1624,29 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
       conv3_diff(R, gdog, R.slot(S_GB), gauss_taps_f(s[3], false), gauss_taps_f(s[4], false), gauss_taps_f(s[5], false),
                  R.slot(S_T1), R.slot(S_T2), R.slot(S_T3), nrm, nullptr);
     }
-    // quotient rule: direct term into grad_vol, g_e -> S_T1, g_d -> S_T2
-    KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<<<nb, 256, 0, st>>>(vol, R.slot(S_E), R.slot(S_D), R.slot(S_GB),
-                                                                       grad_vol, R.slot(S_T1), R.slot(S_T2),
+    // quotient rule: direct term into grad_vol, the box means' gradients into a pair
+    float2 *cur = R.pair(S_PA), *next = R.pair(S_PB);
+    KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<<<nb, 256, 0, st>>>(vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur,
                                                                        p->min_intensity, R.N)));
+    // box means transposed z -> y -> x, then the extremes z -> y -> x, each adding to a zeroed pair but the
+    // last, which adds straight to the input gradient (holding the quotient rule's direct term)
     const int rr[3] = {p->radius_norm_xy, p->radius_norm_xy, p->radius_norm_z};
-    // min side then max side: box means transposed z -> y -> x, then the min / max filters
-    // transposed z -> y -> x, each scattering into a zeroed buffer but the last, which
-    // scatters straight into the input gradient (holding the quotient rule's direct term)
-    int last = -1;   // the axis of the last min / max pass: the lowest one with a window
-    for (int a = 2; a >= 0; a--)
-      if (rr[a] != 0) last = a;
-    for (int side = 0; side < 2; side++) {
-      float *g = R.slot(side == 0 ? S_T1 : S_T2);
-      float *ping = R.slot(S_GA), *pong = R.slot(S_GC);
-      const float *cur = g;
-      for (int a = 2; a >= 0; a--) {
-        float *dst = (cur == ping) ? pong : ping;
-        if (rr[a] == 0) continue;
-        adj_pass(R, cur, nullptr, dst, a, kAdjBox, rr[a]);
-        cur = dst;
-      }
-      // filter inputs of the forward passes x, y, z: vol, *1, *2
-      const float *fin[3] = {vol, R.slot(side == 0 ? S_MN1 : S_MX1), R.slot(side == 0 ? S_MN2 : S_MX2)};
-      for (int a = 2; a >= 0; a--) {
-        if (rr[a] == 0) continue;
-        float *dst = grad_vol;
-        if (a != last) {
-          dst = (cur == ping) ? pong : ping;
-          if (dst == g) dst = R.slot(S_GB);
-          cudaMemsetAsync(dst, 0, R.N * sizeof(float), st);
-        }
-        adj_pass(R, fin[a], cur, dst, a, side == 0 ? kAdjMin : kAdjMax, rr[a]);
-        cur = dst;
-      }
-      if (last < 0) KLAUNCH("k_soft_add", st, (k_soft_add<<<nb, 256, 0, st>>>(grad_vol, cur, R.N)));
+    for (int a = 2; a >= 0; a--) {
+      if (rr[a] == 0) continue;
+      box_pass<true>(R, cur, next, a, rr[a]);
+      std::swap(cur, next);
     }
+    for (int a = 2; a >= 0; a--) {
+      if (rr[a] == 0) continue;
+      if (a == 0) {
+        ext_adj(R, vol, cur, grad_vol, 0, rr[0]);
+      } else {
+        cudaMemsetAsync(next, 0, R.N * sizeof(float2), st);
+        ext_adj(R, R.pair(a == 1 ? S_MM1 : S_MM2), cur, reinterpret_cast<float *>(next), a, rr[a]);
+        std::swap(cur, next);
+      }
+    }
+    if (rr[0] == 0) KLAUNCH("k_soft_add", st, (k_soft_add<<<nb, 256, 0, st>>>(grad_vol, cur, R.N)));
   }
   HDOG_CUDA_TRY(cudaGetLastError());
   return HDOG_OK;

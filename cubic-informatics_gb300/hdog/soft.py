@@ -7,7 +7,7 @@ sample points.  Torch only holds the tensors and the graph; every stage runs in 
                                radius_norm_z=5, min_intensity=50.0, tau=1e-3)
     loss.backward()      # volume.grad, sigma.grad, b.grad
 
-By default the forward's workspace (17 volume-sized float32 buffers) stays alive until the
+By default the forward's workspace (13 volume-sized float32 buffers) stays alive until the
 backward, which then takes the forward chain's intermediates from it instead of recomputing
 them (same results); keep_intermediates=False frees it after the forward and the backward
 recomputes.
