@@ -549,7 +549,34 @@ __device__ __forceinline__ float2 soft_box_ends(int c, int n, int R, LoadF ld, f
     for (int t = max(0, n - R); t < n; t++) acc = soft_fma2((float)(t + R - (n - 1)), ld(t), acc);
   return acc;
 }
-__device__ __forceinline__ float2 soft_div(float2 a, float n) { return make_float2(a.x / n, a.y / n); }
+// the same for K outputs from c0 (a multiple of K) on: only the first of them can be the line's first, any its
+// last, so each loop stands once in the code
+template <int K, class LoadF>
+__device__ __forceinline__ void soft_box_ends_k(int c0, int n, int R, LoadF ld, float2 (&acc)[K]) {
+  if (c0 == 0)
+    for (int t = 0; t < min(n, R); t++) acc[0] = soft_fma2((float)(R - t), ld(t), acc[0]);
+  const int last = n - 1 - c0;
+  if (last >= K) return;
+  float2 e = acc[0];
+#pragma unroll
+  for (int k = 1; k < K; k++) e = k == last ? acc[k] : e;
+  for (int t = max(0, n - R); t < n; t++) e = soft_fma2((float)(t + R - (n - 1)), ld(t), e);
+#pragma unroll
+  for (int k = 0; k < K; k++) acc[k] = k == last ? e : acc[k];
+}
+
+// a / n for a whole number n below 2^24, correctly rounded: with z = 1 / n rounded and q = a z rounded, the remainder
+// a - n q is exact in one FMA and q + remainder z rounds to the quotient (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  An infinite or NaN a
+// leaves no remainder to correct with.
+struct SoftDiv {
+  float n, z;
+  __device__ __forceinline__ SoftDiv(int n_) : n((float)n_), z(1.0f / (float)n_) {}
+  __device__ __forceinline__ float2 operator()(float2 a) const {
+    const float2 zz = make_float2(z, z), q = mul2(a, zz), r = fma2(make_float2(-n, -n), q, a), p = fma2(r, zz, q);
+    return make_float2(r.x == r.x ? p.x : q.x, r.y == r.y ? p.y : q.y);
+  }
+};
 
 // Box mean along x (or its transpose): a tile of 32 rows x kSoftBoxX outputs with the reach on both sides in shared
 // memory (odd pitch: a lane's row starts in its own bank), one row per lane and kSoftBoxK outputs per thread.
@@ -566,9 +593,14 @@ __global__ void __launch_bounds__(256, 2) k_soft_box_x(const float2 *in, float2 
     const float2 *line = in + (row0 + k) * g.W;
     for (int i = lane; i < n0; i += 32) {
       const int x = x0 - R + i;
-      tile2[k * pitch + i] = ADJ && (x < 0 || x >= g.W) ? make_float2(0.0f, 0.0f) : __ldg(line + clampi(x, 0, g.W - 1));
+      // asynchronous, so that all of a thread's loads are in flight at once; outside the line (ADJ) no bytes, zeros
+      const bool zero = ADJ && (x < 0 || x >= g.W);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(tile2 + k * pitch + i)),
+                   "l"(line + clampi(x, 0, g.W - 1)), "r"(zero ? 0 : 8)
+                   : "memory");
     }
   }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   float2 acc[kSoftBoxK];
   const float2 *mine = tile2 + lane * pitch;
@@ -576,12 +608,10 @@ __global__ void __launch_bounds__(256, 2) k_soft_box_x(const float2 *in, float2 
   const bool work = lane < nr && x0 + xw < g.W;
   if (work) {
     box_chain<kSoftBoxK>(2 * R + 1, [&](int i) { return mine[xw + i]; }, acc);
-    const float L = (float)(2 * R + 1);
+    if (ADJ) soft_box_ends_k(x0 + xw, g.W, R, [&](int t) { return mine[t - x0 + R]; }, acc);
+    const SoftDiv div(2 * R + 1);
 #pragma unroll
-    for (int k = 0; k < kSoftBoxK; k++) {
-      if (ADJ) acc[k] = soft_box_ends(x0 + xw + k, g.W, R, [&](int t) { return mine[t - x0 + R]; }, acc[k]);
-      acc[k] = soft_div(acc[k], L);
-    }
+    for (int k = 0; k < kSoftBoxK; k++) acc[k] = div(acc[k]);
   }
   __syncthreads();
   if (work)
@@ -594,15 +624,36 @@ __global__ void __launch_bounds__(256, 2) k_soft_box_x(const float2 *in, float2 
 
 // Box mean along y or z (or its transpose), K outputs of one column per thread; NORM (z, the last
 // pass): also the normalized volume, *bad set when a value of it is not finite (a window without contrast).
-template <int AXIS, int K, bool ADJ, bool NORM>
-__global__ void __launch_bounds__(128) k_soft_box_cols(const float2 *in, float2 *out, SoftGeom g, int R, const float *I,
+// RT: the reach where it is known at compile time (all of a thread's loads are then in flight before the
+// first add), else 0.
+template <int AXIS, int K, bool ADJ, bool NORM, int RT>
+__global__ void __launch_bounds__(128) k_soft_box_cols(const float2 *in, float2 *out, SoftGeom g, int R_, const float *I,
                                                        float *norm, float min_intensity, unsigned *bad) {
   const SoftLine<AXIS> l(g);
   const int c0 = (blockIdx.z * blockDim.y + threadIdx.y) * K;
   if (!l.in || c0 >= l.n) return;
   const float2 *col = in + l.base;
+  const int R = RT ? RT : R_;
   float2 acc[K];
-  if (c0 - R >= 0 && c0 + K + R < l.n) {   // the chain loads one input past its last window
+  float iv[K];
+  if (NORM) {
+#pragma unroll
+    for (int k = 0; k < K; k++) iv[k] = __ldg(I + l.base + (int64_t)min(c0 + k, l.n - 1) * l.s);
+  }
+  if constexpr (RT > 0) {
+    float2 win[K + 2 * RT];
+#pragma unroll
+    for (int i = 0; i < K + 2 * RT; i++) {
+      const int c = c0 - RT + i;
+      win[i] = ADJ && (c < 0 || c >= l.n) ? make_float2(0.0f, 0.0f) : __ldg(col + (int64_t)clampi(c, 0, l.n - 1) * l.s);
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      acc[k] = make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int j = 0; j <= 2 * RT; j++) acc[k] = add2(acc[k], win[k + j]);
+    }
+  } else if (c0 - R >= 0 && c0 + K + R < l.n) {   // the chain loads one input past its last window
     const float2 *p = col + (int64_t)(c0 - R) * l.s;
     box_chain<K>(2 * R + 1, [&](int i) { return __ldg(p + (int64_t)i * l.s); }, acc);
   } else {
@@ -611,18 +662,17 @@ __global__ void __launch_bounds__(128) k_soft_box_cols(const float2 *in, float2 
       return ADJ && (c < 0 || c >= l.n) ? make_float2(0.0f, 0.0f) : __ldg(col + (int64_t)clampi(c, 0, l.n - 1) * l.s);
     }, acc);
   }
-  const float L = (float)(2 * R + 1);
+  if (ADJ) soft_box_ends_k(c0, l.n, R, [&](int t) { return __ldg(col + (int64_t)t * l.s); }, acc);
+  const SoftDiv div(2 * R + 1);
 #pragma unroll
   for (int k = 0; k < K; k++) {
     const int c = c0 + k;
     if (c >= l.n) break;
     const int64_t i = l.base + (int64_t)c * l.s;
-    if (ADJ) acc[k] = soft_box_ends(c, l.n, R, [&](int t) { return __ldg(col + (int64_t)t * l.s); }, acc[k]);
-    const float2 m = soft_div(acc[k], L);
+    const float2 m = div(acc[k]);
     out[i] = m;
     if (NORM) {
-      const float iv = __ldg(I + i);
-      const float v = iv >= min_intensity ? (iv - m.x) / (m.y - m.x) : 0.0f;
+      const float v = iv[k] >= min_intensity ? (iv[k] - m.x) / (m.y - m.x) : 0.0f;
       norm[i] = v;
       if (!isfinite(v)) *bad = 1u;
     }
@@ -689,7 +739,7 @@ __global__ void k_soft_box_far(const float2 *in, float2 *out, SoftGeom g, int ax
   }
   float2 acc = add2(hi, lo);
   if (ADJ) acc = soft_box_ends(c, n, R, [&](int t) { return line[(int64_t)t * s]; }, acc);
-  out[i] = soft_div(acc, (float)(2 * R + 1));
+  out[i] = SoftDiv(2 * R + 1)(acc);
 }
 
 // The normalized volume from the box means where no other pass forms it (see k_soft_box_cols).
@@ -704,20 +754,37 @@ __global__ void k_soft_norm(const float *I, const float2 *ed, float *norm, float
 }
 
 // Quotient rule of the normalization: g_I (direct term, written) and the gradients of both box means.
-__global__ void k_soft_norm_adj(const float *I, const float2 *ed, const float *g_norm, float *g_I, float2 *g_ed,
-                                float min_intensity, int64_t N) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const float g = g_norm[i], v = I[i];
-  const float2 m = ed[i];
+__device__ __forceinline__ void soft_norm_adj_one(float v, float2 m, float g, float min_intensity, float &gi, float2 &ged) {
   if (v >= min_intensity) {
     const float den = m.y - m.x, inv = 1.0f / den, inv2 = inv * inv;
-    g_I[i] = g * inv;
-    g_ed[i] = make_float2(g * (v - m.y) * inv2, -g * (v - m.x) * inv2);
+    gi = g * inv;
+    ged = make_float2(g * (v - m.y) * inv2, -g * (v - m.x) * inv2);
   } else {
-    g_I[i] = 0.0f;
-    g_ed[i] = make_float2(0.0f, 0.0f);
+    gi = 0.0f;
+    ged = make_float2(0.0f, 0.0f);
   }
+}
+
+// VEC 4: four voxels per thread in 16-byte accesses (I and g_I on 16 bytes; the workspace's volumes are)
+template <int VEC>
+__global__ void __launch_bounds__(256) k_soft_norm_adj(const float *I, const float2 *ed, const float *g_norm, float *g_I,
+                                                       float2 *g_ed, float min_intensity, int64_t N) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  if (VEC == 4 && i + 4 <= N) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(I + i)), g = __ldg(reinterpret_cast<const float4 *>(g_norm + i));
+    const float4 m0 = __ldg(reinterpret_cast<const float4 *>(ed + i)), m1 = __ldg(reinterpret_cast<const float4 *>(ed + i) + 1);
+    float4 gi;
+    float2 a, b, c, d;
+    soft_norm_adj_one(v.x, make_float2(m0.x, m0.y), g.x, min_intensity, gi.x, a);
+    soft_norm_adj_one(v.y, make_float2(m0.z, m0.w), g.y, min_intensity, gi.y, b);
+    soft_norm_adj_one(v.z, make_float2(m1.x, m1.y), g.z, min_intensity, gi.z, c);
+    soft_norm_adj_one(v.w, make_float2(m1.z, m1.w), g.w, min_intensity, gi.w, d);
+    *reinterpret_cast<float4 *>(g_I + i) = gi;
+    reinterpret_cast<float4 *>(g_ed + i)[0] = make_float4(a.x, a.y, b.x, b.y);
+    reinterpret_cast<float4 *>(g_ed + i)[1] = make_float4(c.x, c.y, d.x, d.y);
+    return;
+  }
+  for (int64_t k = i; k < min(i + VEC, N); k++) soft_norm_adj_one(I[k], ed[k], g_norm[k], min_intensity, g_I[k], g_ed[k]);
 }
 
 // a += b.x + b.y (no window along any of x and y: both sides' gradients belong where they are)
@@ -1415,16 +1482,29 @@ void box_pass(const SoftRun &R, const float2 *in, float2 *out, int axis, int r, 
     constexpr int K = 16;
     const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)g.D, (unsigned)ceil_div(g.H, 4 * K));
     KLAUNCH(ADJ ? "k_soft_box_adj_y" : "k_soft_box_y", R.st,
-            (k_soft_box_cols<1, K, ADJ, false><<<grid, dim3(32, 4), 0, R.st>>>(in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));
+            (k_soft_box_cols<1, K, ADJ, false, 0><<<grid, dim3(32, 4), 0, R.st>>>(in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));
     return;
   }
   constexpr int K = 8;
   const dim3 grid((unsigned)ceil_div(g.W, 32), (unsigned)g.H, (unsigned)ceil_div(g.D, 4 * K));
+  switch (r) {
+#define HDOG_CASE(RT)                                                                                                   \
+  case RT:                                                                                                              \
+    if (vol)                                                                                                            \
+      KLAUNCH("k_soft_box_z_norm", R.st, (k_soft_box_cols<2, K, false, true, RT><<<grid, dim3(32, 4), 0, R.st>>>(       \
+                                             in, out, g, r, vol, R.slot(S_NORM), R.p.min_intensity, R.flags())));       \
+    else                                                                                                                \
+      KLAUNCH("k_soft_box_adj_z", R.st, (k_soft_box_cols<2, K, true, false, RT><<<grid, dim3(32, 4), 0, R.st>>>(        \
+                                            in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));                          \
+    return;
+    HDOG_CASE(1) HDOG_CASE(2) HDOG_CASE(3) HDOG_CASE(4) HDOG_CASE(5) HDOG_CASE(6) HDOG_CASE(7) HDOG_CASE(8)
+#undef HDOG_CASE
+  }
   if (vol)
-    KLAUNCH("k_soft_box_z_norm", R.st, (k_soft_box_cols<2, K, false, true><<<grid, dim3(32, 4), 0, R.st>>>(
+    KLAUNCH("k_soft_box_z_norm", R.st, (k_soft_box_cols<2, K, false, true, 0><<<grid, dim3(32, 4), 0, R.st>>>(
                                            in, out, g, r, vol, R.slot(S_NORM), R.p.min_intensity, R.flags())));
   else
-    KLAUNCH("k_soft_box_adj_z", R.st, (k_soft_box_cols<2, K, ADJ, false><<<grid, dim3(32, 4), 0, R.st>>>(
+    KLAUNCH("k_soft_box_adj_z", R.st, (k_soft_box_cols<2, K, true, false, 0><<<grid, dim3(32, 4), 0, R.st>>>(
                                           in, out, g, r, nullptr, nullptr, 0.0f, nullptr)));
 }
 
@@ -1626,8 +1706,13 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
     }
     // quotient rule: direct term into grad_vol, the box means' gradients into a pair
     float2 *cur = R.pair(S_PA), *next = R.pair(S_PB);
-    KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<<<nb, 256, 0, st>>>(vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur,
-                                                                       p->min_intensity, R.N)));
+    const auto on16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    if (on16(vol) && on16(grad_vol) && on16(work))
+      KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<4><<<ceil_div(R.N, 1024), 256, 0, st>>>(
+                                         vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur, p->min_intensity, R.N)));
+    else
+      KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<1><<<nb, 256, 0, st>>>(
+                                         vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur, p->min_intensity, R.N)));
     // box means transposed z -> y -> x, then the extremes z -> y -> x, each adding to a zeroed pair but the
     // last, which adds straight to the input gradient (holding the quotient rule's direct term)
     const int rr[3] = {p->radius_norm_xy, p->radius_norm_xy, p->radius_norm_z};

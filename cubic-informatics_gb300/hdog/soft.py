@@ -66,9 +66,9 @@ class SoftLoss(torch.autograd.Function):
         vol, sigma, thresh, pos, neg = ctx.saved_tensors
         p = _params(vol, sigma, thresh, ctx.cfg)
         want_vol, want_sigma, want_thresh = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
-        gv = torch.zeros_like(vol) if want_vol else None
-        gs = torch.zeros(6, dtype=torch.float32, device=vol.device) if want_sigma else None
-        gb = torch.zeros(3, dtype=torch.float32, device=vol.device) if want_thresh else None
+        gv = torch.empty_like(vol) if want_vol else None     # every element is written
+        gs = torch.empty(6, dtype=torch.float32, device=vol.device) if want_sigma else None
+        gb = torch.empty(3, dtype=torch.float32, device=vol.device) if want_thresh else None
         stream = ctypes.c_void_p(torch.cuda.current_stream(vol.device).cuda_stream)
         if ctx.kept is not None:
             ws = ctx.kept
