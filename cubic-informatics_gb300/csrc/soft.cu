@@ -258,15 +258,19 @@ __global__ void __launch_bounds__(32 * NW) k_soft_ext_cols(const float2 *in, flo
 }
 
 // The adjoint along y or z: src the pass's input, gout its output's gradient, added to gin (zeroed before).
-// As ext_cols, with the suffixes' places in their blocks kept beside them.
-template <int AXIS, int NW>
-__global__ void __launch_bounds__(32 * NW) k_soft_ext_adj_cols(const float2 *src, const float2 *gout, float2 *gin,
-                                                               SoftGeom g, int r, int seg) {
+// As ext_cols with the suffixes' places in their blocks kept beside them, but one warp per 32 columns
+// runs down a segment alone: it needs no block barrier, and a run of windows with one extreme goes on from
+// block to block, so that few voxels take an atomic add (interleaved blocks of 8 warps ended a run every
+// 8 outputs).  The next block's inputs and gradients are loaded before this one is worked on.
+// 512x512x128, reaches 20 and 5: y 244 -> 202 us, z 240 -> 150 us.
+template <int AXIS>
+__global__ void __launch_bounds__(32) k_soft_ext_adj_cols(const float2 *src, const float2 *gout, float2 *gin, SoftGeom g,
+                                                          int r, int seg) {
   constexpr int B = kSoftB;
   extern __shared__ float2 ring2[];
   const SoftLine<AXIS> l(g);
-  const int lane = threadIdx.x, w = threadIdx.y, t0 = blockIdx.z * seg, n = min(seg, l.n - t0);
-  const int rows = ext_cols_rows(r, B, NW), total = n + 2 * r, back = (2 * r + B - 1) / B, q = back * B - 2 * r;
+  const int lane = threadIdx.x, t0 = blockIdx.z * seg, n = min(seg, l.n - t0);
+  const int rows = ext_cols_rows(r, B, 1), total = n + 2 * r, back = (2 * r + B - 1) / B, q = back * B - 2 * r;
   uint16_t *place = reinterpret_cast<uint16_t *>(ring2 + rows * 32);
   float *gi = reinterpret_cast<float *>(gin);
   auto put = [&](int side) {
@@ -274,23 +278,41 @@ __global__ void __launch_bounds__(32 * NW) k_soft_ext_adj_cols(const float2 *src
       atomicAdd(gi + 2 * (l.base + (int64_t)clampi(t0 - r + e, 0, l.n - 1) * l.s) + side, v);
     };
   };
-  int pos = w * B;
-  for (int c = 0; c < total; c += NW * B) {
-    const int a = c + w * B;
-    float2 v[B];
-    if (a < total) {
+  RunSum<decltype(put(0))> lo(put(0)), hi(put(1));
+  float2 nv[B], ng[B];
+  auto fetch = [&](int a) {
+    const int y = t0 - r + a;
+    if (y >= 0 && y + B <= l.n) {
+      const float2 *p = src + l.base + (int64_t)y * l.s;
 #pragma unroll
-      for (int j = 0; j < B; j++) v[j] = __ldg(src + l.base + (int64_t)clampi(t0 - r + a + j, 0, l.n - 1) * l.s);
-      ExtAt s{v[B - 1], B - 1, B - 1};
+      for (int j = 0; j < B; j++, p += l.s) nv[j] = __ldg(p);
+    } else {
 #pragma unroll
-      for (int j = B - 1; j >= 0; j--) {
-        if (j < B - 1) s = ext_join(ExtAt{v[j], j, j}, s);
-        ring2[(pos + j) * 32 + lane] = s.v;
-        place[(pos + j) * 32 + lane] = (uint16_t)(s.a | s.b << 8);
-      }
+      for (int j = 0; j < B; j++) nv[j] = __ldg(src + l.base + (int64_t)clampi(y + j, 0, l.n - 1) * l.s);
     }
-    __syncthreads();
-    if (a < total && a + B > 2 * r && l.in) {
+    if (a + B > 2 * r) {
+#pragma unroll
+      for (int j = 0; j < B; j++) ng[j] = __ldg(gout + l.base + (int64_t)clampi(t0 + a + j - 2 * r, 0, l.n - 1) * l.s);
+    }
+  };
+  fetch(0);
+  int pos = 0;
+  for (int a = 0; a < total; a += B) {
+    float2 v[B], go[B];
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+      v[j] = nv[j];
+      go[j] = ng[j];
+    }
+    if (a + B < total) fetch(a + B);
+    ExtAt s{v[B - 1], B - 1, B - 1};
+#pragma unroll
+    for (int j = B - 1; j >= 0; j--) {
+      if (j < B - 1) s = ext_join(ExtAt{v[j], j, j}, s);
+      ring2[(pos + j) * 32 + lane] = s.v;
+      place[(pos + j) * 32 + lane] = (uint16_t)(s.a | s.b << 8);
+    }
+    if (a + B > 2 * r) {   // a lane reads its own column only
       auto row = [&](int d) {
         const int p = pos - d * B;
         return p < 0 ? p + rows : p;
@@ -308,7 +330,6 @@ __global__ void __launch_bounds__(32 * NW) k_soft_ext_adj_cols(const float2 *src
         mid0 = get(row(back - 1), a - (back - 1) * B);
         if (back >= 3) mid0 = ext_join(mid0, mid1);
       }
-      RunSum<decltype(put(0))> lo(put(0)), hi(put(1));
       const int r0 = row(back), r1 = back >= 2 ? row(back - 1) : r0;
       ExtAt p{v[0], a, a};
 #pragma unroll
@@ -320,16 +341,17 @@ __global__ void __launch_bounds__(32 * NW) k_soft_ext_adj_cols(const float2 *src
         ExtAt m = first ? get(r0 + q + o, a - back * B) : get(r1 + q + o - B, a - (back - 1) * B);
         if (first ? back >= 2 : back >= 3) m = ext_join(m, first ? mid0 : mid1);
         m = ext_join(m, p);
-        const float2 go = __ldg(gout + l.base + (int64_t)(t0 + e - 2 * r) * l.s);
-        lo.add(m.a, go.x);
-        hi.add(m.b, go.y);
+        if (l.in) {
+          lo.add(m.a, go[o].x);
+          hi.add(m.b, go[o].y);
+        }
       }
-      lo.flush();
-      hi.flush();
     }
-    pos += NW * B;
+    pos += B;
     if (pos >= rows) pos -= rows;
   }
+  lo.flush();
+  hi.flush();
 }
 
 // 32-byte global accesses where the address allows them (sm_100 on), else entry by entry
@@ -913,7 +935,8 @@ __global__ void k_soft_points(const float *dog, SoftGeom g, const int32_t *pos, 
 // Backward at the points: d loss / d dog scattered into gdog (which must start at zero), and
 // d loss / d thresholds summed into gb[0..2] (double, zeroed first) when gb is given.
 __global__ void k_soft_points_adj(const float *dog, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg,
-                                  int n_neg, float tau, SoftThresh b, float grad_loss, double *gdog, double *gb) {
+                                  int n_neg, float tau, SoftThresh b, float grad_loss, double *gdog,
+                                  double *gb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos + n_neg) return;
   const int32_t *q = i < n_pos ? pos + 3 * i : neg + 3 * (i - n_pos);
@@ -1365,12 +1388,12 @@ void allow_smem(F *fn, size_t bytes) {
 }
 
 // Grid of a column pass: 32 columns x the other coordinate x segments of the line, which is cut while the
-// columns alone leave the chip idle and a segment stays as long as a block's step and a window.
-dim3 col_grid(const SoftGeom &g, int axis, int r, int step, int &seg) {
+// columns alone are fewer than `blocks` blocks, into segments of at least `shortest`.
+dim3 col_grid(const SoftGeom &g, int axis, int shortest, int64_t blocks, int &seg) {
   const int n = axis == 1 ? g.H : g.D, other = axis == 1 ? g.D : g.H;
   const int64_t cols = (int64_t)ceil_div(g.W, 32) * other;
-  const int64_t want = std::max<int64_t>(1, (1216 + cols - 1) / cols);
-  seg = std::min<int64_t>(n, std::max<int64_t>(ceil_div(n, want), std::max(step, 2 * r)));
+  const int64_t want = std::max<int64_t>(1, (blocks + cols - 1) / cols);
+  seg = std::min<int64_t>(n, std::max<int64_t>(ceil_div(n, want), shortest));
   return dim3((unsigned)ceil_div(g.W, 32), (unsigned)other, (unsigned)ceil_div(n, seg));
 }
 
@@ -1406,7 +1429,7 @@ void ext_pass(const SoftRun &R, const void *in, float2 *out, int axis, int r) {
     return;
   }
   int seg;
-  const dim3 grid = col_grid(g, axis, r, nw * kSoftB, seg);
+  const dim3 grid = col_grid(g, axis, std::max(nw * kSoftB, 2 * r), 152 * 8, seg);
   if (axis == 1) {
     allow_smem(k_soft_ext_cols<1, kSoftColWarps[1]>, smem);
     KLAUNCH("k_soft_ext_y", R.st, (k_soft_ext_cols<1, kSoftColWarps[1]><<<grid, dim3(32, nw), smem, R.st>>>(in2, out, g, r, seg)));
@@ -1441,22 +1464,21 @@ void ext_adj(const SoftRun &R, const void *src, const float2 *gout, float *gin, 
     KLAUNCH("k_soft_ext_adj_far", R.st, (k_soft_ext_adj_far<true><<<R.blocks(), 256, 0, R.st>>>(src, gout, gin, g, axis, r, R.N)));
     return;
   }
-  const int nw = kSoftColWarps[axis];
-  const size_t smem = (size_t)ext_cols_rows(r, kSoftB, nw) * 32 * (sizeof(float2) + sizeof(uint16_t));
+  const size_t smem = (size_t)ext_cols_rows(r, kSoftB, 1) * 32 * (sizeof(float2) + sizeof(uint16_t));
   if (2 * r < kSoftB || smem > kSoftMaxSmem) {
     KLAUNCH("k_soft_ext_adj_far", R.st, (k_soft_ext_adj_far<false><<<R.blocks(), 256, 0, R.st>>>(src, gout, gin, g, axis, r, R.N)));
     return;
   }
   int seg;
-  const dim3 grid = col_grid(g, axis, r, nw * kSoftB, seg);
+  const dim3 grid = col_grid(g, axis, std::max(16, r), 152 * 16, seg);   // 16 warps per SM
   const float2 *s2 = static_cast<const float2 *>(src);
   float2 *g2 = reinterpret_cast<float2 *>(gin);
   if (axis == 1) {
-    allow_smem(k_soft_ext_adj_cols<1, kSoftColWarps[1]>, smem);
-    KLAUNCH("k_soft_ext_adj_y", R.st, (k_soft_ext_adj_cols<1, kSoftColWarps[1]><<<grid, dim3(32, nw), smem, R.st>>>(s2, gout, g2, g, r, seg)));
+    allow_smem(k_soft_ext_adj_cols<1>, smem);
+    KLAUNCH("k_soft_ext_adj_y", R.st, (k_soft_ext_adj_cols<1><<<grid, 32, smem, R.st>>>(s2, gout, g2, g, r, seg)));
   } else {
-    allow_smem(k_soft_ext_adj_cols<2, kSoftColWarps[2]>, smem);
-    KLAUNCH("k_soft_ext_adj_z", R.st, (k_soft_ext_adj_cols<2, kSoftColWarps[2]><<<grid, dim3(32, nw), smem, R.st>>>(s2, gout, g2, g, r, seg)));
+    allow_smem(k_soft_ext_adj_cols<2>, smem);
+    KLAUNCH("k_soft_ext_adj_z", R.st, (k_soft_ext_adj_cols<2><<<grid, 32, smem, R.st>>>(s2, gout, g2, g, r, seg)));
   }
 }
 
@@ -1580,8 +1602,8 @@ void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int
   const unsigned grid = (unsigned)std::min<int64_t>(n, 152 * 8);
   KLAUNCH(BWD ? "k_soft_points_local_adj" : "k_soft_points_local", R.st,
           (k_soft_points_local<BWD><<<grid, kSoftPtThreads, smem, R.st>>>(R.slot(S_NORM), R.g, pos, n_pos, neg, n_neg, T,
-                                                                          box, nrm, p.tau, b, grad_loss, scores, acc, gb,
-                                                                          gnorm)));
+                                                                          box, nrm, p.tau, b, grad_loss, scores,
+                                                                          acc, gb, gnorm)));
 }
 
 SoftThresh thresh_of(const hdog_soft_params &p) {
