@@ -1562,6 +1562,18 @@ extern "C" int hdog_soft_backward_kept(const hdog_soft_params *p, const float *d
   return HDOG_OK;
 }
 
+extern "C" int hdog_soft_backward_scaled(const hdog_soft_params *p, const float *d_volume, const int32_t *d_pos,
+                                         int n_pos, const int32_t *d_neg, int n_neg, const float *d_grad_loss,
+                                         int forward_kept, float *d_grad_volume, float *d_grad_sigma,
+                                         float *d_grad_thresh, void *d_workspace, void *stream) {
+  if (!d_grad_loss) return fail(HDOG_ERR_ARG, "hdog_soft_backward_scaled: null loss gradient");
+  const int rc = soft_backward(p, d_volume, d_pos, n_pos, d_neg, n_neg, 0.0f, d_grad_volume, d_grad_sigma,
+                               d_grad_thresh, d_workspace, (cudaStream_t)stream, forward_kept != 0, d_grad_loss);
+  if (rc != HDOG_OK) return fail(rc, "hdog_soft_backward_scaled: bad argument, parameter or sigma");
+  HDOG_CUDA_TRY(cudaGetLastError());
+  return HDOG_OK;
+}
+
 // ------------------------------------------------------------------ after the records
 extern "C" int hdog_records_to_global(const hdog_record *d_records, int64_t n, const hdog_global_params *p,
                                       hdog_global *d_out, void *stream) {

@@ -111,13 +111,14 @@ void launch_scale_merge(const hdog_global *in, int64_t n, const hdog_scalemerge_
                         cudaStream_t s);
 void launch_clf_features(const hdog_record *rec, int64_t n, const hdog_clf_params &p, double *X, cudaStream_t s);
 
-// soft.cu: the differentiable chain (hdog_soft_*); status codes as the C ABI
+// soft.cu: the differentiable chain (hdog_soft_*); status codes as the C ABI.  d_grad_loss, when given,
+// holds the loss's gradient in device memory instead of grad_loss.
 size_t soft_workspace_bytes(const hdog_soft_params &p);
 int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos, int n_pos, const int32_t *neg,
                  int n_neg, float *loss, float *scores, void *work, cudaStream_t st);
 int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *pos, int n_pos, const int32_t *neg,
                   int n_neg, float grad_loss, float *grad_vol, float *grad_sigma, float *grad_thresh, void *work,
-                  cudaStream_t st, bool forward_kept = false);
+                  cudaStream_t st, bool forward_kept = false, const float *d_grad_loss = nullptr);
 
 // Zero `bytes` (a multiple of 4) of device memory on stream s with a kernel.
 void zero_async(void *p, size_t bytes, cudaStream_t s);

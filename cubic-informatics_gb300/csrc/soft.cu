@@ -935,10 +935,11 @@ __global__ void k_soft_points(const float *dog, SoftGeom g, const int32_t *pos, 
 // Backward at the points: d loss / d dog scattered into gdog (which must start at zero), and
 // d loss / d thresholds summed into gb[0..2] (double, zeroed first) when gb is given.
 __global__ void k_soft_points_adj(const float *dog, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg,
-                                  int n_neg, float tau, SoftThresh b, float grad_loss, double *gdog,
+                                  int n_neg, float tau, SoftThresh b, float grad_loss, const float *d_grad_loss, double *gdog,
                                   double *gb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos + n_neg) return;
+  if (d_grad_loss) grad_loss = __ldg(d_grad_loss);
   const int32_t *q = i < n_pos ? pos + 3 * i : neg + 3 * (i - n_pos);
   const SoftPoint p{q[2], q[1], q[0]};
   float h[6], ds[6], db[3];
@@ -1068,12 +1069,13 @@ template <bool BWD>
 __global__ void __launch_bounds__(kSoftPtThreads, 4)
     k_soft_points_local(const float *norm, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
                         const __grid_constant__ SoftTapSet T, SoftBox box, float nrm, float tau, SoftThresh b,
-                        float grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+                        float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
   extern __shared__ float sm[];
   __shared__ float fv[2][4][kSoftStencil];   // per scale: plain, d/dz, d/dy, d/dx
   __shared__ float cube[125], coef[125];     // DoG and d loss / d DoG around the point (0 off the stencil)
   __shared__ float hs[6], ds[6];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (d_grad_loss) grad_loss = __ldg(d_grad_loss);
   const int ex = box.e(0), ey = box.e(1), ez = box.e(2), L = box.lines();
   float *tile = sm;
   float *xl = tile + box.tile();             // [scale][plain, derivative][lines][5]
@@ -1583,7 +1585,7 @@ bool points_local(const SoftRun &R, int64_t n, SoftBox &box) {
 
 template <bool BWD>
 void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
-                   float grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+                   float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
   const hdog_soft_params &p = R.p;
   const int64_t n = (int64_t)n_pos + n_neg;
   if (n == 0) return;
@@ -1602,7 +1604,7 @@ void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int
   const unsigned grid = (unsigned)std::min<int64_t>(n, 152 * 8);
   KLAUNCH(BWD ? "k_soft_points_local_adj" : "k_soft_points_local", R.st,
           (k_soft_points_local<BWD><<<grid, kSoftPtThreads, smem, R.st>>>(R.slot(S_NORM), R.g, pos, n_pos, neg, n_neg, T,
-                                                                          box, nrm, p.tau, b, grad_loss, scores,
+                                                                          box, nrm, p.tau, b, grad_loss, d_grad_loss, scores,
                                                                           acc, gb, gnorm)));
 }
 
@@ -1642,7 +1644,7 @@ int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos
   const bool local = points_local(R, (int64_t)n_pos + n_neg, box);
   forward_chain(R, vol, !local);
   if (local)
-    points_launch<false>(R, box, pos, n_pos, neg, n_neg, 0.0f, scores, R.acc, nullptr, nullptr);
+    points_launch<false>(R, box, pos, n_pos, neg, n_neg, 0.0f, nullptr, scores, R.acc, nullptr, nullptr);
   else if (n_pos + n_neg > 0)
     KLAUNCH("k_soft_points", st, (k_soft_points<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
                                      R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), scores,
@@ -1653,7 +1655,7 @@ int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos
 
 int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *pos, int n_pos, const int32_t *neg,
                   int n_neg, float grad_loss, float *grad_vol, float *grad_sigma, float *grad_thresh, void *work,
-                  cudaStream_t st, bool forward_kept) {
+                  cudaStream_t st, bool forward_kept, const float *d_grad_loss) {
   const int rc = check_params(p, vol, pos, n_pos, neg, n_neg, work);
   if (rc != HDOG_OK) return rc;
   SoftRun R{*p, SoftGeom{p->width, p->height, p->depth}, (int64_t)p->width * p->height * p->depth, st,
@@ -1675,7 +1677,7 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
   if (local) {
     float *gnorm = grad_vol ? R.slot(S_GB) : nullptr;
     if (gnorm) cudaMemsetAsync(gnorm, 0, R.N * sizeof(float), st);
-    points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, nullptr, grad_sigma ? R.acc : nullptr,
+    points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, d_grad_loss, nullptr, grad_sigma ? R.acc : nullptr,
                         grad_thresh ? gb : nullptr, gnorm);
   } else {
     // a forward call with fewer points may have left the DoG slot empty
@@ -1685,7 +1687,7 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
     if (n_pos + n_neg > 0)
       KLAUNCH("k_soft_points_adj", st, (k_soft_points_adj<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
                                            R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), grad_loss,
-                                           gsum, gb)));
+                                           d_grad_loss, gsum, gb)));
     KLAUNCH("k_soft_gdog", st, (k_soft_gdog<<<nb, 256, 0, st>>>(gsum, gdog, R.N)));
   }
   if (grad_thresh) k_soft_to_float<<<1, 32, 0, st>>>(gb, grad_thresh, 3);

@@ -27,9 +27,9 @@ from . import check, hdog_soft_params, lib
 def _params(vol, sigma, thresh, cfg):
     rxy, rz, min_intensity, tau, gamma = cfg
     D, H, W = vol.shape
-    s = [float(v) for v in sigma.detach().cpu().reshape(-1)]
+    s = sigma.detach().reshape(-1).tolist()
     assert len(s) == 6, "sigma holds 6 values: x1, y1, z1, x2, y2, z2"
-    b = [float(v) for v in thresh.detach().cpu().reshape(-1)]
+    b = thresh.detach().reshape(-1).tolist()
     assert len(b) == 3, "thresh holds 3 values: b0, b1, b2"
     return hdog_soft_params(int(W), int(H), int(D), int(rxy), int(rz), float(min_intensity), (ctypes.c_float * 6)(*s),
                             float(gamma), float(tau), (ctypes.c_float * 3)(*b))
@@ -56,7 +56,7 @@ class SoftLoss(torch.autograd.Function):
         check(lib().hdog_soft_forward(ctypes.byref(p), _ptr(vol), _ptr(pos), pos.shape[0], _ptr(neg), neg.shape[0],
                                       _ptr(loss), None, _ptr(ws), stream))
         ctx.save_for_backward(vol, sigma, thresh, pos, neg)
-        ctx.cfg = cfg
+        ctx.params = p               # sigma and thresh as the forward read them
         # the saved tensors' version check already refuses a volume changed in place since
         ctx.kept = ws if keep else None
         return loss[0]
@@ -64,20 +64,28 @@ class SoftLoss(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         vol, sigma, thresh, pos, neg = ctx.saved_tensors
-        p = _params(vol, sigma, thresh, ctx.cfg)
+        p = ctx.params
         want_vol, want_sigma, want_thresh = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
         gv = torch.empty_like(vol) if want_vol else None     # every element is written
-        gs = torch.empty(6, dtype=torch.float32, device=vol.device) if want_sigma else None
-        gb = torch.empty(3, dtype=torch.float32, device=vol.device) if want_thresh else None
-        stream = ctypes.c_void_p(torch.cuda.current_stream(vol.device).cuda_stream)
-        if ctx.kept is not None:
-            ws = ctx.kept
-            fn = lib().hdog_soft_backward_kept
+        together = want_sigma and want_thresh and sigma.device == thresh.device != vol.device
+        if together:
+            small = torch.empty(9, dtype=torch.float32, device=vol.device)
+            gs, gb = small[:6], small[6:]
         else:
+            gs = torch.empty(6, dtype=torch.float32, device=vol.device) if want_sigma else None
+            gb = torch.empty(3, dtype=torch.float32, device=vol.device) if want_thresh else None
+        stream = ctypes.c_void_p(torch.cuda.current_stream(vol.device).cuda_stream)
+        ws = ctx.kept
+        if ws is None:
             ws = torch.empty(lib().hdog_soft_workspace_bytes(ctypes.byref(p)), dtype=torch.uint8, device=vol.device)
-            fn = lib().hdog_soft_backward
-        check(fn(ctypes.byref(p), _ptr(vol), _ptr(pos), pos.shape[0], _ptr(neg), neg.shape[0], float(grad), _ptr(gv),
-                 _ptr(gs), _ptr(gb), _ptr(ws), stream))
+        # the loss's gradient stays on the device: reading it here would wait for the forward
+        scale = grad.detach().to(device=vol.device, dtype=torch.float32).reshape(1).contiguous()
+        check(lib().hdog_soft_backward_scaled(ctypes.byref(p), _ptr(vol), _ptr(pos), pos.shape[0], _ptr(neg), neg.shape[0],
+                                              _ptr(scale), int(ctx.kept is not None), _ptr(gv), _ptr(gs), _ptr(gb),
+                                              _ptr(ws), stream))
+        if together:
+            host = small.to(sigma.device)            # one copy, and one wait for it, for both
+            gs, gb = host[:6].clone(), host[6:].clone()
         if gs is not None:
             gs = gs.to(device=sigma.device, dtype=sigma.dtype).reshape(sigma.shape)
         if gb is not None:

@@ -337,6 +337,14 @@ int hdog_soft_backward_kept(const hdog_soft_params *p, const float *d_volume, co
                             const int32_t *d_neg, int n_neg, float grad_loss, float *d_grad_volume,
                             float *d_grad_sigma, float *d_grad_thresh, void *d_workspace, void *stream);
 
+/* Either of the two (forward_kept 0 or 1) with the loss's gradient in device memory (one float),
+   read on `stream`: a caller whose gradient comes from earlier work on the stream need not wait
+   for it on the host. */
+int hdog_soft_backward_scaled(const hdog_soft_params *p, const float *d_volume, const int32_t *d_pos, int n_pos,
+                              const int32_t *d_neg, int n_neg, const float *d_grad_loss, int forward_kept,
+                              float *d_grad_volume, float *d_grad_sigma, float *d_grad_thresh, void *d_workspace,
+                              void *stream);
+
 /* ---- context options ---- */
 enum {
   HDOG_OPT_FUSED_SWEEP = 1,  /* 1 (default): DoG, Hessian and the PD test in one z-sweep kernel
