@@ -211,6 +211,7 @@ struct hdog_ctx {
   int max_sub = 0;
   int W = 0, H = 0, D = 0;
   int64_t nvox = 0;        // W*H*D
+  int P = 0;               // row pitch of norm and dog: W rounded up to 4 (TMA rows start on 16 bytes)
   int64_t reg_cap = 0;     // region slots per substack (background included)
   int64_t nblk = 0;        // per-substack block slots (voxel blocks and region blocks)
   int64_t nchk = 0;        // per-substack chunk slots
@@ -229,7 +230,7 @@ struct hdog_ctx {
   size_t arena_bytes = 0;
   uint16_t *img = nullptr;       // [max_sub * nvox] staging of host substacks
   float2 *fa = nullptr, *fb = nullptr;   // [max_sub * nvox] temps (min/max, box, DoG)
-  float *norm = nullptr, *dog = nullptr;
+  float *norm = nullptr, *dog = nullptr;   // [max_sub * P*H*D]
   uint8_t *mask = nullptr;
   int32_t *labels = nullptr;
   uint32_t *root_bits = nullptr, *blk_counts = nullptr, *blk_offsets = nullptr, *chunk = nullptr;
@@ -300,6 +301,7 @@ struct Layout {
   }
 };
 
+static int pitch_of(int width) { return (width + 3) & ~3; }
 static int64_t edge_capacity(int64_t nvox) { return nvox / 8 + 1024; }
 static int64_t fg_capacity(int64_t nvox) { return nvox / 8 + 1024; }
 
@@ -314,8 +316,9 @@ static void plan(const hdog_params *p, int max_sub, int64_t &nvox, int64_t &reg_
   L.add(S * nvox * sizeof(uint16_t));        // 0 img
   L.add(S * nvox * sizeof(float2));          // 1 fa
   L.add(S * nvox * sizeof(float2));          // 2 fb
-  L.add(S * nvox * sizeof(float));           // 3 norm
-  L.add(S * nvox * sizeof(float));           // 4 dog
+  const int64_t pvox = (int64_t)pitch_of(p->width) * p->height * p->depth;
+  L.add(S * pvox * sizeof(float));           // 3 norm
+  L.add(S * pvox * sizeof(float));           // 4 dog
   L.add(S * nvox * sizeof(uint8_t));         // 5 mask
   L.add(S * nvox * sizeof(int32_t));         // 6 labels
   L.add(S * nblk * (kScanBlock / 32) * sizeof(uint32_t));   // 7 root bits
@@ -393,6 +396,7 @@ extern "C" int hdog_ctx_create(const hdog_params *p, int max_substacks, hdog_ctx
   c->dev = p->dev_id;
   c->max_sub = max_substacks;
   c->W = p->width; c->H = p->height; c->D = p->depth;
+  c->P = pitch_of(p->width);
   Layout L;
   plan(p, max_substacks, c->nvox, c->reg_cap, c->nblk, c->nchk, L);
   c->slots = (int64_t)max_substacks * c->reg_cap;
@@ -479,6 +483,8 @@ static void set_sub(hdog_ctx *c, int s, const uint16_t *src, int depth_valid, in
   S.z0 = z0;
   S.margin = c->margin;
   S.vox = (int64_t)s * c->nvox;
+  S.P = c->P;
+  S.pvox = (int64_t)s * c->P * c->H * c->D;
   S.reg = (int64_t)s * c->reg_cap;
   S.reg_cap = c->reg_cap;
   S.blk = (int64_t)s * c->nblk;
@@ -571,9 +577,9 @@ static void enqueue_normalize(hdog_ctx *c, int nsub, float *out_norm, cudaStream
 }
 
 // DoG volume: the radius-specialised z-sweep where it applies (bit-identical), else the
-// three separate passes.
-static void enqueue_dog(hdog_ctx *c, int nsub, const float *norm, float *dog, cudaStream_t st) {
-  if (c->use_sweep && launch_dog_sweep(c->d_subs, nsub, c->W, c->H, c->D, c->taps, norm, dog, c->status, c->max_smem, st))
+// three separate passes.  P: the volumes' row pitch, the descriptors'.
+static void enqueue_dog(hdog_ctx *c, int nsub, int P, const float *norm, float *dog, cudaStream_t st) {
+  if (c->use_sweep && launch_dog_sweep(c->d_subs, nsub, c->W, P, c->H, c->D, c->taps, norm, dog, c->status, c->max_smem, st))
     return;
   launch_dog(c->d_subs, nsub, c->W, c->H, c->D, (int64_t)c->H * c->D, c->taps, norm, c->fa, c->fb, dog, st);
 }
@@ -585,10 +591,10 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
   // entry beside the list (fb is free after the normalization)
   int32_t *fg_root = reinterpret_cast<int32_t *>(c->fb);
   if (fused) {
-    launch_dog_hess(c->d_subs, nsub, c->W, c->H, c->D, c->taps, c->norm, c->dog, c->mask, c->fg, fg_root,
-                    c->fg_count, c->status, c->shape, c->qctr, st);
+    launch_dog_hess(c->d_subs, nsub, c->W, c->P, c->H, c->D, c->taps, c->norm, c->fa, c->fb, c->dog, c->mask, c->fg,
+                    fg_root, c->fg_count, c->status, c->shape, c->qctr, c->max_smem, st);
   } else {
-    enqueue_dog(c, nsub, c->norm, c->dog, st);
+    enqueue_dog(c, nsub, c->P, c->norm, c->dog, st);
     launch_hessian_pd(c->d_subs, nsub, c->W, c->H, c->D, c->dog, c->mask, nullptr, st);
   }
   launch_ccl(c->d_subs, nsub, c->W, c->H, c->D, c->nvox, c->mask, c->labels, c->edges, c->edge_count, c->root_bits,
@@ -611,7 +617,7 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
 // the separate passes.
 static bool fused_ok(hdog_ctx *c) {
   return c->use_sweep && c->W <= 65535 && c->H <= 65535 && c->D <= 65535 &&
-         sweep_supported(c->taps, c->W, c->max_smem);
+         sweep_supported(c->max_smem);
 }
 
 // Reads record / region / foreground counts and the status word back (one sync).
@@ -791,6 +797,7 @@ static int copy_out(const RecordBuf &v, hdog_record *out, int64_t cap, int64_t *
 // ------------------------------------------------------------------ stage entry points
 static int single_sub(hdog_ctx *c, const uint16_t *src, cudaStream_t st) {
   set_sub(c, 0, src, c->D, 0);
+  c->h_subs[0].P = c->W;   // the caller's volumes have no padding
   return upload_subs(c, 1, st);
 }
 
@@ -827,7 +834,7 @@ extern "C" int hdog_dog(hdog_ctx *c, const float *d_norm, float *d_dog, void *st
   cudaStream_t st = (cudaStream_t)stream;
   TRY(single_sub(c, nullptr, st));
   zero_async(c->status, sizeof(int), st);
-  enqueue_dog(c, 1, d_norm, d_dog, st);
+  enqueue_dog(c, 1, c->W, d_norm, d_dog, st);
   HDOG_CUDA_TRY(cudaGetLastError());
   // the sweep's bounded TMA waits report through the status word
   int status = 0;

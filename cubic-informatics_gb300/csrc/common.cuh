@@ -100,23 +100,23 @@ __device__ __forceinline__ bool pd_test(float xx, float xy, float xz, float yy, 
 
 // The six Hessian elements at voxel (x, y, z) straight from global memory, with the
 // same zero-halo rule as the tiled kernel: f outside the volume is 0 and a first
-// derivative at a position outside the volume is 0.  Order xx, xy, xz, yy, yz, zz.
-__device__ __forceinline__ float dog_ld(const float *f, int W, int H, int D, int x, int y, int z) {
-  return (x >= 0 && y >= 0 && z >= 0 && x < W && y < H && z < D) ? __ldg(f + ((int64_t)z * H + y) * W + x) : 0.0f;
+// derivative at a position outside the volume is 0.  P: row pitch.  Order xx, xy, xz, yy, yz, zz.
+__device__ __forceinline__ float dog_ld(const float *f, int W, int P, int H, int D, int x, int y, int z) {
+  return (x >= 0 && y >= 0 && z >= 0 && x < W && y < H && z < D) ? __ldg(f + ((int64_t)z * H + y) * P + x) : 0.0f;
 }
-__device__ __forceinline__ float grad1(const float *f, int W, int H, int D, int x, int y, int z, int dx,
+__device__ __forceinline__ float grad1(const float *f, int W, int P, int H, int D, int x, int y, int z, int dx,
                                        int dy, int dz) {
   if (x < 0 || y < 0 || z < 0 || x >= W || y >= H || z >= D) return 0.0f;
-  return cdiff(dog_ld(f, W, H, D, x + dx, y + dy, z + dz), dog_ld(f, W, H, D, x - dx, y - dy, z - dz));
+  return cdiff(dog_ld(f, W, P, H, D, x + dx, y + dy, z + dz), dog_ld(f, W, P, H, D, x - dx, y - dy, z - dz));
 }
-__device__ __forceinline__ void hessian_at(const float *f, int W, int H, int D, int x, int y, int z,
+__device__ __forceinline__ void hessian_at(const float *f, int W, int P, int H, int D, int x, int y, int z,
                                            float h[6]) {
-  h[0] = cdiff(grad1(f, W, H, D, x + 1, y, z, 1, 0, 0), grad1(f, W, H, D, x - 1, y, z, 1, 0, 0));
-  h[1] = cdiff(grad1(f, W, H, D, x, y + 1, z, 1, 0, 0), grad1(f, W, H, D, x, y - 1, z, 1, 0, 0));
-  h[2] = cdiff(grad1(f, W, H, D, x, y, z + 1, 1, 0, 0), grad1(f, W, H, D, x, y, z - 1, 1, 0, 0));
-  h[3] = cdiff(grad1(f, W, H, D, x, y + 1, z, 0, 1, 0), grad1(f, W, H, D, x, y - 1, z, 0, 1, 0));
-  h[4] = cdiff(grad1(f, W, H, D, x, y, z + 1, 0, 1, 0), grad1(f, W, H, D, x, y, z - 1, 0, 1, 0));
-  h[5] = cdiff(grad1(f, W, H, D, x, y, z + 1, 0, 0, 1), grad1(f, W, H, D, x, y, z - 1, 0, 0, 1));
+  h[0] = cdiff(grad1(f, W, P, H, D, x + 1, y, z, 1, 0, 0), grad1(f, W, P, H, D, x - 1, y, z, 1, 0, 0));
+  h[1] = cdiff(grad1(f, W, P, H, D, x, y + 1, z, 1, 0, 0), grad1(f, W, P, H, D, x, y - 1, z, 1, 0, 0));
+  h[2] = cdiff(grad1(f, W, P, H, D, x, y, z + 1, 1, 0, 0), grad1(f, W, P, H, D, x, y, z - 1, 1, 0, 0));
+  h[3] = cdiff(grad1(f, W, P, H, D, x, y + 1, z, 0, 1, 0), grad1(f, W, P, H, D, x, y - 1, z, 0, 1, 0));
+  h[4] = cdiff(grad1(f, W, P, H, D, x, y, z + 1, 0, 1, 0), grad1(f, W, P, H, D, x, y, z - 1, 0, 1, 0));
+  h[5] = cdiff(grad1(f, W, P, H, D, x, y, z + 1, 0, 0, 1), grad1(f, W, P, H, D, x, y, z - 1, 0, 0, 1));
 }
 
 // Region float sums accumulate as 64-bit fixed point with 36 fractional bits: integer

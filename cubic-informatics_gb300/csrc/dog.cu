@@ -31,7 +31,7 @@ __global__ void k_conv_x(const Sub *subs, const __grid_constant__ DogTaps T, con
   const int x0 = (int)(bid % segs) * kConvSeg;
   const int ra = T.r[0], rb = T.r[2], rm = max(ra, rb);
   const int n0 = kConvSeg + 2 * rm;
-  const float *line = in + S.vox + row * S.W;
+  const float *line = in + S.pvox + row * S.P;
   for (int t = threadIdx.x; t < n0; t += blockDim.x) {
     const int x = x0 - rm + t;
     scx[t] = (x >= 0 && x < S.W) ? line[x] : 0.0f;
@@ -118,6 +118,8 @@ __global__ void k_conv_z_dog(const Sub *subs, const __grid_constant__ DogTaps T,
   if (p >= plane) return;
   const int D = S.D;
   const float2 *col = in + S.vox + p;
+  float *o = dog + S.pvox + (S.P == S.W ? p : p + (int64_t)((uint32_t)p / (uint32_t)S.W) * (S.P - S.W));
+  const int64_t pplane = (int64_t)S.P * S.H;
   for (int z0 = 0; z0 < D; z0 += kConvK) {
     float2 acc[kConvK];
     conv_chain(z0, T.k[1], T.r[1], T.k[3], T.r[3],
@@ -125,7 +127,7 @@ __global__ void k_conv_z_dog(const Sub *subs, const __grid_constant__ DogTaps T,
 #pragma unroll
     for (int k = 0; k < kConvK; k++) {
       const int z = z0 + k;
-      if (z < D) dog[S.vox + z * plane + p] = __fmul_rn(__fsub_rn(acc[k].x, acc[k].y), T.normalizer);
+      if (z < D) o[z * pplane] = __fmul_rn(__fsub_rn(acc[k].x, acc[k].y), T.normalizer);
     }
   }
 }
@@ -150,12 +152,13 @@ __global__ void __launch_bounds__(256) k_hessian_pd(const Sub *subs, const float
   const int x0 = bx * kHX, y0 = by * kHY, z0 = bz * kHZ;
   const int W = S.W, H = S.H, D = S.D;
   const int64_t plane = (int64_t)W * H;
-  const float *f = dog + S.vox;
+  const float *f = dog + S.pvox;
+  const int64_t pplane = (int64_t)S.P * H;
   const int tid = threadIdx.x + threadIdx.y * blockDim.x, nt = blockDim.x * blockDim.y;
   for (int i = tid; i < kDZ * kDY * kDX; i += nt) {
     const int lx = i % kDX, ly = (i / kDX) % kDY, lz = i / (kDX * kDY);
     const int x = x0 - 2 + lx, y = y0 - 2 + ly, z = z0 - 2 + lz;
-    sd[i] = (x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D) ? f[z * plane + (int64_t)y * W + x] : 0.0f;
+    sd[i] = (x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D) ? f[z * pplane + (int64_t)y * S.P + x] : 0.0f;
   }
   __syncthreads();
   for (int i = tid; i < kGZ * kGY * kGX; i += nt) {

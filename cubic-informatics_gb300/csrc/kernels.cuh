@@ -14,6 +14,9 @@ struct Sub {
   int z0;                 // global z of slice 0, added to record centroid_z
   int margin;             // depth margin m (records keep m <= cz < depth_valid - m)
   int64_t vox;            // voxel offset of this substack in the batch volume arrays
+  int P;                  // row pitch of the normalized and the DoG volume (TMA wants rows on 16
+                          // bytes: W rounded up to 4 inside the chain; W in callers' volumes)
+  int64_t pvox;           // this substack's offset in those two
   int64_t reg;            // offset of its region slots in the region arrays
   int64_t reg_cap;        // number of region slots (background included)
   int64_t blk;            // offset of its per-block slots in block scratch arrays
@@ -99,9 +102,7 @@ void launch_dog(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d, in
 void launch_hessian_pd(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d,
                        const float *dog, uint8_t *mask, float *hess6, cudaStream_t s);
 // ---- sweep.cu ----
-constexpr int kMaxSweepRxy = 12;
-size_t sweep_smem_bytes(int rxy);
-bool sweep_supported(const DogTaps &T, int W, int max_smem);
+bool sweep_supported(int max_smem);
 // DoG volume by the radius-specialised z-sweep; false (nothing launched) when the radii
 // have no instantiation or the buffers do not suit TMA.
 // records.cu: per-record steps after the records (host-side NumPy in the reference)
@@ -124,14 +125,14 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
 void zero_async(void *p, size_t bytes, cudaStream_t s);
 void pack_fg_counts_async(const unsigned long long *fg_count, int nsub, unsigned long long *packed, cudaStream_t s);
 
-bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int H, int D, const DogTaps &T, const float *norm,
+bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
                       float *dog, int *d_status, int max_smem, cudaStream_t s);
-// DoG + Hessian + PD: the radius-specialised pair (norm -> dog -> mask + list) when the tap
-// radii have an instantiation, else the generic fused sweep (dog untouched).
-// ls / qctr (two device counters): the launch shape of the radius-specialised sweeps.
-int launch_dog_hess(const Sub *d_subs, int nsub, int W, int H, int D, const DogTaps &T, const float *norm,
-                    float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count,
-                    int *d_status, const LaunchShape &ls, unsigned *qctr, cudaStream_t s);
+// DoG + Hessian + PD: norm -> dog by the radius-specialised sweep, or by the separate passes (temporaries
+// fa, fb) where the tap radii have no instantiation, then dog -> mask + list by the Hessian sweep.
+// ls / qctr (two device counters): the launch shape of the sweeps.
+int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
+                    float2 *fa, float2 *fb, float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count,
+                    int *d_status, const LaunchShape &ls, unsigned *qctr, int max_smem, cudaStream_t s);
 // ---- ccl.cu ----
 // Segments of a per-substack scan: substack s scans len[s] counts starting at off[s];
 // chk[s] is its offset in the chunk-sum scratch (one slot per 1024 counts).

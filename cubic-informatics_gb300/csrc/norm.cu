@@ -660,6 +660,11 @@ __global__ void __launch_bounds__(128, 6) k_box_y_t(const Sub *subs, const float
     if (y0 + k < H) *o = mul2(acc[k], make_float2(inv, inv));
 }
 
+// Where plane position p of slice 0 lies in the normalized volume, whose rows may be padded.
+__device__ __forceinline__ int64_t norm_at(const Sub &S, int64_t p) {
+  return S.pvox + (S.P == S.W ? p : p + (int64_t)((uint32_t)p / (uint32_t)S.W) * (S.P - S.W));
+}
+
 // z pass of the box mean fused with Normalize3DKernel (NormalizeFilter.cu:571-586).
 constexpr int kBoxZK = 8;
 
@@ -671,6 +676,8 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
   if (p >= plane) return;
   const float2 *col = in + S.vox + p;
   const int D = S.D, L = 2 * rz + 1;
+  float *nout = norm + norm_at(S, p);
+  const int64_t pplane = (int64_t)S.P * S.H;
   const float inv = 1.0f / (float)L;
   for (int z0 = 0; z0 < D; z0 += kBoxZK) {
     float2 acc[kBoxZK];
@@ -681,7 +688,7 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
       if (z < D) {
         const float2 el = mul2(acc[k], make_float2(inv, inv));
         const float v = z < S.depth_valid ? (float)__ldg(S.src + z * plane + p) : 0.0f;
-        norm[S.vox + z * plane + p] = (v >= min_intensity) ? (v - el.x) / (el.y - el.x) : 0.0f;
+        nout[z * pplane] = (v >= min_intensity) ? (v - el.x) / (el.y - el.x) : 0.0f;
         if (ero_l) {
           ero_l[S.vox + z * plane + p] = el.x;
           dil_l[S.vox + z * plane + p] = el.y;
@@ -716,6 +723,8 @@ __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min
     v[k] = z < S.depth_valid ? (float)__ldg(S.src + z * plane + p) : 0.0f;
   }
   const float inv = 1.0f / (float)L;
+  float *nout = norm + norm_at(S, p);
+  const int64_t pplane = (int64_t)S.P * S.H;
 #pragma unroll
   for (int k = 0; k < kBoxZK; k++) {
     float2 acc = make_float2(0.f, 0.f);
@@ -724,7 +733,7 @@ __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min
     const int z = z0 + k;
     if (z < D) {
       const float2 el = mul2(acc, make_float2(inv, inv));
-      norm[S.vox + z * plane + p] = (v[k] >= min_intensity) ? (v[k] - el.x) / (el.y - el.x) : 0.0f;
+      nout[z * pplane] = (v[k] >= min_intensity) ? (v[k] - el.x) / (el.y - el.x) : 0.0f;
       if (PARTS) {
         ero_l[S.vox + z * plane + p] = el.x;
         dil_l[S.vox + z * plane + p] = el.y;
@@ -741,7 +750,7 @@ __global__ void k_copy_norm(const Sub *subs, float min_intensity, float *norm) {
   if (i >= n) return;
   const int z = (int)(i / plane);
   const float v = z < S.depth_valid ? (float)S.src[i] : 0.0f;
-  norm[S.vox + i] = (v >= min_intensity) ? v : 0.0f;
+  norm[norm_at(S, i - z * plane) + (int64_t)z * S.P * S.H] = (v >= min_intensity) ? v : 0.0f;
 }
 
 // ---------------------------------------------------------------- launchers

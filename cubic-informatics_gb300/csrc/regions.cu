@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) k_accumulate(const Sub *subs, const uint8
       run_reset(a, r);
     }
     const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((int64_t)W * H));
-    const float v = norm[S.vox + i];
+    const float v = norm[S.pvox + ((int64_t)z * H + y) * S.P + x];
     a.count++;
     a.max_ord = max(a.max_ord, f2ord(v));
     a.norm += to_fix(v);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) k_accumulate(const Sub *subs, const uint8
     a.y += (unsigned long long)y;
     a.z += (unsigned long long)z;
     float h[6];
-    hessian_at(dog + S.vox, W, H, S.D, x, y, z, h);
+    hessian_at(dog + S.pvox, W, S.P, H, S.D, x, y, z, h);
 #pragma unroll
     for (int q = 0; q < 6; q++) a.h[q] += to_fix(h[q]);
   }
