@@ -229,7 +229,7 @@ struct hdog_ctx {
   void *arena = nullptr;
   size_t arena_bytes = 0;
   uint16_t *img = nullptr;       // [max_sub * nvox] staging of host substacks
-  float2 *fa = nullptr, *fb = nullptr;   // [max_sub * nvox] temps (min/max, box, DoG)
+  float2 *fa = nullptr, *fb = nullptr;   // [max_sub * P*H*D] temps (min/max and box: rows of W; DoG: rows of P)
   float *norm = nullptr, *dog = nullptr;   // [max_sub * P*H*D]
   uint8_t *mask = nullptr;
   int32_t *labels = nullptr;
@@ -314,9 +314,9 @@ static void plan(const hdog_params *p, int max_sub, int64_t &nvox, int64_t &reg_
   nchk = (nblk + 1023) / 1024 + 1;
   const int64_t S = max_sub, slots = S * reg_cap;
   L.add(S * nvox * sizeof(uint16_t));        // 0 img
-  L.add(S * nvox * sizeof(float2));          // 1 fa
-  L.add(S * nvox * sizeof(float2));          // 2 fb
   const int64_t pvox = (int64_t)pitch_of(p->width) * p->height * p->depth;
+  L.add(S * pvox * sizeof(float2));          // 1 fa
+  L.add(S * pvox * sizeof(float2));          // 2 fb
   L.add(S * pvox * sizeof(float));           // 3 norm
   L.add(S * pvox * sizeof(float));           // 4 dog
   L.add(S * nvox * sizeof(uint8_t));         // 5 mask
@@ -572,7 +572,7 @@ static void enqueue_normalize(hdog_ctx *c, int nsub, float *out_norm, cudaStream
   // min/max (exact) z -> y -> x, box means x -> y -> z; packed u32 in fb's halves
   uint32_t *ma = reinterpret_cast<uint32_t *>(c->fb);
   uint32_t *mb = ma + (int64_t)c->max_sub * c->nvox;
-  launch_normalize(c->d_subs, nsub, c->W, c->H, c->D, p.radius_norm_xy, p.radius_norm_z, (float)p.min_intensity,
+  launch_normalize(c->d_subs, nsub, c->W, c->h_subs[0].P, c->H, c->D, p.radius_norm_xy, p.radius_norm_z, (float)p.min_intensity,
                    srcs_aligned8(c, nsub), ma, mb, c->fa, c->fb, out_norm, st, ero_l, dil_l);
 }
 
@@ -581,7 +581,7 @@ static void enqueue_normalize(hdog_ctx *c, int nsub, float *out_norm, cudaStream
 static void enqueue_dog(hdog_ctx *c, int nsub, int P, const float *norm, float *dog, cudaStream_t st) {
   if (c->use_sweep && launch_dog_sweep(c->d_subs, nsub, c->W, P, c->H, c->D, c->taps, norm, dog, c->status, c->max_smem, st))
     return;
-  launch_dog(c->d_subs, nsub, c->W, c->H, c->D, (int64_t)c->H * c->D, c->taps, norm, c->fa, c->fb, dog, st);
+  launch_dog(c->d_subs, nsub, c->W, P, c->H, c->D, (int64_t)c->H * c->D, c->taps, norm, c->fa, c->fb, dog, st);
 }
 
 // The chain after normalization: DoG + Hessian (fused sweep or separate passes), CCL,

@@ -88,7 +88,8 @@ inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) /
 // ma, mb: packed u32 volumes; fa, fb: float2 volumes (ma/mb may alias fb's two halves).
 // src_aligned8: every substack's src is 8-byte aligned (four-column z loads).
 // ero_l, dil_l (optional): also write the box means of the min and the max.
-void launch_normalize(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, int rz, float min_intensity,
+// P: row pitch of norm (W with ero_l / dil_l).
+void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, int rxy, int rz, float min_intensity,
                       bool src_aligned8, uint32_t *ma, uint32_t *mb, float2 *fa, float2 *fb, float *norm,
                       cudaStream_t s, float *ero_l = nullptr, float *dil_l = nullptr);
 void launch_copy_norm(const Sub *d_subs, int nsub, int64_t max_n, float min_intensity,
@@ -97,7 +98,8 @@ void launch_copy_norm(const Sub *d_subs, int nsub, int64_t max_n, float min_inte
 void launch_erosion(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, int rz, bool src_aligned8,
                     uint32_t *tmp, uint16_t *dst, cudaStream_t s);
 // ---- dog.cu ----
-void launch_dog(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d, int64_t max_rows,
+// t0, t1: temporaries with the rows of norm and dog (pitch)
+void launch_dog(const Sub *d_subs, int nsub, int max_w, int pitch, int max_h, int max_d, int64_t max_rows,
                 const DogTaps &T, const float *norm, float2 *t0, float2 *t1, float *dog, cudaStream_t s);
 void launch_hessian_pd(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d,
                        const float *dog, uint8_t *mask, float *hess6, cudaStream_t s);

@@ -660,9 +660,10 @@ __global__ void __launch_bounds__(128, 6) k_box_y_t(const Sub *subs, const float
     if (y0 + k < H) *o = mul2(acc[k], make_float2(inv, inv));
 }
 
-// Where plane position p of slice 0 lies in the normalized volume, whose rows may be padded.
+// Where plane position p of slice 0 lies in the normalized volume, whose rows may be padded (PAD).
+template <bool PAD>
 __device__ __forceinline__ int64_t norm_at(const Sub &S, int64_t p) {
-  return S.pvox + (S.P == S.W ? p : p + (int64_t)((uint32_t)p / (uint32_t)S.W) * (S.P - S.W));
+  return PAD ? S.pvox + p + (int64_t)((uint32_t)p / (uint32_t)S.W) * (S.P - S.W) : S.vox + p;
 }
 
 // z pass of the box mean fused with Normalize3DKernel (NormalizeFilter.cu:571-586).
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
   if (p >= plane) return;
   const float2 *col = in + S.vox + p;
   const int D = S.D, L = 2 * rz + 1;
-  float *nout = norm + norm_at(S, p);
+  float *nout = norm + norm_at<true>(S, p);
   const int64_t pplane = (int64_t)S.P * S.H;
   const float inv = 1.0f / (float)L;
   for (int z0 = 0; z0 < D; z0 += kBoxZK) {
@@ -702,7 +703,7 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
 // slices), every window input loaded before the first add so that all loads of a thread
 // are in flight together; threadIdx.y picks the chunk, so the chunks of one column share
 // their overlapping inputs through L1.  PARTS also stores the box means (stage dumps).
-template <int RZ, bool PARTS>
+template <int RZ, bool PARTS, bool PAD>
 __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min_intensity, const float2 *in,
                                                       float *norm, float *ero_l, float *dil_l) {
   constexpr int L = 2 * RZ + 1, NW = kBoxZK + 2 * RZ;
@@ -723,8 +724,8 @@ __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min
     v[k] = z < S.depth_valid ? (float)__ldg(S.src + z * plane + p) : 0.0f;
   }
   const float inv = 1.0f / (float)L;
-  float *nout = norm + norm_at(S, p);
-  const int64_t pplane = (int64_t)S.P * S.H;
+  float *nout = norm + norm_at<PAD>(S, p);
+  const int64_t pplane = PAD ? (int64_t)S.P * S.H : plane;
 #pragma unroll
   for (int k = 0; k < kBoxZK; k++) {
     float2 acc = make_float2(0.f, 0.f);
@@ -750,7 +751,7 @@ __global__ void k_copy_norm(const Sub *subs, float min_intensity, float *norm) {
   if (i >= n) return;
   const int z = (int)(i / plane);
   const float v = z < S.depth_valid ? (float)S.src[i] : 0.0f;
-  norm[norm_at(S, i - z * plane) + (int64_t)z * S.P * S.H] = (v >= min_intensity) ? v : 0.0f;
+  norm[norm_at<true>(S, i - z * plane) + (int64_t)z * S.P * S.H] = (v >= min_intensity) ? v : 0.0f;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -875,7 +876,7 @@ static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const 
 
 static int mm_z_vec(bool src_aligned8, int plane) { return !src_aligned8 ? 1 : plane % 4 == 0 ? 4 : plane % 2 == 0 ? 2 : 1; }
 
-void launch_normalize(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, int rz, float min_intensity,
+void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, int rxy, int rz, float min_intensity,
                       bool src_aligned8, uint32_t *ma, uint32_t *mb, float2 *fa, float2 *fb, float *norm,
                       cudaStream_t s, float *ero_l, float *dil_l) {
   const int plane = W * H;
@@ -905,9 +906,11 @@ void launch_normalize(const Sub *d_subs, int nsub, int W, int H, int D, int rxy,
 #define HDOG_BOXZ_CASE(R)                                                                                   \
   case R:                                                                                                   \
     if (ero_l)                                                                                              \
-      KLAUNCH("k_box_z_norm", s, (k_box_z_norm_t<R, true><<<gz, bz, 0, s>>>(d_subs, min_intensity, fb, norm, ero_l, dil_l))); \
+      KLAUNCH("k_box_z_norm", s, (k_box_z_norm_t<R, true, false><<<gz, bz, 0, s>>>(d_subs, min_intensity, fb, norm, ero_l, dil_l))); \
+    else if (P != W)                                                                                        \
+      KLAUNCH("k_box_z_norm", s, (k_box_z_norm_t<R, false, true><<<gz, bz, 0, s>>>(d_subs, min_intensity, fb, norm, ero_l, dil_l))); \
     else                                                                                                    \
-      KLAUNCH("k_box_z_norm", s, (k_box_z_norm_t<R, false><<<gz, bz, 0, s>>>(d_subs, min_intensity, fb, norm, ero_l, dil_l))); \
+      KLAUNCH("k_box_z_norm", s, (k_box_z_norm_t<R, false, false><<<gz, bz, 0, s>>>(d_subs, min_intensity, fb, norm, ero_l, dil_l))); \
     break;
     HDOG_BOXZ_CASE(1) HDOG_BOXZ_CASE(2) HDOG_BOXZ_CASE(3) HDOG_BOXZ_CASE(4)
     HDOG_BOXZ_CASE(5) HDOG_BOXZ_CASE(6) HDOG_BOXZ_CASE(7) HDOG_BOXZ_CASE(8)

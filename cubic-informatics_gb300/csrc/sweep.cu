@@ -395,6 +395,7 @@ constexpr int kHStage = 128;
 // gathered here, once per flush rather than on every slice -- and stores them as
 // consecutive 32-byte entries.  Entries past the list's capacity are dropped but counted,
 // so the host sees the overflow and redoes the batch.
+template <bool PAD>
 __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const Sub &S, const float *norm, FgEntry *fg,
                                             int32_t *fg_idx, unsigned long long *count) {
   __syncwarp();
@@ -404,8 +405,8 @@ __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const S
   base = __shfl_sync(0xFFFFFFFFu, base, 0);
   const int64_t room = S.fg_cap - (int64_t)base;
   const int keep = room <= 0 ? 0 : (room < n ? (int)room : n);
-  const float *nv = norm + S.pvox;
-  const int extra = S.P - S.W;   // rows of the normalized volume are padded by this much
+  const float *nv = norm + (PAD ? S.pvox : S.vox);
+  const int extra = S.P - S.W;   // PAD: rows of the normalized volume are padded by this much
   // every lane's gathers are issued before any of them is used, so a flush waits for one
   // global-load latency rather than one per entry
   constexpr int kPer = kHStage / 32;
@@ -415,7 +416,7 @@ __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const S
   for (int u = 0; u < kPer; u++) {
     const int i = lane + 32 * u;
     idx[u] = i < keep ? stage[i].idx : 0;
-    nvv[u] = i < keep ? __ldg(nv + (extra ? idx[u] + (int64_t)(idx[u] / S.W) * extra : idx[u])) : 0.0f;
+    nvv[u] = i < keep ? __ldg(nv + (PAD ? idx[u] + (int64_t)(idx[u] / S.W) * extra : idx[u])) : 0.0f;
   }
 #pragma unroll
   for (int u = 0; u < kPer; u++) {
@@ -440,8 +441,9 @@ __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const S
 #endif
 // PERSIST: a grid of a few blocks per SM takes (substack, tile) items from the device work
 // queue `q` until it is empty; otherwise one block per tile (blockIdx.x) and substack
-// (blockIdx.y).  Results are the same either way.
-template <bool PERSIST>
+// (blockIdx.y).  Results are the same either way.  PAD: the width is no multiple of 4, so the rows of the
+// DoG and the normalized volume are padded and the mask's are not whole words.
+template <bool PERSIST, bool PAD>
 __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
     k_hess_sweep(const __grid_constant__ CUtensorMap map, const Sub *subs, const float *norm, uint8_t *mask,
                  FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count, int *status, WorkQueue q) {
@@ -625,7 +627,7 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
         hv[2 * j][5] = hzz[j].x; hv[2 * j + 1][5] = hzz[j].y;
       }
       uint8_t *mo = mask + S.vox + i0;
-      if ((W & 3) == 0) {
+      if (!PAD) {
         *reinterpret_cast<uint32_t *>(mo) = mword;
       } else {   // the mask's rows are not padded
 #pragma unroll
@@ -679,7 +681,7 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
       const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
       const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
       if (staged + tot > kHStage) {
-        flush_stage(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
+        flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
         staged = 0;
       }
       int k = staged + excl;
@@ -696,7 +698,7 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
     __syncwarp();
     if ((t & 31) == 0) mbar_arrive(&done[(ibase + (uint32_t)zh) % kHRing]);
   }
-  if (staged) flush_stage(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
+  if (staged) flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
   zbase += (uint32_t)(D + 4);
   ibase += (uint32_t)D;
   if (!PERSIST) break;
@@ -801,19 +803,21 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
   if (si && (int)si->smem <= max_smem && encode_map(&map_n, norm, W, P, H, D, nsub, si->bw, si->bh) == CUDA_SUCCESS)
     dog_sweep_launch(si, map_n, T, d_subs, nsub, W, H, dog, d_status, ls, qctr, s);
   else
-    launch_dog(d_subs, nsub, W, H, D, (int64_t)H * D, T, norm, fa, fb, dog, s);
+    launch_dog(d_subs, nsub, W, P, H, D, (int64_t)H * D, T, norm, fa, fb, dog, s);
   const unsigned tiles_h = ceil_div(W, kHTX) * ceil_div(H, kHTY);
   if (ls.hess_per_sm > 0 && qctr) {
     zero_async(qctr + 1, sizeof(unsigned), s);
     const WorkQueue q{qctr + 1, (int)(tiles_h * (unsigned)nsub), (int)tiles_h};
     const unsigned grid = std::min<unsigned>((unsigned)(ls.hess_per_sm * ls.num_sms), tiles_h * (unsigned)nsub);
-    cudaFuncSetAttribute(k_hess_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
-    KLAUNCH("k_hess_sweep", s, (k_hess_sweep<true><<<grid, kHThreads, kHessSmem, s>>>(
-                                   map_d, d_subs, norm, mask, fg, fg_idx, fg_count, d_status, q)));
+    auto fn = P != W ? k_hess_sweep<true, true> : k_hess_sweep<true, false>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
+    KLAUNCH("k_hess_sweep", s, (fn<<<grid, kHThreads, kHessSmem, s>>>(map_d, d_subs, norm, mask, fg, fg_idx, fg_count,
+                                                                      d_status, q)));
   } else {
-    cudaFuncSetAttribute(k_hess_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
-    KLAUNCH("k_hess_sweep", s, (k_hess_sweep<false><<<dim3(tiles_h, nsub), kHThreads, kHessSmem, s>>>(
-                                   map_d, d_subs, norm, mask, fg, fg_idx, fg_count, d_status, WorkQueue{})));
+    auto fn = P != W ? k_hess_sweep<false, true> : k_hess_sweep<false, false>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
+    KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub), kHThreads, kHessSmem, s>>>(map_d, d_subs, norm, mask, fg, fg_idx,
+                                                                                     fg_count, d_status, WorkQueue{})));
   }
   return 0;
 }
