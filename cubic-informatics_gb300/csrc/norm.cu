@@ -707,12 +707,13 @@ template <int RZ, bool PARTS, bool PAD>
 __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min_intensity, const float2 *in,
                                                       float *norm, float *ero_l, float *dil_l) {
   constexpr int L = 2 * RZ + 1, NW = kBoxZK + 2 * RZ;
-  const Sub S = subs[blockIdx.z];
+  const Sub S = subs[blockIdx.y];
   const int64_t plane = (int64_t)S.W * S.H;
-  const int64_t p = (int64_t)blockIdx.x * 32 + threadIdx.x;
-  const int z0 = (blockIdx.y * blockDim.y + threadIdx.y) * kBoxZK;
+  const int nch = (S.D + kBoxZK - 1) / kBoxZK;
+  const int64_t p = (int64_t)(blockIdx.x / nch) * 128 + threadIdx.x;
+  const int z0 = (int)(blockIdx.x % nch) * kBoxZK;
   const int D = S.D;
-  if (p >= plane || z0 >= D) return;
+  if (p >= plane) return;
   const float2 *col = in + S.vox + p;
   float2 win[NW];
 #pragma unroll
@@ -901,7 +902,7 @@ void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, i
     dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * kBoxYK) * D), nsub);
     KLAUNCH("k_box_y", s, (k_box_y<<<gy, dim3(32, by), 0, s>>>(d_subs, rxy, fa, fb)));
   }
-  const dim3 gz(ceil_div(plane, 32), ceil_div(D, 4 * kBoxZK), nsub), bz(32, 4);
+  const dim3 gz(ceil_div(plane, 128) * ceil_div(D, kBoxZK), nsub), bz(128);
   switch (rz) {
 #define HDOG_BOXZ_CASE(R)                                                                                   \
   case R:                                                                                                   \
