@@ -234,11 +234,11 @@ struct hdog_ctx {
   uint8_t *mask = nullptr;
   int32_t *labels = nullptr;
   uint32_t *root_bits = nullptr, *blk_counts = nullptr, *blk_offsets = nullptr, *chunk = nullptr;
+  uint32_t *rec_counts = nullptr;   // records per block of regions
   int2 *edges = nullptr;
   unsigned long long *edge_count = nullptr;
   FgEntry *fg = nullptr;
   unsigned long long *fg_count = nullptr;
-  unsigned long long *fg_count_packed = nullptr;
   unsigned *qctr = nullptr;      // work-queue counters of the persistent sweeps
   LaunchShape shape;             // launch shape of the sweeps (autotuned per frame shape)
   bool tuned = false;            // shape and graph_batch chosen by the autotuner
@@ -346,7 +346,7 @@ static void plan(const hdog_params *p, int max_sub, int64_t &nvox, int64_t &reg_
   L.add(S * sizeof(unsigned long long));     // 29 edge counts
   L.add(S * fg_capacity(nvox) * sizeof(FgEntry));         // 30 foreground list
   L.add(S * kFgCountStride * sizeof(unsigned long long));   // 31 foreground counts (strided)
-  L.add(S * sizeof(unsigned long long));     // 32 foreground counts, packed for the read-back
+  L.add(S * nblk * sizeof(uint32_t));        // 32 record counts per block of regions
   L.add(4 * sizeof(unsigned));               // 33 work-queue counters
 }
 
@@ -443,7 +443,7 @@ extern "C" int hdog_ctx_create(const hdog_params *p, int max_substacks, hdog_ctx
   c->edge_cap = edge_capacity(c->nvox);
   c->fg = (FgEntry *)at(30);
   c->fg_count = (unsigned long long *)at(31);
-  c->fg_count_packed = (unsigned long long *)at(32);
+  c->rec_counts = (uint32_t *)at(32);
   c->fg_cap = fg_capacity(c->nvox);
   c->qctr = (unsigned *)at(33);
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->dev);
@@ -523,15 +523,33 @@ struct SubsParam {
 };
 
 // substacks [s0, s0 + n) of the context's ms slots: the first nsub of them get descriptors,
-// every slot its six scan-segment entries (seg is [6][ms])
+// every slot its six scan-segment entries (seg is [6][ms]); the blocks together zero z's ranges
 __global__ void k_store_subs(const __grid_constant__ SubsParam P, int s0, int n, int nsub, int ms, Sub *subs,
-                             int64_t *seg) {
+                             int64_t *seg, const __grid_constant__ ClearList z) {
   const int t = threadIdx.x;
+  clear_ranges(z);
+  if (blockIdx.x != 0) return;
   if (t < n && s0 + t < nsub) subs[s0 + t] = P.subs[t];
   if (t < 6 * n) seg[(int64_t)(t / n) * ms + s0 + t % n] = P.seg[t / n][t % n];
 }
 
-static int upload_subs(hdog_ctx *c, int nsub, cudaStream_t st) {
+// What a batch's kernels count up from zero, all in one list: the status word, the list counters, the
+// labelling's edge counters, the root bitmap and its block counts (the list path sets and counts
+// roots one by one), the record counts of blocks without regions.
+static ClearList batch_zeros(hdog_ctx *c, int nsub, bool fused) {
+  ClearList z;
+  z.add(c->status, sizeof(int));
+  z.add(c->edge_count, nsub * sizeof(unsigned long long));
+  z.add(c->rec_counts, (size_t)nsub * c->nblk * sizeof(uint32_t));
+  if (fused) {
+    z.add(c->fg_count, (size_t)nsub * kFgCountStride * sizeof(unsigned long long));
+    z.add(c->root_bits, (size_t)nsub * c->nblk * (kScanBlock / 32) * sizeof(uint32_t));
+    z.add(c->blk_counts, (size_t)nsub * c->nblk * sizeof(uint32_t));
+  }
+  return z;
+}
+
+static int upload_subs(hdog_ctx *c, int nsub, cudaStream_t st, const ClearList &zeros = ClearList()) {
   const int ms = c->max_sub;
   for (int s0 = 0; s0 < ms; s0 += kParamSubs) {
     const int n = std::min(kParamSubs, ms - s0);
@@ -540,7 +558,8 @@ static int upload_subs(hdog_ctx *c, int nsub, cudaStream_t st) {
     const int ns = std::max(0, std::min(n, nsub - s0));
     if (ns > 0) memcpy(P.subs, c->h_subs + s0, ns * sizeof(Sub));
     for (int k = 0; k < 6; k++) memcpy(P.seg[k], c->h_seg + (size_t)k * ms + s0, n * sizeof(int64_t));
-    KLAUNCH("k_store_subs", st, (k_store_subs<<<1, 6 * kParamSubs, 0, st>>>(P, s0, n, nsub, ms, c->d_subs, c->d_seg)));
+    const ClearList z = s0 == 0 ? zeros : ClearList();
+    KLAUNCH("k_store_subs", st, (k_store_subs<<<z.blocks(), 256, 0, st>>>(P, s0, n, nsub, ms, c->d_subs, c->d_seg, z)));
     HDOG_CUDA_TRY(cudaGetLastError());
   }
   return HDOG_OK;
@@ -599,7 +618,7 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
   }
   launch_ccl(c->d_subs, nsub, c->W, c->H, c->D, c->nvox, c->mask, c->labels, c->edges, c->edge_count, c->root_bits,
              c->blk_counts, c->status, c->num_sms, st, fused ? c->fg : nullptr, fused ? c->fg_count : nullptr,
-             c->fg_cap, c->nblk, fg_root);
+             c->fg_cap, fg_root);
   int32_t *rank = reinterpret_cast<int32_t *>(c->fa);
   if (fused)
     launch_regions_fg(c->d_subs, nsub, c->nvox, c->fg_cap, vseg_of(c), fg_root, c->root_bits, c->fg, c->fg_count, rank,
@@ -609,7 +628,7 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
     launch_regions(c->d_subs, nsub, c->nvox, vseg_of(c), c->mask, c->labels, c->root_bits, c->norm, c->dog, rank,
                    c->blk_counts, c->blk_offsets, c->chunk, c->num_regions, c->acc, c->slots, c->status, st);
   launch_finalize(c->d_subs, nsub, c->reg_cap, rseg_of(c), c->num_regions, c->acc, c->slots, c->out, filter_of(c->p),
-                  c->blk_counts, c->blk_offsets, c->chunk, c->num_records, c->records, c->nblk, st);
+                  c->rec_counts, c->blk_offsets, c->chunk, c->num_records, c->records, st);
 }
 
 // The fused sweep and the list-based region sums; the latter add coordinates in 32 bits
@@ -624,16 +643,10 @@ static bool fused_ok(hdog_ctx *c) {
 static int readback(hdog_ctx *c, int nsub, cudaStream_t st) {
   const int ms = c->max_sub;
   HDOG_CUDA_TRY(cudaGetLastError());
-  HDOG_CUDA_TRY(cudaMemcpyAsync(c->h_counts, c->num_records, nsub * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  HDOG_CUDA_TRY(cudaMemcpyAsync(c->h_counts + ms, c->num_regions, nsub * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  // a strided (2D) copy could wait on the copy engine behind a host stack's chunks, so the
-  // counters are packed on the device first
-  pack_fg_counts_async(c->fg_count, nsub, c->fg_count_packed, st);
-  HDOG_CUDA_TRY(cudaMemcpyAsync(c->h_counts + 2 * ms, c->fg_count_packed, nsub * sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                st));
-  HDOG_CUDA_TRY(cudaMemcpyAsync(c->h_counts + 3 * ms, c->status, sizeof(int), cudaMemcpyDeviceToHost, st));
+  report_async(c->num_records, c->num_regions, c->fg_count, c->status, nsub, ms, c->h_counts, st);
+  HDOG_CUDA_TRY(cudaGetLastError());
   HDOG_CUDA_TRY(cudaStreamSynchronize(st));
-  const int status = *(int *)(c->h_counts + 3 * ms);
+  const int status = (int)c->h_counts[3 * ms];
   if (status == HDOG_ERR_CAPACITY) return fail(HDOG_ERR_CAPACITY, "region capacity exceeded");
   if (status != 0) return fail(status, "a bounded device wait or loop hit its limit");
   return HDOG_OK;
@@ -644,8 +657,7 @@ static int readback(hdog_ctx *c, int nsub, cudaStream_t st) {
 // Enqueues the whole chain for nsub substacks whose host descriptors are set, up to the
 // records in c->records (no host synchronization).
 static int enqueue_batch(hdog_ctx *c, int nsub, bool fused, cudaStream_t st) {
-  TRY(upload_subs(c, nsub, st));
-  zero_async(c->status, sizeof(int), st);
+  TRY(upload_subs(c, nsub, st, batch_zeros(c, nsub, fused)));
   if (c->p.erosion_radius_xy > 0 || c->p.erosion_radius_z > 0) {
     // opt-in regional erosion of the input (the reference compiles Erosion3DFilter but
     // never calls it); the eroded substacks replace the inputs in c->img
@@ -658,7 +670,6 @@ static int enqueue_batch(hdog_ctx *c, int nsub, bool fused, cudaStream_t st) {
     TRY(upload_subs(c, nsub, st));
   }
   enqueue_normalize(c, nsub, c->norm, st);
-  if (fused) zero_async(c->fg_count, (size_t)nsub * kFgCountStride * sizeof(unsigned long long), st);
   enqueue_after_norm(c, nsub, fused, st);
   HDOG_CUDA_TRY(cudaGetLastError());
   return HDOG_OK;
@@ -683,7 +694,7 @@ static int run_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
     for (int s = 0; s < nsub; s++) over |= c->h_counts[2 * c->max_sub + s] > c->fg_cap;
     if (over) {
       // more foreground than the list holds: redo this batch with the separate passes
-      zero_async(c->status, sizeof(int), st);
+      clear_async(batch_zeros(c, nsub, false), st);
       enqueue_after_norm(c, nsub, false, st);
       TRY(readback(c, nsub, st));
     }
@@ -795,10 +806,11 @@ static int copy_out(const RecordBuf &v, hdog_record *out, int64_t cap, int64_t *
 }
 
 // ------------------------------------------------------------------ stage entry points
-static int single_sub(hdog_ctx *c, const uint16_t *src, cudaStream_t st) {
+// zeros: also clear what the stage counts up (batch_zeros)
+static int single_sub(hdog_ctx *c, const uint16_t *src, cudaStream_t st, bool zeros = false) {
   set_sub(c, 0, src, c->D, 0);
   c->h_subs[0].P = c->W;   // the caller's volumes have no padding
-  return upload_subs(c, 1, st);
+  return upload_subs(c, 1, st, zeros ? batch_zeros(c, 1, false) : ClearList());
 }
 
 #define CTX_GUARD(c)                                                   \
@@ -832,8 +844,7 @@ extern "C" int hdog_dog(hdog_ctx *c, const float *d_norm, float *d_dog, void *st
   CTX_GUARD(c);
   if (!d_norm || !d_dog) return fail(HDOG_ERR_ARG, "hdog_dog: null buffer");
   cudaStream_t st = (cudaStream_t)stream;
-  TRY(single_sub(c, nullptr, st));
-  zero_async(c->status, sizeof(int), st);
+  TRY(single_sub(c, nullptr, st, true));
   enqueue_dog(c, 1, c->W, d_norm, d_dog, st);
   HDOG_CUDA_TRY(cudaGetLastError());
   // the sweep's bounded TMA waits report through the status word
@@ -858,8 +869,7 @@ extern "C" int hdog_ccl(hdog_ctx *c, const uint8_t *d_mask, int32_t *d_labels, v
   CTX_GUARD(c);
   if (!d_mask || !d_labels) return fail(HDOG_ERR_ARG, "hdog_ccl: null buffer");
   cudaStream_t st = (cudaStream_t)stream;
-  TRY(single_sub(c, nullptr, st));
-  zero_async(c->status, sizeof(int), st);
+  TRY(single_sub(c, nullptr, st, true));
   launch_ccl(c->d_subs, 1, c->W, c->H, c->D, c->nvox, d_mask, d_labels, c->edges, c->edge_count, c->root_bits,
              c->blk_counts, c->status, c->num_sms, st);
   HDOG_CUDA_TRY(cudaGetLastError());
@@ -875,15 +885,14 @@ extern "C" int hdog_regional_features(hdog_ctx *c, const int32_t *d_labels, cons
   CTX_GUARD(c);
   if (!d_labels || !d_norm || !d_dog || !out) return fail(HDOG_ERR_ARG, "hdog_regional_features: null argument");
   cudaStream_t st = (cudaStream_t)stream;
-  TRY(single_sub(c, nullptr, st));
-  zero_async(c->status, sizeof(int), st);
+  TRY(single_sub(c, nullptr, st, true));
   // foreground = nonzero label; roots = voxels labelled with their own index
   launch_roots_from_labels(c->d_subs, 1, c->nvox, d_labels, c->mask, c->root_bits, c->blk_counts, st);
   int32_t *rank = reinterpret_cast<int32_t *>(c->fa);
   launch_regions(c->d_subs, 1, c->nvox, vseg_of(c), c->mask, d_labels, c->root_bits, d_norm, d_dog, rank,
                  c->blk_counts, c->blk_offsets, c->chunk, c->num_regions, c->acc, c->slots, c->status, st);
   launch_finalize(c->d_subs, 1, c->reg_cap, rseg_of(c), c->num_regions, c->acc, c->slots, c->out,
-                  filter_of(c->p, true), c->blk_counts, c->blk_offsets, c->chunk, c->num_records, c->records, c->nblk, st);
+                  filter_of(c->p, true), c->rec_counts, c->blk_offsets, c->chunk, c->num_records, c->records, st);
   HDOG_CUDA_TRY(cudaGetLastError());
   int64_t nr = 0;
   int status = 0;
@@ -1423,21 +1432,36 @@ extern "C" int hdog_graph_create(hdog_ctx *const *ctxs, int n_ctx, const hdog_gr
   // capture every batch of every context, with the record placement after each, on a
   // stream of its own (the caller's may be the legacy default stream, which cannot capture)
   HDOG_CUDA_TRY(cudaStreamSynchronize(st));
-  struct CapStream {
-    cudaStream_t s = nullptr;
-    ~CapStream() {
-      if (s) cudaStreamDestroy(s);
+  // (and one per context: batches of one context follow each other in its scratch, but the contexts share
+  // nothing, so they are parallel branches of the graph)
+  struct CapStreams {
+    std::vector<cudaStream_t> s;
+    std::vector<cudaEvent_t> e;
+    ~CapStreams() {
+      for (cudaStream_t x : s) cudaStreamDestroy(x);
+      for (cudaEvent_t x : e) cudaEventDestroy(x);
     }
   } cap;
-  HDOG_CUDA_TRY(cudaStreamCreateWithFlags(&cap.s, cudaStreamNonBlocking));
-  st = cap.s;
+  for (size_t k = 0; k <= g->ctxs.size(); k++) {   // the last: the capture's own
+    cudaStream_t x;
+    HDOG_CUDA_TRY(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    cap.s.push_back(x);
+    cudaEvent_t ev;
+    HDOG_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cap.e.push_back(ev);
+  }
+  st = cap.s.back();
   KernelTimer *saved_timer = g_timer;
   g_timer = nullptr;
   HDOG_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   int rc = HDOG_OK;
   zero_async(g->dmem, 256, st);
+  cudaEventRecord(cap.e.back(), st);
   for (size_t k = 0; k < g->ctxs.size() && rc == HDOG_OK; k++) {
     hdog_ctx *c = g->ctxs[k];
+    if (items[k].empty()) continue;
+    const cudaStream_t cs = cap.s[k];
+    cudaStreamWaitEvent(cs, cap.e.back(), 0);
     const bool fused = fused_ok(c);
     const size_t per = (size_t)std::max(1, c->graph_batch > 0 ? c->graph_batch : c->max_sub);
     for (size_t b = 0; b < items[k].size() && rc == HDOG_OK; b += per) {
@@ -1447,12 +1471,14 @@ extern "C" int hdog_graph_create(hdog_ctx *const *ctxs, int n_ctx, const hdog_gr
         set_item(c, s, items[k][b + s]);
         ids.id[s] = (int)items[k][b + s].id;
       }
-      rc = enqueue_batch(c, nsub, fused, st);
+      rc = enqueue_batch(c, nsub, fused, cs);
       if (rc != HDOG_OK) break;
       launch_graph_place(nsub, ids, c->num_records, c->fg_count, c->fg_cap, fused, c->status, g->d_total, g->d_table,
-                         g->d_redo, g->out_cap, st);
-      launch_graph_copy(nsub, ids, c->records, c->reg_cap, g->d_table, g->d_out, g->out_cap, st);
+                         g->d_redo, g->out_cap, cs);
+      launch_graph_copy(nsub, ids, c->records, c->reg_cap, g->d_table, g->d_out, g->out_cap, cs);
     }
+    cudaEventRecord(cap.e[k], cs);
+    cudaStreamWaitEvent(st, cap.e[k], 0);
   }
   cudaGraph_t graph = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(st, &graph);

@@ -12,14 +12,16 @@
 namespace hdog {
 
 // One thread: each batch substack's slot in the run's record array, after the running
-// total.  A batch whose foreground list overflowed, whose status word is set, or whose
+// total (batches of other contexts may run at the same time).  A batch whose foreground list overflowed, whose status word is set, or whose
 // records would pass the array's end raises *redo (the host then reruns the call without
 // the graph); the copy below skips what does not fit.
 __global__ void k_graph_place(int nsub, GraphIds ids, const int64_t *num_records, const unsigned long long *fg_count,
                               int64_t fg_cap, int fused, const int *status, int64_t *total, GraphSlot *table, int *redo,
                               int64_t out_cap) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int64_t t = *total;
+  int64_t sum = 0;
+  for (int s = 0; s < nsub; s++) sum += num_records[s];
+  int64_t t = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(total), (unsigned long long)sum);
   int bad = *status != 0;
   for (int s = 0; s < nsub; s++) {
     const int64_t k = num_records[s];
@@ -30,7 +32,6 @@ __global__ void k_graph_place(int nsub, GraphIds ids, const int64_t *num_records
   }
   if (t > out_cap) bad = 1;
   if (bad) *redo = 1;
-  *total = t;
 }
 
 // Copies substack blockIdx.y's records (28-byte structs, as 32-bit words) to its slot.

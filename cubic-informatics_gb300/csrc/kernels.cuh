@@ -123,9 +123,37 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
                   int n_neg, float grad_loss, float *grad_vol, float *grad_sigma, float *grad_thresh, void *work,
                   cudaStream_t st, bool forward_kept = false, const float *d_grad_loss = nullptr);
 
+// Ranges of 32-bit words that one kernel zeroes.
+struct ClearList {
+  static constexpr int kMax = 6;
+  uint32_t *p[kMax];
+  int64_t n[kMax];
+  int count = 0;
+  void add(void *q, size_t bytes) {
+    p[count] = static_cast<uint32_t *>(q);
+    n[count++] = (int64_t)(bytes / 4);
+  }
+  int64_t words() const {
+    int64_t t = 0;
+    for (int i = 0; i < count; i++) t += n[i];
+    return t;
+  }
+  unsigned blocks() const { return words() < 4096 ? 1u : (unsigned)(words() / 2048 < 4096 ? words() / 2048 : 4096); }
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void clear_ranges(const ClearList &z) {
+  for (int r = 0; r < z.count; r++)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < z.n[r]; i += (int64_t)gridDim.x * blockDim.x)
+      z.p[r][i] = 0u;
+}
+#endif
+void clear_async(const ClearList &z, cudaStream_t s);
 // Zero `bytes` (a multiple of 4) of device memory on stream s with a kernel.
 void zero_async(void *p, size_t bytes, cudaStream_t s);
-void pack_fg_counts_async(const unsigned long long *fg_count, int nsub, unsigned long long *packed, cudaStream_t s);
+// A batch's counts straight into page-locked host memory: host[0 .. nsub) records, host[ms ..) regions,
+// host[2 ms ..) list entries, host[3 ms] the status word.
+void report_async(const int64_t *records, const int64_t *regions, const unsigned long long *fg_count, const int *status,
+                  int nsub, int ms, int64_t *host, cudaStream_t s);
 
 bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
                       float *dog, int *d_status, int max_smem, cudaStream_t s);
@@ -144,11 +172,11 @@ struct ScanSeg {
 };
 void launch_scan(const ScanSeg &sg, int nsub, const uint32_t *in, uint32_t *out, uint32_t *chunk,
                  int64_t *totals, int64_t add, cudaStream_t s);
+// edge_count, and on the list path root_bits and blk_counts, must start at zero.
 void launch_ccl(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d, int64_t max_n, const uint8_t *mask,
                 int32_t *labels, int2 *edges, unsigned long long *edge_count, uint32_t *root_bits,
                 uint32_t *blk_counts, int *d_status, int num_sms, cudaStream_t s, const FgEntry *fg = nullptr,
-                const unsigned long long *fg_count = nullptr, int64_t max_fg = 0, int64_t nblk = 0,
-                int32_t *fg_root = nullptr);
+                const unsigned long long *fg_count = nullptr, int64_t max_fg = 0, int32_t *fg_root = nullptr);
 // Foreground mask (label != 0), root bitmap and per-block root counts from labels alone.
 void launch_roots_from_labels(const Sub *d_subs, int nsub, int64_t max_n, const int32_t *labels, uint8_t *mask,
                               uint32_t *root_bits, uint32_t *blk_counts, cudaStream_t s);
@@ -162,10 +190,11 @@ void launch_regions_fg(const Sub *d_subs, int nsub, int64_t max_n, int64_t max_f
                        const unsigned long long *fg_count, int32_t *rank, uint32_t *blk_counts,
                        uint32_t *blk_offsets, uint32_t *chunk, int64_t *d_num_regions, RegionAcc acc, int64_t slots,
                        int *d_status, int num_sms, cudaStream_t s);
+// blk_counts must start at zero.
 void launch_finalize(const Sub *d_subs, int nsub, int64_t max_reg_cap, const ScanSeg &rseg,
                      const int64_t *d_num_regions, RegionAcc acc, int64_t slots, RegionOut out,
                      FilterParams fp, uint32_t *blk_counts, uint32_t *blk_offsets, uint32_t *chunk,
-                     int64_t *d_num_records, hdog_record *records, int64_t blk_stride, cudaStream_t s);
+                     int64_t *d_num_records, hdog_record *records, cudaStream_t s);
 
 // ---- graph.cu: record placement of the batched graph form ----
 constexpr int kGraphMaxBatch = 64;   // substacks per batch in the graph form

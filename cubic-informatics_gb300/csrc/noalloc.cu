@@ -125,7 +125,10 @@ extern "C" int hdog_ccl_noalloc(const uint8_t *d_mask, int32_t *d_labels, int wi
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   HDOG_CUDA_TRY(cudaMemcpyAsync(d_sub, &S, sizeof(Sub), cudaMemcpyHostToDevice, st));
-  HDOG_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));   // the edge counter is cleared by launch_ccl
+  ClearList zeros;
+  zeros.add(d_status, sizeof(int));
+  zeros.add(d_edge_count, sizeof(unsigned long long));
+  clear_async(zeros, st);
   launch_ccl(d_sub, 1, width, height, depth, n, d_mask, d_labels, d_edges, d_edge_count, d_bits, d_blk, d_status,
              num_sms, st);
   HDOG_CUDA_TRY(cudaGetLastError());

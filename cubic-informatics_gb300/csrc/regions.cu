@@ -93,6 +93,26 @@ __global__ void __launch_bounds__(1024) k_scan_p3(const int64_t *seg_off, const 
   if (i < len) out[seg_off[s] + i] = chunk[chk_off[s] + c] + e;
 }
 
+// Both scans of one substack's counts by one block, chunk after chunk with a running carry, for up to
+// kScanOneMax chunks: one launch instead of three (each about as long as this one) where the counts are few.
+constexpr int64_t kScanOneMax = 4;
+
+__global__ void __launch_bounds__(1024) k_scan_one(const int64_t *seg_off, const int64_t *seg_len, const uint32_t *in,
+                                                   uint32_t *out, int64_t *totals, int64_t add) {
+  const int s = blockIdx.x;
+  const int64_t len = seg_len[s], off = seg_off[s];
+  uint32_t carry = 0;
+  for (int64_t b = 0; b < len; b += 1024) {
+    const int64_t i = b + threadIdx.x;
+    const uint32_t v = i < len ? in[off + i] : 0u;
+    uint32_t tot;
+    const uint32_t e = block_excl_scan(v, &tot);
+    if (i < len) out[off + i] = carry + e;
+    carry += tot;
+  }
+  if (threadIdx.x == 0) totals[s] = (int64_t)carry + add;
+}
+
 // ------------------------------------------------------------------ region numbering
 // Region r >= 1 is the r-th root in ascending voxel order (region 0 = background), the
 // order reduce-by-key over sorted labels produces.  Each root initialises its slot.
@@ -552,23 +572,38 @@ void zero_async(void *p, size_t bytes, cudaStream_t s) {
                                static_cast<uint32_t *>(p), n)));
 }
 
-// The substacks' list counters (kFgCountStride apart) into consecutive slots, for one
-// plain device-to-host copy.
-__global__ void k_pack_fg_counts(const unsigned long long *fg_count, int nsub, unsigned long long *packed) {
-  for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < nsub; i += (int)(gridDim.x * blockDim.x))
-    packed[i] = fg_count[(int64_t)i * kFgCountStride];
+__global__ void __launch_bounds__(256) k_clear(const __grid_constant__ ClearList z) { clear_ranges(z); }
+
+void clear_async(const ClearList &z, cudaStream_t s) {
+  KLAUNCH("k_clear", s, (k_clear<<<z.blocks(), 256, 0, s>>>(z)));
 }
 
-void pack_fg_counts_async(const unsigned long long *fg_count, int nsub, unsigned long long *packed, cudaStream_t s) {
-  if (nsub > 0)
-    KLAUNCH("k_pack_fg_counts", s, (k_pack_fg_counts<<<std::min<unsigned>(ceil_div(nsub, 256), 64u), 256, 0, s>>>(
-                                       fg_count, nsub, packed)));
+// The list counters sit kFgCountStride apart.  Written through to the host: no copies to queue behind a host
+// stack's chunks, and one launch where there were five.
+__global__ void k_report(const int64_t *records, const int64_t *regions, const unsigned long long *fg_count,
+                         const int *status, int nsub, int ms, int64_t *host) {
+  for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < nsub; i += (int)(gridDim.x * blockDim.x)) {
+    host[i] = records[i];
+    host[ms + i] = regions[i];
+    host[2 * ms + i] = (int64_t)fg_count[(int64_t)i * kFgCountStride];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) host[3 * ms] = *status;
+}
+
+void report_async(const int64_t *records, const int64_t *regions, const unsigned long long *fg_count, const int *status,
+                  int nsub, int ms, int64_t *host, cudaStream_t s) {
+  KLAUNCH("k_report", s, (k_report<<<std::min<unsigned>(ceil_div(std::max(nsub, 1), 64), 64u), 64, 0, s>>>(
+                             records, regions, fg_count, status, nsub, ms, host)));
 }
 
 // ------------------------------------------------------------------ launchers
 void launch_scan(const ScanSeg &sg, int nsub, const uint32_t *in, uint32_t *out, uint32_t *chunk,
                  int64_t *totals, int64_t add, cudaStream_t s) {
   const unsigned nch = ceil_div(sg.max_len, 1024);
+  if (nch <= kScanOneMax) {
+    KLAUNCH("k_scan_one", s, (k_scan_one<<<nsub, 1024, 0, s>>>(sg.off, sg.len, in, out, totals, add)));
+    return;
+  }
   KLAUNCH("k_scan_p1", s, (k_scan_p1<<<dim3(nch, nsub), 1024, 0, s>>>(sg.off, sg.len, sg.chk, in, chunk)));
   KLAUNCH("k_scan_p2", s, (k_scan_p2<<<nsub, 1024, 0, s>>>(sg.len, sg.chk, chunk, totals, add)));
   KLAUNCH("k_scan_p3", s, (k_scan_p3<<<dim3(nch, nsub), 1024, 0, s>>>(sg.off, sg.len, sg.chk, in, chunk, out)));
@@ -605,11 +640,10 @@ void launch_regions_fg(const Sub *d_subs, int nsub, int64_t max_n, int64_t max_f
 void launch_finalize(const Sub *d_subs, int nsub, int64_t max_reg_cap, const ScanSeg &rseg,
                      const int64_t *d_num_regions, RegionAcc acc, int64_t slots, RegionOut out,
                      FilterParams fp, uint32_t *blk_counts, uint32_t *blk_offsets, uint32_t *chunk,
-                     int64_t *d_num_records, hdog_record *records, int64_t blk_stride, cudaStream_t s) {
+                     int64_t *d_num_records, hdog_record *records, cudaStream_t s) {
   // the kernels visit only the blocks that hold regions (the count is on the device): the
-  // other blocks' counts are zero for the record scan
+  // other blocks' counts stay zero for the record scan
   const int64_t nb = ceil_div(max_reg_cap, kFinalizeBlock);
-  zero_async(blk_counts, (size_t)((nsub - 1) * blk_stride + nb) * sizeof(uint32_t), s);
   const unsigned grid = (unsigned)std::min<int64_t>(nb, 2048);
   KLAUNCH("k_finalize", s, (k_finalize<<<dim3(grid, nsub), kFinalizeBlock, 0, s>>>(d_subs, d_num_regions, acc, slots, out, fp, blk_counts)));
   launch_scan(rseg, nsub, blk_counts, blk_offsets, chunk, d_num_records, 0, s);

@@ -796,7 +796,6 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
                     float2 *fa, float2 *fb, float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx,
                     unsigned long long *fg_count, int *d_status, const LaunchShape &ls, unsigned *qctr, int max_smem,
                     cudaStream_t s) {
-  zero_async(fg_count, (size_t)nsub * kFgCountStride * sizeof(unsigned long long), s);
   const SweepInst *si = find_inst(T);
   CUtensorMap map_n, map_d;
   if (encode_map(&map_d, dog, W, P, H, D, nsub, kHPX, kHPY) != CUDA_SUCCESS) return -1;
