@@ -74,9 +74,12 @@ __device__ __forceinline__ void back_offset(int k, int &dz, int &dy, int &dx) {
 }
 
 // ------------------------------------------------------------------ pass 1: tile-local
-constexpr int kTX = 64, kTY = 16, kTZ = 32;
-constexpr int kTileVox = kTX * kTY * kTZ;     // 32768 voxels
-constexpr int kCclThreads = 256;              // thread = 4 x-consecutive voxels of one row, all kTZ slices
+// Tiles of 64 x 16 voxels and TZ slices.  A block works through its tile's layers one after the other, so
+// where the 32-slice tiles would leave most of the chip idle (fewer than two per SM) they are 16 slices
+// deep, and 8 where even those are fewer than one for two SMs: more cross-tile edges, but shorter blocks and
+// more of them.  One 128x96x16 substack 27 -> 16 us, one of 256x256x32 50 -> 31 us.
+constexpr int kTX = 64, kTY = 16;
+constexpr int kCclThreads = 256;              // thread = 4 x-consecutive voxels of one row, all TZ slices
 
 // Shared-memory union-find over the tile's cells, 32-bit parents (native shared atomics;
 // kBg32 marks a background cell).  Find with path halving (stores an ancestor of the
@@ -122,13 +125,14 @@ struct CclTile {
   int x0, y0, z0, tz;     // origin, slices in this tile
 };
 
+template <int TZ>
 __device__ __forceinline__ bool ccl_tile(const Sub &S, int64_t bid, CclTile &T) {
-  const int nx = (S.W + kTX - 1) / kTX, ny = (S.H + kTY - 1) / kTY, nz = (S.D + kTZ - 1) / kTZ;
+  const int nx = (S.W + kTX - 1) / kTX, ny = (S.H + kTY - 1) / kTY, nz = (S.D + TZ - 1) / TZ;
   if (bid >= (int64_t)nx * ny * nz) return false;
   T.x0 = (int)(bid % nx) * kTX;
   T.y0 = (int)((bid / nx) % ny) * kTY;
-  T.z0 = (int)(bid / ((int64_t)nx * ny)) * kTZ;
-  T.tz = min(kTZ, S.D - T.z0);
+  T.z0 = (int)(bid / ((int64_t)nx * ny)) * TZ;
+  T.tz = min(TZ, S.D - T.z0);
   return true;
 }
 
@@ -154,8 +158,7 @@ constexpr int kEdgeBuf = 2048;                // cross-tile edges staged per til
 // connected exactly when each has a foreground voxel on the side facing the other --
 // two mask tests per pair.  A component's label is then the minimum voxel index over
 // its cells, found with one shared-memory atomicMin per cell.
-constexpr int kCX = kTX / 2, kCY = kTY / 2, kCZ = kTZ / 2;
-constexpr int kCells = kCX * kCY * kCZ;       // 4096
+constexpr int kCX = kTX / 2, kCY = kTY / 2;
 
 // Occupancy bits of a cell whose voxels have local coordinate `side` along one axis
 // (0 or 1); axis 0 = x, 1 = y, 2 = z.
@@ -187,8 +190,7 @@ __constant__ CellNb kCellNb[13] = {
 
 // Occupancy of a halo-framed block of cells: the tile's cells plus one cell on each x
 // and y side and one layer below (cell coordinates -1 .. kC? along each axis).
-constexpr int kHX = kCX + 2, kHY = kCY + 2, kHZ = kCZ + 1;
-constexpr int kHalo = kHX * kHY * kHZ;        // 5780
+constexpr int kHX = kCX + 2, kHY = kCY + 2;
 __device__ __forceinline__ int halo_of(int cx, int cy, int cz) { return ((cz + 1) * kHY + (cy + 1)) * kHX + (cx + 1); }
 __device__ __forceinline__ int cell_bit(int lx, int ly, int lz) { return ((lz & 1) << 2) | ((ly & 1) << 1) | (lx & 1); }
 
@@ -282,8 +284,10 @@ __device__ __forceinline__ uint32_t prune_links(uint32_t todo, const uint32_t (&
   return todo;
 }
 
+template <int TZ>
 __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, const uint8_t *mask, int32_t *labels,
                                                           int2 *edges, unsigned long long *edge_count) {
+  constexpr int kCZ = TZ / 2, kCells = kCX * kCY * kCZ, kHZ = kCZ + 1, kHalo = kHX * kHY * kHZ;   // 4096 cells, 5780 with halo at TZ 32
   __shared__ uint32_t par[kCells];
   __shared__ uint8_t occ[kHalo];
   __shared__ uint32_t minv[kCells];
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
   __shared__ unsigned long long edge_base;
   const Sub S = subs[blockIdx.y];
   CclTile T;
-  if (!ccl_tile(S, blockIdx.x, T)) return;
+  if (!ccl_tile<TZ>(S, blockIdx.x, T)) return;
   const int t = threadIdx.x;
   const int64_t WH = (int64_t)S.W * S.H;
   const int64_t N = WH * S.D;
@@ -468,6 +472,17 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
         if (nz < 0 && !zface) continue;
         if ((oc & nb.self) && (occ[halo_of(nx, ny, nz)] & nb.other)) todo |= 1u << k;
       }
+      if (todo & (1u << 4)) {
+        // linked to the cell below, in the tile below: that tile's own unions join it to those of its eight
+        // neighbours it touches inside the same footprint, so the edges to these add nothing
+        const uint32_t below = occ[halo_of(fx, fy, fz - 1)];
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+          const int dy = k / 3 - 1, dx = k % 3 - 1;
+          if (k == 4 || fx + dx < 0 || fx + dx >= kCX || fy + dy < 0 || fy + dy >= kCY) continue;
+          if (touches(below, occ[halo_of(fx + dx, fy + dy, fz - 1)], cell_nb(0, dy, dx))) todo &= ~(1u << k);
+        }
+      }
       if (!todo) continue;
       const int64_t a = first_voxel(fx, fy, fz, oc);
       while (todo) {
@@ -484,12 +499,21 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
   // 4b. the reference's wrap-around edges: backward linear offsets of a voxel in the first
   //     or last column or row that leave the row or slice (only border tiles hold such voxels)
   if (T.x0 == 0 || T.x0 + kTX >= S.W || T.y0 == 0 || T.y0 + kTY >= S.H) {
-    const int lastx = min(kTX - 1, S.W - 1 - T.x0), lasty = min(kTY - 1, S.H - 1 - T.y0);
-    for (int v = t; v < kTX * kTY * T.tz; v += kCclThreads) {
-      const int lx = v % kTX, ly = (v / kTX) % kTY, lz = v / (kTX * kTY);
-      if (lx > lastx || ly > lasty) continue;
+    // per layer: the first and last column of the volume (all rows), then the first and last row
+    constexpr int kRing = 2 * kTY + 2 * kTX;
+    for (int v = t; v < kRing * T.tz; v += kCclThreads) {
+      const int lz = v / kRing, j = v % kRing;
+      int lx, ly;
+      if (j < 2 * kTY) {
+        lx = (j & 1 ? S.W - 1 : 0) - T.x0;
+        ly = j >> 1;
+      } else {
+        ly = ((j & 1) ? S.H - 1 : 0) - T.y0;
+        lx = (j - 2 * kTY) >> 1;
+        if (T.x0 + lx == 0 || T.x0 + lx == S.W - 1) continue;   // done with the columns
+      }
       const int x = T.x0 + lx, y = T.y0 + ly, z = T.z0 + lz;
-      if (x != 0 && x != S.W - 1 && y != 0 && y != S.H - 1) continue;
+      if (lx < 0 || lx >= kTX || ly < 0 || ly >= kTY || x >= S.W || y >= S.H) continue;
       if (!((occ[halo_of(lx >> 1, ly >> 1, lz >> 1)] >> cell_bit(lx, ly, lz)) & 1u)) continue;
       const int64_t g = z * WH + (int64_t)y * S.W + x;
       for (int o = 0; o < 13; o++) {
@@ -565,13 +589,14 @@ __global__ void k_ccl_edges(const Sub *subs, const int2 *edges, const unsigned l
 }
 
 // The same cross-tile edges straight from the mask, for a substack whose list overflowed.
+template <int TZ>
 __global__ void __launch_bounds__(kCclThreads) k_ccl_cross_direct(const Sub *subs, const uint8_t *mask,
                                                                  const unsigned long long *edge_count,
                                                                  int32_t *labels, int *status) {
   const Sub S = subs[blockIdx.y];
   if (edge_count[blockIdx.y] <= (unsigned long long)S.edge_cap) return;
   CclTile T;
-  if (!ccl_tile(S, blockIdx.x, T)) return;
+  if (!ccl_tile<TZ>(S, blockIdx.x, T)) return;
   const int t = threadIdx.x;
   const int lx0 = (t % (kTX / 4)) * 4, ly = t / (kTX / 4);
   const int x = T.x0 + lx0, y = T.y0 + ly;
@@ -708,14 +733,17 @@ void launch_ccl(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d, in
                 int32_t *labels, int2 *edges, unsigned long long *edge_count, uint32_t *root_bits,
                 uint32_t *blk_counts, int *d_status, int num_sms, cudaStream_t s, const FgEntry *fg,
                 const unsigned long long *fg_count, int64_t max_fg, int32_t *fg_root) {
-  const int64_t tiles = (int64_t)ceil_div(max_w, kTX) * ceil_div(max_h, kTY) * ceil_div(max_d, kTZ);
-  KLAUNCH("k_ccl_local", s, (k_ccl_local<<<dim3((unsigned)tiles, nsub), kCclThreads, 0, s>>>(
-                                d_subs, mask, labels, edges, edge_count)));
+  const int64_t cols = (int64_t)ceil_div(max_w, kTX) * ceil_div(max_h, kTY);
+  const auto tiles_of = [&](int tz) { return cols * ceil_div(max_d, tz); };
+  const int tz = tiles_of(32) * nsub >= 2 * (int64_t)num_sms ? 32 : tiles_of(16) * nsub * 2 >= num_sms ? 16 : 8;
+  const dim3 grid((unsigned)tiles_of(tz), nsub);
+  auto local = tz == 32 ? k_ccl_local<32> : tz == 16 ? k_ccl_local<16> : k_ccl_local<8>;
+  auto cross = tz == 32 ? k_ccl_cross_direct<32> : tz == 16 ? k_ccl_cross_direct<16> : k_ccl_cross_direct<8>;
+  KLAUNCH("k_ccl_local", s, (local<<<grid, kCclThreads, 0, s>>>(d_subs, mask, labels, edges, edge_count)));
   const unsigned eb = (unsigned)max(1, (8 * num_sms + nsub - 1) / nsub);
   KLAUNCH("k_ccl_edges", s, (k_ccl_edges<<<dim3(eb, nsub), 256, 0, s>>>(d_subs, edges, edge_count, labels,
                                                                         d_status)));
-  KLAUNCH("k_ccl_cross_direct", s, (k_ccl_cross_direct<<<dim3((unsigned)tiles, nsub), kCclThreads, 0, s>>>(
-                                       d_subs, mask, edge_count, labels, d_status)));
+  KLAUNCH("k_ccl_cross_direct", s, (cross<<<grid, kCclThreads, 0, s>>>(d_subs, mask, edge_count, labels, d_status)));
   if (fg) {
     const int64_t want = std::min((int64_t)ceil_div(max_fg, 256 * kFlatFgPerThread),
                                   (int64_t)(8 * num_sms / (nsub > 0 ? nsub : 1) + 1));

@@ -441,12 +441,14 @@ __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const S
 #endif
 // PERSIST: a grid of a few blocks per SM takes (substack, tile) items from the device work
 // queue `q` until it is empty; otherwise one block per tile (blockIdx.x) and substack
-// (blockIdx.y).  Results are the same either way.  PAD: the width is no multiple of 4, so the rows of the
+// (blockIdx.y).  SPLIT: the latter, with zlen slices per block (blockIdx.z) where the tiles alone leave most of
+// the chip idle (a block's slices follow one another).  One 128x96x16 substack 28 -> 12 us, one of 256x256x32 63 ->
+// 30 us.  Results are the same either way.  PAD: the width is no multiple of 4, so the rows of the
 // DoG and the normalized volume are padded and the mask's are not whole words.
-template <bool PERSIST, bool PAD>
-__global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
+template <bool PERSIST, bool PAD, bool SPLIT>
+__global__ void __launch_bounds__(kHThreads, SPLIT ? HDOG_HESS_BLOCKS - 1 : HDOG_HESS_BLOCKS)
     k_hess_sweep(const __grid_constant__ CUtensorMap map, const Sub *subs, const float *norm, uint8_t *mask,
-                 FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count, int *status, WorkQueue q) {
+                 FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count, int *status, WorkQueue q, int zlen) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PL = kHPX * kHPY;
   constexpr uint32_t tma_bytes = (uint32_t)(PL * 4);
@@ -494,16 +496,17 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
   const int D = S.D, W = S.W, H = S.H;
   const int32_t WH = W * H;
   const int tx = x0 - 4, ty = y0 - 2;
-  // ring slot of DoG slice z (z = -2 .. D+1; slices outside the volume arrive zero-filled)
-  auto slot = [zbase](int z) { return (int)((zbase + (uint32_t)(z + 2)) % kHRing); };
+  const int zb = SPLIT ? (int)blockIdx.z * zlen : 0, ze = SPLIT ? min(D, zb + zlen) : D;   // this block's slices
+  // ring slot of DoG slice z (z = zb-2 .. ze+1; slices outside the volume arrive zero-filled)
+  auto slot = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) % kHRing); };
   // use k of slot s (k-th slice loaded into it) completes barrier phase k & 1
-  auto use = [zbase](int z) { return (int)((zbase + (uint32_t)(z + 2)) / kHRing); };
-  // slices -2 .. 4 up front, then slice zh + 5 while slice zh is tested: the slot it
+  auto use = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) / kHRing); };
+  // slices zb-2 .. zb+4 up front, then slice zh + 5 while slice zh is tested: the slot it
   // reuses held slice zh - 3, last read one barrier earlier
   if (t == 0 && ok)
-    for (int z = -2; z <= 4 && z <= D + 1; z++)
+    for (int z = zb - 2; z <= zb + 4 && z <= ze + 1; z++)
       tma_slice(&map, ring + slot(z) * PL, &bar[slot(z)], tx, ty, z, sub, tma_bytes);
-  for (int z = -2; z <= 1; z++)
+  for (int z = zb - 2; z <= zb + 1; z++)
     if (ok && !mbar_wait(&bar[slot(z)], use(z) & 1)) {
       ok = false;
       atomicExch(status, HDOG_ERR_TIMEOUT);
@@ -522,8 +525,8 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
   float2 gym[2] = {zero2, zero2}, gy0[2], gzm[2] = {zero2, zero2}, gz0[2];
   float2 fm[2] = {zero2, zero2}, f0[2];
   if (interior) {
-    // slice 0: gx, gy on row Y; gz from slices 1 and -1 (zero)
-    const float *P0 = ring + slot(0) * PL + b, *P1 = ring + slot(1) * PL + b;
+    // slice zb: gx, gy on row Y; gz from slices zb+1 and zb-1 (zero below the volume)
+    const float *P0 = ring + slot(zb) * PL + b, *P1 = ring + slot(zb + 1) * PL + b;
     float2 l, r, u0, u1, d0, d1;
     ld_row(P0, l, f0[0], f0[1], r);
     gx_g(l, f0[0], f0[1], r, gx0);
@@ -533,18 +536,34 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
     gy0[1] = hd2(d1, u1);
     float2 p0, p1;
     ld_quad(P1, p0, p1);
-    gz0[0] = hd2(p0, zero2);
-    gz0[1] = hd2(p1, zero2);
+    if (!SPLIT || zb == 0) {
+      gz0[0] = hd2(p0, zero2);
+      gz0[1] = hd2(p1, zero2);
+    } else {   // a block that starts inside the volume: the derivatives of slice zb-1 as well
+      const float *M1 = ring + slot(zb - 1) * PL + b, *M2 = ring + slot(zb - 2) * PL + b;
+      float2 c0, c1, q0, q1;
+      ld_row(M1, l, c0, c1, r);
+      gx_g(l, c0, c1, r, gxm);
+      gz0[0] = hd2(p0, c0);
+      gz0[1] = hd2(p1, c1);
+      ld_quad(M1 - kHPX, u0, u1);
+      ld_quad(M1 + kHPX, d0, d1);
+      gym[0] = hd2(d0, u0);
+      gym[1] = hd2(d1, u1);
+      ld_quad(M2, q0, q1);
+      gzm[0] = hd2(f0[0], q0);
+      gzm[1] = hd2(f0[1], q1);
+    }
     fm[0] = f0[0]; fm[1] = f0[1];
     f0[0] = p0; f0[1] = p1;
   }
-  for (int zh = 0; zh < D; zh++) {
+  for (int zh = zb; zh < ze; zh++) {
     // DoG slice zh+5 reuses the slot of slice zh-3, read for the last time in iteration
     // zh-1: the producer waits until every warp is past it (warps otherwise run up to the
     // ring's depth apart)
-    if (t == 0 && ok && zh + 5 <= D + 1) {
-      const uint32_t prev = ibase + (uint32_t)zh - 1u;
-      if (zh >= 1 && !mbar_wait(&done[prev % kHRing], (prev / kHRing) & 1)) {
+    if (t == 0 && ok && zh + 5 <= ze + 1) {
+      const uint32_t prev = ibase + (uint32_t)(zh - zb) - 1u;
+      if (zh > zb && !mbar_wait(&done[prev % kHRing], (prev / kHRing) & 1)) {
         ok = false;
         atomicExch(status, HDOG_ERR_TIMEOUT);
       }
@@ -634,33 +653,23 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
         for (int o = 0; o < 4; o++) mo[o] = (uint8_t)(mword >> (8 * o));
       }
     } else {
+      const bool ym = Y >= 1, yp = Y + 1 < H, zm = zh >= 1, zp = zh + 1 < D;
+      const int p0 = slot(zh) * PL + b, p1 = slot(zh + 1) * PL + b, p2 = slot(zh + 2) * PL + b;
+      const int m1 = slot(zh - 1) * PL + b, m2 = slot(zh - 2) * PL + b;
 #pragma unroll
       for (int o = 0; o < 4; o++) {
         const int X = X0 + o;
         if (X >= W || Y >= H) continue;
-        const int ex = 4 * q + o + 4, ey = ly + 2;
-        auto Dv = [&](int ddx, int ddy, int ddz) -> float {
-          return ring[slot(zh + ddz) * PL + (ey + ddy) * kHPX + (ex + ddx)];
-        };
-        auto in_vol = [&](int ddx, int ddy, int ddz) -> bool {
-          const int xx = X + ddx, yy = Y + ddy, zz = zh + ddz;
-          return xx >= 0 && xx < W && yy >= 0 && yy < H && zz >= 0 && zz < D;
-        };
-        auto GX = [&](int ddx, int ddy, int ddz) -> float {
-          return in_vol(ddx, ddy, ddz) ? hdiff(Dv(ddx + 1, ddy, ddz), Dv(ddx - 1, ddy, ddz)) : 0.0f;
-        };
-        auto GY = [&](int ddx, int ddy, int ddz) -> float {
-          return in_vol(ddx, ddy, ddz) ? hdiff(Dv(ddx, ddy + 1, ddz), Dv(ddx, ddy - 1, ddz)) : 0.0f;
-        };
-        auto GZ = [&](int ddz) -> float {
-          return in_vol(0, 0, ddz) ? hdiff(Dv(0, 0, ddz + 1), Dv(0, 0, ddz - 1)) : 0.0f;
-        };
-        hv[o][0] = hdiff(GX(1, 0, 0), GX(-1, 0, 0));
-        hv[o][1] = hdiff(GX(0, 1, 0), GX(0, -1, 0));
-        hv[o][2] = hdiff(GX(0, 0, 1), GX(0, 0, -1));
-        hv[o][3] = hdiff(GY(0, 1, 0), GY(0, -1, 0));
-        hv[o][4] = hdiff(GY(0, 0, 1), GY(0, 0, -1));
-        hv[o][5] = hdiff(GZ(1), GZ(-1));
+        // the slices hold zeros outside the volume, so a first derivative only needs the zero of its own
+        // position outside: past the frame's sides (xm .. yp) or the first and last slice (zm, zp)
+        const bool xm = X >= 1, xp = X + 1 < W;
+        const float *c0 = ring + p0 + o, *cu = ring + p1 + o, *cd = ring + m1 + o;
+        hv[o][0] = hdiff(xp ? hdiff(c0[2], c0[0]) : 0.0f, xm ? hdiff(c0[0], c0[-2]) : 0.0f);
+        hv[o][1] = hdiff(yp ? hdiff(c0[kHPX + 1], c0[kHPX - 1]) : 0.0f, ym ? hdiff(c0[1 - kHPX], c0[-1 - kHPX]) : 0.0f);
+        hv[o][2] = hdiff(zp ? hdiff(cu[1], cu[-1]) : 0.0f, zm ? hdiff(cd[1], cd[-1]) : 0.0f);
+        hv[o][3] = hdiff(yp ? hdiff(c0[2 * kHPX], c0[0]) : 0.0f, ym ? hdiff(c0[0], c0[-2 * kHPX]) : 0.0f);
+        hv[o][4] = hdiff(zp ? hdiff(cu[kHPX], cu[-kHPX]) : 0.0f, zm ? hdiff(cd[kHPX], cd[-kHPX]) : 0.0f);
+        hv[o][5] = hdiff(zp ? hdiff(ring[p2 + o], c0[0]) : 0.0f, zm ? hdiff(c0[0], ring[m2 + o]) : 0.0f);
         const bool pdv = pd_test(hv[o][0], hv[o][1], hv[o][2], hv[o][3], hv[o][4], hv[o][5]);
         mask[S.vox + i0 + o] = pdv ? 1 : 0;
         // voxel 0 is background (its label is 0 in the reference's CCL)
@@ -696,7 +705,7 @@ __global__ void __launch_bounds__(kHThreads, HDOG_HESS_BLOCKS)
       staged += tot;
     }
     __syncwarp();
-    if ((t & 31) == 0) mbar_arrive(&done[(ibase + (uint32_t)zh) % kHRing]);
+    if ((t & 31) == 0) mbar_arrive(&done[(ibase + (uint32_t)(zh - zb)) % kHRing]);
   }
   if (staged) flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
   zbase += (uint32_t)(D + 4);
@@ -808,15 +817,21 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
     zero_async(qctr + 1, sizeof(unsigned), s);
     const WorkQueue q{qctr + 1, (int)(tiles_h * (unsigned)nsub), (int)tiles_h};
     const unsigned grid = std::min<unsigned>((unsigned)(ls.hess_per_sm * ls.num_sms), tiles_h * (unsigned)nsub);
-    auto fn = P != W ? k_hess_sweep<true, true> : k_hess_sweep<true, false>;
+    auto fn = P != W ? k_hess_sweep<true, true, false> : k_hess_sweep<true, false, false>;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
     KLAUNCH("k_hess_sweep", s, (fn<<<grid, kHThreads, kHessSmem, s>>>(map_d, d_subs, norm, mask, fg, fg_idx, fg_count,
-                                                                      d_status, q)));
+                                                                      d_status, q, D)));
   } else {
-    auto fn = P != W ? k_hess_sweep<false, true> : k_hess_sweep<false, false>;
+    // split z while the blocks about fit the chip at once (four per SM, and half as many again while those run), down
+    // to six slices: a piece spends about two slices' time on the four it loads around its own.  256x256x32 alone: one
+    // piece 63 us, five 30 us; 683x517x75, whose tiles fill the chip, 221 us unsplit
+    const int64_t room = (int64_t)6 * ls.num_sms / ((int64_t)tiles_h * nsub);
+    const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(room, D / 6)), zlen = (int)ceil_div(D, pieces);
+    auto fn = zlen < D ? (P != W ? k_hess_sweep<false, true, true> : k_hess_sweep<false, false, true>)
+                       : (P != W ? k_hess_sweep<false, true, false> : k_hess_sweep<false, false, false>);
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
-    KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub), kHThreads, kHessSmem, s>>>(map_d, d_subs, norm, mask, fg, fg_idx,
-                                                                                     fg_count, d_status, WorkQueue{})));
+    KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub, ceil_div(D, zlen)), kHThreads, kHessSmem, s>>>(
+                                   map_d, d_subs, norm, mask, fg, fg_idx, fg_count, d_status, WorkQueue{}, zlen)));
   }
   return 0;
 }
