@@ -542,6 +542,7 @@ static ClearList batch_zeros(hdog_ctx *c, int nsub, bool fused) {
   z.add(c->edge_count, nsub * sizeof(unsigned long long));
   z.add(c->rec_counts, (size_t)nsub * c->nblk * sizeof(uint32_t));
   if (fused) {
+    z.add(c->qctr, 2 * sizeof(unsigned));
     z.add(c->fg_count, (size_t)nsub * kFgCountStride * sizeof(unsigned long long));
     z.add(c->root_bits, (size_t)nsub * c->nblk * (kScanBlock / 32) * sizeof(uint32_t));
     z.add(c->blk_counts, (size_t)nsub * c->nblk * sizeof(uint32_t));
@@ -1217,8 +1218,8 @@ static int tune_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
   struct Cand {
     int dog, hess;
   };
-  // grid form, and persistent grids at and below the sweeps' occupancy (three DoG blocks,
-  // five Hessian blocks per SM)
+  // grid form, and persistent grids at and below the sweeps' occupancy (two or three DoG blocks by its tile,
+  // five Hessian blocks per SM; blocks beyond it find the queue empty)
   const Cand cands[] = {{0, 0}, {3, 5}, {2, 4}};
   double dog_ms[3] = {0, 0, 0}, hess_ms[3] = {0, 0, 0}, all_ms[3] = {0, 0, 0};
   c->shape = LaunchShape{};

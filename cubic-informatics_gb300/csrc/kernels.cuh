@@ -125,7 +125,7 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
 
 // Ranges of 32-bit words that one kernel zeroes.
 struct ClearList {
-  static constexpr int kMax = 6;
+  static constexpr int kMax = 8;   // a fused batch adds seven
   uint32_t *p[kMax];
   int64_t n[kMax];
   int count = 0;
@@ -159,7 +159,7 @@ bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int P, int H, int D, c
                       float *dog, int *d_status, int max_smem, cudaStream_t s);
 // DoG + Hessian + PD: norm -> dog by the radius-specialised sweep, or by the separate passes (temporaries
 // fa, fb) where the tap radii have no instantiation, then dog -> mask + list by the Hessian sweep.
-// ls / qctr (two device counters): the launch shape of the sweeps.
+// ls / qctr (two device counters, zero at the call): the launch shape of the sweeps.
 int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
                     float2 *fa, float2 *fb, float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count,
                     int *d_status, const LaunchShape &ls, unsigned *qctr, int max_smem, cudaStream_t s);

@@ -29,14 +29,15 @@ __device__ __forceinline__ void tma_slice(const CUtensorMap *map, float *dst, ui
 // For common sigma pairs the chain runs as two z-sweeps with the four tap radii as
 // template parameters (RA/RB: xy radius of the small/large scale, ZA/ZB: z radius):
 //
-//   k_dog_sweep   normalized -> DoG volume.  A block owns a kDTX x kDTY tile and sweeps
+//   k_dog_sweep   normalized -> DoG volume.  A block owns a 32 x 24 tile (32 x 16 of
+//                 a small batch) and sweeps
 //                 z; stage A filters slice it along x (TMA-loaded, double-buffered), stage
 //                 B filters slice it-1 along y and feeds the z shift register, which emits
 //                 DoG slice it-1-RZ straight to global memory.  One barrier per slice.
 //                 Tap pairs shared by both scales sit in per-thread registers, the taps of
 //                 the wider scale alone are constant-bank operands.  The z shift
-//                 register never moves: output zo lives in slot zo mod (2RZ+1), and a
-//                 switch on the step's phase picks the compile-time slot of every tap.
+//                 register never moves: output zo lives in slot zo mod (2RZ+1), and the loop
+//                 is unrolled over one turn, so the slot of every tap is known when compiling.
 //                 Every output is the reference's FMA chain, zero taps at the borders
 //                 included, so the volume equals the separate passes bit for bit.
 //   k_hess_sweep  DoG -> mask + foreground list.  A block owns a kHTX x kHTY tile; DoG slices
@@ -48,7 +49,7 @@ __device__ __forceinline__ void tma_slice(const CUtensorMap *map, float *dst, ui
 //
 // The split costs one write and one read of the DoG volume but frees the Hessian stage
 // from the z shift register's registers, so several Hessian blocks share an SM.
-constexpr int kDTX = 32, kDTY = 16;     // DoG tile (three 256-thread blocks per SM, 80 registers)
+constexpr int kDTX = 32;                // DoG tile width
 constexpr int kHTX = 32, kHTY = 16;     // Hessian tile (six blocks per SM)
 constexpr int kHPX = kHTX + 8;          // Hessian ring row: columns x0-4 .. x0+kHTX+3 (16-byte aligned start)
 constexpr int kHPY = kHTY + 4;
@@ -63,20 +64,26 @@ constexpr int kHThreads = kHTX / 4 * kHTY;   // one x quad per thread
 #endif
 constexpr int kDogIn = HDOG_DOG_STAGES;
 
-template <int RA, int RB, int ZA, int ZB>
+// ROWS: rows of the tile's columns a thread takes through the y pass and the z register.  The y pass reads 2R + ROWS
+// x-filtered values for ROWS outputs from shared memory and the x pass filters 2R halo rows for a tile of NT / 32 * ROWS,
+// so with two rows (a 32 x 16 tile, 80 registers, three blocks of 256 per SM) the shared-memory pipe was the limit (73%);
+// four rows (32 x 24, 138 registers, two blocks of 192) leave it at 58% and the issue slots at 59%.  1.42 G voxels of
+// radii (4, 6, 3, 5) 6.30 -> 5.63 ms, 0.71 G of (8, 12, 4, 5) 5.30 -> 4.29 ms.  Three rows (5.84 ms), five (6.07), one
+// copy of the code for all z phases (6.37) and x pairs instead of scale pairs in the x pass (6.8) were slower.
+template <int RA, int RB, int ZA, int ZB, int ROWS>
 struct DogT {
   static constexpr int RXY = RA > RB ? RA : RB;
   static constexpr int RZ = ZA > ZB ? ZA : ZB;
   static constexpr int WIN = 2 * RZ + 1;
+  static constexpr int NT = ROWS == 4 ? 192 : 256, BLOCKS = ROWS == 4 ? 2 : 3;
+  static constexpr int TY = NT / kDTX * ROWS;                 // tile height
   static constexpr int HX = (RXY + 3) / 4 * 4;                // x halo, 16-byte aligned
   static constexpr int BW = kDTX + 2 * HX;                    // staged input box
-  static constexpr int BH = kDTY + 2 * RXY;
+  static constexpr int BH = TY + 2 * RXY;
   static constexpr int IN_FLOATS = (BW * BH + 31) / 32 * 32;  // 128-byte multiple
-  static constexpr int XQ = kDTX / 4;                         // x-pass items per row
+  static constexpr int XQ = kDTX / 4;                         // x-pass items of four outputs per row
   static constexpr int XITEMS = BH * XQ;
-  static constexpr int OFF = HX - RXY;                        // item q reads from column 4q + OFF
-  static constexpr int NV = (OFF + 2 * RXY + 4 + 3) / 4 * 4;  // inputs staged per item
-  static constexpr int NT = kDTX * kDTY / 2;                  // 256: two z columns per thread
+  static constexpr int NV = (HX + RXY + 4 + 3) / 4 * 4;       // inputs of an item, from column 4q
   static constexpr size_t SMEM = (size_t)kDogIn * IN_FLOATS * 4 + (size_t)2 * BH * kDTX * 8 + 8 * kDogIn + 64;
 };
 
@@ -87,18 +94,14 @@ struct DogT {
 template <int RA, int RB>
 struct TapPairs {
   static constexpr int RS = RA < RB ? RA : RB;
-  float2 k[2 * RS + 1];
-  static constexpr int N = 2 * RS + 1;
-  __device__ __forceinline__ void load(const DogTaps &T, int ka, int kb) {
-#pragma unroll
-    for (int j = -RS; j <= RS; j++) k[j + RS] = make_float2(T.k[ka][RA - j], T.k[kb][RB - j]);
-  }
+  static constexpr int N = RS + 1;
+  float2 k[N];   // pair |j|: the taps are symmetric
   // The pairs as written by stage(): read back from shared memory, they are per-thread
   // registers, so the f32x2 FMAs use them directly instead of copying each pair out of
   // the uniform registers a kernel-parameter value would live in.
   __device__ __forceinline__ static void stage(const DogTaps &T, int ka, int kb, float2 *sh) {
 #pragma unroll
-    for (int j = -RS; j <= RS; j++) sh[j + RS] = make_float2(T.k[ka][RA - j], T.k[kb][RB - j]);
+    for (int j = 0; j <= RS; j++) sh[j] = make_float2(T.k[ka][RA - j], T.k[kb][RB - j]);
   }
   __device__ __forceinline__ void load_shared(const float2 *sh) {
 #pragma unroll
@@ -112,7 +115,7 @@ template <int RA, int RB, int J>
 __device__ __forceinline__ void tap2(const DogTaps &T, const TapPairs<RA, RB> &K, int ka, int kb, float2 v,
                                      float2 &acc) {
   constexpr bool a = J >= -RA && J <= RA, b = J >= -RB && J <= RB;
-  if (a && b) acc = fma2(K.k[J + TapPairs<RA, RB>::RS], v, acc);
+  if (a && b) acc = fma2(K.k[J < 0 ? -J : J], v, acc);
   else if (b) acc.y = __fmaf_rn(T.k[kb][RB - J], v.y, acc.y);
   else if (a) acc.x = __fmaf_rn(T.k[ka][RA - J], v.x, acc.x);
 }
@@ -135,33 +138,23 @@ struct XIn {
   }
 };
 
-template <int RA, int RB, int J, int N>
-struct TapLoop {
-  // x pass: taps J .. J+N-1 for the four outputs of an item
-  template <int NV>
-  __device__ __forceinline__ static void x4(const DogTaps &T, const TapPairs<RA, RB> &K, const float (&w)[NV],
-                                            int base, float2 (&a)[4]) {
-    if constexpr (N > 0) {
-#pragma unroll
-      for (int o = 0; o < 4; o++) {
-        const float x = w[base + o + J];
-        tap2<RA, RB, J>(T, K, 0, 2, make_float2(x, x), a[o]);
-      }
-      TapLoop<RA, RB, J + 1, N - 1>::x4(T, K, w, base, a);
+// y pass of ROWS rows, input row by input row: row I is tap I - R - o of output row o, read once, and every
+// output still takes its taps in ascending order.
+template <int RA, int RB, int ROWS, int I, int N>
+struct YIn {
+  static constexpr int R = RA > RB ? RA : RB;
+  template <int O>
+  __device__ __forceinline__ static void taps(const DogTaps &T, const TapPairs<RA, RB> &K, float2 v, float2 (&g)[ROWS]) {
+    if constexpr (O < ROWS) {
+      if constexpr (I - R - O >= -R && I - R - O <= R) tap2<RA, RB, I - R - O>(T, K, 0, 2, v, g[O]);
+      taps<O + 1>(T, K, v, g);
     }
   }
-  // y pass of rows cy (g0) and cy + 1 (g1): input row i is tap i - R of g0 and tap
-  // i - R - 1 of g1, loaded once, in ascending tap order for both
-  template <int STRIDE>
-  __device__ __forceinline__ static void y2(const DogTaps &T, const TapPairs<RA, RB> &K, const float2 *col,
-                                            float2 &g0, float2 &g1) {
-    if constexpr (N > 0) {
-      constexpr int R = RA > RB ? RA : RB;
-      const float2 v = col[(J + R) * STRIDE];
-      tap2<RA, RB, J>(T, K, 0, 2, v, g0);
-      if constexpr (J > -R) tap2<RA, RB, J - 1>(T, K, 0, 2, v, g1);
-      if constexpr (N == 1) tap2<RA, RB, J>(T, K, 0, 2, col[(J + R + 1) * STRIDE], g1);
-      TapLoop<RA, RB, J + 1, N - 1>::template y2<STRIDE>(T, K, col, g0, g1);
+  __device__ __forceinline__ static void run(const DogTaps &T, const TapPairs<RA, RB> &K, const float2 *col,
+                                             float2 (&g)[ROWS]) {
+    if constexpr (I < N) {
+      taps<0>(T, K, col[I * kDTX], g);
+      YIn<RA, RB, ROWS, I + 1, N>::run(T, K, col, g);
     }
   }
 };
@@ -169,28 +162,29 @@ struct TapLoop {
 // z step of phase P = zy mod WIN: input slice zy is tap d of output zo = zy - d, which
 // lives in slot (zo mod WIN); then output zy - RZ is complete and its slot is cleared for
 // output zy - RZ + WIN.
-template <class C, int ZA, int ZB, int P, int D0, int N>
+template <class C, int ZA, int ZB, int ROWS, int P, int D0, int N>
 struct ZTaps {
-  __device__ __forceinline__ static void run(const DogTaps &T, const TapPairs<ZA, ZB> &K, float2 (&a0)[C::WIN],
-                                             float2 (&a1)[C::WIN], float2 g0, float2 g1) {
+  __device__ __forceinline__ static void run(const DogTaps &T, const TapPairs<ZA, ZB> &K, float2 (&a)[ROWS][C::WIN],
+                                             const float2 (&g)[ROWS]) {
     if constexpr (N > 0) {
       constexpr int s = ((P - D0) % C::WIN + C::WIN) % C::WIN;
-      tap2<ZA, ZB, D0>(T, K, 1, 3, g0, a0[s]);
-      tap2<ZA, ZB, D0>(T, K, 1, 3, g1, a1[s]);
-      ZTaps<C, ZA, ZB, P, D0 + 1, N - 1>::run(T, K, a0, a1, g0, g1);
+#pragma unroll
+      for (int o = 0; o < ROWS; o++) tap2<ZA, ZB, D0>(T, K, 1, 3, g[o], a[o][s]);
+      ZTaps<C, ZA, ZB, ROWS, P, D0 + 1, N - 1>::run(T, K, a, g);
     }
   }
 };
 
-template <class C, int ZA, int ZB, int P>
-__device__ __forceinline__ void z_step(const DogTaps &T, const TapPairs<ZA, ZB> &K, float2 (&a0)[C::WIN],
-                                       float2 (&a1)[C::WIN], float2 g0, float2 g1, float &d0, float &d1) {
-  ZTaps<C, ZA, ZB, P, -C::RZ, C::WIN>::run(T, K, a0, a1, g0, g1);
+template <class C, int ZA, int ZB, int ROWS, int P>
+__device__ __forceinline__ void z_step(const DogTaps &T, const TapPairs<ZA, ZB> &K, float2 (&a)[ROWS][C::WIN],
+                                       const float2 (&g)[ROWS], float (&d)[ROWS]) {
+  ZTaps<C, ZA, ZB, ROWS, P, -C::RZ, C::WIN>::run(T, K, a, g);
   constexpr int se = ((P - C::RZ) % C::WIN + C::WIN) % C::WIN;
-  d0 = __fmul_rn(__fsub_rn(a0[se].x, a0[se].y), T.normalizer);
-  d1 = __fmul_rn(__fsub_rn(a1[se].x, a1[se].y), T.normalizer);
-  a0[se] = make_float2(0.f, 0.f);
-  a1[se] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int o = 0; o < ROWS; o++) {
+    d[o] = __fmul_rn(__fsub_rn(a[o][se].x, a[o][se].y), T.normalizer);
+    a[o][se] = make_float2(0.f, 0.f);
+  }
 }
 
 // Calls f(base + P, integral_constant<P>) for P = 0 .. N-1 while base + P < limit (the
@@ -212,15 +206,15 @@ __device__ __forceinline__ void unroll_steps(F &f, int base, int limit) {
 // PERSIST: a grid of a few blocks per SM takes (substack, tile) items from the device work
 // queue `q` until it is empty; otherwise one block per tile (blockIdx.x) and substack
 // (blockIdx.y).  Results are the same either way.
-template <int RA, int RB, int ZA, int ZB, bool PERSIST>
-__global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
+template <int RA, int RB, int ZA, int ZB, int ROWS, bool PERSIST>
+__global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB, ROWS>::NT, DogT<RA, RB, ZA, ZB, ROWS>::BLOCKS)
     k_dog_sweep(const __grid_constant__ CUtensorMap map, const __grid_constant__ DogTaps T, const Sub *subs,
                 float *dog, int *status, WorkQueue q) {
-  using C = DogT<RA, RB, ZA, ZB>;
+  using C = DogT<RA, RB, ZA, ZB, ROWS>;
   extern __shared__ __align__(128) unsigned char smem[];
   float *inb = reinterpret_cast<float *>(smem);
-  float2 *xb = reinterpret_cast<float2 *>(smem + (size_t)kDogIn * C::IN_FLOATS * 4);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kDogIn * C::IN_FLOATS * 4 + (size_t)2 * C::BH * kDTX * 8);
+  float2 *xb = reinterpret_cast<float2 *>(inb + kDogIn * C::IN_FLOATS);   // two x-filtered slices, both scales
+  uint64_t *bar = reinterpret_cast<uint64_t *>(xb + 2 * C::BH * kDTX);
   const int t = threadIdx.x;
   __shared__ float2 tap_sh[TapPairs<RA, RB>::N + TapPairs<ZA, ZB>::N];
   __shared__ int s_item;
@@ -249,12 +243,12 @@ __global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
     tile = blockIdx.x;
   }
   const Sub S = subs[sub];
-  const int ntx = (S.W + kDTX - 1) / kDTX, nty = (S.H + kDTY - 1) / kDTY;
+  const int ntx = (S.W + kDTX - 1) / kDTX, nty = (S.H + C::TY - 1) / C::TY;
   if (tile >= ntx * nty) {
     if (PERSIST) continue;
     break;
   }
-  const int x0 = (tile % ntx) * kDTX, y0 = (tile / ntx) * kDTY;
+  const int x0 = (tile % ntx) * kDTX, y0 = (tile / ntx) * C::TY;
   const int D = S.D, W = S.W, H = S.H;
   constexpr uint32_t tma_bytes = (uint32_t)(C::BW * C::BH * 4);
   const int tx = x0 - C::HX, ty = y0 - C::RXY;
@@ -263,15 +257,18 @@ __global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
       const uint32_t g = gbase + (uint32_t)z;
       tma_slice(&map, inb + (g % kDogIn) * C::IN_FLOATS, &bar[g % kDogIn], tx, ty, z, sub, tma_bytes);
     }
-  // stage B ownership: columns (cx, cy) and (cx, cy + 1) of the tile
-  const int cx = t % kDTX, cy = 2 * (t / kDTX);
+  // stage B ownership: columns (cx, cy .. cy + ROWS - 1) of the tile
+  const int cx = t % kDTX, cy = ROWS * (t / kDTX);
   const int gx = x0 + cx, gy = y0 + cy;
-  const bool w0 = gx < W && gy < H, w1 = gx < W && gy + 1 < H;
+  const float2 *yin = xb + cy * kDTX + cx;
+  const int nrow = gx < W ? H - gy : 0;   // rows of them inside the frame
   float *out0 = dog + S.pvox + (int64_t)gy * S.P + gx;
   const int64_t WH = (int64_t)S.P * H;
-  float2 acc0[C::WIN], acc1[C::WIN];
+  float2 acc[ROWS][C::WIN];
 #pragma unroll
-  for (int s = 0; s < C::WIN; s++) { acc0[s] = make_float2(0.f, 0.f); acc1[s] = make_float2(0.f, 0.f); }
+  for (int o = 0; o < ROWS; o++)
+#pragma unroll
+    for (int s = 0; s < C::WIN; s++) acc[o][s] = make_float2(0.f, 0.f);
   TapPairs<RA, RB> kxy;
   TapPairs<ZA, ZB> kz;
   kxy.load_shared(tap_sh);
@@ -290,16 +287,18 @@ __global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
     // z shift register, DoG slice zy - RZ
     const int zy = it - 1;
     if (zy >= 0) {
-      float2 g0 = make_float2(0.f, 0.f), g1 = make_float2(0.f, 0.f);
+      float2 g[ROWS];
+#pragma unroll
+      for (int o = 0; o < ROWS; o++) g[o] = make_float2(0.f, 0.f);
       if (zy < D)
-        TapLoop<RA, RB, -C::RXY, 2 * C::RXY + 1>::template y2<kDTX>(
-            T, kxy, xb + (zy & 1) * C::BH * kDTX + cy * kDTX + cx, g0, g1);
-      float d0, d1;
-      z_step<C, ZA, ZB, PH>(T, kz, acc0, acc1, g0, g1, d0, d1);
+        YIn<RA, RB, ROWS, 0, 2 * C::RXY + ROWS>::run(T, kxy, yin + (zy & 1) * C::BH * kDTX, g);
+      float d[ROWS];
+      z_step<C, ZA, ZB, ROWS, PH>(T, kz, acc, g, d);
       const int zo = zy - C::RZ;
       if (zo >= 0) {
-        if (w0) out0[zo * WH] = d0;
-        if (w1) out0[zo * WH + S.P] = d1;
+#pragma unroll
+        for (int o = 0; o < ROWS; o++)
+          if (o < nrow) out0[zo * WH + o * S.P] = d[o];
       }
     }
     // ---- A: x pass of slice it
@@ -311,7 +310,6 @@ __global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
       }
       const float *ib = inb + (gi % kDogIn) * C::IN_FLOATS;
       float2 *xo = xb + (it & 1) * C::BH * kDTX;
-      // one item per thread when the items fit the block (no loop, no reconvergence)
       for (int item = t; item < C::XITEMS; item += (C::XITEMS <= C::NT ? C::XITEMS : C::NT)) {
         const int row = item / C::XQ, q = item % C::XQ;
         const float *in = ib + row * C::BW + 4 * q;
@@ -321,9 +319,9 @@ __global__ void __launch_bounds__(DogT<RA, RB, ZA, ZB>::NT, 3)
           const float4 f = *reinterpret_cast<const float4 *>(in + i);
           w[i] = f.x; w[i + 1] = f.y; w[i + 2] = f.z; w[i + 3] = f.w;
         }
-        float2 a[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        XIn<RA, RB, C::OFF + C::RXY, 0, C::NV>::run(T, kxy, w, a);
         float4 *o = reinterpret_cast<float4 *>(xo + row * kDTX + 4 * q);
+        float2 a[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        XIn<RA, RB, C::HX, 0, C::NV>::run(T, kxy, w, a);
         o[0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
         o[1] = make_float4(a[2].x, a[2].y, a[3].x, a[3].y);
       }
@@ -734,23 +732,33 @@ static EncodeTiledFn encode_fn() {
 // Radius-specialised instantiations: (small xy, large xy, small z, large z) tap radii.
 // (4, 6, 3, 5): sigma (2.0, 1.5) / (3.2, 2.4); (8, 12, 4, 5): sigma (4.0, 1.8) / (6.0, 2.7).
 typedef void (*DogSweepKernel)(CUtensorMap, DogTaps, const Sub *, float *, int *, WorkQueue);
-struct SweepInst {
-  int ra, rb, za, zb;
+struct SweepForm {
   DogSweepKernel fn, fn_persist;
   size_t smem;
-  int threads, bw, bh, hx, rxy;
+  int threads, ty, bw, bh;
 };
+struct SweepInst {
+  int ra, rb, za, zb;
+  SweepForm form[2];   // two and four rows per thread
+};
+template <int RA, int RB, int ZA, int ZB, int ROWS>
+constexpr SweepForm sweep_form() {
+  using C = DogT<RA, RB, ZA, ZB, ROWS>;
+  return SweepForm{k_dog_sweep<RA, RB, ZA, ZB, ROWS, false>, k_dog_sweep<RA, RB, ZA, ZB, ROWS, true>,
+                   C::SMEM, C::NT, C::TY, C::BW, C::BH};
+}
 template <int RA, int RB, int ZA, int ZB>
 constexpr SweepInst sweep_inst() {
-  using C = DogT<RA, RB, ZA, ZB>;
-  return SweepInst{RA, RB, ZA, ZB, k_dog_sweep<RA, RB, ZA, ZB, false>, k_dog_sweep<RA, RB, ZA, ZB, true>,
-                   C::SMEM, C::NT, C::BW, C::BH, C::HX, C::RXY};
+  return SweepInst{RA, RB, ZA, ZB, {sweep_form<RA, RB, ZA, ZB, 2>(), sweep_form<RA, RB, ZA, ZB, 4>()}};
 }
 static const SweepInst kSweepInst[] = {sweep_inst<4, 6, 3, 5>(), sweep_inst<8, 12, 4, 5>()};
 
-static const SweepInst *find_inst(const DogTaps &T) {
+// The sweep for these taps, or none.  The four-row form where its 32 x 24 tiles give every SM its two blocks; below
+// that the two-row form's smaller ones, whose blocks take a slice sooner (one 128x96x16 substack 11.9 against 13.9 us).
+static const SweepForm *find_form(const DogTaps &T, int W, int H, int nsub, int num_sms) {
   for (const SweepInst &s : kSweepInst)
-    if (s.ra == T.r[0] && s.rb == T.r[2] && s.za == T.r[1] && s.zb == T.r[3]) return &s;
+    if (s.ra == T.r[0] && s.rb == T.r[2] && s.za == T.r[1] && s.zb == T.r[3])
+      return &s.form[(int64_t)ceil_div(W, kDTX) * ceil_div(H, s.form[1].ty) * nsub >= 2 * (int64_t)num_sms];
   return nullptr;
 }
 
@@ -772,13 +780,12 @@ static CUresult encode_map(CUtensorMap *map, const float *base, int W, int P, in
 }
 
 // One launch of a radius-specialised DoG sweep: a block per tile and substack, or (per_sm > 0)
-// per_sm blocks per SM over the work queue whose counter is *qctr (zeroed here first).
-static void dog_sweep_launch(const SweepInst *si, const CUtensorMap &map_n, const DogTaps &T, const Sub *d_subs,
+// per_sm blocks per SM over the work queue whose counter is *qctr (zero at the launch).
+static void dog_sweep_launch(const SweepForm *si, const CUtensorMap &map_n, const DogTaps &T, const Sub *d_subs,
                              int nsub, int W, int H, float *dog, int *d_status, const LaunchShape &ls,
                              unsigned *qctr, cudaStream_t s) {
-  const unsigned tiles_d = ceil_div(W, kDTX) * ceil_div(H, kDTY);
+  const unsigned tiles_d = ceil_div(W, kDTX) * ceil_div(H, si->ty);
   if (ls.dog_per_sm > 0 && qctr) {
-    zero_async(qctr, sizeof(unsigned), s);
     const WorkQueue q{qctr, (int)(tiles_d * (unsigned)nsub), (int)tiles_d};
     const unsigned grid = std::min<unsigned>((unsigned)(ls.dog_per_sm * ls.num_sms), tiles_d * (unsigned)nsub);
     cudaFuncSetAttribute(si->fn_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)si->smem);
@@ -792,7 +799,7 @@ static void dog_sweep_launch(const SweepInst *si, const CUtensorMap &map_n, cons
 
 bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
                       float *dog, int *d_status, int max_smem, cudaStream_t s) {
-  const SweepInst *si = find_inst(T);
+  const SweepForm *si = find_form(T, W, H, nsub, LaunchShape{}.num_sms);
   if (!si || P % 4 != 0 || (int)si->smem > max_smem || encode_fn() == nullptr) return false;
   if ((reinterpret_cast<uintptr_t>(norm) & 15) != 0) return false;
   CUtensorMap map_n;
@@ -805,7 +812,7 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
                     float2 *fa, float2 *fb, float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx,
                     unsigned long long *fg_count, int *d_status, const LaunchShape &ls, unsigned *qctr, int max_smem,
                     cudaStream_t s) {
-  const SweepInst *si = find_inst(T);
+  const SweepForm *si = find_form(T, W, H, nsub, ls.num_sms);
   CUtensorMap map_n, map_d;
   if (encode_map(&map_d, dog, W, P, H, D, nsub, kHPX, kHPY) != CUDA_SUCCESS) return -1;
   if (si && (int)si->smem <= max_smem && encode_map(&map_n, norm, W, P, H, D, nsub, si->bw, si->bh) == CUDA_SUCCESS)
@@ -814,7 +821,6 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
     launch_dog(d_subs, nsub, W, P, H, D, (int64_t)H * D, T, norm, fa, fb, dog, s);
   const unsigned tiles_h = ceil_div(W, kHTX) * ceil_div(H, kHTY);
   if (ls.hess_per_sm > 0 && qctr) {
-    zero_async(qctr + 1, sizeof(unsigned), s);
     const WorkQueue q{qctr + 1, (int)(tiles_h * (unsigned)nsub), (int)tiles_h};
     const unsigned grid = std::min<unsigned>((unsigned)(ls.hess_per_sm * ls.num_sms), tiles_h * (unsigned)nsub);
     auto fn = P != W ? k_hess_sweep<true, true, false> : k_hess_sweep<true, false, false>;

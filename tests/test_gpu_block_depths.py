@@ -1,5 +1,5 @@
 """The component labelling at each of its tile depths (csrc/ccl.cu: 8, 16 and 32 slices by how many tiles there are) and
-the Hessian sweep with its slices split among blocks (csrc/sweep.cu), at depths around a tile's and a piece's end,
+the sweeps of csrc/sweep.cu (the Hessian with its slices split among blocks, the DoG in both its tiles), around their ends,
 against the oracle."""
 import numpy as np
 import pytest
@@ -39,3 +39,23 @@ def test_gpu_records_over_split_slices(W, H, D):
     assert len(got) == len(ref)
     for f in ("local_x", "local_y", "local_z", "intensity", "size"):
         assert np.array_equal(got[f], ref[f]), f
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sig", [(2.0, 1.5, 3.2, 2.4), (4.0, 1.8, 6.0, 2.7)])
+@pytest.mark.parametrize("W,H,D", [(640, 365, 5), (641, 361, 12), (1283, 192, 11), (639, 383, 23), (67, 47, 13), (70, 25, 1)])
+def test_gpu_dog_sweep_tiles(W, H, D, sig):
+    """32 x 24 tiles (at least 304 of them) and 32 x 16 ones, rows and columns left over on every side, depths around
+    one turn of the z register (11)."""
+    import hdog
+    norm = np.random.default_rng(W + H + D).normal(0, 1, (D, H, W)).astype(np.float32)
+    norm[D // 2, H // 2, W // 2] = np.inf
+    norm[0, 1, 2] = np.nan
+    p = hdog.make_params(width=W, height=H, depth=D, sigma_xy_small=sig[0], sigma_z_small=sig[1], sigma_xy_large=sig[2],
+                         sigma_z_large=sig[3])
+    with hdog.Context(p) as ctx:
+        got = ctx.dog(torch.from_numpy(norm).cuda()).cpu().numpy()
+    ref = orc.dog(norm, *sig)
+    nan = np.isnan(ref)
+    assert np.array_equal(np.isnan(got), nan)
+    assert np.array_equal(got[~nan].view(np.uint32), ref[~nan].view(np.uint32))
