@@ -595,32 +595,40 @@ __device__ __forceinline__ void box_chain_t(LoadF load, float2 (&acc)[K]) {
   }
 }
 
-constexpr int kBoxYK = 12;   // y outputs per thread
+// K outputs of a column per thread: a window of K inputs moves through registers, (K + 2r) loads for K (2r + 1) f32x2
+// adds.  The adds are the reference's chains and cannot be shared, so at long reaches the FMA pipe is the bound (reach
+// 100: 7.6 ms of adds in 8.4) and at short ones HBM; running pointers keep the address arithmetic out of it.  2560 x 2160
+// x 16 at reach 16: K = 12 305 us, 16 273, 20 304; reach 64: 760, 720, 718; reach 127: 1421, 1372, 1337.
 
+template <int K>
 __global__ void __launch_bounds__(128) k_box_y(const Sub *subs, int r, const float2 *in, float2 *out) {
   const Sub S = subs[blockIdx.y];
-  const int rows_per_blk = blockDim.y * kBoxYK;
+  const int rows_per_blk = blockDim.y * K;
   const int tx_n = (S.W + 31) / 32, ty_n = (S.H + rows_per_blk - 1) / rows_per_blk;
   const int64_t bid = blockIdx.x;
   if (bid >= (int64_t)tx_n * ty_n * S.D) return;
   const int z = (int)(bid / ((int64_t)tx_n * ty_n));
   const int rem = (int)(bid % ((int64_t)tx_n * ty_n));
   const int x = (rem % tx_n) * 32 + threadIdx.x;
-  const int y0 = (rem / tx_n) * rows_per_blk + threadIdx.y * kBoxYK;
+  const int y0 = (rem / tx_n) * rows_per_blk + threadIdx.y * K;
   if (x >= S.W || y0 >= S.H) return;
   const int H = S.H, W = S.W, L = 2 * r + 1;
   const float2 *col = in + S.vox + (int64_t)z * W * H + x;
-  float2 acc[kBoxYK];
-  if (y0 - r >= 0 && y0 + kBoxYK + r <= H) {
+  float2 acc[K];
+  if (y0 - r >= 0 && y0 + K + r <= H) {
     const float2 *p = col + (int64_t)(y0 - r) * W;
-    box_chain<kBoxYK>(L, [&](int i) { return __ldg(p + (int64_t)i * W); }, acc);
+    box_chain<K>(L, [&](int) {   // loads its inputs in order
+      const float2 v = __ldg(p);
+      p += W;
+      return v;
+    }, acc);
   } else {
-    box_chain<kBoxYK>(L, [&](int i) { return __ldg(col + (int64_t)clampi(y0 - r + i, 0, H - 1) * W); }, acc);
+    box_chain<K>(L, [&](int i) { return __ldg(col + (int64_t)clampi(y0 - r + i, 0, H - 1) * W); }, acc);
   }
   const float inv = 1.0f / (float)L;
   float2 *o = out + S.vox + (int64_t)z * W * H + x;
 #pragma unroll
-  for (int k = 0; k < kBoxYK; k++)
+  for (int k = 0; k < K; k++)
     if (y0 + k < H) o[(int64_t)(y0 + k) * W] = mul2(acc[k], make_float2(inv, inv));
 }
 
@@ -699,34 +707,46 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
   }
 }
 
-// The same pass specialised on the z radius: one thread per (column, chunk of kBoxZK
-// slices), every window input loaded before the first add so that all loads of a thread
-// are in flight together; threadIdx.y picks the chunk, so the chunks of one column share
-// their overlapping inputs through L1.  PARTS also stores the box means (stage dumps).
+// The same pass specialised on the z radius: one thread per (column, chunk of kBoxZK slices), every window input loaded
+// before the first add so that all loads of a thread are in flight together; neighbouring blocks take the chunks of the
+// same columns, which share their overlapping inputs through the caches.  Bound by HBM (14 bytes a voxel) once the
+// instructions around the loads are few: chunks whose window lies inside the volume walk two pointers instead of clamping
+// and multiplying every index, and ten blocks fit an SM.  1.42 G voxels at reach 5: 4.23 -> 3.60 ms (5.5 TB/s); chunks of
+// 6 (3.88 ms), 10 (4.48) and 12 (4.42), and a register ring down the column (5.9) are slower.  PARTS also stores the box
+// means (stage dumps).
 template <int RZ, bool PARTS, bool PAD>
-__global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min_intensity, const float2 *in,
+__global__ void __launch_bounds__(128, RZ <= 5 ? 10 : 6) k_box_z_norm_t(const Sub *subs, float min_intensity, const float2 *in,
                                                       float *norm, float *ero_l, float *dil_l) {
   constexpr int L = 2 * RZ + 1, NW = kBoxZK + 2 * RZ;
   const Sub S = subs[blockIdx.y];
-  const int64_t plane = (int64_t)S.W * S.H;
-  const int nch = (S.D + kBoxZK - 1) / kBoxZK;
-  const int64_t p = (int64_t)(blockIdx.x / nch) * 128 + threadIdx.x;
+  const int plane = S.W * S.H, D = S.D;
+  const int nch = (D + kBoxZK - 1) / kBoxZK;
+  const int p = (int)(blockIdx.x / nch) * 128 + threadIdx.x;
   const int z0 = (int)(blockIdx.x % nch) * kBoxZK;
-  const int D = S.D;
   if (p >= plane) return;
   const float2 *col = in + S.vox + p;
+  const uint16_t *src = S.src + p;
   float2 win[NW];
-#pragma unroll
-  for (int i = 0; i < NW; i++) win[i] = __ldg(col + clampi(z0 - RZ + i, 0, D - 1) * plane);
   float v[kBoxZK];
+  if (z0 >= RZ && z0 + kBoxZK + RZ <= D && z0 + kBoxZK <= S.depth_valid) {
+    const float2 *c = col + (int64_t)(z0 - RZ) * plane;
+    const uint16_t *s = src + (int64_t)z0 * plane;
 #pragma unroll
-  for (int k = 0; k < kBoxZK; k++) {
-    const int z = min(z0 + k, D - 1);
-    v[k] = z < S.depth_valid ? (float)__ldg(S.src + z * plane + p) : 0.0f;
+    for (int i = 0; i < NW; i++) { win[i] = __ldg(c); c += plane; }
+#pragma unroll
+    for (int k = 0; k < kBoxZK; k++) { v[k] = (float)__ldg(s); s += plane; }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NW; i++) win[i] = __ldg(col + (int64_t)clampi(z0 - RZ + i, 0, D - 1) * plane);
+#pragma unroll
+    for (int k = 0; k < kBoxZK; k++) {
+      const int z = min(z0 + k, D - 1);
+      v[k] = z < S.depth_valid ? (float)__ldg(src + (int64_t)z * plane) : 0.0f;
+    }
   }
   const float inv = 1.0f / (float)L;
-  float *nout = norm + norm_at<PAD>(S, p);
-  const int64_t pplane = PAD ? (int64_t)S.P * S.H : plane;
+  const int pplane = PAD ? S.P * S.H : plane;
+  float *nout = norm + norm_at<PAD>(S, p) + (int64_t)z0 * pplane;
 #pragma unroll
   for (int k = 0; k < kBoxZK; k++) {
     float2 acc = make_float2(0.f, 0.f);
@@ -735,10 +755,11 @@ __global__ void __launch_bounds__(128) k_box_z_norm_t(const Sub *subs, float min
     const int z = z0 + k;
     if (z < D) {
       const float2 el = mul2(acc, make_float2(inv, inv));
-      nout[z * pplane] = (v[k] >= min_intensity) ? (v[k] - el.x) / (el.y - el.x) : 0.0f;
+      *nout = (v[k] >= min_intensity) ? (v[k] - el.x) / (el.y - el.x) : 0.0f;
+      nout += pplane;
       if (PARTS) {
-        ero_l[S.vox + z * plane + p] = el.x;
-        dil_l[S.vox + z * plane + p] = el.y;
+        ero_l[S.vox + (int64_t)z * plane + p] = el.x;
+        dil_l[S.vox + (int64_t)z * plane + p] = el.y;
       }
     }
   }
@@ -899,8 +920,9 @@ void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, i
     dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * K) * D), nsub);
     KLAUNCH("k_box_y", s, (k_box_y_t<20, K><<<gy, dim3(32, by), 0, s>>>(d_subs, fa, fb)));
   } else {
-    dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * kBoxYK) * D), nsub);
-    KLAUNCH("k_box_y", s, (k_box_y<<<gy, dim3(32, by), 0, s>>>(d_subs, rxy, fa, fb)));
+    const int K = rxy < 64 ? 16 : 20;
+    dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * K) * D), nsub);
+    KLAUNCH("k_box_y", s, ((K == 16 ? k_box_y<16> : k_box_y<20>)<<<gy, dim3(32, by), 0, s>>>(d_subs, rxy, fa, fb)));
   }
   const dim3 gz(ceil_div(plane, 128) * ceil_div(D, kBoxZK), nsub), bz(128);
   switch (rz) {
