@@ -77,7 +77,8 @@ __device__ __forceinline__ void back_offset(int k, int &dz, int &dy, int &dx) {
 // Tiles of 64 x 16 voxels and TZ slices.  A block works through its tile's layers one after the other, so
 // where the 32-slice tiles would leave most of the chip idle (fewer than two per SM) they are 16 slices
 // deep, and 8 where even those are fewer than one for two SMs: more cross-tile edges, but shorter blocks and
-// more of them.  One 128x96x16 substack 27 -> 16 us, one of 256x256x32 50 -> 31 us.
+// more of them.  One 128x96x16 substack 27 -> 16 us, one of 256x256x32 50 -> 31 us
+// (13.6 and 24.6 with the cells' tests packed as below).
 constexpr int kTX = 64, kTY = 16;
 constexpr int kCclThreads = 256;              // thread = 4 x-consecutive voxels of one row, all TZ slices
 
@@ -182,16 +183,65 @@ __host__ __device__ constexpr CellNb cell_nb(int dz, int dy, int dx) {
                 (uint8_t)(cell_face(0, dx, true) & cell_face(1, dy, true) & cell_face(2, dz, true)),
                 (uint8_t)(cell_face(0, dx, false) & cell_face(1, dy, false) & cell_face(2, dz, false))};
 }
-// The 13 backward cell neighbours (the other 13 are their mirror images).
-__constant__ CellNb kCellNb[13] = {
-    cell_nb(-1, -1, -1), cell_nb(-1, -1, 0), cell_nb(-1, -1, 1), cell_nb(-1, 0, -1), cell_nb(-1, 0, 0),
-    cell_nb(-1, 0, 1),   cell_nb(-1, 1, -1), cell_nb(-1, 1, 0),  cell_nb(-1, 1, 1),  cell_nb(0, -1, -1),
-    cell_nb(0, -1, 0),   cell_nb(0, -1, 1),  cell_nb(0, 0, -1)};
+// The 13 backward cell neighbours (the other 13 are their mirror images) as four words of occupancy bytes: the layer
+// below at dx = -1, 0, +1, each with dy = -1, 0, +1 in bytes 0 .. 2, and this layer's (dy, dx) = (-1, -1), (-1, 0),
+// (-1, +1), (0, -1).  A link list has bit 8 b + w for byte b of word w, so a word's tests are a few operations on all its
+// bytes at once instead of two masks and two branches a neighbour.  The kernel is bound by its ALU
+// instructions, of which these tests and the cells' occupancy were the most: 1.42 G voxels 4.07 -> 2.91 ms with both packed,
+// a row's eight cells stored at once and a column's neighbours read from the next lanes.
+struct CellWords {
+  uint32_t w[4];
+};
+__host__ __device__ constexpr CellNb word_nb(int w, int b) {
+  return w < 3 ? cell_nb(-1, b - 1, w - 1) : (b < 3 ? cell_nb(0, -1, b - 1) : cell_nb(0, 0, -1));
+}
+// self / other masks of a word's bytes; flat: the cells as neighbours of the one below instead (dz = 0)
+__host__ __device__ constexpr uint32_t word_mask(int w, bool self, bool flat) {
+  uint32_t m = 0;
+  for (int b = 0; b < (w < 3 ? 3 : 4); b++) {
+    const CellNb n = flat ? cell_nb(0, b - 1, w - 1) : word_nb(w, b);
+    m |= (uint32_t)(self ? n.self : n.other) << (8 * b);
+  }
+  return m;
+}
+// 0x80 in every nonzero byte
+__device__ __forceinline__ uint32_t byte_flags(uint32_t x) {
+  return (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
+}
+// Link list of a cell with occupancy oc.
+__device__ __forceinline__ uint32_t cell_links(uint32_t oc, const CellWords &n) {
+  constexpr uint32_t own[4] = {word_mask(0, true, false), word_mask(1, true, false), word_mask(2, true, false), word_mask(3, true, false)};
+  constexpr uint32_t nbr[4] = {word_mask(0, false, false), word_mask(1, false, false), word_mask(2, false, false), word_mask(3, false, false)};
+  const uint32_t r = oc * 0x01010101u;
+  uint32_t todo = 0;
+#pragma unroll
+  for (int w = 0; w < 4; w++) todo |= (byte_flags(r & own[w]) & byte_flags(n.w[w] & nbr[w])) >> (7 - w);
+  return todo;
+}
+constexpr uint32_t kLinkBelow = 1u << 9, kLinkBehind = 1u << 11, kLinkLeft = 1u << 27;   // (-1,0,0), (0,-1,0), (0,0,-1)
+// Links to the layer below whose cell the cell directly below touches in that layer.
+__device__ __forceinline__ uint32_t below_touches(const CellWords &n) {
+  constexpr uint32_t own[3] = {word_mask(0, true, true), word_mask(1, true, true), word_mask(2, true, true)};
+  constexpr uint32_t nbr[3] = {word_mask(0, false, true), word_mask(1, false, true), word_mask(2, false, true)};
+  const uint32_t r = ((n.w[1] >> 8) & 0xFFu) * 0x01010101u;
+  uint32_t t = 0;
+#pragma unroll
+  for (int w = 0; w < 3; w++) t |= (byte_flags(r & own[w]) & byte_flags(n.w[w] & nbr[w])) >> (7 - w);
+  return t & ~kLinkBelow;
+}
+// Cell offset of list bit p.
+__device__ __forceinline__ void link_offset(int p, int &dz, int &dy, int &dx) {
+  const int w = p & 7, b = p >> 3;
+  dz = w < 3 ? -1 : 0;
+  dy = w < 3 ? b - 1 : (b < 3 ? -1 : 0);
+  dx = w < 3 ? w - 1 : (b < 3 ? b - 1 : -1);
+}
 
 // Occupancy of a halo-framed block of cells: the tile's cells plus one cell on each x
 // and y side and one layer below (cell coordinates -1 .. kC? along each axis).
-constexpr int kHX = kCX + 2, kHY = kCY + 2;
-__device__ __forceinline__ int halo_of(int cx, int cy, int cz) { return ((cz + 1) * kHY + (cy + 1)) * kHX + (cx + 1); }
+// Rows of 40 bytes with cell 0 at byte 8: eight cells of a row are one 8-byte store.
+constexpr int kHX = kCX + 8, kHY = kCY + 2;
+__device__ __forceinline__ int halo_of(int cx, int cy, int cz) { return ((cz + 1) * kHY + (cy + 1)) * kHX + (cx + 8); }
 __device__ __forceinline__ int cell_bit(int lx, int ly, int lz) { return ((lz & 1) << 2) | ((ly & 1) << 1) | (lx & 1); }
 
 // Occupancy of the cell whose first voxel is (x, y, z) (volume coordinates; voxels outside
@@ -221,11 +271,10 @@ __device__ __forceinline__ uint32_t cell_occ(const Sub &S, const uint8_t *m, int
   return o;
 }
 
-// Occupancy of the 8 cells whose first voxels are (x + 2k, y, z), k = 0..7, from one
+// Occupancy bytes of the 8 cells whose first voxels are (x + 2k, y, z), k = 0..7, from one
 // 16-byte load of each of the 4 voxel rows they cover (x 16-byte aligned, x + 15 < W;
 // rows outside the volume read as background).
-__device__ __forceinline__ void cell_occ8(const Sub &S, const uint8_t *m, int64_t WH, int x, int y, int z,
-                                          uint32_t (&o)[8]) {
+__device__ __forceinline__ uint2 cell_occ8(const Sub &S, const uint8_t *m, int64_t WH, int x, int y, int z) {
   uint4 r[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -234,52 +283,46 @@ __device__ __forceinline__ void cell_occ8(const Sub &S, const uint8_t *m, int64_
                ? __ldg(reinterpret_cast<const uint4 *>(m + zz * WH + (int64_t)yy * S.W + x))
                : make_uint4(0u, 0u, 0u, 0u);
   }
-#pragma unroll
-  for (int k = 0; k < 8; k++) o[k] = 0;
+  uint32_t o[4] = {0u, 0u, 0u, 0u};   // cells 2j and 2j + 1 in bytes 0 and 2
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int sh = 4 * (q >> 1) + 2 * (q & 1);   // bit of the row's first voxel: 4 dz + 2 dy
     const uint32_t w[4] = {r[q].x, r[q].y, r[q].z, r[q].w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const uint32_t nz = __vcmpne4(w[j], 0u);   // 0xFF per foreground byte
-      o[2 * j] |= ((nz & 1u) | ((nz >> 7) & 2u)) << sh;
-      o[2 * j + 1] |= (((nz >> 16) & 1u) | ((nz >> 23) & 2u)) << sh;
+      const uint32_t f = byte_flags(w[j]);   // voxels 0, 1 at bits 7, 15 and 2, 3 at 23, 31
+      o[j] |= (((f >> 7) | (f >> 14)) & 0x00030003u) << sh;
     }
   }
+  return make_uint2(__byte_perm(o[0], o[1], 0x6420), __byte_perm(o[2], o[3], 0x6420));
 }
 
 // Drops links that other links of the tile already imply.  Every tile edge is linked by
 // the later of its two cells, so with cell c linked to B (a backward neighbour) and B
 // touching A (another backward neighbour of c), the edge B-A is linked too and c-A adds
-// nothing.  Links kept unconditionally: k = 4 (dz -1), 10 (dy -1), 12 (dx -1).  Pruned:
-//   via k = 4  (the cell below):  the other eight cells of the layer below, through the
-//              in-plane edges of that layer;
-//   via k = 10 (the cell behind): k = 9, 11 through that row's x edges (kept by rule) and
-//              k = 1 through its own link k = 4 (kept);
-//   via k = 12 (the cell left):   k = 9 through its link k = 10 and k = 3 through its
-//              link k = 4 (both kept).
+// nothing.  Links kept unconditionally: below (dz -1), behind (dy -1), left (dx -1).  Pruned:
+//   via below:   the other eight cells of the layer below, through the
+//                in-plane edges of that layer;
+//   via behind:  its left and right neighbours through that row's x edges (kept by rule) and
+//                the cell below it through its own link below (kept);
+//   via left:    the cell behind it and the one below it through its links (both kept).
 // Each pruned link rests on links that are kept or pruned only by the rules for
 // in-layer edges, which rest on kept links: the implied connectivity is exact.
 // The component minima are unchanged (they come from the final trees, not the links).
 __device__ __forceinline__ bool touches(uint32_t a, uint32_t b, CellNb e) { return (a & e.self) && (b & e.other); }
 
-__device__ __forceinline__ uint32_t prune_links(uint32_t todo, const uint32_t (&on)[13]) {
-  if (todo & (1u << 4)) {
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      if (k == 4) continue;
-      if (touches(on[4], on[k], cell_nb(0, k / 3 - 1, k % 3 - 1))) todo &= ~(1u << k);
-    }
+__device__ __forceinline__ uint32_t prune_links(uint32_t todo, const CellWords &n) {
+  if (todo & kLinkBelow) todo &= ~below_touches(n);
+  if (todo & kLinkBehind) {
+    const uint32_t on10 = (n.w[3] >> 8) & 0xFFu;
+    if (touches(on10, n.w[3] & 0xFFu, cell_nb(0, 0, -1))) todo &= ~(1u << 3);
+    if (touches(on10, (n.w[3] >> 16) & 0xFFu, cell_nb(0, 0, 1))) todo &= ~(1u << 19);
+    if (touches(on10, n.w[1] & 0xFFu, cell_nb(-1, 0, 0))) todo &= ~(1u << 1);
   }
-  if (todo & (1u << 10)) {
-    if (touches(on[10], on[9], cell_nb(0, 0, -1))) todo &= ~(1u << 9);
-    if (touches(on[10], on[11], cell_nb(0, 0, 1))) todo &= ~(1u << 11);
-    if (touches(on[10], on[1], cell_nb(-1, 0, 0))) todo &= ~(1u << 1);
-  }
-  if (todo & (1u << 12)) {
-    if (touches(on[12], on[9], cell_nb(0, -1, 0))) todo &= ~(1u << 9);
-    if (touches(on[12], on[3], cell_nb(-1, 0, 0))) todo &= ~(1u << 3);
+  if (todo & kLinkLeft) {
+    const uint32_t on12 = n.w[3] >> 24;
+    if (touches(on12, n.w[3] & 0xFFu, cell_nb(0, -1, 0))) todo &= ~(1u << 3);
+    if (touches(on12, (n.w[0] >> 8) & 0xFFu, cell_nb(-1, 0, 0))) todo &= ~(1u << 8);
   }
   return todo;
 }
@@ -287,9 +330,10 @@ __device__ __forceinline__ uint32_t prune_links(uint32_t todo, const uint32_t (&
 template <int TZ>
 __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, const uint8_t *mask, int32_t *labels,
                                                           int2 *edges, unsigned long long *edge_count) {
-  constexpr int kCZ = TZ / 2, kCells = kCX * kCY * kCZ, kHZ = kCZ + 1, kHalo = kHX * kHY * kHZ;   // 4096 cells, 5780 with halo at TZ 32
-  __shared__ uint32_t par[kCells];
-  __shared__ uint8_t occ[kHalo];
+  constexpr int kCZ = TZ / 2, kCells = kCX * kCY * kCZ, kHZ = kCZ + 1, kHalo = kHX * kHY * kHZ;   // 4096 cells, 6800 bytes with halo at TZ 32
+  static_assert(kCX == 32, "a warp is a row of cells");
+  __shared__ __align__(16) uint32_t par[kCells];
+  __shared__ __align__(8) uint8_t occ[kHalo + 8];   // cell 32 of a row is byte 0 of the next
   __shared__ uint32_t minv[kCells];
   __shared__ int2 ebuf[kEdgeBuf];
   __shared__ uint32_t n_local_edges;
@@ -313,39 +357,31 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
     for (int it = t; it < kHY * kHZ * kSeg; it += kCclThreads) {
       const int seg = it % kSeg, hy = (it / kSeg) % kHY, hz = it / (kSeg * kHY);
       const int cy = hy - 1, cz = hz - 1, cx0 = seg * 8;
-      uint32_t o[8];
+      uint2 o = make_uint2(0u, 0u);
       if (cz < ncz && (cz >= 0 || T.z0 > 0)) {
-        cell_occ8(S, m, WH, T.x0 + 2 * cx0, T.y0 + 2 * cy, T.z0 + 2 * cz, o);
-        if (T.x0 == 0 && T.y0 + 2 * cy == 0 && T.z0 + 2 * cz == 0 && cx0 == 0) o[0] &= ~1u;   // voxel 0
-        if (cz >= 0 && 2 * cz + 1 >= T.tz)
-#pragma unroll
-          for (int k = 0; k < 8; k++) o[k] &= 0x0Fu;
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; k++) o[k] = 0;
+        o = cell_occ8(S, m, WH, T.x0 + 2 * cx0, T.y0 + 2 * cy, T.z0 + 2 * cz);
+        if (T.x0 == 0 && T.y0 + 2 * cy == 0 && T.z0 + 2 * cz == 0 && cx0 == 0) o.x &= ~1u;   // voxel 0
+        if (cz >= 0 && 2 * cz + 1 >= T.tz) { o.x &= 0x0F0F0F0Fu; o.y &= 0x0F0F0F0Fu; }
       }
-#pragma unroll
-      for (int k = 0; k < 8; k++) occ[halo_of(cx0 + k, cy, cz)] = (uint8_t)o[k];
+      *reinterpret_cast<uint2 *>(occ + halo_of(cx0, cy, cz)) = o;
       if (cy >= 0 && cy < kCY && cz >= 0) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int c = (cz * kCY + cy) * kCX + cx0 + k;
-          par[c] = o[k] ? (uint32_t)c : kBg32;
-          minv[c] = 0xFFFFFFFFu;
-        }
+        const uint32_t c = (cz * kCY + cy) * kCX + cx0;
+        uint4 *pc = reinterpret_cast<uint4 *>(par + c);
+        pc[0] = make_uint4(o.x & 0xFFu ? c : kBg32, o.x & 0xFF00u ? c + 1 : kBg32, o.x & 0xFF0000u ? c + 2 : kBg32, o.x >> 24 ? c + 3 : kBg32);
+        pc[1] = make_uint4(o.y & 0xFFu ? c + 4 : kBg32, o.y & 0xFF00u ? c + 5 : kBg32, o.y & 0xFF0000u ? c + 6 : kBg32, o.y >> 24 ? c + 7 : kBg32);
       }
     }
   }
-  for (int h = t; h < (rows16 ? kHY * kHZ * 2 : kHalo); h += kCclThreads) {
+  for (int h = t; h < kHY * kHZ * (rows16 ? 2 : kCX + 2); h += kCclThreads) {
     int hx, hy, hz;
     if (rows16) {   // the side columns cx = -1 and cx = kCX
-      hx = (h & 1) ? kHX - 1 : 0;
+      hx = (h & 1) ? kCX + 1 : 0;
       hy = (h >> 1) % kHY;
       hz = (h >> 1) / kHY;
     } else {
-      hx = h % kHX;
-      hy = (h / kHX) % kHY;
-      hz = h / (kHX * kHY);
+      hx = h % (kCX + 2);
+      hy = (h / (kCX + 2)) % kHY;
+      hz = h / ((kCX + 2) * kHY);
     }
     const int cx = hx - 1, cy = hy - 1, cz = hz - 1;
     uint32_t o = 0;
@@ -353,11 +389,10 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
       o = cell_occ(S, m, WH, T.x0 + 2 * cx, T.y0 + 2 * cy, T.z0 + 2 * cz);
       if (cz >= 0 && 2 * cz + 1 >= T.tz) o &= 0x0Fu;   // a tile's last odd slice: no second layer
     }
-    occ[(hz * kHY + hy) * kHX + hx] = (uint8_t)o;
+    occ[halo_of(cx, cy, cz)] = (uint8_t)o;
     if (cx >= 0 && cx < kCX && cy >= 0 && cy < kCY && cz >= 0) {
       const int c = (cz * kCY + cy) * kCX + cx;
       par[c] = o ? (uint32_t)c : kBg32;
-      minv[c] = 0xFFFFFFFFu;
     }
   }
   __syncthreads();
@@ -369,23 +404,27 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
   //    others idle for that layer alone.  Union order does not change the components.
   const int cx = t % kCX, cy = t / kCX;
   uint32_t layers = 0;   // bit cz: the cell of layer cz has links
-  for (int cz = 0; cz < ncz; cz++) {
-    const int c = (cz * kCY + cy) * kCX + cx;
-    const uint32_t oc = occ[halo_of(cx, cy, cz)];
-    uint32_t todo = 0;
-    if (oc) {
-      uint32_t on[13];   // occupancy of the backward neighbours inside the tile (0 outside)
-#pragma unroll
-      for (int k = 0; k < 13; k++) {
-        const CellNb nb = kCellNb[k];
-        const int nx = cx + nb.dx, ny = cy + nb.dy, nz = cz + nb.dz;
-        on[k] = (nx < 0 || nx >= kCX || ny < 0 || ny >= kCY || nz < 0) ? 0u : occ[halo_of(nx, ny, nz)];
-        if ((oc & nb.self) && (on[k] & nb.other)) todo |= 1u << k;
+  {
+    // the column's cells of rows cy - 1 .. cy + 1 (0 outside the tile) in bytes 0 .. 2, its neighbours' by shuffles; a
+    // layer's words stay in registers as the next one's layer below
+    const uint32_t rows = (cy > 0 ? 0xFFu : 0u) | 0xFF00u | (cy < kCY - 1 ? 0xFF0000u : 0u);
+    CellWords n = {{0u, 0u, 0u, 0u}};
+    for (int cz = 0; cz < ncz; cz++) {
+      const uint8_t *o = occ + halo_of(cx, cy - 1, cz);
+      const uint32_t cur = (o[0] | (uint32_t)o[kHX] << 8 | (uint32_t)o[2 * kHX] << 16) & rows;
+      uint32_t left = __shfl_up_sync(0xFFFFFFFFu, cur, 1), right = __shfl_down_sync(0xFFFFFFFFu, cur, 1);
+      if (cx == 0) left = 0;
+      if (cx == kCX - 1) right = 0;
+      const uint32_t oc = (cur >> 8) & 0xFFu;
+      uint32_t todo = 0;
+      if (oc) {
+        n.w[3] = __byte_perm(__byte_perm(left, cur, 0x1040), right, 0x3410);
+        todo = prune_links(cell_links(oc, n), n);
       }
-      todo = prune_links(todo, on);
+      minv[(cz * kCY + cy) * kCX + cx] = todo;
+      layers |= (todo ? 1u : 0u) << cz;
+      n.w[0] = left; n.w[1] = cur; n.w[2] = right;
     }
-    minv[c] = todo;
-    layers |= (todo ? 1u : 0u) << cz;
   }
   {
     uint32_t todo = 0;
@@ -400,10 +439,8 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
       if (todo) {
         const int k = __ffs(todo) - 1;
         todo &= todo - 1;
-        // backward cell offset k: (dz, dy, dx) as in kCellNb
-        const int dz = k < 9 ? -1 : 0;
-        const int dy = k < 9 ? k / 3 - 1 : (k < 12 ? -1 : 0);
-        const int dx = k < 9 ? k % 3 - 1 : (k < 12 ? k - 10 : -1);
+        int dz, dy, dx;
+        link_offset(k, dz, dy, dx);
         const int cn = c + (dz * kCY + dy) * kCX + dx;
         if (par[cn] != par[c]) sunion(par, c, cn, 2 * kCells);
       }
@@ -463,34 +500,26 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
       }
       const uint32_t oc = occ[halo_of(fx, fy, fz)];
       if (!oc) continue;
-      uint32_t todo = 0;
+      const uint8_t *o = occ + halo_of(fx, fy, fz), *below = o - kHX * kHY;
+      CellWords n;
 #pragma unroll
-      for (int k = 0; k < 13; k++) {
-        const CellNb nb = kCellNb[k];
-        const int nx = fx + nb.dx, ny = fy + nb.dy, nz = fz + nb.dz;
-        if (nx >= 0 && nx < kCX && ny >= 0 && ny < kCY && nz >= 0) continue;   // inside the tile
-        if (nz < 0 && !zface) continue;
-        if ((oc & nb.self) && (occ[halo_of(nx, ny, nz)] & nb.other)) todo |= 1u << k;
-      }
-      if (todo & (1u << 4)) {
-        // linked to the cell below, in the tile below: that tile's own unions join it to those of its eight
-        // neighbours it touches inside the same footprint, so the edges to these add nothing
-        const uint32_t below = occ[halo_of(fx, fy, fz - 1)];
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-          const int dy = k / 3 - 1, dx = k % 3 - 1;
-          if (k == 4 || fx + dx < 0 || fx + dx >= kCX || fy + dy < 0 || fy + dy >= kCY) continue;
-          if (touches(below, occ[halo_of(fx + dx, fy + dy, fz - 1)], cell_nb(0, dy, dx))) todo &= ~(1u << k);
-        }
-      }
+      for (int w = 0; w < 3; w++)
+        n.w[w] = below[w - 1 - kHX] | (uint32_t)below[w - 1] << 8 | (uint32_t)below[w - 1 + kHX] << 16;
+      n.w[3] = o[-1 - kHX] | (uint32_t)o[-kHX] << 8 | (uint32_t)o[1 - kHX] << 16 | (uint32_t)o[-1] << 24;
+      // links to cells beyond the tile's x and y faces, and to the layer below it
+      const uint32_t side = (fx == 0 ? 0x08010109u : 0u) | (fx == kCX - 1 ? 0x000C0404u : 0u) |
+                            (fy == 0 ? 0x0008080Fu : 0u) | (fy == kCY - 1 ? 0x00070000u : 0u);
+      uint32_t todo = cell_links(oc, n) & (side | (fz == 0 ? 0x00070707u : 0u));
+      // linked to the cell below, in the tile below: that tile's own unions join it to those of its eight
+      // neighbours it touches inside the same footprint, so the edges to these add nothing
+      if (todo & kLinkBelow) todo &= ~(below_touches(n) & ~side);
       if (!todo) continue;
       const int64_t a = first_voxel(fx, fy, fz, oc);
       while (todo) {
         const int k = __ffs(todo) - 1;
         todo &= todo - 1;
-        const int dz = k < 9 ? -1 : 0;
-        const int dy = k < 9 ? k / 3 - 1 : (k < 12 ? -1 : 0);
-        const int dx = k < 9 ? k % 3 - 1 : (k < 12 ? k - 10 : -1);
+        int dz, dy, dx;
+        link_offset(k, dz, dy, dx);
         const int nx = fx + dx, ny = fy + dy, nz = fz + dz;
         emit(a, first_voxel(nx, ny, nz, occ[halo_of(nx, ny, nz)]));
       }
