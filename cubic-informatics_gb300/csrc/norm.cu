@@ -310,6 +310,61 @@ __global__ void __launch_bounds__(256) k_mm_x(const Sub *subs, int r, int ry, in
   }
 }
 
+// ---------------------------------------------------------------- reaches below 4
+// Windows of at most seven entries are folded in registers: they are shorter than the blocks of the passes below, and
+// chains in shared memory cost more than their few mins.  HBM-bound.  2560x2160x16, reaches 1 to 3: y 215 -> 119 to
+// 137 us.  640x720x32 erosion at reach 2: y 54 -> 25 us, x 45 -> 17.  (The x box of these reaches and rows of other
+// widths stay with k_mm_x: a load an entry and an output takes 410 to 790 us where it takes 380.)
+template <int BORDER>
+__device__ __forceinline__ uint32_t mm_at(const uint32_t *line, int i, int n, int64_t step) {
+  return BORDER == 1 && (i < 0 || i >= n) ? kZeroPacked : __ldg(line + clampi(i, 0, n - 1) * step);
+}
+
+// A warp takes kShortRows rows of 32 columns.
+constexpr int kShortRows = 8;
+template <int BORDER, int R>
+__global__ void __launch_bounds__(256) k_mm_y_short(const Sub *subs, const uint32_t *in, uint32_t *out) {
+  const Sub S = subs[blockIdx.y];
+  const int W = S.W, H = S.H, tx_n = (W + 31) / 32, ty_n = (H + 8 * kShortRows - 1) / (8 * kShortRows);
+  const int64_t bid = blockIdx.x;
+  if (bid >= (int64_t)tx_n * ty_n * S.D) return;
+  const int z = (int)(bid / ((int64_t)tx_n * ty_n)), rem = (int)(bid % ((int64_t)tx_n * ty_n));
+  const int x = (rem % tx_n) * 32 + (threadIdx.x & 31), y0 = ((rem / tx_n) * 8 + (threadIdx.x >> 5)) * kShortRows;
+  if (x >= W || y0 >= H) return;
+  const int64_t sl = S.vox + (int64_t)z * W * H + x;
+  uint32_t v[kShortRows + 2 * R];
+#pragma unroll
+  for (int j = 0; j < kShortRows + 2 * R; j++) v[j] = mm_at<BORDER>(in + sl, y0 - R + j, H, W);
+#pragma unroll
+  for (int k = 0; k < kShortRows; k++) {
+    uint32_t m = v[k];
+#pragma unroll
+    for (int j = 1; j <= 2 * R; j++) m = __vminu2(m, v[k + j]);
+    if (y0 + k < H) out[sl + (int64_t)(y0 + k) * W] = m;
+  }
+}
+
+// The erosion's x pass on rows of whole, aligned quads: a thread reads its quad and the two beside it.
+template <int R>
+__global__ void __launch_bounds__(256) k_erode_x_quad(const Sub *subs, const uint32_t *in, uint16_t *out) {
+  const Sub S = subs[blockIdx.y];
+  const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4;
+  if (i >= (int64_t)S.W * S.H * S.D) return;
+  const int x = (int)((uint32_t)i % (uint32_t)S.W);
+  const uint4 *p = reinterpret_cast<const uint4 *>(in + S.vox + i);
+  const uint4 zero = make_uint4(kZeroPacked, kZeroPacked, kZeroPacked, kZeroPacked);
+  const uint4 c = __ldg(p), a = x > 0 ? __ldg(p - 1) : zero, b = x + 4 < S.W ? __ldg(p + 1) : zero;
+  const uint32_t v[12] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w, b.x, b.y, b.z, b.w};
+  uint32_t m[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    m[k] = v[4 + k - R];
+#pragma unroll
+    for (int j = 1 - R; j <= R; j++) m[k] = __vminu2(m[k], v[4 + k + j]);
+  }
+  *reinterpret_cast<uint2 *>(out + S.vox + i) = make_uint2(__byte_perm(m[0], m[1], 0x5410), __byte_perm(m[2], m[3], 0x5410));
+}
+
 // ---------------------------------------------------------------- y / x passes for any reach
 // Windows from short blocks (window.cuh), for reaches from 4 up.
 struct PackedMin {
@@ -844,8 +899,15 @@ static bool mm_y_cols(const Sub *d_subs, int nsub, int W, int H, int D, int r, c
 template <int BORDER>
 static void mm_y(const Sub *d_subs, int nsub, int W, int H, int D, int r, const uint32_t *in, uint32_t *out,
                  cudaStream_t s) {
+  if (r < 4) {
+    const dim3 grid((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, 8 * kShortRows) * D), nsub);
+    const auto fn = r == 0 ? k_mm_y_short<BORDER, 0> : r == 1 ? k_mm_y_short<BORDER, 1>
+                  : r == 2 ? k_mm_y_short<BORDER, 2> : k_mm_y_short<BORDER, 3>;
+    KLAUNCH("k_mm_y", s, (fn<<<grid, 256, 0, s>>>(d_subs, in, out)));
+    return;
+  }
   if (r >= 8 && mm_y_cols<BORDER, 16>(d_subs, nsub, W, H, D, r, in, out, s)) return;
-  if (r >= 4 && r < 8 && mm_y_cols<BORDER, 8>(d_subs, nsub, W, H, D, r, in, out, s)) return;
+  if (r < 8 && mm_y_cols<BORDER, 8>(d_subs, nsub, W, H, D, r, in, out, s)) return;
   // rows per block: 128, fewer when the staged window would not fit in shared memory
   const int cap_rows = max_optin_smem() / (2 * 32 * 4);
   int ty = 128;
@@ -870,6 +932,11 @@ static size_t mm_x_smem(int mode, int r, int ry, int tx) {
 template <int BORDER, int MODE>
 static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const uint32_t *in, void *out,
                  cudaStream_t s) {
+  if (MODE == 1 && r < 4 && W % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) {
+    const auto fn = r == 0 ? k_erode_x_quad<0> : r == 1 ? k_erode_x_quad<1> : r == 2 ? k_erode_x_quad<2> : k_erode_x_quad<3>;
+    KLAUNCH("k_mm_x", s, (fn<<<dim3((unsigned)ceil_div(rows * W / 4, 256), nsub), 256, 0, s>>>(d_subs, in, static_cast<uint16_t *>(out))));
+    return;
+  }
   if (r >= 4 && r <= (MODE == 0 ? 127 : 255)) {
     switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
 #define HDOG_MMX_CASE(Q)                                                                                     \
