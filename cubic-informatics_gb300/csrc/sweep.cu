@@ -42,7 +42,7 @@ __device__ __forceinline__ void tma_slice(const CUtensorMap *map, float *dst, ui
 //                 included, so the volume equals the separate passes bit for bit.
 //   k_hess_sweep  DoG -> mask + foreground list.  A block owns a kHTX x kHTY tile; DoG slices
 //                 (tile + 2-voxel halo, zero outside the volume) arrive by TMA into an
-//                 8-slot ring, up to five slices ahead; each thread tests one x quad.  No
+//                 ring of six or eight slots, as far ahead; each thread tests an x quad of one or two rows.  No
 //                 block barrier per slice: warps release ring slots through mbarriers.
 //                 The normalized values the list carries are read from global memory by
 //                 the threads whose quad has foreground.
@@ -50,11 +50,17 @@ __device__ __forceinline__ void tma_slice(const CUtensorMap *map, float *dst, ui
 // The split costs one write and one read of the DoG volume but frees the Hessian stage
 // from the z shift register's registers, so several Hessian blocks share an SM.
 constexpr int kDTX = 32;                // DoG tile width
-constexpr int kHTX = 32, kHTY = 16;     // Hessian tile (six blocks per SM)
+constexpr int kHTX = 32, kHTY = 16;     // Hessian tile
 constexpr int kHPX = kHTX + 8;          // Hessian ring row: columns x0-4 .. x0+kHTX+3 (16-byte aligned start)
 constexpr int kHPY = kHTY + 4;
-constexpr int kHRing = 8;              // ring slots; a slot is 40 x 20 floats = 25 x 128 bytes
-constexpr int kHThreads = kHTX / 4 * kHTY;   // one x quad per thread
+// Rows of an x quad that a thread of the Hessian sweep takes, and the shape that goes with them: threads, ring slots (a
+// slot is 40 x 20 floats = 25 x 128 bytes) and blocks per SM.
+template <int ROWS>
+struct HessT {
+  static constexpr int NT = kHTX / 4 * kHTY / ROWS;
+  static constexpr int RING = ROWS == 2 ? 6 : 8;
+  static constexpr size_t SMEM = (size_t)RING * kHPX * kHPY * 4 + (2 * RING) * 8 + (size_t)(NT / 32) * 128 * sizeof(FgEntry);
+};
 
 // Input slices of the DoG sweep in flight: slice it + kDogIn - 1 is requested while slice it
 // is filtered (2, 3 and 4 measured the same on the camera stack; 2 keeps the buffer index a
@@ -432,36 +438,34 @@ __device__ __forceinline__ void flush_stage(const FgEntry *stage, int n, const S
   __syncwarp();
 }
 
-// Blocks per SM the Hessian sweep is compiled for: five fit its z pipeline in 96
-// registers without spilling.
-#ifndef HDOG_HESS_BLOCKS
-#define HDOG_HESS_BLOCKS 5
-#endif
 // PERSIST: a grid of a few blocks per SM takes (substack, tile) items from the device work
 // queue `q` until it is empty; otherwise one block per tile (blockIdx.x) and substack
 // (blockIdx.y).  SPLIT: the latter, with zlen slices per block (blockIdx.z) where the tiles alone leave most of
 // the chip idle (a block's slices follow one another).  One 128x96x16 substack 28 -> 12 us, one of 256x256x32 63 ->
 // 30 us.  Results are the same either way.  PAD: the width is no multiple of 4, so the rows of the
 // DoG and the normalized volume are padded and the mask's are not whole words.
-template <bool PERSIST, bool PAD, bool SPLIT>
-__global__ void __launch_bounds__(kHThreads, SPLIT ? HDOG_HESS_BLOCKS - 1 : HDOG_HESS_BLOCKS)
+// ROWS 2: the two rows share the rows around them, 16 shared-memory reads and 32 wavefronts a row instead of 13 and
+// 52, in 128 registers; 1.42 G voxels 5.11 -> 4.60 ms.  Blocks are half as wide in threads and take a slice as long,
+// so batches without four waves of them keep one row (128x96x16: 12 us against 20; twelve small substacks: 155 against 187).
+template <bool PERSIST, bool PAD, bool SPLIT, int ROWS>
+__global__ void __launch_bounds__(HessT<ROWS>::NT, ROWS == 2 ? 7 : SPLIT ? 4 : 5)
     k_hess_sweep(const __grid_constant__ CUtensorMap map, const Sub *subs, const float *norm, uint8_t *mask,
                  FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count, int *status, WorkQueue q, int zlen) {
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int PL = kHPX * kHPY;
+  constexpr int PL = kHPX * kHPY, RING = HessT<ROWS>::RING;
   constexpr uint32_t tma_bytes = (uint32_t)(PL * 4);
   float *ring = reinterpret_cast<float *>(smem);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kHRing * PL * 4);
-  // done[i % kHRing] completes when every warp has finished the block's i-th iteration, with
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)RING * PL * 4);
+  // done[i % RING] completes when every warp has finished the block's i-th iteration, with
   // its last reads of that iteration's DoG slice zh-2
-  uint64_t *done = bar + kHRing;
+  uint64_t *done = bar + RING;
   const int t = threadIdx.x;
   // this warp's staging of list entries (flushed to the global list kHStage at a time at most)
-  FgEntry *stage = reinterpret_cast<FgEntry *>(smem + (size_t)kHRing * PL * 4 + 2 * kHRing * 8) + (t >> 5) * kHStage;
+  FgEntry *stage = reinterpret_cast<FgEntry *>(smem + (size_t)RING * PL * 4 + 2 * RING * 8) + (t >> 5) * kHStage;
   __shared__ int s_item;
   if (t == 0) {
-    for (int i = 0; i < kHRing; i++) mbar_init(&bar[i], 1);
-    for (int i = 0; i < kHRing; i++) mbar_init(&done[i], kHThreads / 32);
+    for (int i = 0; i < RING; i++) mbar_init(&bar[i], 1);
+    for (int i = 0; i < RING; i++) mbar_init(&done[i], HessT<ROWS>::NT / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   bool ok = true;
@@ -496,214 +500,218 @@ __global__ void __launch_bounds__(kHThreads, SPLIT ? HDOG_HESS_BLOCKS - 1 : HDOG
   const int tx = x0 - 4, ty = y0 - 2;
   const int zb = SPLIT ? (int)blockIdx.z * zlen : 0, ze = SPLIT ? min(D, zb + zlen) : D;   // this block's slices
   // ring slot of DoG slice z (z = zb-2 .. ze+1; slices outside the volume arrive zero-filled)
-  auto slot = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) % kHRing); };
+  auto slot = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) % RING); };
   // use k of slot s (k-th slice loaded into it) completes barrier phase k & 1
-  auto use = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) / kHRing); };
-  // slices zb-2 .. zb+4 up front, then slice zh + 5 while slice zh is tested: the slot it
-  // reuses held slice zh - 3, last read one barrier earlier
+  auto use = [zbase, zb](int z) { return (int)((zbase + (uint32_t)(z - zb + 2)) / RING); };
+  // the ring's slices but one up front, then slice zh + RING - 3 while slice zh is tested: the slot it
+  // reuses held slice zh - 3, last read one iteration earlier
   if (t == 0 && ok)
-    for (int z = zb - 2; z <= zb + 4 && z <= ze + 1; z++)
+    for (int z = zb - 2; z <= zb + RING - 4 && z <= ze + 1; z++)
       tma_slice(&map, ring + slot(z) * PL, &bar[slot(z)], tx, ty, z, sub, tma_bytes);
   for (int z = zb - 2; z <= zb + 1; z++)
     if (ok && !mbar_wait(&bar[slot(z)], use(z) & 1)) {
       ok = false;
       atomicExch(status, HDOG_ERR_TIMEOUT);
     }
-  const int q = t % (kHTX / 4), ly = t / (kHTX / 4);
-  const int X0 = x0 + 4 * q, Y = y0 + ly;
+  const int q = t % (kHTX / 4), ly = ROWS * (t / (kHTX / 4));
+  const int X0 = x0 + 4 * q, Y = y0 + ly;      // the quad's column and first row
   const int b = (ly + 2) * kHPX + 4 * q + 4;   // ring index of column X0 on row Y
-  // every in-plane gradient position of the quad inside the volume: the z-pipelined
+  // every in-plane gradient position of the quads inside the volume: the z-pipelined
   // stencil below (only the z neighbours can fall outside); the frame's edges take the
   // literal zero-halo path voxel by voxel.  Fixed per thread for the whole sweep.
-  const bool interior = X0 >= 1 && X0 + 3 <= W - 2 && Y >= 1 && Y <= H - 2;
-  // z pipeline of the interior path: first derivatives of slices zh-1 and zh on row Y
-  // (gx in the G frame, gy and gz in the C frame) and DoG of slices zh and zh+1 on row Y
+  const bool interior = X0 >= 1 && X0 + 3 <= W - 2 && Y >= 1 && Y + ROWS <= H - 1;
+  // z pipeline of the interior path, per row: first derivatives of slices zh-1 and zh
+  // (gx in the G frame, gy and gz in the C frame) and DoG of slices zh and zh+1
   const float2 zero2 = make_float2(0.0f, 0.0f);
-  float2 gxm[3] = {zero2, zero2, zero2}, gx0[3];
-  float2 gym[2] = {zero2, zero2}, gy0[2], gzm[2] = {zero2, zero2}, gz0[2];
-  float2 fm[2] = {zero2, zero2}, f0[2];
+  float2 gxm[ROWS][3], gx0[ROWS][3], gym[ROWS][2], gy0[ROWS][2], fm[ROWS][2], f0[ROWS][2];
+#pragma unroll
+  for (int r = 0; r < ROWS; r++) {
+    gxm[r][0] = gxm[r][1] = gxm[r][2] = zero2;
+    gym[r][0] = gym[r][1] = zero2;
+  }
   if (interior) {
-    // slice zb: gx, gy on row Y; gz from slices zb+1 and zb-1 (zero below the volume)
-    const float *P0 = ring + slot(zb) * PL + b, *P1 = ring + slot(zb + 1) * PL + b;
-    float2 l, r, u0, u1, d0, d1;
-    ld_row(P0, l, f0[0], f0[1], r);
-    gx_g(l, f0[0], f0[1], r, gx0);
-    ld_quad(P0 - kHPX, u0, u1);
-    ld_quad(P0 + kHPX, d0, d1);
-    gy0[0] = hd2(d0, u0);
-    gy0[1] = hd2(d1, u1);
-    float2 p0, p1;
-    ld_quad(P1, p0, p1);
-    if (!SPLIT || zb == 0) {
-      gz0[0] = hd2(p0, zero2);
-      gz0[1] = hd2(p1, zero2);
-    } else {   // a block that starts inside the volume: the derivatives of slice zb-1 as well
-      const float *M1 = ring + slot(zb - 1) * PL + b, *M2 = ring + slot(zb - 2) * PL + b;
-      float2 c0, c1, q0, q1;
-      ld_row(M1, l, c0, c1, r);
-      gx_g(l, c0, c1, r, gxm);
-      gz0[0] = hd2(p0, c0);
-      gz0[1] = hd2(p1, c1);
-      ld_quad(M1 - kHPX, u0, u1);
-      ld_quad(M1 + kHPX, d0, d1);
-      gym[0] = hd2(d0, u0);
-      gym[1] = hd2(d1, u1);
-      ld_quad(M2, q0, q1);
-      gzm[0] = hd2(f0[0], q0);
-      gzm[1] = hd2(f0[1], q1);
+    // slice zb: gx, gy on the thread's rows
+    auto first = [&](const float *P, float2 (&gx)[ROWS][3], float2 (&gy)[ROWS][2], float2 (&c)[ROWS][2]) {
+      float2 l, rr, u[2], d[2];
+#pragma unroll
+      for (int r = 0; r < ROWS; r++) {
+        ld_row(P + r * kHPX, l, c[r][0], c[r][1], rr);
+        gx_g(l, c[r][0], c[r][1], rr, gx[r]);
+      }
+      ld_quad(P - kHPX, u[0], u[1]);
+      ld_quad(P + ROWS * kHPX, d[0], d[1]);
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        gy[0][j] = hd2(ROWS == 2 ? c[ROWS - 1][j] : d[j], u[j]);
+        if (ROWS == 2) gy[ROWS - 1][j] = hd2(d[j], c[0][j]);
+      }
+    };
+    first(ring + slot(zb) * PL + b, gx0, gy0, fm);
+    const float *P1 = ring + slot(zb + 1) * PL + b;
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) ld_quad(P1 + r * kHPX, f0[r][0], f0[r][1]);
+    if (SPLIT && zb > 0) {   // a block that starts inside the volume: the derivatives of slice zb-1 as well
+      float2 c[ROWS][2];
+      first(ring + slot(zb - 1) * PL + b, gxm, gym, c);
     }
-    fm[0] = f0[0]; fm[1] = f0[1];
-    f0[0] = p0; f0[1] = p1;
   }
   for (int zh = zb; zh < ze; zh++) {
-    // DoG slice zh+5 reuses the slot of slice zh-3, read for the last time in iteration
+    // DoG slice zh+RING-3 reuses the slot of slice zh-3, read for the last time in iteration
     // zh-1: the producer waits until every warp is past it (warps otherwise run up to the
     // ring's depth apart)
-    if (t == 0 && ok && zh + 5 <= ze + 1) {
+    const int zn = zh + RING - 3;
+    if (t == 0 && ok && zn <= ze + 1) {
       const uint32_t prev = ibase + (uint32_t)(zh - zb) - 1u;
-      if (zh > zb && !mbar_wait(&done[prev % kHRing], (prev / kHRing) & 1)) {
+      if (zh > zb && !mbar_wait(&done[prev % RING], (prev / RING) & 1)) {
         ok = false;
         atomicExch(status, HDOG_ERR_TIMEOUT);
       }
-      if (ok) tma_slice(&map, ring + slot(zh + 5) * PL, &bar[slot(zh + 5)], tx, ty, zh + 5, sub, tma_bytes);
+      if (ok) tma_slice(&map, ring + slot(zn) * PL, &bar[slot(zn)], tx, ty, zn, sub, tma_bytes);
     }
     // slices zh-2 .. zh+1 were waited for already; zh+2 is new
     if (ok && !mbar_wait(&bar[slot(zh + 2)], use(zh + 2) & 1)) {
       ok = false;
       atomicExch(status, HDOG_ERR_TIMEOUT);
     }
-    uint32_t mword = 0;
     const int32_t i0 = zh * WH + Y * W + X0;
-    float hv[4][6];
-    if (interior) {
-      const float *P0 = ring + slot(zh) * PL + b, *P1 = ring + slot(zh + 1) * PL + b;
-      const float *P2 = ring + slot(zh + 2) * PL + b;
-      // ---- in-plane second derivatives of slice zh
-      float2 hxx[2], hxy[3], hyy[2];
-      hxx[0] = hd2(gx0[1], gx0[0]);
-      hxx[1] = hd2(gx0[2], gx0[1]);
-      {
-        float2 l, c0, c1, r, gu[3], gd[3];
-        ld_row(P0 - kHPX, l, c0, c1, r);
-        gx_g(l, c0, c1, r, gu);
-        float2 e0, e1;
-        ld_quad(P0 - 2 * kHPX, e0, e1);
-        const float2 gyu0 = hd2(fm[0], e0), gyu1 = hd2(fm[1], e1);   // gy on row Y-1
-        ld_row(P0 + kHPX, l, c0, c1, r);
-        gx_g(l, c0, c1, r, gd);
-        ld_quad(P0 + 2 * kHPX, e0, e1);
-        const float2 gyd0 = hd2(e0, fm[0]), gyd1 = hd2(e1, fm[1]);                      // gy on row Y+1
 #pragma unroll
-        for (int i = 0; i < 3; i++) hxy[i] = hd2(gd[i], gu[i]);
-        hyy[0] = hd2(gyd0, gyu0);
-        hyy[1] = hd2(gyd1, gyu1);
-      }
-      // ---- first derivatives of slice zh+1 on row Y, then the z second derivatives
-      float2 gxp[3], gyp[2], gzp[2], fp[2];
-      {
-        float2 l, r, u0, u1, d0, d1;
+    for (int r = 0; r < ROWS; r++) {
+      uint32_t mword = 0;
+      float hv[4][6];
+      const int32_t ir = i0 + r * W;
+      if (interior) {
+        // row 1 comes after row 0's advance: row 0's derivatives of slice zh are gxm[0] and gym[0] then, its DoG of
+        // slice zh+1 is fm[0]
+        const float *P0 = ring + slot(zh) * PL + b + r * kHPX, *P1 = ring + slot(zh + 1) * PL + b + r * kHPX;
+        float2 hxx[2], hxy[3], hyy[2], hxz[3], hyz[2], hzz[2], gxp[3], gyp[2], fp[2], l, rr, c[2], e[2];
+        hxx[0] = hd2(gx0[r][1], gx0[r][0]);
+        hxx[1] = hd2(gx0[r][2], gx0[r][1]);
+        // ---- in-plane second derivatives: the row beyond this one and the other row's first derivatives
+        {
+          float2 g[3];
+          ld_row(r == 0 ? P0 - kHPX : P0 + kHPX, l, c[0], c[1], rr);
+          gx_g(l, c[0], c[1], rr, g);
+          ld_quad(r == 0 ? P0 - 2 * kHPX : P0 + 2 * kHPX, e[0], e[1]);
+          if constexpr (ROWS == 2) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) hxy[i] = r == 0 ? hd2(gx0[ROWS - 1][i], g[i]) : hd2(g[i], gxm[0][i]);
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+              hyy[j] = r == 0 ? hd2(gy0[ROWS - 1][j], hd2(fm[0][j], e[j])) : hd2(hd2(e[j], fm[r][j]), gym[0][j]);
+          } else {
+            float2 gd[3], k[2];
+            ld_row(P0 + kHPX, l, c[0], c[1], rr);
+            gx_g(l, c[0], c[1], rr, gd);
+            ld_quad(P0 + 2 * kHPX, k[0], k[1]);
+#pragma unroll
+            for (int i = 0; i < 3; i++) hxy[i] = hd2(gd[i], g[i]);
+#pragma unroll
+            for (int j = 0; j < 2; j++) hyy[j] = hd2(hd2(k[j], fm[r][j]), hd2(fm[r][j], e[j]));
+          }
+        }
+        // ---- first derivatives of slice zh+1, then the z second derivatives
         l = *reinterpret_cast<const float2 *>(P1 - 2);
-        r = *reinterpret_cast<const float2 *>(P1 + 4);
-        gx_g(l, f0[0], f0[1], r, gxp);
-        ld_quad(P1 - kHPX, u0, u1);
-        ld_quad(P1 + kHPX, d0, d1);
-        gyp[0] = hd2(d0, u0);
-        gyp[1] = hd2(d1, u1);
-        ld_quad(P2, fp[0], fp[1]);
-        const bool zin = zh + 1 < D;   // gz outside the volume is zero
-        gzp[0] = zin ? hd2(fp[0], fm[0]) : zero2;
-        gzp[1] = zin ? hd2(fp[1], fm[1]) : zero2;
-      }
-      float2 hxz[3], hyz[2], hzz[2];
+        rr = *reinterpret_cast<const float2 *>(P1 + 4);
+        gx_g(l, f0[r][0], f0[r][1], rr, gxp);
+        ld_quad(r == 0 ? P1 - kHPX : P1 + kHPX, c[0], c[1]);
+        float2 d[2];
+        if (ROWS == 1) ld_quad(P1 + kHPX, d[0], d[1]);
+        ld_quad(ring + slot(zh + 2) * PL + b + r * kHPX, fp[0], fp[1]);
+        ld_quad(ring + slot(zh - 2) * PL + b + r * kHPX, e[0], e[1]);
+        const bool zin = zh + 1 < D, zim = zh >= 1;   // gz outside the volume is zero
 #pragma unroll
-      for (int i = 0; i < 3; i++) hxz[i] = hd2(gxp[i], gxm[i]);
-      hyz[0] = hd2(gyp[0], gym[0]);
-      hyz[1] = hd2(gyp[1], gym[1]);
-      hzz[0] = hd2(gzp[0], gzm[0]);
-      hzz[1] = hd2(gzp[1], gzm[1]);
-      // advance the pipeline
+        for (int j = 0; j < 2; j++) {
+          gyp[j] = ROWS == 1 ? hd2(d[j], c[j]) : r == 0 ? hd2(f0[ROWS - 1][j], c[j]) : hd2(c[j], fm[0][j]);
+          hyz[j] = hd2(gyp[j], gym[r][j]);
+          hzz[j] = hd2(zin ? hd2(fp[j], fm[r][j]) : zero2, zim ? hd2(fm[r][j], e[j]) : zero2);
+        }
 #pragma unroll
-      for (int i = 0; i < 3; i++) { gxm[i] = gx0[i]; gx0[i] = gxp[i]; }
+        for (int i = 0; i < 3; i++) hxz[i] = hd2(gxp[i], gxm[r][i]);
+        // advance the pipeline
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        gym[j] = gy0[j]; gy0[j] = gyp[j];
-        gzm[j] = gz0[j]; gz0[j] = gzp[j];
-        fm[j] = f0[j]; f0[j] = fp[j];
-      }
-      // G frame -> C frame for the two elements that live there (voxel 2j+h)
-      const float2 cxy[2] = {make_float2(hxy[0].y, hxy[1].x), make_float2(hxy[1].y, hxy[2].x)};
-      const float2 cxz[2] = {make_float2(hxz[0].y, hxz[1].x), make_float2(hxz[1].y, hxz[2].x)};
+        for (int i = 0; i < 3; i++) { gxm[r][i] = gx0[r][i]; gx0[r][i] = gxp[i]; }
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        mword |= pd_test2(hxx[j], cxy[j], cxz[j], hyy[j], hyz[j], hzz[j]) << (16 * j);
-        hv[2 * j][0] = hxx[j].x; hv[2 * j + 1][0] = hxx[j].y;
-        hv[2 * j][1] = cxy[j].x; hv[2 * j + 1][1] = cxy[j].y;
-        hv[2 * j][2] = cxz[j].x; hv[2 * j + 1][2] = cxz[j].y;
-        hv[2 * j][3] = hyy[j].x; hv[2 * j + 1][3] = hyy[j].y;
-        hv[2 * j][4] = hyz[j].x; hv[2 * j + 1][4] = hyz[j].y;
-        hv[2 * j][5] = hzz[j].x; hv[2 * j + 1][5] = hzz[j].y;
-      }
-      uint8_t *mo = mask + S.vox + i0;
-      if (!PAD) {
-        *reinterpret_cast<uint32_t *>(mo) = mword;
-      } else {   // the mask's rows are not padded
+        for (int j = 0; j < 2; j++) {
+          gym[r][j] = gy0[r][j]; gy0[r][j] = gyp[j];
+          fm[r][j] = f0[r][j]; f0[r][j] = fp[j];
+        }
+        // G frame -> C frame for the two elements that live there (voxel 2j+h)
+        const float2 cxy[2] = {make_float2(hxy[0].y, hxy[1].x), make_float2(hxy[1].y, hxy[2].x)};
+        const float2 cxz[2] = {make_float2(hxz[0].y, hxz[1].x), make_float2(hxz[1].y, hxz[2].x)};
 #pragma unroll
-        for (int o = 0; o < 4; o++) mo[o] = (uint8_t)(mword >> (8 * o));
-      }
-    } else {
-      const bool ym = Y >= 1, yp = Y + 1 < H, zm = zh >= 1, zp = zh + 1 < D;
-      const int p0 = slot(zh) * PL + b, p1 = slot(zh + 1) * PL + b, p2 = slot(zh + 2) * PL + b;
-      const int m1 = slot(zh - 1) * PL + b, m2 = slot(zh - 2) * PL + b;
+        for (int j = 0; j < 2; j++) {
+          mword |= pd_test2(hxx[j], cxy[j], cxz[j], hyy[j], hyz[j], hzz[j]) << (16 * j);
+          hv[2 * j][0] = hxx[j].x; hv[2 * j + 1][0] = hxx[j].y;
+          hv[2 * j][1] = cxy[j].x; hv[2 * j + 1][1] = cxy[j].y;
+          hv[2 * j][2] = cxz[j].x; hv[2 * j + 1][2] = cxz[j].y;
+          hv[2 * j][3] = hyy[j].x; hv[2 * j + 1][3] = hyy[j].y;
+          hv[2 * j][4] = hyz[j].x; hv[2 * j + 1][4] = hyz[j].y;
+          hv[2 * j][5] = hzz[j].x; hv[2 * j + 1][5] = hzz[j].y;
+        }
+        uint8_t *mo = mask + S.vox + ir;
+        if (!PAD) {
+          *reinterpret_cast<uint32_t *>(mo) = mword;
+        } else {   // the mask's rows are not padded
 #pragma unroll
-      for (int o = 0; o < 4; o++) {
-        const int X = X0 + o;
-        if (X >= W || Y >= H) continue;
-        // the slices hold zeros outside the volume, so a first derivative only needs the zero of its own
-        // position outside: past the frame's sides (xm .. yp) or the first and last slice (zm, zp)
-        const bool xm = X >= 1, xp = X + 1 < W;
-        const float *c0 = ring + p0 + o, *cu = ring + p1 + o, *cd = ring + m1 + o;
-        hv[o][0] = hdiff(xp ? hdiff(c0[2], c0[0]) : 0.0f, xm ? hdiff(c0[0], c0[-2]) : 0.0f);
-        hv[o][1] = hdiff(yp ? hdiff(c0[kHPX + 1], c0[kHPX - 1]) : 0.0f, ym ? hdiff(c0[1 - kHPX], c0[-1 - kHPX]) : 0.0f);
-        hv[o][2] = hdiff(zp ? hdiff(cu[1], cu[-1]) : 0.0f, zm ? hdiff(cd[1], cd[-1]) : 0.0f);
-        hv[o][3] = hdiff(yp ? hdiff(c0[2 * kHPX], c0[0]) : 0.0f, ym ? hdiff(c0[0], c0[-2 * kHPX]) : 0.0f);
-        hv[o][4] = hdiff(zp ? hdiff(cu[kHPX], cu[-kHPX]) : 0.0f, zm ? hdiff(cd[kHPX], cd[-kHPX]) : 0.0f);
-        hv[o][5] = hdiff(zp ? hdiff(ring[p2 + o], c0[0]) : 0.0f, zm ? hdiff(c0[0], ring[m2 + o]) : 0.0f);
-        const bool pdv = pd_test(hv[o][0], hv[o][1], hv[o][2], hv[o][3], hv[o][4], hv[o][5]);
-        mask[S.vox + i0 + o] = pdv ? 1 : 0;
-        // voxel 0 is background (its label is 0 in the reference's CCL)
-        mword |= (pdv && i0 + o != 0 ? 1u : 0u) << (8 * o);
-      }
-    }
-    // the foreground voxels go to the warp's staging buffer in shared memory; a full buffer
-    // goes to the global list with one slot reservation and coalesced stores (and the
-    // entries' normalized values).  Warps without foreground skip all of it; each lane's
-    // place comes from three bit-sliced ballots of its count.
-    const int nfg = __popc(mword);
-    const unsigned any = __ballot_sync(0xFFFFFFFFu, nfg != 0);
-    if (any) {
-      const int lane = t & 31;
-      const unsigned b0 = __ballot_sync(0xFFFFFFFFu, nfg & 1), b1 = __ballot_sync(0xFFFFFFFFu, nfg & 2),
-                     b2 = __ballot_sync(0xFFFFFFFFu, nfg & 4);
-      const unsigned lt = (1u << lane) - 1u;
-      const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
-      const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-      if (staged + tot > kHStage) {
-        flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
-        staged = 0;
-      }
-      int k = staged + excl;
+          for (int o = 0; o < 4; o++) mo[o] = (uint8_t)(mword >> (8 * o));
+        }
+      } else {
+        const int yr = Y + r;
+        const bool ym = yr >= 1, yp = yr + 1 < H, zm = zh >= 1, zp = zh + 1 < D;
+        const int br = b + r * kHPX;
+        const int p0 = slot(zh) * PL + br, p1 = slot(zh + 1) * PL + br, p2 = slot(zh + 2) * PL + br;
+        const int m1 = slot(zh - 1) * PL + br, m2 = slot(zh - 2) * PL + br;
 #pragma unroll
-      for (int o = 0; o < 4; o++) {
-        if (!((mword >> (8 * o)) & 1u)) continue;
-        float4 *dst = reinterpret_cast<float4 *>(stage + k);
-        dst[0] = make_float4(__int_as_float(i0 + o), 0.0f, hv[o][0], hv[o][1]);
-        dst[1] = make_float4(hv[o][2], hv[o][3], hv[o][4], hv[o][5]);
-        k++;
+        for (int o = 0; o < 4; o++) {
+          const int X = X0 + o;
+          if (X >= W || yr >= H) continue;
+          // the slices hold zeros outside the volume, so a first derivative only needs the zero of its own
+          // position outside: past the frame's sides (xm .. yp) or the first and last slice (zm, zp)
+          const bool xm = X >= 1, xp = X + 1 < W;
+          const float *c0 = ring + p0 + o, *cu = ring + p1 + o, *cd = ring + m1 + o;
+          hv[o][0] = hdiff(xp ? hdiff(c0[2], c0[0]) : 0.0f, xm ? hdiff(c0[0], c0[-2]) : 0.0f);
+          hv[o][1] = hdiff(yp ? hdiff(c0[kHPX + 1], c0[kHPX - 1]) : 0.0f, ym ? hdiff(c0[1 - kHPX], c0[-1 - kHPX]) : 0.0f);
+          hv[o][2] = hdiff(zp ? hdiff(cu[1], cu[-1]) : 0.0f, zm ? hdiff(cd[1], cd[-1]) : 0.0f);
+          hv[o][3] = hdiff(yp ? hdiff(c0[2 * kHPX], c0[0]) : 0.0f, ym ? hdiff(c0[0], c0[-2 * kHPX]) : 0.0f);
+          hv[o][4] = hdiff(zp ? hdiff(cu[kHPX], cu[-kHPX]) : 0.0f, zm ? hdiff(cd[kHPX], cd[-kHPX]) : 0.0f);
+          hv[o][5] = hdiff(zp ? hdiff(ring[p2 + o], c0[0]) : 0.0f, zm ? hdiff(c0[0], ring[m2 + o]) : 0.0f);
+          const bool pdv = pd_test(hv[o][0], hv[o][1], hv[o][2], hv[o][3], hv[o][4], hv[o][5]);
+          mask[S.vox + ir + o] = pdv ? 1 : 0;
+          // voxel 0 is background (its label is 0 in the reference's CCL)
+          mword |= (pdv && ir + o != 0 ? 1u : 0u) << (8 * o);
+        }
       }
-      staged += tot;
+      // the foreground voxels go to the warp's staging buffer in shared memory; a full buffer
+      // goes to the global list with one slot reservation and coalesced stores (and the
+      // entries' normalized values).  Warps without foreground skip all of it; each lane's
+      // place comes from three bit-sliced ballots of its count.
+      const int nfg = __popc(mword);
+      const unsigned any = __ballot_sync(0xFFFFFFFFu, nfg != 0);
+      if (any) {
+        const int lane = t & 31;
+        const unsigned b0 = __ballot_sync(0xFFFFFFFFu, nfg & 1), b1 = __ballot_sync(0xFFFFFFFFu, nfg & 2),
+                       b2 = __ballot_sync(0xFFFFFFFFu, nfg & 4);
+        const unsigned lt = (1u << lane) - 1u;
+        const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+        const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+        if (staged + tot > kHStage) {
+          flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
+          staged = 0;
+        }
+        int k = staged + excl;
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          if (!((mword >> (8 * o)) & 1u)) continue;
+          float4 *dst = reinterpret_cast<float4 *>(stage + k);
+          dst[0] = make_float4(__int_as_float(ir + o), 0.0f, hv[o][0], hv[o][1]);
+          dst[1] = make_float4(hv[o][2], hv[o][3], hv[o][4], hv[o][5]);
+          k++;
+        }
+        staged += tot;
+      }
     }
     __syncwarp();
-    if ((t & 31) == 0) mbar_arrive(&done[(ibase + (uint32_t)(zh - zb)) % kHRing]);
+    if ((t & 31) == 0) mbar_arrive(&done[(ibase + (uint32_t)(zh - zb)) % RING]);
   }
   if (staged) flush_stage<PAD>(stage, staged, S, norm, fg, fg_idx, &fg_count[sub * kFgCountStride]);
   zbase += (uint32_t)(D + 4);
@@ -762,12 +770,10 @@ static const SweepForm *find_form(const DogTaps &T, int W, int H, int nsub, int 
   return nullptr;
 }
 
-static constexpr size_t kHessSmem =
-    (size_t)kHRing * kHPX * kHPY * 4 + (2 * kHRing) * 8 + (size_t)(kHThreads / 32) * kHStage * sizeof(FgEntry);
 static_assert((kHPX * kHPY * 4) % 128 == 0, "TMA ring slots must start on 128-byte boundaries");
 
 // Whether the Hessian sweep can run at all (its volumes are the context's own, padded for TMA).
-bool sweep_supported(int max_smem) { return encode_fn() != nullptr && (int)kHessSmem <= max_smem; }
+bool sweep_supported(int max_smem) { return encode_fn() != nullptr && (int)HessT<1>::SMEM <= max_smem; }
 
 static CUresult encode_map(CUtensorMap *map, const float *base, int W, int P, int H, int D, int nsub, int bw, int bh) {
   const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)nsub};
@@ -823,9 +829,9 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
   if (ls.hess_per_sm > 0 && qctr) {
     const WorkQueue q{qctr + 1, (int)(tiles_h * (unsigned)nsub), (int)tiles_h};
     const unsigned grid = std::min<unsigned>((unsigned)(ls.hess_per_sm * ls.num_sms), tiles_h * (unsigned)nsub);
-    auto fn = P != W ? k_hess_sweep<true, true, false> : k_hess_sweep<true, false, false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
-    KLAUNCH("k_hess_sweep", s, (fn<<<grid, kHThreads, kHessSmem, s>>>(map_d, d_subs, norm, mask, fg, fg_idx, fg_count,
+    auto fn = P != W ? k_hess_sweep<true, true, false, 1> : k_hess_sweep<true, false, false, 1>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HessT<1>::SMEM);
+    KLAUNCH("k_hess_sweep", s, (fn<<<grid, HessT<1>::NT, HessT<1>::SMEM, s>>>(map_d, d_subs, norm, mask, fg, fg_idx, fg_count,
                                                                       d_status, q, D)));
   } else {
     // split z while the blocks about fit the chip at once (four per SM, and half as many again while those run), down
@@ -833,10 +839,14 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
     // piece 63 us, five 30 us; 683x517x75, whose tiles fill the chip, 221 us unsplit
     const int64_t room = (int64_t)6 * ls.num_sms / ((int64_t)tiles_h * nsub);
     const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(room, D / 6)), zlen = (int)ceil_div(D, pieces);
-    auto fn = zlen < D ? (P != W ? k_hess_sweep<false, true, true> : k_hess_sweep<false, false, true>)
-                       : (P != W ? k_hess_sweep<false, true, false> : k_hess_sweep<false, false, false>);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHessSmem);
-    KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub, ceil_div(D, zlen)), kHThreads, kHessSmem, s>>>(
+    const bool two = (int64_t)tiles_h * nsub >= 28 * (int64_t)ls.num_sms;   // four waves of seven blocks per SM
+    auto fn = two        ? (P != W ? k_hess_sweep<false, true, false, 2> : k_hess_sweep<false, false, false, 2>)
+              : zlen < D ? (P != W ? k_hess_sweep<false, true, true, 1> : k_hess_sweep<false, false, true, 1>)
+                         : (P != W ? k_hess_sweep<false, true, false, 1> : k_hess_sweep<false, false, false, 1>);
+    const unsigned nt = two ? HessT<2>::NT : HessT<1>::NT;
+    const size_t smem = two ? HessT<2>::SMEM : HessT<1>::SMEM;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub, ceil_div(D, zlen)), nt, smem, s>>>(
                                    map_d, d_subs, norm, mask, fg, fg_idx, fg_count, d_status, WorkQueue{}, zlen)));
   }
   return 0;

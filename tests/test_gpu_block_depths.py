@@ -59,3 +59,20 @@ def test_gpu_dog_sweep_tiles(W, H, D, sig):
     nan = np.isnan(ref)
     assert np.array_equal(np.isnan(got), nan)
     assert np.array_equal(got[~nan].view(np.uint32), ref[~nan].view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,D", [(1280, 1712, 4), (1283, 1701, 5)])
+def test_gpu_records_over_two_row_threads(W, H, D):
+    """Enough 32 x 16 tiles (4256) for the Hessian sweep's two-row form, with an odd last row and a padded width."""
+    import hdog
+    rng = np.random.default_rng(W + D)
+    vol = np.clip(300 + 60 * rng.normal(size=(D, H, W)), 0, 65535).astype(np.uint16)
+    p = hdog.make_params(width=W, height=H, depth=D, left_margin=0, right_margin=0, top_margin=0, bottom_margin=0,
+                         extra_depth_margin=0, radius_norm_xy=6, radius_norm_z=2, min_intensity=0, min_size=0)
+    with hdog.Context(p) as ctx:
+        got = ctx.run_substack(torch.from_numpy(vol).cuda(), D, 0)
+    ref = orc.substack(orc.params_from(p), vol, D, 0)[0]
+    assert len(got) == len(ref)
+    for f in ("local_x", "local_y", "local_z", "intensity", "size"):
+        assert np.array_equal(got[f], ref[f]), f
