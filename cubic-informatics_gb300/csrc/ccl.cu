@@ -8,9 +8,9 @@
 // which voxel 0 is background (label = index * mask).
 //
 // Here the same labels come from union-find in three passes, with no host round trip:
-//   1. k_ccl_local: a 64 x 16 x 32 tile (a whole 32-slice substack column) is labelled in
+//   1. k_ccl_local: a 64 x 16 tile of 32 slices (16 or 8 in small batches) is labelled in
 //      shared memory over its 2 x 2 x 2 cells (see below); the foreground edges that
-//      leave the tile (its x and y faces, and the wrap-around offsets) go to an edge list.
+//      leave the tile (its faces, and the wrap-around offsets) go to an edge list.
 //   2. k_ccl_edges: a persistent pass merges those edges in the global label array.
 //      If the list overflowed, k_ccl_cross_direct merges the same edges from the mask.
 //   3. k_ccl_flatten: every foreground voxel gets its root (a read-only walk, so every
