@@ -45,16 +45,16 @@ WORKLOAD = ("camera stack uint16 2560x2160x128, 60k nuclei (10% touching pairs),
 # Stage totals: normalize 56 (five passes), DoG 8, Hessian + mask 5, CCL 5, features ~0.
 KERNEL_BYTES_PER_VOXEL = {
     "k_mm_z": 2 + 4, "k_mm_y": 4 + 4, "k_mm_x": 4 + 8, "k_box_y": 8 + 8, "k_box_z_norm": 8 + 2 + 4,
-    "k_dog_sweep": 4 + 4, "k_hess_sweep": 4 + 1, "k_dog_hess": 4 + 1, "k_conv_x": 4 + 8, "k_conv_y": 8 + 8, "k_conv_z_dog": 8 + 4,
+    "k_dog_sweep": 4 + 4, "k_hess_sweep": 4 + 1, "k_conv_x": 4 + 8, "k_conv_y": 8 + 8, "k_conv_z_dog": 8 + 4,
     "k_hessian_pd": 4 + 1, "k_ccl_local": 1 + 4, "k_ccl_flatten": 1 + 0.125, "k_rank": 0.125,
     "k_accumulate": 1,
 }
 E2E_ALG_BYTES_PER_VOXEL = 6      # 2 B uint16 in + 4 B labels out per processed voxel
 # FP32 lane operations (an FMA or an add counts one) the DoG sweep spends per output voxel
 # with the workload's tap radii (xy 4 / 6, z 3 / 5): the x pass of both scales (9 + 13 taps)
-# over the 16-row tile and its 12 halo rows, the y pass (9 + 13), the z pass (7 + 11), the
+# over the 24-row tile and its 12 halo rows, the y pass (9 + 13), the z pass (7 + 11), the
 # difference and the scale.
-DOG_FP32_LANE_OPS_PER_VOXEL = (9 + 13) * (16 + 12) / 16 + (9 + 13) + (7 + 11) + 2
+DOG_FP32_LANE_OPS_PER_VOXEL = (9 + 13) * (24 + 12) / 24 + (9 + 13) + (7 + 11) + 2
 
 
 def peaks():
