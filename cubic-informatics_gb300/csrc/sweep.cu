@@ -53,13 +53,15 @@ constexpr int kDTX = 32;                // DoG tile width
 constexpr int kHTX = 32, kHTY = 16;     // Hessian tile
 constexpr int kHPX = kHTX + 8;          // Hessian ring row: columns x0-4 .. x0+kHTX+3 (16-byte aligned start)
 constexpr int kHPY = kHTY + 4;
+// Staged list entries per warp: one iteration adds at most 128 (four voxels per lane).
+constexpr int kHStage = 128;
 // Rows of an x quad that a thread of the Hessian sweep takes, and the shape that goes with them: threads, ring slots (a
 // slot is 40 x 20 floats = 25 x 128 bytes) and blocks per SM.
 template <int ROWS>
 struct HessT {
   static constexpr int NT = kHTX / 4 * kHTY / ROWS;
   static constexpr int RING = ROWS == 2 ? 6 : 8;
-  static constexpr size_t SMEM = (size_t)RING * kHPX * kHPY * 4 + (2 * RING) * 8 + (size_t)(NT / 32) * 128 * sizeof(FgEntry);
+  static constexpr size_t SMEM = (size_t)RING * kHPX * kHPY * 4 + (2 * RING) * 8 + (size_t)(NT / 32) * kHStage * sizeof(FgEntry);
 };
 
 // Input slices of the DoG sweep in flight: slice it + kDogIn - 1 is requested while slice it
@@ -391,8 +393,6 @@ __device__ __forceinline__ void ld_quad(const float *p, float2 &c0, float2 &c1) 
   c1 = make_float2(c.z, c.w);
 }
 
-// Staged list entries per warp: one iteration adds at most 128 (four voxels per lane).
-constexpr int kHStage = 128;
 
 // Moves a warp's `n` staged entries to the substack's list: one slot reservation, then
 // each lane completes whole entries -- the normalized value at the entry's voxel is
