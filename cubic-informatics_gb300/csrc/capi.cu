@@ -316,7 +316,8 @@ static void plan(const hdog_params *p, int max_sub, int64_t &nvox, int64_t &reg_
   L.add(S * nvox * sizeof(uint16_t));        // 0 img
   const int64_t pvox = (int64_t)pitch_of(p->width) * p->height * p->depth;
   L.add(S * pvox * sizeof(float2));          // 1 fa
-  L.add(S * pvox * sizeof(float2));          // 2 fb
+  // 2 fb; later the foreground list's roots, which take more room in substacks of a few hundred voxels
+  L.add(std::max<int64_t>(S * pvox * sizeof(float2), S * fg_capacity(nvox) * sizeof(int32_t)));
   L.add(S * pvox * sizeof(float));           // 3 norm
   L.add(S * pvox * sizeof(float));           // 4 dog
   L.add(S * nvox * sizeof(uint8_t));         // 5 mask
