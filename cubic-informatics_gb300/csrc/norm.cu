@@ -833,19 +833,20 @@ __global__ void k_copy_norm(const Sub *subs, float min_intensity, float *norm) {
 
 // ---------------------------------------------------------------- launchers
 static int max_optin_smem() {
-  static int v = 0;
-  if (!v) {
-    int dev = 0;
+  static const int v = [] {
+    int dev = 0, n = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (v <= 0) v = 48 * 1024;
-  }
+    cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return n > 0 ? n : 48 * 1024;
+  }();
   return v;
 }
 
+// The allowance belongs to the kernel, not to the launch, so it is the largest of any call: a smaller one could take
+// away what another host thread has just asked for.
 template <class F>
 static void allow_smem(F *fn, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin_smem());
 }
 
 // vec: the widest of 4, 2, 1 neighbouring columns that the inputs' alignment allows

@@ -1434,9 +1434,11 @@ void conv3_diff(const SoftRun &R, const float *in, float *out, const SoftTaps &t
 constexpr size_t kSoftMaxSmem = 220 * 1024;
 constexpr int kSoftColWarps[3] = {0, 8, 4};   // warps of the column passes along y and z
 
+// The allowance belongs to the kernel, not to the launch, so it is the largest of any call: a smaller one could take
+// away what another host thread has just asked for.
 template <class F>
 void allow_smem(F *fn, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoftMaxSmem);
 }
 
 // Grid of a column pass: 32 columns x the other coordinate x segments of the line, which is cut while the
