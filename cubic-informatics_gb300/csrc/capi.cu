@@ -241,7 +241,8 @@ struct hdog_ctx {
   unsigned long long *fg_count = nullptr;
   unsigned *qctr = nullptr;      // work-queue counters of the persistent sweeps
   LaunchShape shape;             // launch shape of the sweeps (autotuned per frame shape)
-  bool tuned = false;            // shape and graph_batch chosen by the autotuner
+  int tuned_on = 0;              // substacks of the batch the autotuner chose shape and graph_batch on (0: none)
+  bool tuned_fused = false;      // and whether the sweeps ran
   int graph_batch = 0;           // substacks per launch in the graph form (0: max_sub)
   std::string tune_report;       // JSON of the autotuner's timings
   RegionAcc acc{};
@@ -612,8 +613,13 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
   // entry beside the list (fb is free after the normalization)
   int32_t *fg_root = reinterpret_cast<int32_t *>(c->fb);
   if (fused) {
+    LaunchShape shape = c->shape;
+    if (c->tuned_on > 0 && nsub > c->tuned_on) {   // found on a smaller batch: here the tiles decide
+      shape = LaunchShape{};
+      shape.num_sms = c->num_sms;
+    }
     launch_dog_hess(c->d_subs, nsub, c->W, c->P, c->H, c->D, c->taps, c->norm, c->fa, c->fb, c->dog, c->mask, c->fg,
-                    fg_root, c->fg_count, c->status, c->shape, c->qctr, c->max_smem, st);
+                    fg_root, c->fg_count, c->status, shape, c->qctr, c->max_smem, st);
   } else {
     enqueue_dog(c, nsub, c->P, c->norm, c->dog, st);
     launch_hessian_pd(c->d_subs, nsub, c->W, c->H, c->D, c->dog, c->mask, nullptr, st);
@@ -1164,8 +1170,9 @@ extern "C" int hdog_run_stacks(hdog_ctx *c, const hdog_stack_in *stacks, int n_s
 // Launch shapes of the two sweeps (one block per tile, or a persistent grid of a few
 // blocks per SM over the device work queue) and the substacks per launch of the graph
 // form, chosen by timing the caller's own first batch with CUDA events.  Results are cached
-// per device, frame shape, depth, tap radii, normalization radii and context size: every
-// candidate gives the same output, only the time differs.
+// per device, frame shape, depth, tap radii, normalization radii, context size, substacks of the batch and
+// whether the sweeps ran (what wins on one substack may lose on many: the Hessian sweep's two-row form and its z split
+// are grid forms, chosen by the batch's tiles): every candidate gives the same output, only the time differs.
 struct TuneResult {
   LaunchShape shape;
   int batch = 0;
@@ -1174,24 +1181,25 @@ struct TuneResult {
 static std::mutex g_tune_mu;
 static std::vector<std::pair<std::string, TuneResult>> g_tune_cache;
 
-static std::string tune_key(const hdog_ctx *c) {
+static std::string tune_key(const hdog_ctx *c, int nsub, bool fused) {
   char k[256];
-  snprintf(k, sizeof(k), "%d:%dx%dx%d:%d,%d,%d,%d:%d,%d:%d:%d", c->dev, c->W, c->H, c->D, c->taps.r[0], c->taps.r[1],
+  snprintf(k, sizeof(k), "%d:%dx%dx%d:%d,%d,%d,%d:%d,%d:%d:%d:%d:%d", c->dev, c->W, c->H, c->D, c->taps.r[0], c->taps.r[1],
            c->taps.r[2], c->taps.r[3], c->p.radius_norm_xy, c->p.radius_norm_z, c->max_sub,
-           (c->p.erosion_radius_xy || c->p.erosion_radius_z) ? 1 : 0);
+           (c->p.erosion_radius_xy || c->p.erosion_radius_z) ? 1 : 0, nsub, fused ? 1 : 0);
   return k;
 }
 
-static bool tune_lookup(hdog_ctx *c) {
+static bool tune_lookup(hdog_ctx *c, int nsub, bool fused) {
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  const std::string k = tune_key(c);
+  const std::string k = tune_key(c, nsub, fused);
   for (auto &e : g_tune_cache)
     if (e.first == k) {
       c->shape = e.second.shape;
       c->shape.num_sms = c->num_sms;
       c->graph_batch = e.second.batch;
       c->tune_report = e.second.report;
-      c->tuned = true;
+      c->tuned_on = nsub;
+      c->tuned_fused = fused;
       return true;
     }
   return false;
@@ -1207,7 +1215,9 @@ static double timer_ms(EventTimer &t, const char *name) {
 // Tunes the context on the batch of nsub substacks whose host descriptors are set (their
 // inputs in device memory).  Leaves the context's scratch with one of the runs' results.
 static int tune_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
-  if (c->tuned || tune_lookup(c)) return HDOG_OK;
+  const bool fused = fused_ok(c);
+  if ((c->tuned_on == nsub && c->tuned_fused == fused) || tune_lookup(c, nsub, fused)) return HDOG_OK;
+  c->tuned_on = 0;
   KernelTimer *saved = g_timer;
   EventTimer timer;
   g_timer = &timer;
@@ -1215,7 +1225,6 @@ static int tune_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
     KernelTimer *saved;
     ~Restore() { g_timer = saved; }
   } restore{saved};
-  const bool fused = fused_ok(c);
   struct Cand {
     int dog, hess;
   };
@@ -1276,9 +1285,10 @@ static int tune_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
            c->W, c->H, c->D, nsub, dog_ms[0], dog_ms[1], dog_ms[2], hess_ms[0], hess_ms[1], hess_ms[2],
            c->shape.dog_per_sm, c->shape.hess_per_sm, full_ms, half_ms, batch);
   c->tune_report = rep;
-  c->tuned = true;
+  c->tuned_on = nsub;
+  c->tuned_fused = fused;
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tune_cache.emplace_back(tune_key(c), TuneResult{c->shape, batch, c->tune_report});
+  g_tune_cache.emplace_back(tune_key(c, nsub, fused), TuneResult{c->shape, batch, c->tune_report});
   return HDOG_OK;
 }
 
@@ -1292,10 +1302,10 @@ extern "C" int hdog_autotune(hdog_ctx *c, const uint16_t *d_stack, int length, v
   const size_t plane = (size_t)c->W * c->H;
   for (int s = 0; s < nsub; s++)
     set_sub(c, s, d_stack + (size_t)z0s[s] * plane, std::min(c->D, length - z0s[s]), z0s[s]);
-  c->tuned = false;
+  c->tuned_on = 0;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    const std::string k = tune_key(c);
+    const std::string k = tune_key(c, nsub, fused_ok(c));
     for (size_t i = 0; i < g_tune_cache.size(); i++)
       if (g_tune_cache[i].first == k) {
         g_tune_cache.erase(g_tune_cache.begin() + i);
@@ -1308,7 +1318,7 @@ extern "C" int hdog_autotune(hdog_ctx *c, const uint16_t *d_stack, int length, v
 extern "C" int hdog_ctx_tuning(hdog_ctx *c, char *buf, size_t cap) {
   if (!c || !buf || cap == 0) return fail(HDOG_ERR_ARG, "hdog_ctx_tuning: bad argument");
   std::lock_guard<std::mutex> lock(c->mu);
-  const std::string &r = c->tuned ? c->tune_report : std::string("{}");
+  const std::string &r = c->tuned_on > 0 ? c->tune_report : std::string("{}");
   if (r.size() + 1 > cap) return fail(HDOG_ERR_CAPACITY, "hdog_ctx_tuning: buffer too small");
   memcpy(buf, r.c_str(), r.size() + 1);
   return HDOG_OK;

@@ -209,9 +209,10 @@ int hdog_graph_destroy(hdog_graph *g);
    Times the context's first batch of a device stack with each candidate launch shape of the
    two sweeps (one block per tile, or persistent grids of 3 / 2 DoG and 5 / 4 Hessian blocks
    per SM over the device work queue) and the full batch against half of it, keeps the
-   fastest for the context (and for later contexts of the same frame shape, depth, radii and
-   size in this process), and writes the timings as JSON for hdog_ctx_tuning.  No counterpart
-   in the reference.  Every choice gives the same records. */
+   fastest for the context (and for later batches of as many substacks on contexts of the same
+   frame shape, depth, radii and size in this process), and writes the timings as JSON for
+   hdog_ctx_tuning.  A larger batch runs without the choice.  No counterpart in the
+   reference.  Every choice gives the same records. */
 int hdog_autotune(hdog_ctx *ctx, const uint16_t *d_stack, int length, void *stream);
 int hdog_ctx_tuning(hdog_ctx *ctx, char *buf, size_t cap);
 
