@@ -19,7 +19,7 @@ namespace hdog {
 
 // Largest volume hdog_ccl_noalloc accepts: 2^22 voxels (for example 256 x 256 x 64).
 constexpr int64_t kNoAllocMaxVoxels = (int64_t)1 << 22;
-constexpr int64_t kNoAllocEdges = kNoAllocMaxVoxels / 8 + 1024;
+constexpr int64_t kNoAllocEdges = kNoAllocMaxVoxels / 16 * 3 + 1024;   // as a context's (capi.cu)
 constexpr int64_t kNoAllocBlocks = kNoAllocMaxVoxels / kScanBlock;
 
 // Scratch layout, byte offsets (each part 256-byte aligned).
@@ -29,7 +29,7 @@ constexpr size_t kNaEdgeCount = 512;                                      // uns
 constexpr size_t kNaBlkCounts = 768;                                      // uint32 per 4096 voxels
 constexpr size_t kNaRootBits = kNaBlkCounts + ((kNoAllocBlocks * 4 + 255) / 256) * 256;
 constexpr size_t kNaEdges = kNaRootBits + ((kNoAllocBlocks * (kScanBlock / 32) * 4 + 255) / 256) * 256;
-constexpr size_t kNoAllocScratchBytes = kNaEdges + kNoAllocEdges * sizeof(int2);   // about 4.7 MB
+constexpr size_t kNoAllocScratchBytes = kNaEdges + kNoAllocEdges * sizeof(int2);   // about 6.8 MB
 
 static_assert(sizeof(Sub) <= kNaStatus, "descriptor slot too small");
 

@@ -221,7 +221,7 @@ int hdog_ctx_tuning(hdog_ctx *ctx, char *buf, size_t cap);
    themselves (a host framework that owns all device memory through its own allocator,
    or a service with a fixed memory budget reserved at start-up): the same labels as
    hdog_ccl for a mask of at most 2^22 voxels (width * height * depth), with all scratch
-   in one fixed 4.7 MB device array inside the library (per device, for the life of the
+   in one fixed 6.8 MB device array inside the library (per device, for the life of the
    process).  Larger volumes return HDOG_ERR_SHAPE.  Calls share that array: calls that
    overlap on the GPU (other streams or host threads) race; calls in sequence on one
    stream do not.  The first call on a device (and the first after a cudaDeviceReset,
