@@ -25,6 +25,7 @@
 // Erosion and dilation travel as one packed u32 per voxel: low half the running min,
 // high half 65535 minus the running max, so one __vminu2 combines both.
 #include <algorithm>
+#include <climits>
 
 #include "kernels.cuh"
 #include "window.cuh"
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(32 * kColWarps) k_mm_y_cols(const Sub *subs, i
 // the lanes' totals, and the prefix at the one place of a block where its windows start, from the lane
 // that many blocks back); the other seven slide, taking the extremes that leave from a second ring. All in
 // wrapping integers; the row's first and last extreme stand for the positions outside it.
-// G = 8 for reaches up to 31: chunks of 64 entries waste less of a short row, and the scan is three steps.
+// G = 8 (row_of_8): chunks of 64 entries waste less of a short row, and the scan is three steps.
 // Bound by instruction issue and the shared-memory pipe.
 // 2560x2160x32 substacks: eight with reach 20 3.85 -> 3.41 ms (against rows of 41 entries in
 // registers), four with reach 100 9.85 -> 1.62 ms (against chains of 201 in shared memory); 256x256
@@ -930,6 +931,17 @@ static size_t mm_x_smem(int mode, int r, int ry, int tx) {
   return words * 4;
 }
 
+// Whether the tiles of k_mm_x beat a warp a row: a row takes about 0.6 us (erosion 0.5) for each 256 columns, one after
+// the other, however few rows there are, and tiles share a long row among many blocks, at a cost per voxel that grows
+// with the reach.  us, rows / tiles, at reach 20: 64 rows of 2560 columns 14/12, of 20000 54/15, 608 of 5000 19/25, of
+// 20000 62/78; erosion, 256 rows of 20000 51/21, 2160 95/142.
+template <int MODE>
+static bool mm_x_tiles(int W, int64_t rows, int r) {
+  const double by_row = MODE == 0 ? 2.4e-3 : 2.0e-3;                          // us a column
+  const double by_voxel = MODE == 0 ? 3.5e-6 + 1e-7 * r : 1.6e-6 + 5e-8 * r;   // us
+  return W * (by_row - by_voxel * (double)rows) > 5.0;
+}
+
 template <int BORDER, int MODE>
 static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const uint32_t *in, void *out,
                  cudaStream_t s) {
@@ -938,8 +950,8 @@ static void mm_x(const Sub *d_subs, int nsub, int W, int64_t rows, int r, const 
     KLAUNCH("k_mm_x", s, (fn<<<dim3((unsigned)ceil_div(rows * W / 4, 256), nsub), 256, 0, s>>>(d_subs, in, static_cast<uint16_t *>(out))));
     return;
   }
-  if (r >= 4 && r <= (MODE == 0 ? 127 : 255)) {
-    switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+  if (r >= 4 && r <= (MODE == 0 ? 127 : 255) && !mm_x_tiles<MODE>(W, rows * nsub, r)) {
+    switch ((8 - 2 * r % 8) % 8 + (row_of_8(r, W, rows * nsub, MODE == 0 ? INT_MAX : 128) ? 1 : 0)) {
 #define HDOG_MMX_CASE(Q)                                                                                     \
   case Q:                                                                                                    \
     KLAUNCH("k_mm_x", s, (k_mm_x_rows<BORDER, MODE, 32, Q><<<dim3(ceil_div(rows, kRowWarps), nsub), 32 * kRowWarps, 0, s>>>( \

@@ -27,6 +27,7 @@
 // Tap radii are (int)(2 sigma + 0.5), held fixed for the derivatives.
 //
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "kernels.cuh"
@@ -1464,7 +1465,7 @@ void ext_pass(const SoftRun &R, const void *in, float2 *out, int axis, int r) {
     const float *v = static_cast<const float *>(in);
     const int64_t rows = (int64_t)g.H * g.D;
     if (r >= 4 && r <= 255) {
-      switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+      switch ((8 - 2 * r % 8) % 8 + (row_of_8(r, g.W, rows, INT_MAX) ? 1 : 0)) {
 #define HDOG_CASE(Q)                                                                                                  \
   case Q:                                                                                                             \
     KLAUNCH("k_soft_ext_rows", R.st, (k_soft_ext_rows<32, Q><<<ceil_div(rows, kSoftRowWarps), 32 * kSoftRowWarps, 0,  \
@@ -1514,7 +1515,7 @@ void ext_adj(const SoftRun &R, const void *src, const float2 *gout, float *gin, 
     const float *v = static_cast<const float *>(src);
     const int64_t rows = (int64_t)g.H * g.D;
     if (r >= 4 && r <= 255) {
-      switch ((8 - 2 * r % 8) % 8 + (r <= RowRing<8>::MAX_R ? 1 : 0)) {
+      switch ((8 - 2 * r % 8) % 8 + (row_of_8(r, g.W, rows, INT_MAX) ? 1 : 0)) {
 #define HDOG_CASE(Q)                                                                                                      \
   case Q:                                                                                                                 \
     KLAUNCH("k_soft_ext_adj_rows", R.st, (k_soft_ext_adj_rows<32, Q><<<ceil_div(rows, kSoftRowWarps), 32 * kSoftRowWarps, \

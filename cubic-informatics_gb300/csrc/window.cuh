@@ -90,6 +90,15 @@ struct RowRing {
   static constexpr int MAX_R = G == 8 ? 31 : 255;     // window of 2r + 1 entries within the reach
 };
 
+// Whether 8 lanes a row serve a pass best, or 32.  Eight waste less of a short row's last chunk and start four rows a
+// warp, but a row then takes four times as many steps one after the other, which only many rows hide: from 32 rows per SM
+// on, 64 where rows are long.  us with 8 / 32 lanes at reach 20: min/max and box of 2560 columns 33/20 in 2160 rows,
+// 71/60 in 9728; of 256 columns 12/10 in 2160, 14/18 in 8192, 62/109 in 69120.  narrow: rows wider than this never
+// take 8 lanes (the erosion's chunks carry little: 128 columns 29/30 in 69120 rows, 256 columns 52/49).
+inline bool row_of_8(int r, int W, int64_t rows, int narrow) {
+  return r <= RowRing<8>::MAX_R && W <= narrow && rows >= (W <= 1024 ? 32 : 64) * 152;
+}
+
 // The value of the group's lane `lag` lanes back (1 .. G): cur in this chunk, prev in the one before.
 template <int G, class T>
 __device__ __forceinline__ T row_lag(T cur, T prev, int lag) {
