@@ -850,11 +850,14 @@ static void allow_smem(F *fn, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin_smem());
 }
 
-// vec: the widest of 4, 2, 1 neighbouring columns that the inputs' alignment allows
+// vec: the widest of 4, 2, 1 neighbouring columns that the inputs' alignment allows.  The streaming form loads and
+// combines whole blocks of 2 rz + 1 slices, two of them at least, so volumes of few slices take the windows' own loads
+// (one slice of 2560x2160 at reach 5: 31 against 10 us).
 template <int BORDER>
-static void mm_z(const Sub *d_subs, int nsub, int plane, int rz, int vec, uint32_t *mm, cudaStream_t s) {
+static void mm_z(const Sub *d_subs, int nsub, int plane, int D, int rz, int vec, uint32_t *mm, cudaStream_t s) {
   const dim3 g2(ceil_div(plane / 2, 128), nsub), g1(ceil_div(plane, 128), nsub);
-  switch (rz) {
+  const int L = 2 * rz + 1;
+  switch ((int64_t)D * std::min(D, L) <= 2 * L ? 0 : rz) {
 #define HDOG_MMZ_CASE(R)                                                                      \
   case R:                                                                                     \
     if (vec >= 2)                                                                             \
@@ -983,7 +986,7 @@ void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, i
                       cudaStream_t s, float *ero_l, float *dil_l) {
   const int plane = W * H;
   const int64_t rows = (int64_t)H * D;
-  mm_z<0>(d_subs, nsub, plane, rz, mm_z_vec(src_aligned8, plane), ma, s);
+  mm_z<0>(d_subs, nsub, plane, D, rz, mm_z_vec(src_aligned8, plane), ma, s);
   mm_y<0>(d_subs, nsub, W, H, D, rxy, ma, mb, s);
   if (2 * rxy + 1 <= 256) {
     mm_x<0, 0>(d_subs, nsub, W, rows, rxy, mb, fa, s);
@@ -1037,7 +1040,7 @@ void launch_erosion(const Sub *d_subs, int nsub, int W, int H, int D, int rxy, i
   const int plane = W * H;
   const int64_t n = (int64_t)plane * D;
   uint32_t *a = tmp, *b = tmp + n * nsub;
-  mm_z<1>(d_subs, nsub, plane, rz, mm_z_vec(src_aligned8, plane), a, s);
+  mm_z<1>(d_subs, nsub, plane, D, rz, mm_z_vec(src_aligned8, plane), a, s);
   mm_y<1>(d_subs, nsub, W, H, D, rxy, a, b, s);
   mm_x<1, 1>(d_subs, nsub, W, (int64_t)H * D, rxy, b, dst, s);
 }
