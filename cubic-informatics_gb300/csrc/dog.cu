@@ -297,18 +297,21 @@ __global__ void __launch_bounds__(128) k_conv_z_dog_t(const Sub *subs, const __g
 // of a column from it, the first derivatives along z in registers: 13 reads a voxel, where planes of first derivatives beside the tile cost 61 KB of shared memory
 // (three blocks per SM), a second barrier and as many reads.  640x720x32 with planes: 200 -> 96 us, its 29 bytes a voxel
 // 64.
-constexpr int kHX = 32, kHY = 8, kHZ = 16;         // outputs per block
-constexpr int kDX = kHX + 8, kDY = kHY + 4, kDZ = kHZ + 4;   // dog tile (halo 2, whole quads along x)
+// HZ: slices of a block, 16, or 8 where 16 leave SMs without one (a block works through its slices one after the other).
+constexpr int kHX = 32, kHY = 8;                   // outputs per block and slice
+constexpr int kDX = kHX + 8, kDY = kHY + 4;        // dog tile (halo 2, whole quads along x)
 
+template <int HZ>
 __global__ void __launch_bounds__(256) k_hessian_pd(const Sub *subs, const float *dog, uint8_t *mask,
                                                     float *hess6) {
+  constexpr int kDZ = HZ + 4;
   __shared__ __align__(16) float sd[kDZ * kDY * kDX];
   const Sub S = subs[blockIdx.y];
-  const int nx = (S.W + kHX - 1) / kHX, ny = (S.H + kHY - 1) / kHY, nz = (S.D + kHZ - 1) / kHZ;
+  const int nx = (S.W + kHX - 1) / kHX, ny = (S.H + kHY - 1) / kHY, nz = (S.D + HZ - 1) / HZ;
   const int64_t bid = blockIdx.x;
   if (bid >= (int64_t)nx * ny * nz) return;
   const int bx = (int)(bid % nx), by = (int)((bid / nx) % ny), bz = (int)(bid / ((int64_t)nx * ny));
-  const int x0 = bx * kHX, y0 = by * kHY, z0 = bz * kHZ;
+  const int x0 = bx * kHX, y0 = by * kHY, z0 = bz * HZ;
   const int W = S.W, H = S.H, D = S.D;
   const int64_t plane = (int64_t)W * H, pplane = (int64_t)S.P * H;
   const int lx = threadIdx.x, ly = threadIdx.y;
@@ -322,14 +325,11 @@ __global__ void __launch_bounds__(256) k_hessian_pd(const Sub *subs, const float
               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   } else {
-    for (int row = ly; row < kDZ * kDY; row += kHY) {
-      const int y = y0 - 2 + row % kDY, z = z0 - 2 + row / kDY;
-      const bool in = y >= 0 && y < H && z >= 0 && z < D;
-      const float *f = dog + S.pvox + z * pplane + (int64_t)y * S.P;
-      for (int i = lx; i < kDX; i += 32) {
-        const int x = x0 - 4 + i;
-        sd[row * kDX + i] = in && x >= 0 && x < W ? f[x] : 0.0f;
-      }
+#pragma unroll 8
+    for (int i = ly * 32 + lx; i < kDZ * kDY * kDX; i += 256) {
+      const int row = i / kDX, x = x0 - 4 + i % kDX, y = y0 - 2 + row % kDY, z = z0 - 2 + row / kDY;
+      const bool in = y >= 0 && y < H && z >= 0 && z < D && x >= 0 && x < W;
+      sd[i] = in ? __ldg(dog + S.pvox + z * pplane + (int64_t)y * S.P + x) : 0.0f;
     }
   }
   __syncthreads();
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) k_hessian_pd(const Sub *subs, const float
   // first derivatives of slices z - 1 and z, the column's DoG of z and z + 1
   float gxm = slice_x(c - sz, z0 >= 1), gx0 = slice_x(c, true), gym = slice_y(c - sz, z0 >= 1), gy0 = slice_y(c, true);
   float gzm = z0 >= 1 ? cdiff(c[0], c[-2 * sz]) : 0.0f, gz0 = cdiff(c[sz], c[-sz]), c0 = c[0], c1 = c[sz];
-  for (int lz = 0; lz < kHZ && z0 + lz < D; lz++, c += sz) {
+  for (int lz = 0; lz < HZ && z0 + lz < D; lz++, c += sz) {
     const int z = z0 + lz;
     const bool zp = z + 1 < D;
     const float c2 = c[2 * sz], gxp = slice_x(c + sz, zp), gyp = slice_y(c + sz, zp), gzp = zp ? cdiff(c2, c0) : 0.0f;
@@ -417,8 +417,10 @@ void launch_dog(const Sub *d_subs, int nsub, int max_w, int pitch, int max_h, in
 
 void launch_hessian_pd(const Sub *d_subs, int nsub, int max_w, int max_h, int max_d, const float *dog,
                        uint8_t *mask, float *hess6, cudaStream_t s) {
-  const int64_t tiles = (int64_t)ceil_div(max_w, kHX) * ceil_div(max_h, kHY) * ceil_div(max_d, kHZ);
-  KLAUNCH("k_hessian_pd", s, (k_hessian_pd<<<dim3((unsigned)tiles, nsub), dim3(kHX, kHY), 0, s>>>(d_subs, dog, mask, hess6)));
+  const int64_t cols = (int64_t)ceil_div(max_w, kHX) * ceil_div(max_h, kHY);
+  const int hz = cols * ceil_div(max_d, 16) * nsub >= 152 ? 16 : 8;
+  const dim3 grid((unsigned)(cols * ceil_div(max_d, hz)), nsub);
+  KLAUNCH("k_hessian_pd", s, ((hz == 16 ? k_hessian_pd<16> : k_hessian_pd<8>)<<<grid, dim3(kHX, kHY), 0, s>>>(d_subs, dog, mask, hess6)));
 }
 
 }  // namespace hdog
