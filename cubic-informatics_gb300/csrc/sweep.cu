@@ -763,10 +763,18 @@ static const SweepInst kSweepInst[] = {sweep_inst<4, 6, 3, 5>(), sweep_inst<8, 1
 
 // The sweep for these taps, or none.  The four-row form where its 32 x 24 tiles give every SM its two blocks; below
 // that the two-row form's smaller ones, whose blocks take a slice sooner (one 128x96x16 substack 11.9 against 13.9 us).
+// A wave of either covers as many voxels (two blocks of 24 rows, three of 16), the four-row one in 0.81 to 0.89 of the
+// time, so heights that fill the 24-row tiles badly, or start another wave of them, stay with 16 rows.  us, 24 / 16
+// rows, radii (4, 6, 3, 5), 8 slices: 70000x8 75/57, 10000x32 29/23, 4000x100 29/26, 10000x40 30/30; 16 slices of
+// 4000x112 48/43, of 2560x2160 389/420.
 static const SweepForm *find_form(const DogTaps &T, int W, int H, int nsub, int num_sms) {
   for (const SweepInst &s : kSweepInst)
-    if (s.ra == T.r[0] && s.rb == T.r[2] && s.za == T.r[1] && s.zb == T.r[3])
-      return &s.form[(int64_t)ceil_div(W, kDTX) * ceil_div(H, s.form[1].ty) * nsub >= 2 * (int64_t)num_sms];
+    if (s.ra == T.r[0] && s.rb == T.r[2] && s.za == T.r[1] && s.zb == T.r[3]) {
+      const int64_t cols = (int64_t)ceil_div(W, kDTX) * nsub;
+      const int64_t tall = cols * ceil_div(H, s.form[1].ty), flat = cols * ceil_div(H, s.form[0].ty);
+      const auto waves = [](int64_t tiles, int64_t room) { return 0.5 * ((double)tiles / room + (double)((tiles + room - 1) / room)); };
+      return &s.form[tall >= 2 * (int64_t)num_sms && 0.85 * waves(tall, 2 * num_sms) <= waves(flat, 3 * num_sms)];
+    }
   return nullptr;
 }
 
