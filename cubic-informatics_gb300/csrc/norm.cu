@@ -1003,9 +1003,11 @@ void launch_normalize(const Sub *d_subs, int nsub, int W, int P, int H, int D, i
     dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * K) * D), nsub);
     KLAUNCH("k_box_y", s, (k_box_y_t<20, K><<<gy, dim3(32, by), 0, s>>>(d_subs, fa, fb)));
   } else {
-    const int K = rxy < 64 ? 16 : 20;
+    // fewer outputs a thread, and so more threads, where there are too few to fill the chip
+    const int K = (int64_t)W * H * D * nsub < ((int64_t)8 << 20) ? 12 : rxy < 64 ? 16 : 20;
+    const auto fn = K == 12 ? k_box_y<12> : K == 16 ? k_box_y<16> : k_box_y<20>;
     dim3 gy((unsigned)((int64_t)ceil_div(W, 32) * ceil_div(H, by * K) * D), nsub);
-    KLAUNCH("k_box_y", s, ((K == 16 ? k_box_y<16> : k_box_y<20>)<<<gy, dim3(32, by), 0, s>>>(d_subs, rxy, fa, fb)));
+    KLAUNCH("k_box_y", s, (fn<<<gy, dim3(32, by), 0, s>>>(d_subs, rxy, fa, fb)));
   }
   const dim3 gz(ceil_div(plane, 128) * ceil_div(D, kBoxZK), nsub), bz(128);
   switch (rz) {
