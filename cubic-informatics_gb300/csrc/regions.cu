@@ -164,9 +164,12 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(const Sub *subs, const ui
 // order, adding field f to a running sum that leaves by one atomic when the region changes.  The three groups
 // walk three stretches of the block's foreground, so runs go on from batch to batch.  All sums are integers (fixed
 // point for the float ones), so neither the grouping nor the order changes them.
-// Fields: 0 count << 32 | x, 1 y << 32 | z, 2 ordered max, 3 norm, 4-9 Hessian.  The packed halves hold a
-// stretch's sums (at most 171 voxels of coordinates below 2^16); in frames of 2^16 and more along an axis
-// every voxel leaves by itself.
+// Fields: 0 count << 56 | x, 1 y << s | z, 2 ordered max, 3 norm, 4-9 Hessian.  The packed parts hold a stretch's sums,
+// at most 171 voxels: of x 39 bits, of y and z together 47 (a volume has less than 2^31 voxels), z's below 24 where the
+// depth is below 2^16 (s = 24) and y's where it is not (s = 40).
+// A batch of several runs, whose ends would stop the groups one after the other, is summed by a segmented scan over its
+// lanes instead, the runs' last lanes adding side by side: components of 640x720x32 127 -> 107 us, random labels of 39
+// regions there 13.4 -> 7.9 ms (2 and 12 runs as the line: 108 and 114 us).
 // Bound by the stencil's gathers (24 per voxel).  640x720x32: 382 -> 116 us against a thread walking 16
 // neighbouring voxels, most of them background.  (On the Hessian sweep's list, whose runs are about three
 // entries long, the same walk took 6.4 ms where the scan of k_accumulate_fg takes 2.4: every run's end
@@ -179,40 +182,67 @@ struct AccStage {
   int32_t key[kAccBatch + 2];
 };
 
+constexpr int kAccShort = 4;   // runs of a batch from which its lanes sum them, one lane a voxel
+
 struct AccWalk {
   int f, g;                 // the lane's field and group (lanes 30, 31: none)
+  int zbits;                // z's bits in field 1
   int32_t cur = -1;         // region of the running sum
   unsigned long long sum = 0ull;
-  __device__ __forceinline__ AccWalk() {
+  __device__ __forceinline__ AccWalk(int depth) {
     const int lane = threadIdx.x & 31;
     g = lane / 10;
     f = lane - 10 * g;
+    zbits = depth < 65536 ? 24 : 40;
   }
-  __device__ __forceinline__ void flush(const Sub &S, const RegionAcc &acc, int64_t slots) const {
-    if (cur <= 0 || cur >= S.reg_cap || g > 2) return;
-    const int64_t i = S.reg + cur;
-    if (f == 0) {
-      atomicAdd(&acc.count[i], (uint32_t)(sum >> 32));
-      atomicAdd(&acc.sum_xyz[i], sum & 0xFFFFFFFFull);
-    } else if (f == 1) {
-      atomicAdd(&acc.sum_xyz[slots + i], sum >> 32);
-      atomicAdd(&acc.sum_xyz[2 * slots + i], sum & 0xFFFFFFFFull);
-    } else if (f == 2) {
-      atomicMax(&acc.max_ord[i], (uint32_t)sum);
+  __device__ __forceinline__ void add(const Sub &S, const RegionAcc &acc, int64_t slots, int32_t key, int field,
+                                      unsigned long long v) const {
+    if (key <= 0 || key >= S.reg_cap) return;
+    const int64_t i = S.reg + key;
+    if (field == 0) {
+      atomicAdd(&acc.count[i], (uint32_t)(v >> 56));
+      atomicAdd(&acc.sum_xyz[i], v & ((1ull << 56) - 1));
+    } else if (field == 1) {
+      atomicAdd(&acc.sum_xyz[slots + i], v >> zbits);
+      atomicAdd(&acc.sum_xyz[2 * slots + i], v & ((1ull << zbits) - 1));
+    } else if (field == 2) {
+      atomicMax(&acc.max_ord[i], (uint32_t)v);
     } else {
-      atomicAdd(f == 3 ? &acc.sum_norm[i] : &acc.hess[(f - 4) * slots + i], sum);
+      atomicAdd(field == 3 ? &acc.sum_norm[i] : &acc.hess[(field - 4) * slots + i], v);
     }
   }
+  __device__ __forceinline__ void flush(const Sub &S, const RegionAcc &acc, int64_t slots) const {
+    if (g <= 2) add(S, acc, slots, cur, f, sum);
+  }
   // a batch: st as written by its lanes (key -1: no voxel)
-  __device__ __forceinline__ void walk(const AccStage &st, const Sub &S, const RegionAcc &acc, int64_t slots,
-                                       bool one_by_one = false) {
+  __device__ __forceinline__ void walk(const AccStage &st, const Sub &S, const RegionAcc &acc, int64_t slots) {
     __syncwarp();
-    if (g <= 2) {
+    const int lane = threadIdx.x & 31;
+    const int32_t mine = st.key[min(lane, kAccBatch - 1)], before = __shfl_up_sync(0xFFFFFFFFu, mine, 1);
+    const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || mine != before);
+    if (__popc(heads) >= kAccShort) {
+      flush(S, acc, slots);
+      cur = -1;
+      sum = 0ull;
+      const int start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));   // first lane of this lane's run
+      const bool last = lane < kAccBatch && (lane == kAccBatch - 1 || ((heads >> (lane + 1)) & 1u));
+      int reach = 1;   // as far as the longest run
+      while (__any_sync(0xFFFFFFFFu, lane - reach >= start)) reach *= 2;
+#pragma unroll
+      for (int k = 0; k < 10; k++) {
+        unsigned long long v = st.v[k * kAccPitch + min(lane, kAccBatch - 1)];
+        for (int d = 1; d < reach; d *= 2) {
+          const unsigned long long u = __shfl_up_sync(0xFFFFFFFFu, v, d);
+          if (lane - d >= start) v = k == 2 ? max(u, v) : v + u;
+        }
+        if (last) add(S, acc, slots, mine, k, v);
+      }
+    } else if (g <= 2) {
 #pragma unroll
       for (int i = 0; i < 10; i++) {
         const int32_t k = st.key[10 * g + i];
         const unsigned long long v = st.v[f * kAccPitch + 10 * g + i];
-        if (k != cur || one_by_one) {
+        if (k != cur) {
           flush(S, acc, slots);
           cur = k;
           sum = 0ull;
@@ -224,12 +254,12 @@ struct AccWalk {
   }
 };
 
-__device__ __forceinline__ void acc_put(AccStage &st, int lane, int32_t key, int x, int y, int z, float norm,
+__device__ __forceinline__ void acc_put(AccStage &st, int lane, int32_t key, int x, int y, int z, int zbits, float norm,
                                         const float (&h)[6]) {
   st.key[lane] = key;
   unsigned long long *v = st.v + lane;
-  v[0] = 1ull << 32 | (uint32_t)x;
-  v[kAccPitch] = (unsigned long long)(uint32_t)y << 32 | (uint32_t)z;
+  v[0] = 1ull << 56 | (uint32_t)x;
+  v[kAccPitch] = (unsigned long long)(uint32_t)y << zbits | (uint32_t)z;
   v[2 * kAccPitch] = f2ord(norm);
   v[3 * kAccPitch] = to_fix(norm);
 #pragma unroll
@@ -277,7 +307,7 @@ __global__ void __launch_bounds__(32 * kAccWarps) k_accumulate(const Sub *subs, 
   if (total == 0) return;
   const int W = S.W, H = S.H, cnt = (int)total;
   const int per = (cnt + 3 * kAccWarps - 1) / (3 * kAccWarps);   // voxels per group
-  AccWalk walk;
+  AccWalk walk(S.D);
   for (int b = 0; b < per; b += 10) {
     if (lane < kAccBatch) {
       const int in = b + walk.f, e = (3 * w + walk.g) * per + in;
@@ -293,9 +323,9 @@ __global__ void __launch_bounds__(32 * kAccWarps) k_accumulate(const Sub *subs, 
         v = norm[S.pvox + ((int64_t)z * H + y) * S.P + x];
         hessian_at(dog + S.pvox, W, S.P, H, S.D, x, y, z, h);
       }
-      acc_put(stage[w], lane, key, x, y, z, v, h);
+      acc_put(stage[w], lane, key, x, y, z, walk.zbits, v, h);
     }
-    walk.walk(stage[w], S, acc, slots, W > 65535 || H > 65535 || S.D > 65535);
+    walk.walk(stage[w], S, acc, slots);
   }
   walk.flush(S, acc, slots);
 }
