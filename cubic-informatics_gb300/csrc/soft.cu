@@ -838,13 +838,21 @@ __device__ __forceinline__ void soft_norm_adj_one(float v, float2 m, float g, fl
   }
 }
 
-// VEC 4: four voxels per thread in 16-byte accesses (I and g_I on 16 bytes; the workspace's volumes are)
-template <int VEC>
-__global__ void __launch_bounds__(256) k_soft_norm_adj(const float *I, const float2 *ed, const float *g_norm, float *g_I,
+// Four neighbouring gradients of the normalized volume
+__device__ __forceinline__ float4 soft_ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 soft_ld4(const double *p) {
+  const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+  return make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+}
+
+// VEC 4: four voxels per thread in 16-byte accesses (I and g_I on 16 bytes; the workspace's volumes are).  g_norm in
+// doubles may lie where g_ed goes: a voxel's eight bytes are read before they are written.
+template <int VEC, class GT>
+__global__ void __launch_bounds__(256) k_soft_norm_adj(const float *I, const float2 *ed, const GT *g_norm, float *g_I,
                                                        float2 *g_ed, float min_intensity, int64_t N) {
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (VEC == 4 && i + 4 <= N) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(I + i)), g = __ldg(reinterpret_cast<const float4 *>(g_norm + i));
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(I + i)), g = soft_ld4(g_norm + i);
     const float4 m0 = __ldg(reinterpret_cast<const float4 *>(ed + i)), m1 = __ldg(reinterpret_cast<const float4 *>(ed + i) + 1);
     float4 gi;
     float2 a, b, c, d;
@@ -857,7 +865,7 @@ __global__ void __launch_bounds__(256) k_soft_norm_adj(const float *I, const flo
     reinterpret_cast<float4 *>(g_ed + i)[1] = make_float4(c.x, c.y, d.x, d.y);
     return;
   }
-  for (int64_t k = i; k < min(i + VEC, N); k++) soft_norm_adj_one(I[k], ed[k], g_norm[k], min_intensity, g_I[k], g_ed[k]);
+  for (int64_t k = i; k < min(i + VEC, N); k++) soft_norm_adj_one(I[k], ed[k], (float)g_norm[k], min_intensity, g_I[k], g_ed[k]);
 }
 
 // a += b.x + b.y (no window along any of x and y: both sides' gradients belong where they are)
@@ -1025,7 +1033,7 @@ __global__ void k_soft_gdog(const double *in, float *out, int64_t N) {
 // dense passes' fold, tap by tap in the same order; a tap outside the volume multiplies a staged
 // zero instead of being skipped, which leaves the sum as it is.  The adjoint spreads the stencil's
 // gradient through the same taps (z, y, then x) and adds the patch to the normalized volume's
-// gradient, one float reduction per voxel and point.
+// gradient, one reduction per voxel and point: in float32, or (GT) in doubles where many points may share a voxel.
 // What bounds it: the phases' latency (twelve barriers a point) and shared-memory loads; 48 KB and
 // 256 threads a block at sigmas 2.0 / 3.2, four blocks per SM.  128x512x512, 4000 points, sigmas
 // (2.0, 2.0, 1.5, 3.2, 3.2, 2.4): 98 us forward and 209 us backward, where the 28 dense passes took
@@ -1116,11 +1124,11 @@ __device__ __forceinline__ float soft_hessian_coef(const SoftGeom &g, SoftPoint 
 // gradients are formed from into acc[0..6] (as soft_backward's dense passes leave them), the
 // threshold gradients into gb[0..2], and, when gnorm is given, the gradient of the normalized volume
 // added to it.  All sums are doubles that must start at zero.
-template <bool BWD>
+template <bool BWD, class GT>
 __global__ void __launch_bounds__(kSoftPtThreads, 4)
     k_soft_points_local(const float *norm, SoftGeom g, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
                         const __grid_constant__ SoftTapSet T, SoftBox box, float nrm, float tau, SoftThresh b,
-                        float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+                        float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, GT *gnorm) {
   extern __shared__ float sm[];
   __shared__ float fv[2][4][kSoftStencil];   // per scale: plain, d/dz, d/dy, d/dx
   __shared__ float cube[125], coef[125];     // DoG and d loss / d DoG around the point (0 off the stencil)
@@ -1319,7 +1327,7 @@ __global__ void __launch_bounds__(kSoftPtThreads, 4)
     for (int k = t, xi = xi0, yi = yi0, zi = zi0; k < box.tile(); k += kSoftPtThreads) {
       const int x = x0 + xi, y = y0 + yi, z = z0 + zi;
       const float v = tile[k];
-      if (v != 0.0f && soft_in(g, x, y, z)) atomicAdd(gnorm + ((int64_t)z * g.H + y) * g.W + x, v);
+      if (v != 0.0f && soft_in(g, x, y, z)) atomicAdd(gnorm + ((int64_t)z * g.H + y) * g.W + x, (GT)v);
       xi += sx;
       yi += sl;
       if (xi >= ex) { xi -= ex; yi++; }
@@ -1659,9 +1667,13 @@ bool points_local(const SoftRun &R, int64_t n, SoftBox &box) {
   return (double)n * (20.0 + 0.011 * box.tile()) <= 0.16 * (double)R.N + 150e3;
 }
 
-template <bool BWD>
+// Points from which the gradient of the normalized volume is summed in doubles: a float32 sum of n like terms is off by up
+// to n / 2^25 of itself (60 k points at one place: 4e-4).  Doubles take 50 of 2490 us more at 512x512x128.
+constexpr int64_t kSoftManyPoints = 4096;
+
+template <bool BWD, class GT = float>
 void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int n_pos, const int32_t *neg, int n_neg,
-                   float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, float *gnorm) {
+                   float grad_loss, const float *d_grad_loss, float *scores, double *acc, double *gb, GT *gnorm) {
   const hdog_soft_params &p = R.p;
   const int64_t n = (int64_t)n_pos + n_neg;
   if (n == 0) return;
@@ -1676,10 +1688,10 @@ void points_launch(const SoftRun &R, const SoftBox &box, const int32_t *pos, int
   const float nrm = (float)pow((double)s[0] * s[1] * s[2], (double)p.gamma);
   const size_t smem = (size_t)box.floats() * sizeof(float);
   if (smem > 44 * 1024)   // 48 KB without it, static shared memory included
-    cudaFuncSetAttribute(k_soft_points_local<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoftLocalSmem);
+    cudaFuncSetAttribute(k_soft_points_local<BWD, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoftLocalSmem);
   const unsigned grid = (unsigned)std::min<int64_t>(n, 152 * 8);
   KLAUNCH(BWD ? "k_soft_points_local_adj" : "k_soft_points_local", R.st,
-          (k_soft_points_local<BWD><<<grid, kSoftPtThreads, smem, R.st>>>(R.slot(S_NORM), R.g, pos, n_pos, neg, n_neg, T,
+          (k_soft_points_local<BWD, GT><<<grid, kSoftPtThreads, smem, R.st>>>(R.slot(S_NORM), R.g, pos, n_pos, neg, n_neg, T,
                                                                           box, nrm, p.tau, b, grad_loss, d_grad_loss, scores,
                                                                           acc, gb, gnorm)));
 }
@@ -1720,7 +1732,7 @@ int soft_forward(const hdog_soft_params *p, const float *vol, const int32_t *pos
   const bool local = points_local(R, (int64_t)n_pos + n_neg, box);
   forward_chain(R, vol, !local);
   if (local)
-    points_launch<false>(R, box, pos, n_pos, neg, n_neg, 0.0f, nullptr, scores, R.acc, nullptr, nullptr);
+    points_launch<false>(R, box, pos, n_pos, neg, n_neg, 0.0f, nullptr, scores, R.acc, nullptr, static_cast<float *>(nullptr));
   else if (n_pos + n_neg > 0)
     KLAUNCH("k_soft_points", st, (k_soft_points<<<ceil_div(n_pos + n_neg, 128), 128, 0, st>>>(
                                      R.slot(S_DOG), R.g, pos, n_pos, neg, n_neg, p->tau, thresh_of(*p), scores,
@@ -1750,11 +1762,18 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
   double *gb = R.acc + 8;   // threshold gradients
   cudaMemsetAsync(R.acc, 0, 14 * sizeof(double), st);
   float *gdog = R.slot(S_GDOG);
+  const bool many = local && (int64_t)n_pos + n_neg > kSoftManyPoints;
   if (local) {
-    float *gnorm = grad_vol ? R.slot(S_GB) : nullptr;
-    if (gnorm) cudaMemsetAsync(gnorm, 0, R.N * sizeof(float), st);
-    points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, d_grad_loss, nullptr, grad_sigma ? R.acc : nullptr,
-                        grad_thresh ? gb : nullptr, gnorm);
+    double *sums = grad_sigma ? R.acc : nullptr, *thr = grad_thresh ? gb : nullptr;
+    if (many) {
+      double *gnorm = grad_vol ? reinterpret_cast<double *>(R.slot(S_PA)) : nullptr;   // a pair's two slots
+      if (gnorm) cudaMemsetAsync(gnorm, 0, R.N * sizeof(double), st);
+      points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, d_grad_loss, nullptr, sums, thr, gnorm);
+    } else {
+      float *gnorm = grad_vol ? R.slot(S_GB) : nullptr;
+      if (gnorm) cudaMemsetAsync(gnorm, 0, R.N * sizeof(float), st);
+      points_launch<true>(R, box, pos, n_pos, neg, n_neg, grad_loss, d_grad_loss, nullptr, sums, thr, gnorm);
+    }
   } else {
     // a forward call with fewer points may have left the DoG slot empty
     if (forward_kept) dense_dog(R, R.flags() + 1);
@@ -1807,11 +1826,14 @@ int soft_backward(const hdog_soft_params *p, const float *vol, const int32_t *po
     // quotient rule: direct term into grad_vol, the box means' gradients into a pair
     float2 *cur = R.pair(S_PA), *next = R.pair(S_PB);
     const auto on16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    if (on16(vol) && on16(grad_vol) && on16(work))
-      KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<4><<<ceil_div(R.N, 1024), 256, 0, st>>>(
-                                         vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur, p->min_intensity, R.N)));
+    const bool by4 = on16(vol) && on16(grad_vol) && on16(work);
+    const unsigned blocks = by4 ? ceil_div(R.N, 1024) : nb;
+    if (many)
+      KLAUNCH("k_soft_norm_adj", st, ((by4 ? k_soft_norm_adj<4, double> : k_soft_norm_adj<1, double>)<<<blocks, 256, 0, st>>>(
+                                         vol, R.pair(S_ED), reinterpret_cast<const double *>(cur), grad_vol, cur,
+                                         p->min_intensity, R.N)));
     else
-      KLAUNCH("k_soft_norm_adj", st, (k_soft_norm_adj<1><<<nb, 256, 0, st>>>(
+      KLAUNCH("k_soft_norm_adj", st, ((by4 ? k_soft_norm_adj<4, float> : k_soft_norm_adj<1, float>)<<<blocks, 256, 0, st>>>(
                                          vol, R.pair(S_ED), R.slot(S_GB), grad_vol, cur, p->min_intensity, R.N)));
     // box means transposed z -> y -> x, then the extremes z -> y -> x, each adding to a zeroed pair but the
     // last, which adds straight to the input gradient (holding the quotient rule's direct term)
