@@ -612,7 +612,7 @@ static void enqueue_dog(hdog_ctx *c, int nsub, int P, const float *norm, float *
 
 // The chain after normalization: DoG + Hessian (fused sweep or separate passes), CCL,
 // region numbering and accumulation, features and record compaction.
-static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t st) {
+static int enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t st) {
   // each foreground entry's voxel index, then its root (written by the CCL flatten), per
   // entry beside the list (fb is free after the normalization)
   int32_t *fg_root = reinterpret_cast<int32_t *>(c->fb);
@@ -622,8 +622,9 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
       shape = LaunchShape{};
       shape.num_sms = c->num_sms;
     }
-    launch_dog_hess(c->d_subs, nsub, c->W, c->P, c->H, c->D, c->taps, c->norm, c->fa, c->fb, c->dog, c->mask, c->fg,
-                    fg_root, c->fg_count, c->status, shape, c->qctr, c->max_smem, st);
+    const int rc = launch_dog_hess(c->d_subs, nsub, c->W, c->P, c->H, c->D, c->taps, c->norm, c->fa, c->fb, c->dog, c->mask,
+                                   c->fg, fg_root, c->fg_count, c->status, shape, c->qctr, c->max_smem, st);
+    if (rc != HDOG_OK) return fail(rc, "the Hessian sweep's tensor map was refused");
   } else {
     enqueue_dog(c, nsub, c->P, c->norm, c->dog, st);
     launch_hessian_pd(c->d_subs, nsub, c->W, c->H, c->D, c->dog, c->mask, nullptr, st);
@@ -641,6 +642,7 @@ static void enqueue_after_norm(hdog_ctx *c, int nsub, bool fused, cudaStream_t s
                    c->blk_counts, c->blk_offsets, c->chunk, c->num_regions, c->acc, c->slots, c->status, st);
   launch_finalize(c->d_subs, nsub, c->reg_cap, rseg_of(c), c->num_regions, c->acc, c->slots, c->out, filter_of(c->p),
                   c->rec_counts, c->blk_offsets, c->chunk, c->num_records, c->records, st);
+  return HDOG_OK;
 }
 
 // The fused sweep and the list-based region sums; the latter add coordinates in 32 bits
@@ -682,7 +684,7 @@ static int enqueue_batch(hdog_ctx *c, int nsub, bool fused, cudaStream_t st) {
     TRY(upload_subs(c, nsub, st));
   }
   enqueue_normalize(c, nsub, c->norm, st);
-  enqueue_after_norm(c, nsub, fused, st);
+  TRY(enqueue_after_norm(c, nsub, fused, st));
   HDOG_CUDA_TRY(cudaGetLastError());
   return HDOG_OK;
 }
@@ -707,7 +709,7 @@ static int run_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
     if (over) {
       // more foreground than the list holds: redo this batch with the separate passes
       clear_async(batch_zeros(c, nsub, false), st);
-      enqueue_after_norm(c, nsub, false, st);
+      TRY(enqueue_after_norm(c, nsub, false, st));
       TRY(readback(c, nsub, st));
     }
   }

@@ -160,7 +160,8 @@ bool launch_dog_sweep(const Sub *d_subs, int nsub, int W, int P, int H, int D, c
 // DoG + Hessian + PD: norm -> dog by the radius-specialised sweep, or by the separate passes (temporaries
 // fa, fb) where the tap radii have no instantiation, then dog -> mask + list by the Hessian sweep.
 // ls / qctr (two device counters, zero at the call): the launch shape of the sweeps.
-int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
+// A status of the C ABI; nothing is launched unless it is HDOG_OK.
+[[nodiscard]] int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, const DogTaps &T, const float *norm,
                     float2 *fa, float2 *fb, float *dog, uint8_t *mask, FgEntry *fg, int32_t *fg_idx, unsigned long long *fg_count,
                     int *d_status, const LaunchShape &ls, unsigned *qctr, int max_smem, cudaStream_t s);
 // ---- ccl.cu ----

@@ -784,6 +784,7 @@ static_assert((kHPX * kHPY * 4) % 128 == 0, "TMA ring slots must start on 128-by
 bool sweep_supported(int max_smem) { return encode_fn() != nullptr && (int)HessT<1>::SMEM <= max_smem; }
 
 static CUresult encode_map(CUtensorMap *map, const float *base, int W, int P, int H, int D, int nsub, int bw, int bh) {
+  if (encode_fn() == nullptr) return CUDA_ERROR_NOT_SUPPORTED;
   const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)nsub};
   const cuuint64_t strides[3] = {(cuuint64_t)P * 4, (cuuint64_t)P * H * 4, (cuuint64_t)P * H * D * 4};
   const cuuint32_t box[4] = {(cuuint32_t)bw, (cuuint32_t)bh, 1, 1};
@@ -828,7 +829,7 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
                     cudaStream_t s) {
   const SweepForm *si = find_form(T, W, H, nsub, ls.num_sms);
   CUtensorMap map_n, map_d;
-  if (encode_map(&map_d, dog, W, P, H, D, nsub, kHPX, kHPY) != CUDA_SUCCESS) return -1;
+  if (encode_map(&map_d, dog, W, P, H, D, nsub, kHPX, kHPY) != CUDA_SUCCESS) return HDOG_ERR_CUDA;
   if (si && (int)si->smem <= max_smem && encode_map(&map_n, norm, W, P, H, D, nsub, si->bw, si->bh) == CUDA_SUCCESS)
     dog_sweep_launch(si, map_n, T, d_subs, nsub, W, H, dog, d_status, ls, qctr, s);
   else
@@ -857,7 +858,7 @@ int launch_dog_hess(const Sub *d_subs, int nsub, int W, int P, int H, int D, con
     KLAUNCH("k_hess_sweep", s, (fn<<<dim3(tiles_h, nsub, ceil_div(D, zlen)), nt, smem, s>>>(
                                    map_d, d_subs, norm, mask, fg, fg_idx, fg_count, d_status, WorkQueue{}, zlen)));
   }
-  return 0;
+  return HDOG_OK;
 }
 
 }  // namespace hdog
