@@ -558,6 +558,7 @@ static ClearList batch_zeros(hdog_ctx *c, int nsub, bool fused) {
 
 static int upload_subs(hdog_ctx *c, int nsub, cudaStream_t st, const ClearList &zeros = ClearList()) {
   const int ms = c->max_sub;
+  if (zeros.over) return fail(HDOG_ERR_CAPACITY, "too many ranges to clear");
   for (int s0 = 0; s0 < ms; s0 += kParamSubs) {
     const int n = std::min(kParamSubs, ms - s0);
     SubsParam P;
@@ -708,7 +709,8 @@ static int run_batch(hdog_ctx *c, int nsub, cudaStream_t st) {
     for (int s = 0; s < nsub; s++) over |= c->h_counts[2 * c->max_sub + s] > c->fg_cap;
     if (over) {
       // more foreground than the list holds: redo this batch with the separate passes
-      clear_async(batch_zeros(c, nsub, false), st);
+      const int rc = clear_async(batch_zeros(c, nsub, false), st);
+      if (rc != HDOG_OK) return fail(rc, "too many ranges to clear");
       TRY(enqueue_after_norm(c, nsub, false, st));
       TRY(readback(c, nsub, st));
     }

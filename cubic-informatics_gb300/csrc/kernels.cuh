@@ -129,7 +129,12 @@ struct ClearList {
   uint32_t *p[kMax];
   int64_t n[kMax];
   int count = 0;
+  bool over = false;   // a range had no place: the launchers refuse the list
   void add(void *q, size_t bytes) {
+    if (count == kMax) {
+      over = true;
+      return;
+    }
     p[count] = static_cast<uint32_t *>(q);
     n[count++] = (int64_t)(bytes / 4);
   }
@@ -147,7 +152,8 @@ __device__ __forceinline__ void clear_ranges(const ClearList &z) {
       z.p[r][i] = 0u;
 }
 #endif
-void clear_async(const ClearList &z, cudaStream_t s);
+// HDOG_ERR_CAPACITY, nothing launched, when a range had no place in the list.
+[[nodiscard]] int clear_async(const ClearList &z, cudaStream_t s);
 // Zero `bytes` (a multiple of 4) of device memory on stream s with a kernel.
 void zero_async(void *p, size_t bytes, cudaStream_t s);
 // A batch's counts straight into page-locked host memory: host[0 .. nsub) records, host[ms ..) regions,

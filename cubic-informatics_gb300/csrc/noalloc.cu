@@ -128,7 +128,8 @@ extern "C" int hdog_ccl_noalloc(const uint8_t *d_mask, int32_t *d_labels, int wi
   ClearList zeros;
   zeros.add(d_status, sizeof(int));
   zeros.add(d_edge_count, sizeof(unsigned long long));
-  clear_async(zeros, st);
+  const int cleared = clear_async(zeros, st);
+  if (cleared != HDOG_OK) return hdog_set_error(cleared, "hdog_ccl_noalloc: too many ranges to clear");
   launch_ccl(d_sub, 1, width, height, depth, n, d_mask, d_labels, d_edges, d_edge_count, d_bits, d_blk, d_status,
              num_sms, st);
   HDOG_CUDA_TRY(cudaGetLastError());

@@ -604,8 +604,10 @@ void zero_async(void *p, size_t bytes, cudaStream_t s) {
 
 __global__ void __launch_bounds__(256) k_clear(const __grid_constant__ ClearList z) { clear_ranges(z); }
 
-void clear_async(const ClearList &z, cudaStream_t s) {
+int clear_async(const ClearList &z, cudaStream_t s) {
+  if (z.over) return HDOG_ERR_CAPACITY;
   KLAUNCH("k_clear", s, (k_clear<<<z.blocks(), 256, 0, s>>>(z)));
+  return HDOG_OK;
 }
 
 // The list counters sit kFgCountStride apart.  Written through to the host: no copies to queue behind a host

@@ -31,3 +31,20 @@ def test_a_volume_that_no_tensor_map_takes_is_refused(tmp_path):
   printf("%d\\n", rc);
   return rc == HDOG_ERR_CUDA ? 0 : 1;""")
     assert rc == 0, (rc, out)
+
+
+def test_a_list_of_more_ranges_than_it_holds_is_refused(tmp_path):
+    """One range too many leaves the others as they are and the list refused."""
+    rc, out = run(tmp_path, """
+  struct { ClearList z; uint32_t guard[64]; } s;
+  for (uint32_t &g : s.guard) g = 7;
+  uint32_t words[4];
+  for (int i = 0; i < ClearList::kMax; i++) s.z.add(words, 4 * (i + 1));
+  const ClearList full = s.z;
+  if (full.over) return 2;
+  s.z.add(words + 1, 16);
+  bool same = s.z.count == full.count;
+  for (int i = 0; i < ClearList::kMax; i++) same &= s.z.p[i] == full.p[i] && s.z.n[i] == i + 1;
+  for (uint32_t g : s.guard) same &= g == 7;
+  return same && s.z.over && clear_async(s.z, nullptr) == HDOG_ERR_CAPACITY ? 0 : 1;""")
+    assert rc == 0, (rc, out)
