@@ -588,19 +588,6 @@ __device__ __forceinline__ void soft_box_ends_k(int c0, int n, int R, LoadF ld, 
   for (int k = 0; k < K; k++) acc[k] = k == last ? e : acc[k];
 }
 
-// a / n for a whole number n below 2^24, correctly rounded: with z = 1 / n rounded and q = a z rounded, the remainder
-// a - n q is exact in one FMA and q + remainder z rounds to the quotient (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  An infinite or NaN a
-// leaves no remainder to correct with.
-struct SoftDiv {
-  float n, z;
-  __device__ __forceinline__ SoftDiv(int n_) : n((float)n_), z(1.0f / (float)n_) {}
-  __device__ __forceinline__ float2 operator()(float2 a) const {
-    const float2 zz = make_float2(z, z), q = mul2(a, zz), r = fma2(make_float2(-n, -n), q, a), p = fma2(r, zz, q);
-    return make_float2(r.x == r.x ? p.x : q.x, r.y == r.y ? p.y : q.y);
-  }
-};
-
 // Box mean along x (or its transpose): a tile of 32 rows x kSoftBoxX outputs with the reach on both sides in shared
 // memory (odd pitch: a lane's row starts in its own bank), one row per lane and kSoftBoxK outputs per thread.
 constexpr int kSoftBoxK = 16, kSoftBoxX = 128;

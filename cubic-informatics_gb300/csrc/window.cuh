@@ -167,6 +167,22 @@ __device__ __forceinline__ void ext_row_chunk(typename Op::T *suf, int pc, int r
   }
 }
 
+// a / n for an odd whole number n below 2^20, correctly rounded for every finite a (a window's length): with z = 1 / n
+// rounded and q = a z rounded, q + r z rounds to the quotient, r = a - n q being the remainder (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  q is within two units in
+// its last place, u, of a / n, and a and n q are multiples of u (of 2^-149 among the subnormals), so r is one too, of at
+// most 2n of them, and exact in one FMA.  a / n - q is then k u / n for a whole k, which for odd n stays at least u / (4n)
+// away from every rounding midpoint, while r z differs from it by less than u / 2^22.  An infinite or NaN a leaves no
+// remainder to correct with; a zero's sign is not kept (sums that start at +0 never are -0).
+struct SoftDiv {
+  float n, z;
+  __device__ __forceinline__ SoftDiv(int n_) : n((float)n_), z(1.0f / (float)n_) {}
+  __device__ __forceinline__ float2 operator()(float2 a) const {
+    const float2 zz = make_float2(z, z), q = mul2(a, zz), r = fma2(make_float2(-n, -n), q, a), p = fma2(r, zz, q);
+    return make_float2(r.x == r.x ? p.x : q.x, r.y == r.y ? p.y : q.y);
+  }
+};
+
 // Register-blocked sequential sums: a thread produces K consecutive outputs along the
 // axis; slot (u + k) % K of a K-entry rotating window feeds output k at tap u of each
 // block of K taps, so the window never moves between registers.  Every output still
