@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(128) k_soft_box_cols(const float2 *in, float2 
 #pragma unroll
       for (int j = 0; j <= 2 * RT; j++) acc[k] = add2(acc[k], win[k + j]);
     }
-  } else if (c0 - R >= 0 && c0 + K + R < l.n) {   // the chain loads one input past its last window
+  } else if (c0 - R >= 0 && c0 + K + R <= l.n) {
     const float2 *p = col + (int64_t)(c0 - R) * l.s;
     box_chain<K>(2 * R + 1, [&](int i) { return __ldg(p + (int64_t)i * l.s); }, acc);
   } else {
@@ -780,7 +780,7 @@ __global__ void k_soft_ext_adj_far(const void *src, const float2 *gout, float *g
   if (go.y != 0.0f) atomicAdd(gin + step * (base + (int64_t)m.b * s) + step - 1, go.y);
 }
 
-// (sums of over 731 values: compensated, a plain float32 chain that long is off by 1e-5 of a score)
+// (sums of 753 values and more: compensated, a plain float32 chain that long is off by 1e-5 of a score)
 template <bool ADJ>
 __global__ void k_soft_box_far(const float2 *in, float2 *out, SoftGeom g, int axis, int R, int64_t N) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1560,7 +1560,7 @@ template <bool ADJ>
 void box_pass(const SoftRun &R, const float2 *in, float2 *out, int axis, int r, const float *vol = nullptr) {
   const SoftGeom &g = R.g;
   const size_t smem = (size_t)32 * ((kSoftBoxX + 2 * r) | 1) * sizeof(float2);
-  if (smem > kSoftMaxSmem) {   // reaches above 365
+  if (smem > kSoftMaxSmem) {   // reaches from 376
     KLAUNCH("k_soft_box_far", R.st, (k_soft_box_far<ADJ><<<R.blocks(), 256, 0, R.st>>>(in, out, g, axis, r, R.N)));
     if (vol)
       KLAUNCH("k_soft_norm", R.st, (k_soft_norm<<<R.blocks(), 256, 0, R.st>>>(vol, out, R.slot(S_NORM), R.p.min_intensity, R.N,

@@ -187,9 +187,11 @@ struct SoftDiv {
 // axis; slot (u + k) % K of a K-entry rotating window feeds output k at tap u of each
 // block of K taps, so the window never moves between registers.  Every output still
 // sums its 2r+1 inputs from 0.0f in the reference order.  load(i) returns input
-// c0 - r + i.
+// c0 - r + i, i = 0 .. L + K - 2 in order: an even K never divides the odd L, so the last block of
+// taps is the guarded one and no load goes past the last window.
 template <int K, class LoadF>
 __device__ __forceinline__ void box_chain(int L, LoadF load, float2 (&acc)[K]) {
+  static_assert(K % 2 == 0, "an odd K could divide L and load one input past the last window");
   float2 win[K];
 #pragma unroll
   for (int k = 0; k < K; k++) {
