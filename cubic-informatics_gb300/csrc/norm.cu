@@ -767,9 +767,9 @@ __global__ void __launch_bounds__(128) k_box_z_norm(const Sub *subs, int rz, flo
 // before the first add so that all loads of a thread are in flight together; neighbouring blocks take the chunks of the
 // same columns, which share their overlapping inputs through the caches.  Bound by HBM (14 bytes a voxel) once the
 // instructions around the loads are few: chunks whose window lies inside the volume walk two pointers instead of clamping
-// and multiplying every index, and ten blocks fit an SM.  1.42 G voxels at reach 5: 4.23 -> 3.60 ms (5.5 TB/s); chunks of
-// 6 (3.88 ms), 10 (4.48) and 12 (4.42), and a register ring down the column (5.9) are slower.  PARTS also stores the box
-// means (stage dumps).
+// and multiplying every index, and ten blocks fit an SM (for which a thread spills 52 bytes at reach 5, 16 at 4).  1.42 G
+// voxels at reach 5: 4.23 -> 3.60 ms (5.5 TB/s); chunks of 6 (3.88 ms), 10 (4.48) and 12 (4.42), and a register ring down
+// the column (5.9) are slower.  PARTS also stores the box means (stage dumps).
 template <int RZ, bool PARTS, bool PAD>
 __global__ void __launch_bounds__(128, RZ <= 5 ? 10 : 6) k_box_z_norm_t(const Sub *subs, float min_intensity, const float2 *in,
                                                       float *norm, float *ero_l, float *dil_l) {

@@ -321,7 +321,8 @@ class Context:
         return torch.empty(self.shape, dtype=dtype, device="cuda:%d" % self.params.dev_id)
 
     def set_fused_sweep(self, on):
-        """DoG + Hessian + PD in one z-sweep kernel (default) or as separate passes."""
+        """Hessian + PD + foreground list (and, for tap radii that have one, the DoG) as z-sweeps (default), or
+        separate passes."""
         check(lib().hdog_ctx_set_option(self._h, HDOG_OPT_FUSED_SWEEP, int(bool(on))))
 
     def set_host_batch(self, n):

@@ -348,8 +348,8 @@ int hdog_soft_backward_scaled(const hdog_soft_params *p, const float *d_volume, 
 
 /* ---- context options ---- */
 enum {
-  HDOG_OPT_FUSED_SWEEP = 1,  /* 1 (default): DoG, Hessian and the PD test in one z-sweep kernel
-                                when the radii allow; 0: separate passes (same results) */
+  HDOG_OPT_FUSED_SWEEP = 1,  /* 1 (default): Hessian, PD test and foreground list by a z-sweep, the DoG by
+                                one for the tap radii that have it; 0: separate passes (same results) */
   HDOG_OPT_HOST_BATCH = 2,   /* substacks in the first batch when hdog_run_stack gets its stack
                                 in host memory (default 1; 0: as many as the context holds);
                                 each later batch holds at most twice as many as the one before
