@@ -249,7 +249,8 @@ __device__ __forceinline__ int cell_bit(int lx, int ly, int lz) { return ((lz & 
 __device__ __forceinline__ uint32_t cell_occ(const Sub &S, const uint8_t *m, int64_t WH, int x, int y, int z) {
   uint32_t o = 0;
   if (x + 1 < 0 || x >= S.W || y + 1 < 0 || y >= S.H || z + 1 < 0 || z >= S.D) return 0;
-  const bool pair = x >= 0 && x + 1 < S.W && (S.W % 2 == 0);
+  // both voxels in one load: x is even, so a caller's mask on an even address and an even width put them on two bytes
+  const bool pair = x >= 0 && x + 1 < S.W && S.W % 2 == 0 && (reinterpret_cast<uintptr_t>(m) & 1u) == 0;
 #pragma unroll
   for (int dz = 0; dz < 2; dz++)
 #pragma unroll
@@ -582,8 +583,8 @@ __global__ void __launch_bounds__(kCclThreads, 4) k_ccl_local(const Sub *subs, c
   const int lx0 = (t % (kTX / 4)) * 4, ly = t / (kTX / 4);
   const int x = T.x0 + lx0, y = T.y0 + ly;
   if (y >= S.H) return;
-  const bool vec = x + 3 < S.W && (S.W % 4 == 0);
   int32_t *L = labels + S.vox;
+  const bool vec = x + 3 < S.W && S.W % 4 == 0 && (reinterpret_cast<uintptr_t>(L) & 15u) == 0;
   const int c0x = lx0 >> 1;   // the quad's voxels lie in cells c0x (first two) and c0x + 1
   for (int lz = 0; lz < T.tz; lz++) {
     const int64_t g = (T.z0 + lz) * WH + (int64_t)y * S.W + x;
